@@ -147,12 +147,7 @@ __device__ __forceinline__ uint32_t quantize_query_word(uint4 km, float4 q4, flo
 #pragma unroll
   for (int x = 0; x < 4; ++x) { z[x] = __fmul_rn(qf[x], ks[x]); amax = fmaxf(amax, fabsf(z[x])); dot = fmaf(qf[x], kb[x], dot); }
   amax = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(amax)));  // amax >= 0: the bit patterns order as the values
-  // r = fl(127 / amax), correctly rounded: reciprocal seed, one Newton step, quotient and its residual correction
-  float rc;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(amax));
-  rc = fmaf(fmaf(-amax, rc, 1.f), rc, rc);
-  const float q0 = __fmul_rn(127.f, rc);
-  const float r = amax > 0.f ? fmaf(fmaf(-amax, q0, 127.f), rc, q0) : 0.f;
+  const float r = quotient_127(amax);
   uint32_t word = 0;
 #pragma unroll
   for (int x = 0; x < 4; ++x)  // rint(z r) in the low mantissa bits: one rounding of the exact product

@@ -74,6 +74,19 @@ __device__ __forceinline__ float2 isum2(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
 
+// fl(127 / a) for a = max |q step|, both BF16, so that a has at most 16 significand bits; 0 for a = 0. One refinement step
+// on an approximate reciprocal r (at most 1 ulp off): q0 = fl(127 r) is within 2 ulp of the quotient, its residual
+// e = 127 - a q0 is exact in an FMA (40-bit product, 18 bits left of it), and q0 + e r is within 2^-21 ulp of the quotient.
+// A quotient by a 16-bit number is never closer than 2^-17 ulp to the midpoint of two floats (|127 2^k - (2 n + 1) a| is a
+// whole number, and not 0), so the last rounding gives the correctly rounded quotient
+// (tests/test_quotient_cpu.py goes through every significand).
+__device__ __forceinline__ float quotient_127(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  const float q0 = __fmul_rn(127.f, r);
+  return a > 0.f ? fmaf(fmaf(-a, q0, 127.f), r, q0) : 0.f;
+}
+
 __device__ __forceinline__ float warp_max(float x) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) x = fmaxf(x, __shfl_xor_sync(FULL, x, o));

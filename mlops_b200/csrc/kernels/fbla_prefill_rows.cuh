@@ -113,10 +113,7 @@ __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_
 #pragma unroll
       for (int x = 0; x < 4; ++x) { z[x] = __fmul_rn(qf[x], ks[x]); amax = fmaxf(amax, fabsf(z[x])); dot = fmaf(qf[x], kb[x], dot); }
       amax = warp_max(amax);
-      float rc;
-      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(amax));
-      rc = fmaf(fmaf(-amax, rc, 1.f), rc, rc);
-      const float q0 = __fmul_rn(127.f, rc), rr = amax > 0.f ? fmaf(fmaf(-amax, q0, 127.f), rc, q0) : 0.f;
+      const float rr = quotient_127(amax);
       uint32_t word = 0;
 #pragma unroll
       for (int x = 0; x < 4; ++x) word |= (__float_as_uint(fmaf(z[x], rr, MAGICF)) & 255u) << (8 * x);

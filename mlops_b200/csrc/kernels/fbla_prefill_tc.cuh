@@ -364,12 +364,8 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           const float am = amax[k];
-          float rc;
-          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(am));
-          rc = fmaf(fmaf(-am, rc, 1.f), rc, rc);
-          const float q0_ = __fmul_rn(127.f, rc);
           // rint(z r) as the exact float (t - 1.5 * 2^23), then FP16 (an integer of magnitude <= 127: exact)
-          const float2 rr2 = splat(am > 0.f ? fmaf(fmaf(-am, q0_, 127.f), rc, q0_) : 0.f);
+          const float2 rr2 = splat(quotient_127(am));
           const float2 t0 = add2(fma2(z[k][0], rr2, mg), ng), t1 = add2(fma2(z[k][1], rr2, mg), ng);
           const float2 t2 = add2(fma2(z[k][2], rr2, mg), ng), t3 = add2(fma2(z[k][3], rr2, mg), ng);
           *reinterpret_cast<uint4 *>(sm.qp[X] + off[k]) = make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
