@@ -139,6 +139,12 @@ mlops_fbla_status mlops_fbla_prefill(const mlops_fbla_config *cfg, int count, co
                                      const uint16_t *k, const uint16_t *v, const mlops_fbla_cache *cache,
                                      uint16_t *output, cudaStream_t stream);
 
+/* As mlops_fbla_prefill of `count` tokens without queries into an empty cache (cfg->tokens 0) whose arrays have no
+ * initial contents: what the tokens do not fill of the units up to cfg->capacity and of the windows is zeroed by the same
+ * launch. No counterpart in the reference interface. */
+mlops_fbla_status mlops_fbla_encode(const mlops_fbla_config *cfg, int count, const uint16_t *k, const uint16_t *v,
+                                    const mlops_fbla_cache *cache, cudaStream_t stream);
+
 /* As mlops_fbla_prefill with the start (*length + cfg->tokens) and *count read on the device when the kernels run;
  * launches are sized by max_count alone. cfg->capacity > 0. reference: mlops_fbla.h:142-144 */
 mlops_fbla_status mlops_fbla_prefill_at(const mlops_fbla_config *cfg, const int *length, const int *count, int max_count,

@@ -53,6 +53,8 @@ _lib.mlops_fbla_decode_at.restype = ctypes.c_int
 _lib.mlops_fbla_decode_at.argtypes = [_cp, _vp, _vp, ctypes.POINTER(Cache), _vp, _vp, ctypes.c_size_t, _vp]
 _lib.mlops_fbla_prefill.restype = ctypes.c_int
 _lib.mlops_fbla_prefill.argtypes = [_cp, ctypes.c_int, _vp, _vp, _vp, ctypes.POINTER(Cache), _vp, _vp]
+_lib.mlops_fbla_encode.restype = ctypes.c_int
+_lib.mlops_fbla_encode.argtypes = [_cp, ctypes.c_int, _vp, _vp, ctypes.POINTER(Cache), _vp]
 _lib.mlops_fbla_prefill_at.restype = ctypes.c_int
 _lib.mlops_fbla_prefill_at.argtypes = [_cp, _vp, _vp, ctypes.c_int, _vp, _vp, _vp, ctypes.POINTER(Cache), _vp, _vp]
 _lib.mlops_fbla_append_at.restype = ctypes.c_int
@@ -157,3 +159,15 @@ def prefill(q, k, v, coarse, fine, meta, sink_k, sink_v, open_k, open_v, tokens,
                                      ctypes.byref(cache), out.data_ptr() if out is not None else None, _stream(dev))
     _raise(st, "mlops_fbla_prefill")
     return out
+
+
+def encode(k, v, coarse, fine, meta, sink_k, sink_v, open_k, open_v, capacity, format):
+    """Stores k / v [B, Hkv, n, 128], n > 0, into an empty cache for `capacity` tokens; its arrays need no initial contents."""
+    dev = k.device
+    _tensor(k, dev, torch.bfloat16, "k")
+    _tensor(v, dev, torch.bfloat16, "v")
+    cfg = _config(k.size(0), k.size(1), k.size(1), 0, format, capacity, 0.0, 0.0)
+    cache = _cache(coarse, fine, meta, sink_k, sink_v, open_k, open_v)
+    with torch.cuda.device(dev):
+        st = _lib.mlops_fbla_encode(ctypes.byref(cfg), k.size(2), k.data_ptr(), v.data_ptr(), ctypes.byref(cache), _stream(dev))
+    _raise(st, "mlops_fbla_encode")

@@ -43,27 +43,29 @@ def _require_kv(k, v):
         raise ValueError(f"k and v have to live on the same CUDA device (k: {k.device}, v: {v.device})")
 
 
-def empty(batch: int, kv_heads: int, capacity: int, mode: str = "3+3", device="cuda") -> FBLACache:
-    """A cache with room for ``capacity`` tokens and none stored. All arrays start as zeros."""
+def _allocate(make, batch, kv_heads, capacity, mode, device) -> FBLACache:
+    """The arrays of a cache for ``capacity`` tokens, each from ``make(shape, dtype=, device=)``."""
     planes = _PLANES.get(mode)
     if planes is None:
         raise ValueError(f"unknown mode {mode!r}: choose '3+3' or '4+2'")
     coarse_bits, fine_bits, fmt = planes
     groups = -(-capacity // GROUP)
-
-    def zeros(shape, dtype):
-        return torch.zeros(shape, dtype=dtype, device=device)
-
     records = 8 * groups
-    windows = [zeros((batch, kv_heads, GROUP, HEAD_DIM), torch.bfloat16) for _ in ("sink_k", "sink_v", "open_k", "open_v")]
+    sink_k, sink_v, open_k, open_v = make((4, batch, kv_heads, GROUP, HEAD_DIM), dtype=torch.bfloat16, device=device).unbind(0)
+    return FBLACache(coarse=make((batch, kv_heads, records, 512 * coarse_bits), dtype=torch.uint8, device=device),
+                     fine=make((batch, kv_heads, records, 512 * fine_bits), dtype=torch.uint8, device=device),
+                     meta=make((batch, kv_heads, groups, 512), dtype=torch.bfloat16, device=device),
+                     sink_k=sink_k, sink_v=sink_v, open_k=open_k, open_v=open_v, tokens=0, capacity=capacity, format=fmt)
+
+
+def empty(batch: int, kv_heads: int, capacity: int, mode: str = "3+3", device="cuda") -> FBLACache:
+    """A cache with room for ``capacity`` tokens and none stored. All arrays start as zeros."""
+    cache = _allocate(torch.zeros, batch, kv_heads, capacity, mode, device)
     with torch.cuda.device(torch.device(device)):
-        image_bytes = _C.images_bytes(batch, kv_heads, groups * GROUP)
-    return FBLACache(coarse=zeros((batch, kv_heads, records, 512 * coarse_bits), torch.uint8),
-                     fine=zeros((batch, kv_heads, records, 512 * fine_bits), torch.uint8),
-                     meta=zeros((batch, kv_heads, groups, 512), torch.bfloat16),
-                     sink_k=windows[0], sink_v=windows[1], open_k=windows[2], open_v=windows[3],
-                     tokens=0, capacity=capacity, format=fmt,
-                     images=zeros((image_bytes,), torch.uint8) if image_bytes > 0 else None)
+        image_bytes = _C.images_bytes(batch, kv_heads, -(-capacity // GROUP) * GROUP)
+    if image_bytes > 0:
+        cache.images = torch.zeros((image_bytes,), dtype=torch.uint8, device=device)
+    return cache
 
 
 def _extend(cache, k, v, q=None, scale=0.0):
@@ -91,8 +93,15 @@ def encode(k: torch.Tensor, v: torch.Tensor, mode: str = "3+3", capacity: Option
     room = n if capacity is None else int(capacity)
     if room < n:
         raise ValueError(f"a capacity of {room} tokens cannot hold the {n} given")
-    cache = empty(batch, kv_heads, room, mode, k.device)
-    _extend(cache, k, v)
+    if n == 0 or batch == 0 or kv_heads == 0:
+        cache = empty(batch, kv_heads, room, mode, k.device)
+        _extend(cache, k, v)
+        return cache
+    # (the call that stores the tokens also zeroes what they leave of the arrays)
+    cache = _allocate(torch.empty, batch, kv_heads, room, mode, k.device)
+    _C.encode(k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous(), cache.coarse, cache.fine, cache.meta, cache.sink_k,
+              cache.sink_v, cache.open_k, cache.open_v, room, cache.format)
+    cache.tokens = n
     return cache
 
 

@@ -251,10 +251,14 @@ void fill_chunk(const mlops_fbla_config *c, int count, long long room, const uin
   a.sl = log2_scale(c);
 }
 // The passes in the order that keeps them correct: closing groups reads the windows as they were, the attention reads
-// them too, and only then are the windows rewritten.
+// them too, and only then are the windows rewritten. Without queries one launch does both (fbla_close.cuh: write_item).
 mlops_fbla_status enqueue_chunk(const char *fn, const fbla_k_prefill &a, int closable_groups, cudaStream_t stream) {
+  if (!a.q) {
+    const cudaError_t e = fbla_k_write_launch(&a, closable_groups, stream);
+    return e == cudaSuccess ? accepted() : device_failure(fn, e);
+  }
   cudaError_t e = fbla_k_close_launch(&a, closable_groups, stream);
-  if (e == cudaSuccess && a.q) e = fbla_k_attend_launch(&a, stream);
+  if (e == cudaSuccess) e = fbla_k_attend_launch(&a, stream);
   if (e == cudaSuccess) e = fbla_k_finish_launch(&a, stream);
   return e == cudaSuccess ? accepted() : device_failure(fn, e);
 }
@@ -337,9 +341,9 @@ int mlops_fbla_cache_sizes(const mlops_fbla_config *c, mlops_fbla_sizes *out) {
   return 1;
 }
 
-mlops_fbla_status mlops_fbla_prefill(const mlops_fbla_config *c, int count, const uint16_t *q, const uint16_t *k, const uint16_t *v,
-                                     const mlops_fbla_cache *cache, uint16_t *out, cudaStream_t stream) {
-  constexpr const char *fn = "mlops_fbla_prefill";
+// `fresh`: the cache's arrays have no initial contents (mlops_fbla_encode)
+static mlops_fbla_status run_chunk(const char *fn, const mlops_fbla_config *c, int count, const uint16_t *q, const uint16_t *k, const uint16_t *v,
+                                   const mlops_fbla_cache *cache, uint16_t *out, bool fresh, cudaStream_t stream) {
   if (!c || !cache || !k || !v) return refuse(fn, "a required pointer is null");
   if (q && !out) return refuse(fn, "queries were given but no output to write their attention to");
   const long long end = (long long)c->tokens + count;
@@ -351,10 +355,24 @@ mlops_fbla_status mlops_fbla_prefill(const mlops_fbla_config *c, int count, cons
   const mlops_fbla_status st = check_chunk_operands(fn, c, q, k, v, cache, out);
   if (st != MLOPS_FBLA_OK) return st;
   fbla_k_prefill a{};
-  fill_chunk(c, count, c->capacity ? c->capacity : end, q, k, v, cache, out, a);
+  const long long room = c->capacity ? c->capacity : end;
+  fill_chunk(c, count, room, q, k, v, cache, out, a);
+  a.clear_groups = fresh ? (int)groups_of(room) : 0;
   // groups completed by this chunk: those whose last token lies before `end` and that were still open before it
   const int first_open = c->tokens == 0 ? 0 : (c->tokens - 1) / kGroup, last_open = (int)((end - 1) / kGroup);
   return enqueue_chunk(fn, a, last_open - first_open, stream);
+}
+
+mlops_fbla_status mlops_fbla_prefill(const mlops_fbla_config *c, int count, const uint16_t *q, const uint16_t *k, const uint16_t *v,
+                                     const mlops_fbla_cache *cache, uint16_t *out, cudaStream_t stream) {
+  return run_chunk("mlops_fbla_prefill", c, count, q, k, v, cache, out, false, stream);
+}
+
+mlops_fbla_status mlops_fbla_encode(const mlops_fbla_config *c, int count, const uint16_t *k, const uint16_t *v, const mlops_fbla_cache *cache,
+                                    cudaStream_t stream) {
+  constexpr const char *fn = "mlops_fbla_encode";
+  if (c && c->tokens != 0) return refuse(fn, "starts a cache: tokens has to be 0");
+  return run_chunk(fn, c, count, nullptr, k, v, cache, nullptr, true, stream);
 }
 
 mlops_fbla_status mlops_fbla_prefill_at(const mlops_fbla_config *c, const int *length, const int *count, int max_count, const uint16_t *q,

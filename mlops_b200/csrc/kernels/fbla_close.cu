@@ -1,4 +1,4 @@
-// Launchers of the close / finish passes (bodies: fbla_close.cuh).
+// Launchers of the close / finish passes and of the chunk without queries (bodies: fbla_close.cuh).
 #include "fbla_close.cuh"
 #include <stdio.h>
 
@@ -15,44 +15,65 @@ template <class K> cudaError_t pass_of(K kernel, int gx, int gy, int threads, si
 
 namespace fbla {
 template <int CB, int FB>
-__global__ void __launch_bounds__(256) close_kernel(const fbla_k_prefill a) {
+__global__ void __launch_bounds__(CLOSE_THREADS, 2) close_kernel(const fbla_k_prefill a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   close_item<CB, FB>(a, smem_raw);
 }
 
-__global__ void __launch_bounds__(256) finish_kernel(const fbla_k_prefill a) {
+template <int CB, int FB>
+__global__ void __launch_bounds__(CLOSE_THREADS, 2) write_kernel(const fbla_k_prefill a) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  write_item<CB, FB>(a, smem_raw);
+}
+
+__global__ void __launch_bounds__(CLOSE_THREADS) finish_kernel(const fbla_k_prefill a) {
   finish_item(a, nullptr);
+}
+
+// the kernels' shared memory is above the default limit: asked for once per device and host thread
+static cudaError_t configure() {
+  static thread_local int configured[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  for (auto kernel : {close_kernel<3, 3>, close_kernel<4, 2>, write_kernel<3, 3>, write_kernel<4, 2>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CloseSmem));
+  if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = 1;
+  return e;
 }
 }  // namespace fbla
 
 extern "C" cudaError_t fbla_k_close_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream) {
   if (close_blocks <= 0) return cudaSuccess;
+  const cudaError_t e = fbla::configure();
+  if (e != cudaSuccess) return e;
   const dim3 grid(close_blocks, a->batch * a->kv_heads);
-  const size_t smem = sizeof(fbla::CloseSmem);
-  cudaError_t e;
-  if (a->cb == 3) {
-    e = cudaFuncSetAttribute(fbla::close_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    fbla::close_kernel<3, 3><<<grid, 256, smem, stream>>>(*a);
-  } else {
-    e = cudaFuncSetAttribute(fbla::close_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    fbla::close_kernel<4, 2><<<grid, 256, smem, stream>>>(*a);
-  }
+  if (a->cb == 3) fbla::close_kernel<3, 3><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
+  else fbla::close_kernel<4, 2><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
+  return cudaGetLastError();
+}
+
+extern "C" cudaError_t fbla_k_write_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream) {
+  const cudaError_t e = fbla::configure();
+  if (e != cudaSuccess) return e;
+  const dim3 grid(close_blocks > 0 ? close_blocks : 1, a->batch * a->kv_heads);
+  if (a->cb == 3) fbla::write_kernel<3, 3><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
+  else fbla::write_kernel<4, 2><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
   return cudaGetLastError();
 }
 
 extern "C" cudaError_t fbla_k_finish_launch(const fbla_k_prefill *a, cudaStream_t stream) {
-  fbla::finish_kernel<<<a->batch * a->kv_heads, 256, 0, stream>>>(*a);
+  fbla::finish_kernel<<<a->batch * a->kv_heads, fbla::CLOSE_THREADS, 0, stream>>>(*a);
   return cudaGetLastError();
 }
 
 extern "C" cudaError_t fbla_k_close_pass(const fbla_k_prefill *a, int close_blocks, fbla_k_pass *info) {
   const int heads = a->batch * a->kv_heads;
-  if (a->cb == 3) return pass_of(fbla::close_kernel<3, 3>, close_blocks, heads, 256, sizeof(fbla::CloseSmem), "fbla::close_item<3, 3>", info);
-  return pass_of(fbla::close_kernel<4, 2>, close_blocks, heads, 256, sizeof(fbla::CloseSmem), "fbla::close_item<4, 2>", info);
+  if (a->cb == 3) return pass_of(fbla::close_kernel<3, 3>, close_blocks, heads, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), "fbla::close_item<3, 3>", info);
+  return pass_of(fbla::close_kernel<4, 2>, close_blocks, heads, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), "fbla::close_item<4, 2>", info);
 }
 
 extern "C" cudaError_t fbla_k_finish_pass(const fbla_k_prefill *a, fbla_k_pass *info) {
-  return pass_of(fbla::finish_kernel, a->batch * a->kv_heads, 1, 256, 0, "fbla::finish_item", info);
+  return pass_of(fbla::finish_kernel, a->batch * a->kv_heads, 1, fbla::CLOSE_THREADS, 0, "fbla::finish_item", info);
 }

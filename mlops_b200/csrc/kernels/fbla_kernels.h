@@ -133,11 +133,16 @@ typedef struct {
   // head >= tc_min_rows, the warp-per-row pass below that -- so that a device-count call takes the kernel the host-count
   // call of the same chunk takes and the two stay bit-identical.
   int tc_min_rows;
+  // > 0 (a chunk that starts a cache whose arrays have no initial contents): the groups per KV head that the layout has
+  // room for; what the chunk does not write of their units and of the sink window is zeroed (fbla_k_write_launch)
+  int clear_groups;
 } fbla_k_prefill;
 
 // close_blocks: grid x of the close pass (groups the chunk can close); 0 skips it
 FBLA_HOST_API(cudaError_t fbla_k_close_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_finish_launch(const fbla_k_prefill *a, cudaStream_t stream);)
+// close and finish of a chunk without queries as one launch
+FBLA_HOST_API(cudaError_t fbla_k_write_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream);)
 // Attention of the chunk's rows: the tensor-core kernel (tcgen05, 128 rows per CTA), or -- for chunks of fewer than
 // FBLA_K_TC_MIN_ROWS rows, or when the environment variable MLOPS_FBLA_PREFILL=rows asks for it -- one warp per row.
 // fbla_k_attend_plan splits a chunk's attention into its one or two passes (two when the count is on the device and

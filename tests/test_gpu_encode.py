@@ -1,0 +1,39 @@
+"""mlops_fbla_encode into arrays without initial contents gives the bytes of a zeroed cache and an append: lengths around
+the group boundary, capacities beyond the tokens, both formats."""
+import ctypes
+
+import pytest
+import torch
+
+from mlops_b200 import attention
+from mlops_b200.attention import _C
+
+pytestmark = pytest.mark.gpu
+ARRAYS = ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v")
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("n,capacity", [(1, 1), (5, 700), (127, 127), (128, 128), (129, 129), (129, 1000), (300, 384), (1025, 4096)])
+def test_encode_needs_no_initial_contents(mode, n, capacity):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    k, v = (torch.randn((2, 3, n, 128), generator=gen, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    want = attention.append(attention.empty(2, 3, capacity, mode), k, v)
+    got = attention.empty(2, 3, capacity, mode)
+    for a in ARRAYS:
+        getattr(got, a).view(torch.uint8).fill_(0xA5)
+    _C.encode(k, v, *[getattr(got, a) for a in ARRAYS], capacity, got.format)
+    whole = attention.encode(k, v, mode, capacity)
+    for a in ARRAYS:
+        x = getattr(want, a).view(torch.uint8)
+        assert torch.equal(getattr(got, a).view(torch.uint8), x), a
+        assert torch.equal(getattr(whole, a).view(torch.uint8), x), a
+    assert whole.tokens == want.tokens == n
+
+
+def test_encode_starts_an_empty_cache_only():
+    c = attention.empty(1, 1, 256)
+    kc = _C._cache(*[getattr(c, a) for a in ARRAYS])
+    cfg = _C._config(1, 1, 1, 5, 0, 256, 0.0, 0.0)
+    assert _C.lib.mlops_fbla_encode(ctypes.byref(cfg), 1, c.open_k.data_ptr(), c.open_v.data_ptr(), ctypes.byref(kc), None) == _C.INVALID_VALUE
+    assert "tokens has to be 0" in _C.last_error()
