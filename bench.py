@@ -59,7 +59,6 @@ WORKLOADS = {
 # under profiles/ (1 GPU); reported with their source, never as a measurement of the run that prints them
 NCU_TRAFFIC = {
     "decode_128k": dict(kernel="coarse_kernel<3,3,4,2>", bytes=113223424, file="profiles/decode_b1_ctx128k_3p3_launches.md"),
-    "decode_b8": dict(kernel="refine_kernel<4,2,4>", bytes=164004352, file="profiles/decode_b8_ctx16k_4p2_launches.md"),
 }
 SUBS = ["decode_128k_4p2", "decode_b8", "prefill_b4", "serving_b64"]
 MIN_TIMED_S = 0.5
@@ -235,14 +234,21 @@ def time_passes(D, _C, passes, reps=30):
     return [float(np.median(t[3:])) for t in times]
 
 
-def refined_share(scratch, vheads, closed_blocks):
-    """Fraction of closed (virtual head, sub-block) pairs the select pass listed. The refine pass leaves the total at the end
-    of its item_off array, which sits just before the 256-byte status block that ends the scratch."""
+def refined_share(passes, scratch, lengths, heads_per_row, mode):
+    """Fraction of closed (virtual head, sub-block) pairs that some query of the head selected in the last decode on this
+    scratch: the sub-blocks' log2 masses against the rows' own (both left in the scratch, at the plan's offsets)."""
     import torch
-    up = lambda n: (n + 255) // 256 * 256
-    off = scratch.numel() - 256 - up((vheads + 1) * 4) + vheads * 4
-    total = int(scratch[off:off + 4].view(torch.int32).item())
-    return total / max(1, closed_blocks)
+    geom = passes[0].geom
+    nblocks, vheads = 8 * geom[22], heads_per_row * len(lengths)
+    merge_rows = passes[3].items  # one per (virtual head, query)
+    qg = merge_rows // vheads
+    at = lambda off, shape: scratch[off:off + 4 * int(np.prod(shape))].view(torch.float32).view(shape)
+    lse, mass = at(geom[25], (vheads, nblocks, qg)), at(geom[28], (vheads, 1, qg))
+    chosen = (lse - mass > np.log2({"3+3": 3e-4, "4+2": 1e-3}[mode])).any(-1).view(len(lengths), heads_per_row, nblocks)
+    last = torch.tensor([8 * max((int(n) + 127) // 128 - 1, 1) for n in lengths], device=scratch.device).view(-1, 1, 1)
+    block = torch.arange(nblocks, device=scratch.device).view(1, 1, -1)
+    closed = ((block >= 8) & (block < last)).expand_as(chosen)
+    return float((chosen & closed).sum()) / max(1, int(closed.sum()))
 
 
 def run_decode(D, cfg, args, headline):
@@ -289,9 +295,10 @@ def run_decode(D, cfg, args, headline):
     status = scratch[-256:].view(torch.int32)[:2].tolist()
     if status[0]:
         raise RuntimeError(f"a bounded wait gave up: status {status}")
-    vheads = B * kh * max(1, g // 4)
-    closed_blocks = vheads * max((N + 127) // 128 - 2, 0) * 8
-    share = refined_share(scratch, vheads, closed_blocks)
+    length = torch.tensor([N], dtype=torch.int32, device=D.dev)
+    cs_at = _C.Config(B, qh, kh, 0, 0.0, 0.0, c0.format, c0.capacity, 0, 0, 0, 0, 0)
+    passes = decode_plan(_C, cs_at, length, qd, caches[0], out, scratch)
+    share = refined_share(passes, scratch, [N] * B, kh * max(1, g // 4), cfg["mode"])
 
     # ---- end to end through the Python interface: host q -> device, decode, output -> host, every step -----------------
     out_host = torch.empty(q_host.shape, dtype=torch.bfloat16).pin_memory()
@@ -305,9 +312,6 @@ def run_decode(D, cfg, args, headline):
     # ---- the passes one by one, and the reference's CUDA library on the same cache (rank 0 of a 1-GPU run) ----------------
     pass_us = ref_us = None
     if D.world == 1:
-        length = torch.tensor([N], dtype=torch.int32, device=D.dev)
-        cs_at = _C.Config(B, qh, kh, 0, 0.0, 0.0, c0.format, c0.capacity, 0, 0, 0, 0, 0)
-        passes = decode_plan(_C, cs_at, length, qd, caches[0], out, scratch)
         step(0)
         torch.cuda.synchronize()
         pass_us = time_passes(D, _C, passes)
@@ -316,7 +320,8 @@ def run_decode(D, cfg, args, headline):
     abytes, parts = decode_bytes(cfg, share)
     peak, peak_kind = hbm_peak()
     rec = dict(ms_per_step=ms, blocks=blocks, clocks=clocks, share=share, ms_e2e=ms_e2e, h2d=q_host.numel() * 2 * world, d2h=out_host.numel() * 2 * world,
-               abytes=abytes, parts=parts, peak=peak, peak_kind=peak_kind, pass_us=pass_us, ref_us=ref_us, world=world)
+               abytes=abytes, parts=parts, peak=peak, peak_kind=peak_kind, pass_us=pass_us, ref_us=ref_us, world=world,
+               dense=b"dense" in passes[0].entry)
     return rec
 
 
@@ -355,11 +360,16 @@ def decode_record(cfg, rec, n_gpus):
                 traffic_source=(f"ncu capture of {captured['kernel']} on this workload, one launch, not this run: {captured['file']}" if captured
                                 else "not captured for this workload; ncu captures of other workloads are summarised under profiles/"),
                 peak_kind=rec["peak_kind"] + (f", x {rec['world']} GPUs" if rec["world"] > 1 else ""),
-                kernel="decode call: coarse, select, refine, merge", algorithmic_bytes=rec["abytes"], bytes_parts=rec["parts"])
+                kernel="decode call, all passes", algorithmic_bytes=rec["abytes"], bytes_parts=rec["parts"])
     if rec["pass_us"]:
-        names = ["coarse_kernel", "select_kernel", "refine_kernel", "merge_kernel"]
-        us = rec["pass_us"]
-        bytes_of = [rec["parts"]["coarse_and_meta"] + rec["parts"]["bf16_windows"], None, rec["parts"]["refine"], None]
+        us, parts = rec["pass_us"], rec["parts"]
+        if rec["dense"]:  # scores: K's half of the coarse records and of the metadata; values: everything once
+            names = ["score_kernel", "mass_kernel", "value_kernel", "gather_kernel"]
+            fine = (3, 2)[cfg["mode"] == "4+2"] / 6  # the fine records' share of a refined sub-block's bytes
+            bytes_of = [parts["coarse_and_meta"] / 2 + parts["bf16_windows"], None, parts["coarse_and_meta"] + fine * parts["refine"], None]
+        else:
+            names = ["coarse_kernel", "select_kernel", "refine_kernel", "merge_kernel"]
+            bytes_of = [parts["coarse_and_meta"] + parts["bf16_windows"], None, parts["refine"], None]
         top = int(np.argmax(us))
         roof["passes_us"] = dict(zip(names, us))
         roof["dominant_kernel"] = dict(name=names[top], us=us[top], share_of_passes=us[top] / sum(us))
@@ -427,9 +437,8 @@ def run_serving(D, cfg, args):
             raise RuntimeError(_C.last_error())
 
     ms, blocks, clocks = timed_blocks(D, step, args.steps, args.warmup)  # (the cache itself, ~0.8 GB per KV head, exceeds L2)
-    vheads = B * kh
     closed_blocks = int(sum(max((int(n) + 127) // 128 - 2, 0) for n in lengths)) * kh * 8
-    share = refined_share(scratch, vheads, closed_blocks)
+    share = refined_share(decode_plan(_C, cs, ld, qd, kc, out, scratch), scratch, lengths, kh, "3+3")
 
     def step_e2e(i):  # the device-length call through the C ABI with host q and output (the Python interface has no per-row lengths)
         dq = q_host.to(D.dev, non_blocking=True)
@@ -451,7 +460,7 @@ def run_serving(D, cfg, args):
                             sharding=("KV heads over %d GPUs, no exchange" % world) if D.world > 1 else "one GPU"),
                 e2e=dict(value=B / (ms_e2e * 1e-3), unit=UNIT, h2d_bytes_per_step=q_host.numel() * 2 * world, d2h_bytes_per_step=out_host.numel() * 2 * world),
                 roofline=dict(bound="hbm", achieved=achieved, peak=peak * world, unit="GB/s", frac=achieved / (peak * world), traffic=None,
-                              peak_kind=peak_kind, kernel="decode_at call: coarse, select, refine, merge", algorithmic_bytes=abytes,
+                              peak_kind=peak_kind, kernel="decode_at call, all passes", algorithmic_bytes=abytes,
                               bytes_parts=dict(coarse_and_meta=coarse, bf16_windows=windows, refine=refine)),
                 dtype="u8")
 

@@ -9,6 +9,7 @@
 #define FBLA_POS ::mlops_fbla::Pos
 #include "../mlops_b200/csrc/kernels/fbla_close.cuh"
 #include "../mlops_b200/csrc/kernels/fbla_decode.cuh"
+#include "../mlops_b200/csrc/kernels/fbla_dense.cuh"
 #include "../mlops_b200/csrc/kernels/fbla_prefill_rows.cuh"
 #include "../mlops_b200/csrc/kernels/fbla_prefill_tc.cuh"
 #include "../mlops_b200/csrc/kernels/fbla_qkv.cuh"

@@ -198,8 +198,10 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   // Which coarse kernel runs is decided by the cache's room where it has one, for host and device lengths alike: both
   // calls on one cache then run the same kernels and return the same bits.
   fbla_k_decode_split(&a, room);
-  const float threshold = c->tau != 0.f ? c->tau : (c->format == MLOPS_FBLA_3P3 ? 3e-4f : 1e-3f);
+  const float usual = c->format == MLOPS_FBLA_3P3 ? 3e-4f : 1e-3f, threshold = c->tau != 0.f ? c->tau : usual;
   a.log2_tau = log2f(threshold);
+  // (a shard's two phases share the scratch but only the second one uses tau: they decide by the format's own)
+  a.dense = (short)fbla_k_decode_dense(&a, room, wants_output ? threshold : usual);
   return MLOPS_FBLA_OK;
 }
 mlops_fbla_status enqueue_decode(const char *fn, fbla_k_decode &a, cudaStream_t stream) {
@@ -533,6 +535,7 @@ mlops_fbla_status mlops_fbla_shard_partial(const mlops_fbla_config *c, const mlo
   if (st == MLOPS_FBLA_OK) st = apply_shard(fn, sh, a);
   if (st != MLOPS_FBLA_OK) return st;
   a.phase = 2;
+  a.mass_given = 1;
   a.row_r = const_cast<float *>(row_mass_total);
   a.out_partial = partial;
   return enqueue_decode(fn, a, stream);
@@ -575,6 +578,7 @@ mlops_fbla_status mlops_fbla_shard_step(const mlops_fbla_config *c, const mlops_
   mass_pass.phase = 1;  // coarse pass; the rows' local masses
   mass_pass.row_r = reinterpret_cast<float *>(own + M.local_mass);
   mass_pass.status_cleared = 1;
+  sum_pass.mass_given = 1;
   sum_pass.phase = 2;   // select with the common masses, refine, the shard's sums
   sum_pass.row_r = reinterpret_cast<float *>(own + M.total);
   sum_pass.out_partial = reinterpret_cast<float *>(own + M.local_part);
@@ -673,6 +677,7 @@ int mlops_fbla_decode_at_items(const mlops_fbla_config *c, const int *length, co
   if (c && c->capacity <= 0) { refuse(fn, "a device-length decode is laid out by capacity, which has to be positive"); return -1; }
   fbla_k_decode a;
   if (make_decode(fn, c, length, q, k, out, true, scratch, scratch_bytes, a) != MLOPS_FBLA_OK) return -1;
+  a.mass_given = a.dense;  // (the plan's second pass leaves the rows' masses for the later ones)
   if (max == 0) { accepted(); return 4; }
   if (!passes || max < 4) { refuse(fn, "the plan has 4 passes: `max` is too small or `passes` is null"); return -1; }
   fbla_k_pass info[4];
@@ -793,6 +798,31 @@ int mlops_fbla_item_access(const mlops_fbla_items *passes, int npasses, int pass
     const long long row_r = p.geom[MLOPS_FBLA_GEOM_ROW_LSE], items = p.geom[MLOPS_FBLA_GEOM_ITEMS], counts = p.geom[MLOPS_FBLA_GEOM_COUNTS];
     const long long item_off = p.geom[3], status = p.geom[4];
     r.add(MLOPS_FBLA_ARG_LENGTH, 0, 0, 4, 4, a.lstride ? a.batch : 1);
+    if (a.dense) {  // part .. row_r holds the window rows, the value rows, the (m, l) pairs and the batch's prefix sums
+      const bool scores = p.kind == MLOPS_FBLA_ITEM_COARSE, values = p.kind == MLOPS_FBLA_ITEM_REFINE;
+      if (scores || values) {
+        r.add(MLOPS_FBLA_ARG_Q, 0, 0, (long long)a.batch * a.q_heads * row);
+        for (int h = 0; h < heads; ++h) head_units(r, p, h, 0, true, values, true);
+        r.add(MLOPS_FBLA_ARG_SCRATCH, scores, lse, part - lse);
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 1, status, 16);
+      }
+      if (scores)
+        for (int h = 0; h < heads; ++h) head_windows(r, h, 0, true, true);
+      else
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 0, part, row_r - part);
+      if (scores || values) r.add(MLOPS_FBLA_ARG_SCRATCH, 1, part, row_r - part);
+      if (p.kind == MLOPS_FBLA_ITEM_SELECT) {
+        const int first = 8 * x, n = vheads - first < 8 ? vheads - first : 8;
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 1, row_r + (long long)first * a.qg * 4, (long long)n * a.qg * 4);
+      } else if (!scores) {
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 0, row_r, (long long)vheads * a.qg * 4);
+      }
+      if (p.kind == MLOPS_FBLA_ITEM_MERGE) {
+        const int vh = item / a.qg, qi = item % a.qg, b = vh / hpr, hir = vh % hpr;
+        r.add(MLOPS_FBLA_ARG_OUT, 1, ((long long)b * a.q_heads + (hir / a.vg) * (a.qg * a.vg) + (hir % a.vg) * a.qg + qi) * row, row);
+      }
+      return r.n;
+    }
     if (p.kind == MLOPS_FBLA_ITEM_COARSE || p.kind == MLOPS_FBLA_ITEM_REFINE) {
       // a persistent CTA's unit range depends on the device length: every head's units are the envelope
       r.add(MLOPS_FBLA_ARG_Q, 0, 0, (long long)a.batch * a.q_heads * row);

@@ -210,6 +210,7 @@ extern "C" void fbla_k_decode_split_of(int cb, int batch, int kv_heads, int vg, 
 }
 
 extern "C" cudaError_t fbla_k_decode_launch(const fbla_k_decode *a, cudaStream_t stream) {
+  if (a->dense) return fbla_k_dense_launch(a, stream);
   using namespace fbla;
   if (a->cb == 3) {
     switch (a->qg) {
@@ -227,6 +228,7 @@ extern "C" cudaError_t fbla_k_decode_launch(const fbla_k_decode *a, cudaStream_t
 
 // (after one whole fbla_k_decode_launch on this device: that call sets the kernels' shared-memory attributes)
 extern "C" cudaError_t fbla_k_decode_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream) {
+  if (a->dense) return fbla_k_dense_pass_launch(a, pass, stream);
   using namespace fbla;
   if (a->cb == 3) {
     switch (a->qg) {
@@ -243,6 +245,7 @@ extern "C" cudaError_t fbla_k_decode_pass_launch(const fbla_k_decode *a, int pas
 }
 
 extern "C" cudaError_t fbla_k_decode_passes(const fbla_k_decode *a, fbla_k_pass info[4]) {
+  if (a->dense) return fbla_k_dense_passes(a, info);
   using namespace fbla;
   if (a->cb == 3) {
     switch (a->qg) {

@@ -267,18 +267,18 @@ struct WindowTile {
   uint4 v[8];
   int count;  // attended tokens of the sub-block (1 .. 16)
 };
-// the window sub-blocks [lo, hi) of the flattened list; the partial rows go to window slot xw + virtual head
-template <int QG>
-__device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, long long lo, long long hi, int xw) {
+// The window sub-blocks [lo, hi) of the flattened list, c the cursor of `lo`; the partial rows of virtual head vh go to
+// rows + vh QG PSTRIDE. AHEAD: the next sub-block's loads are issued before the current one is computed (64 registers
+// more: for the kernels with few warps per SM).
+template <int QG, bool AHEAD>
+__device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, long long lo, long long hi, Cursor c, float *rows) {
   const int hpr = a.kv_heads * a.vg;
   if (lo >= hi) return;
-  const int slot0 = a.coarse_ctas * a.coarse_warps + a.batch * hpr;  // after the coarse slots
   const int gid = lane >> 2, tig = lane & 3;
-  Cursor c = locate<true>(a, hpr, lo);
   int cur_vh = -1;
   float m[2], l[2], o[8][4];  // queries 2 tig + e; o[tile]: channels 16 tile + gid (.0, .1), + 8 (.2, .3) x the two queries
   auto flush = [&]() {
-    float *p = a.part + (size_t)(slot0 + xw + cur_vh) * QG * PSTRIDE;
+    float *p = rows + (size_t)cur_vh * QG * PSTRIDE;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int qi = 2 * tig + e;
@@ -315,8 +315,9 @@ __device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, lon
   };
   for (int i = lane; i < 8 * (D + 8) / 2; i += 32) reinterpret_cast<uint32_t *>(&sm.q[0][0])[i] = 0u;
   WindowTile cur, nxt;
-  load(c, cur);
+  if (AHEAD) load(c, cur);
   for (long long u = lo; u < hi; ++u) {
+    if (!AHEAD) load(c, cur);
     const int vh = c.b * hpr + c.hir;
     if (vh != cur_vh) {
       if (cur_vh >= 0) flush();
@@ -342,7 +343,7 @@ __device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, lon
     }
     const int count = cur.count;
     advance<true>(a, hpr, c);
-    if (u + 1 < hi) load(c, nxt);
+    if (AHEAD && u + 1 < hi) load(c, nxt);
     // x[2 r + e]: token gid + 8 r, query 2 tig + e
     float al[2], w[2];
 #pragma unroll
@@ -375,15 +376,19 @@ __device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, lon
       o[mt][0] = fmaf(al[0], o[mt][0], w[0] * y[0]); o[mt][1] = fmaf(al[1], o[mt][1], w[1] * y[1]);
       o[mt][2] = fmaf(al[0], o[mt][2], w[0] * y[2]); o[mt][3] = fmaf(al[1], o[mt][3], w[1] * y[3]);
     }
-    cur = nxt;
+    if (AHEAD) cur = nxt;
   }
   flush();
+}
+// window slots lie after the coarse slots: slot xw + virtual head of window warp xw
+__device__ __forceinline__ float *window_rows(const fbla_k_decode &a, int qg, int xw) {
+  return a.part + (size_t)(a.coarse_ctas * a.coarse_warps + a.batch * a.kv_heads * a.vg + xw) * qg * PSTRIDE;
 }
 // window warp xw of nxw: an equal contiguous run of the sub-blocks
 template <int QG>
 __device__ __forceinline__ void exact_warp(const fbla_k_decode &a, ExactWarp &sm, int lane, int xw, int nxw) {
   const long long total = total_units<true>(a, a.kv_heads * a.vg), per = ceil_div(total, nxw), lo = (long long)xw * per;
-  exact_range<QG>(a, sm, lane, lo, min(total, lo + per), xw);
+  if (lo < total) exact_range<QG, true>(a, sm, lane, lo, min(total, lo + per), locate<true>(a, a.kv_heads * a.vg, lo), window_rows(a, QG, xw));
 }
 
 // ---- one closed group on the tensor cores ----------------------------------------------------------------------------------
@@ -679,7 +684,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
     long long xlo, xhi;
     gw = (long long)FBLA_POS::x() * sw + warp;
     deal_range(d, gw, xlo, xhi, lo, hi);
-    exact_range<QG>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, xlo, xhi, (int)gw);
+    if (xlo < xhi) exact_range<QG, true>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, xlo, xhi, locate<true>(a, hpr, xlo), window_rows(a, QG, (int)gw));
     __syncwarp();
   }
   StreamWarp<CB> &w = sm.w[warp];

@@ -1,0 +1,116 @@
+// Launchers of the dense decode (bodies: fbla_dense.cuh).
+#include "fbla_dense.cuh"
+#include <stdio.h>
+
+namespace fbla {
+namespace dense {
+template <int CB, int FB, int QG>
+__global__ void __launch_bounds__(32 * SCORE_WARPS, 1) score_kernel(const fbla_k_decode a) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  score_item<CB, FB, QG>(a, smem_raw);
+}
+
+template <int QG>
+__global__ void __launch_bounds__(256) mass_kernel(const fbla_k_decode a) {
+  mass_item<QG>(a, nullptr);
+}
+
+template <int CB, int FB, int QG>
+__global__ void __launch_bounds__(32 * VALUE_WARPS, 1) value_kernel(const fbla_k_decode a) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  value_item<CB, FB, QG>(a, smem_raw);
+}
+
+template <int QG>
+__global__ void __launch_bounds__(128) gather_kernel(const fbla_k_decode a) {
+  gather_item<QG>(a, nullptr);
+}
+
+// a launch that may begin while the previous kernel of the stream still runs (the kernel calls wait_previous_pass)
+template <class... P, class... A>
+cudaError_t launch(bool dependent, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int CB, int FB, int QG> struct Kernels {
+  static constexpr size_t SCORE_SMEM = sizeof(ScoreSmem), VALUE_SMEM = sizeof(ValueSmem<CB, FB>);
+  static cudaError_t configure() {  // once per device and host thread
+    static thread_local int configured[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(score_kernel<CB, FB, QG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCORE_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(value_kernel<CB, FB, QG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VALUE_SMEM);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = 1;
+    return e;
+  }
+  static cudaError_t pass(const fbla_k_decode &a, int which, bool dependent, cudaStream_t stream) {
+    const int vheads = a.batch * a.kv_heads * a.vg;
+    switch (which) {
+      case 0: return launch(dependent, score_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * SCORE_WARPS, SCORE_SMEM, stream, a);
+      case 1: return launch(dependent, mass_kernel<QG>, dim3((vheads + 7) / 8), 256, 0, stream, a);
+      case 2: return launch(dependent, value_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * VALUE_WARPS, VALUE_SMEM, stream, a);
+      case 3: return launch(dependent, gather_kernel<QG>, dim3(vheads * QG), 128, 0, stream, a);
+    }
+    return cudaErrorInvalidValue;
+  }
+  static cudaError_t all(const fbla_k_decode &a, cudaStream_t stream) {
+    cudaError_t e = configure();
+    if (a.phase != 2 && e == cudaSuccess) e = pass(a, 0, false, stream);
+    if (a.phase == 1) return e == cudaSuccess ? pass(a, 1, true, stream) : e;
+    if (e == cudaSuccess) e = pass(a, 2, a.phase != 2, stream);
+    return e == cudaSuccess ? pass(a, 3, true, stream) : e;
+  }
+  template <class K> static cudaError_t describe(K kernel, int items, int threads, size_t smem, fbla_k_pass *p) {
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    p->gx = items; p->gy = p->gz = 1; p->threads = threads; p->smem_bytes = (int)smem; p->regs = fa.numRegs;
+    return cudaSuccess;
+  }
+  static cudaError_t passes(const fbla_k_decode &a, fbla_k_pass *p) {
+    const int vheads = a.batch * a.kv_heads * a.vg;
+    cudaError_t e = describe(score_kernel<CB, FB, QG>, a.coarse_ctas, 32 * SCORE_WARPS, SCORE_SMEM, p + 0);
+    if (e == cudaSuccess) e = describe(mass_kernel<QG>, (vheads + 7) / 8, 256, 0, p + 1);
+    if (e == cudaSuccess) e = describe(value_kernel<CB, FB, QG>, a.coarse_ctas, 32 * VALUE_WARPS, VALUE_SMEM + 128, p + 2);
+    if (e == cudaSuccess) e = describe(gather_kernel<QG>, vheads * QG, 128, 0, p + 3);
+    snprintf(p[0].entry, sizeof p[0].entry, "fbla::dense::score_item<%d, %d, %d>", CB, FB, QG);
+    snprintf(p[1].entry, sizeof p[1].entry, "fbla::dense::mass_item<%d>", QG);
+    snprintf(p[2].entry, sizeof p[2].entry, "fbla::dense::value_item<%d, %d, %d>", CB, FB, QG);
+    snprintf(p[3].entry, sizeof p[3].entry, "fbla::dense::gather_item<%d>", QG);
+    return e;
+  }
+};
+
+template <class F> cudaError_t dispatch(const fbla_k_decode &a, F f) {
+  if (a.cb == 3) return a.qg == 1 ? f(Kernels<3, 3, 1>{}) : a.qg == 2 ? f(Kernels<3, 3, 2>{}) : f(Kernels<3, 3, 4>{});
+  return a.qg == 1 ? f(Kernels<4, 2, 1>{}) : a.qg == 2 ? f(Kernels<4, 2, 2>{}) : f(Kernels<4, 2, 4>{});
+}
+}  // namespace dense
+}  // namespace fbla
+
+extern "C" cudaError_t fbla_k_dense_launch(const fbla_k_decode *a, cudaStream_t stream) {
+  return fbla::dense::dispatch(*a, [&](auto k) { return decltype(k)::all(*a, stream); });
+}
+extern "C" cudaError_t fbla_k_dense_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream) {
+  return fbla::dense::dispatch(*a, [&](auto k) { return decltype(k)::pass(*a, pass, false, stream); });
+}
+extern "C" cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pass info[4]) {
+  return fbla::dense::dispatch(*a, [&](auto k) { return decltype(k)::passes(*a, info); });
+}
+
+// A sub-block of a row of N tokens holds 16 / N of the mass on average. Where that is at least half of tau most sub-blocks
+// are selected (the mass is spread unevenly) and computing each once is the faster way; beyond, the coarse planes alone
+// carry most of the sum and are read once instead of one and a half times. Measured on B200 with 32 query / 8 KV heads, us per
+// step coarse-first / dense: 3+3 (tau 3e-4) batch 8 x 32K 247 / 159, x 64K 349 / 274, x 128K 406 / 456; 4+2 (1e-3) batch
+// 8 x 16K 123 / 88, x 32K 132 / 130, x 64K 168 / 212.
+extern "C" int fbla_k_decode_dense(const fbla_k_decode *a, long long tokens, float tau) {
+  const long long groups = (tokens + fbla::G - 1) / fbla::G, pairs = (long long)a->batch * a->kv_heads * a->vg * groups * fbla::dense::PAIRS;
+  return a->batch <= FBLA_K_DENSE_MAX_BATCH && pairs < (1ll << 29) && (double)tokens * tau <= 2 * 16;
+}

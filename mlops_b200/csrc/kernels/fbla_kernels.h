@@ -51,16 +51,21 @@ typedef struct {
   // [sh_first, sh_first + sh_count) of its local cache, the BF16 sink window if sh_windows & 1, the open window if & 2.
   // phase 0: a whole decode. phase 1: coarse pass, then only the rows' local log2 mass into row_r. phase 2: select with
   // the given (global) row_r, refine, and the rows' unnormalised sums (o[128], l, relative to row_r) into out_partial.
-  int shard_on, sh_first, sh_count, sh_windows, phase;
+  int sh_first, sh_count;
+  short shard_on, sh_windows, phase;
+  short mass_given;    // dense: the rows' masses are in row_r (a pass before, or a shard's caller) instead of formed by the passes that need them
   float *out_partial;  // [rows][FBLA_K_PSTRIDE] floats (phase 2)
-  int status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
+  short status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
   short fold;          // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
+  short dense;         // 1: scores first, then every sub-block's value once (fbla_dense.cuh); 0: coarse sums, then corrections
   short deal;          // how the coarse pass's warps share the work, FBLA_K_DEAL_*
 } fbla_k_decode;
 #define FBLA_K_DEAL_LENGTHS 0 /* a CTA's warps are split between windows and groups by the rows' lengths (short contexts) */
 #define FBLA_K_DEAL_FIXED 1   /* seven warps of a CTA stream groups, the eighth serves windows */
 #define FBLA_K_DEAL_COST 2    /* every warp takes an equal cost share of windows and groups (long contexts) */
 
+#define FBLA_K_DENSE_MAX_BATCH 1024  /* batch rows of a dense decode: their prefix sums lie in shared memory */
+#define FBLA_K_DENSE_VALUE_WARPS 12
 #define FBLA_K_PSTRIDE 132 /* floats of one partial row: o[128], then (m, l) or (dl) and padding */
 #define FBLA_K_SLICE 1024  /* sub-blocks per select slice */
 
@@ -71,6 +76,11 @@ FBLA_HOST_API(cudaError_t fbla_k_decode_launch(const fbla_k_decode *a, cudaStrea
 FBLA_HOST_API(cudaError_t fbla_k_decode_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)
 // chooses the split of the coarse CTAs' warps for rows of about `tokens` tokens (after fbla_k_decode_shape; the scratch layout holds either)
 FBLA_HOST_API(void fbla_k_decode_split(fbla_k_decode *a, long long tokens);)
+// 1 if a decode of rows of about `tokens` tokens with selection threshold tau runs dense
+FBLA_HOST_API(int fbla_k_decode_dense(const fbla_k_decode *a, long long tokens, float tau);)
+// the dense passes (0 scores, 1 rows' masses, 2 values, 3 merge): a whole decode or shard phase; one pass
+FBLA_HOST_API(cudaError_t fbla_k_dense_launch(const fbla_k_decode *a, cudaStream_t stream);)
+FBLA_HOST_API(cudaError_t fbla_k_dense_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)
 // the same choice for a shape given by its numbers (pure host arithmetic: no device is touched): deal and fold as fbla_k_decode_split sets them
 FBLA_HOST_API(void fbla_k_decode_split_of(int cb, int batch, int kv_heads, int vg, long long tokens, int *deal, int *fold);)
 // out[row][ch] = bf16(partial[row][ch] / partial[row][128]) for rows rows of FBLA_K_PSTRIDE floats
@@ -181,6 +191,7 @@ typedef struct {
   char entry[96];    // the device function (kernels/*.cuh), called as entry(args, shared memory)
 } fbla_k_pass;
 FBLA_HOST_API(cudaError_t fbla_k_decode_passes(const fbla_k_decode *a, fbla_k_pass info[4]);)  // coarse, select, refine, merge
+FBLA_HOST_API(cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pass info[4]);)
 FBLA_HOST_API(cudaError_t fbla_k_close_pass(const fbla_k_prefill *a, int close_blocks, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_finish_pass(const fbla_k_prefill *a, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_attend_rows_pass(const fbla_k_prefill *a, fbla_k_pass *info);)

@@ -1,0 +1,48 @@
+"""The dense decode (scores first, then every sub-block's value once) and the decode that corrects coarse sums, at the
+lengths where dealing or table look-ups can go wrong, against the oracle: no closed group, one, runs that end inside a
+group; 1, 2 and 4 queries per virtual head; ragged rows; selection of none, some and all sub-blocks; shards of such rows."""
+import numpy as np
+import pytest
+import torch
+
+from tests import datagen
+from tests import gpu_util as gu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ours():
+    return gu.CLib(gu.OURS)
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("B,QH,KH,N,tau", [(1, 1, 1, 1, 0.0), (1, 4, 1, 128, 0.0), (2, 8, 2, 256, 1e-6), (1, 2, 1, 257, 0.0), (1, 2, 2, 385, 2e-2),
+                                           (3, 8, 2, 1025, 4e-3), (1, 24, 2, 700, 1e-3), (17, 4, 1, 3000, 0.0), (2, 16, 8, 9001, 1e-3), (1, 1, 1, 20011, 1e-9)])
+def test_dense_sizes(ours, oracle, mode, B, QH, KH, N, tau):
+    q, k, v = datagen.baseline_case(7 + N, B, QH, KH, N)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode)
+    got = ours.decode(c, gu.bf16_tensor(q), tau=tau)
+    again = ours.decode(c, gu.bf16_tensor(q), tau=tau)
+    torch.cuda.synchronize()
+    assert torch.equal(got, again)
+    gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode), tau=tau), f"{mode} {N}")
+
+
+@pytest.mark.parametrize("lens", [[1, 2000, 129, 16], [300] * 3 + [1], [256, 257, 4000, 255, 31]])
+def test_dense_ragged_rows(ours, oracle, lens):
+    B, QH, KH, cap, mode = len(lens), 8, 2, 4096, "3+3"
+    q, k, v = datagen.uneven_case(3, B, QH, KH, max(lens))
+    c, o = ours.empty(B, KH, cap, mode), oracle.empty(B, KH, cap, mode)
+    for b, n in enumerate(lens):
+        row = ours.encode(gu.bf16_tensor(k[b:b + 1, :, :n]), gu.bf16_tensor(v[b:b + 1, :, :n]), mode, capacity=cap)
+        orow = oracle.encode(k[b:b + 1, :, :n], v[b:b + 1, :, :n], mode, capacity=cap)
+        for key in ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v"):
+            c[key][b].copy_(row[key][0])
+            o[key][b * KH:(b + 1) * KH] = orow[key]
+    got = ours.decode_at(c, gu.bf16_tensor(q), torch.tensor(lens, dtype=torch.int32, device="cuda"), length_stride=1)
+    torch.cuda.synchronize()
+    o["tokens"] = max(lens)
+    want = oracle.decode(q, o, lengths=np.array(lens, np.int32))
+    for b in range(B):
+        gu.check_close(gu.bits_of(got)[b], want[b], f"row {b} of {lens}")
