@@ -34,7 +34,7 @@ extern "C" {
 #endif
 
 /* Pass kinds (values as the reference's). This library emits: CLOSE (one group the chunk may close, x, of KV head y),
- * STREAM (8 query rows of KV head y on CUDA cores: chunks of fewer than 64 rows), TC (256 query rows of KV head y on
+ * STREAM (8 query rows of KV head y, every share of their groups: chunks of fewer than 64 rows), TC (256 query rows of KV head y on
  * tcgen05 tensor cores; no split pieces, no TC_MERGE pass, no TRANSCODE: this library keeps no images; a prefill plan whose
  * count lives on the device and may reach 64 rows has a TC and a STREAM pass, of which the count activates one), FINISH (one KV
  * head's windows), COARSE / REFINE (CTA x of the persistent pass), SELECT (slice x of virtual head y), MERGE (one output

@@ -251,6 +251,7 @@ void fill_chunk(const mlops_fbla_config *c, int count, long long room, const uin
   a.cb = coarse_bits(c);
   a.fb = fine_bits(c);
   a.sl = log2_scale(c);
+  a.room = (int)room;
 }
 // The passes in the order that keeps them correct: closing groups reads the windows as they were, the attention reads
 // them too, and only then are the windows rewritten. Without queries one launch does both (fbla_close.cuh: write_item).

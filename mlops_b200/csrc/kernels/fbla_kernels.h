@@ -146,6 +146,8 @@ typedef struct {
   // > 0 (a chunk that starts a cache whose arrays have no initial contents): the groups per KV head that the layout has
   // room for; what the chunk does not write of their units and of the sink window is zeroed (fbla_k_write_launch)
   int clear_groups;
+  int room;     // tokens the cache is laid out for
+  int cluster;  // few-row pass: CTAs per tile, one per share of its groups (fbla_prefill_rows.cuh); 1: a CTA takes all shares
 } fbla_k_prefill;
 
 // close_blocks: grid x of the close pass (groups the chunk can close); 0 skips it
@@ -154,7 +156,7 @@ FBLA_HOST_API(cudaError_t fbla_k_finish_launch(const fbla_k_prefill *a, cudaStre
 // close and finish of a chunk without queries as one launch
 FBLA_HOST_API(cudaError_t fbla_k_write_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream);)
 // Attention of the chunk's rows: the tensor-core kernel (tcgen05, 128 rows per CTA), or -- for chunks of fewer than
-// FBLA_K_TC_MIN_ROWS rows, or when the environment variable MLOPS_FBLA_PREFILL=rows asks for it -- one warp per row.
+// FBLA_K_TC_MIN_ROWS rows, or when the environment variable MLOPS_FBLA_PREFILL=rows asks for it -- the few-row kernel.
 // fbla_k_attend_plan splits a chunk's attention into its one or two passes (two when the count is on the device and
 // its ceiling reaches the tensor-core kernel, see tc_min_rows): args[i] / tensor[i] for pass i; returns their number.
 FBLA_HOST_API(int fbla_k_attend_plan(const fbla_k_prefill *a, fbla_k_prefill args[2], int tensor[2]);)
@@ -165,6 +167,7 @@ FBLA_HOST_API(cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaS
 // error. A CTA whose wait gave up also writes NaN to every output row it owns, so the failure shows in the data.
 FBLA_HOST_API(int fbla_k_attend_tc_status(void);)
 #define FBLA_K_TC_MIN_ROWS 64
+#define FBLA_K_ROW_SHARES 8  /* CTAs of a few-row tile's cluster at most */
 
 // ---- fused QKV step: RMSNorm + rotary embedding of new tokens (+ the window stores of the one-token step) ------------------
 typedef struct {
@@ -194,7 +197,7 @@ FBLA_HOST_API(cudaError_t fbla_k_decode_passes(const fbla_k_decode *a, fbla_k_pa
 FBLA_HOST_API(cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pass info[4]);)
 FBLA_HOST_API(cudaError_t fbla_k_close_pass(const fbla_k_prefill *a, int close_blocks, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_finish_pass(const fbla_k_prefill *a, fbla_k_pass *info);)
-FBLA_HOST_API(cudaError_t fbla_k_attend_rows_pass(const fbla_k_prefill *a, fbla_k_pass *info);)
+FBLA_HOST_API(cudaError_t fbla_k_attend_rows_pass(fbla_k_prefill *a, fbla_k_pass *info);)  // (sets a->cluster)
 FBLA_HOST_API(cudaError_t fbla_k_attend_tc_pass(const fbla_k_prefill *a, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_qkv_token_pass(const fbla_k_token *a, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_qkv_chunk_pass(const fbla_k_token *a, fbla_k_pass *info);)

@@ -1,35 +1,61 @@
-// Launcher of the warp-per-row prefill attention (body: fbla_prefill_rows.cuh).
+// Launcher of the few-row prefill attention (body: fbla_prefill_rows.cuh).
 #include "fbla_prefill_rows.cuh"
 #include <stdio.h>
 
-namespace {
-template <class K> cudaError_t pass_of(K kernel, int gx, int gy, int threads, size_t smem, const char *entry, fbla_k_pass *p) {
-  cudaFuncAttributes fa;
-  const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  p->gx = gx; p->gy = gy; p->gz = 1; p->threads = threads; p->smem_bytes = (int)smem; p->regs = fa.numRegs;
-  snprintf(p->entry, sizeof p->entry, "%s", entry);
-  return cudaSuccess;
-}
-}  // namespace
-
 namespace fbla {
 template <int CB, int FB>
-__global__ void __launch_bounds__(256) attend_rows_kernel(const fbla_k_prefill a) {
-  attend_rows_item<CB, FB>(a, nullptr);
+__global__ void __launch_bounds__(32 * rows::WARPS, 1) attend_rows_kernel(const fbla_k_prefill a) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  attend_rows_item<CB, FB>(a, smem_raw);
+}
+
+template <int CB, int FB> static cudaError_t launch_rows(const fbla_k_prefill &a, int tiles, cudaStream_t stream) {
+  constexpr int smem = (int)sizeof(rows::RowSmem<CB, FB>);
+  static thread_local int configured[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(attend_rows_kernel<CB, FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * a.cluster, a.batch * a.kv_heads); cfg.blockDim = dim3(32 * rows::WARPS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = a.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = a.cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, attend_rows_kernel<CB, FB>, a);
+}
+
+// tiles of the launch: with a device count that goes to the tensor-core pass from tc_min_rows rows on, no more than it leaves here
+static int row_tiles(const fbla_k_prefill &a) {
+  const int rows = a.count * (a.q_heads / a.kv_heads), most = a.tc_min_rows && rows >= a.tc_min_rows ? a.tc_min_rows - 1 : rows;
+  return (most + rows::COLS - 1) / rows::COLS;
 }
 }  // namespace fbla
 
 extern "C" cudaError_t fbla_k_attend_rows_launch(const fbla_k_prefill *a, cudaStream_t stream) {
-  const int qg = a->q_heads / a->kv_heads;
-  const dim3 grid((a->count * qg + 7) / 8, a->batch * a->kv_heads);
-  if (a->cb == 3) fbla::attend_rows_kernel<3, 3><<<grid, 256, 0, stream>>>(*a);
-  else fbla::attend_rows_kernel<4, 2><<<grid, 256, 0, stream>>>(*a);
-  return cudaGetLastError();
+  const int tiles = fbla::row_tiles(*a);
+  fbla_k_prefill args = *a;
+  if (a->length) {  // the shares follow from the device's length and count: the cluster has room for as many as they can become
+    const long long most = (a->room / fbla::G + fbla::rows::WARPS - 1) / fbla::rows::WARPS;
+    args.cluster = most < 1 ? 1 : most > FBLA_K_ROW_SHARES ? FBLA_K_ROW_SHARES : (int)most;
+  } else {
+    args.cluster = fbla::rows::row_shares((long long)tiles * a->batch * a->kv_heads, (a->n0 + a->count - 1) / fbla::G);
+  }
+  return a->cb == 3 ? fbla::launch_rows<3, 3>(args, tiles, stream) : fbla::launch_rows<4, 2>(args, tiles, stream);
 }
 
-extern "C" cudaError_t fbla_k_attend_rows_pass(const fbla_k_prefill *a, fbla_k_pass *info) {
-  const int rows = a->count * (a->q_heads / a->kv_heads), heads = a->batch * a->kv_heads;
-  if (a->cb == 3) return pass_of(fbla::attend_rows_kernel<3, 3>, (rows + 7) / 8, heads, 256, 0, "fbla::attend_rows_item<3, 3>", info);
-  return pass_of(fbla::attend_rows_kernel<4, 2>, (rows + 7) / 8, heads, 256, 0, "fbla::attend_rows_item<4, 2>", info);
+extern "C" cudaError_t fbla_k_attend_rows_pass(fbla_k_prefill *a, fbla_k_pass *info) {
+  using namespace fbla;
+  a->cluster = 1;
+  cudaFuncAttributes fa;
+  const cudaError_t e = a->cb == 3 ? cudaFuncGetAttributes(&fa, attend_rows_kernel<3, 3>) : cudaFuncGetAttributes(&fa, attend_rows_kernel<4, 2>);
+  if (e != cudaSuccess) return e;
+  info->gx = row_tiles(*a); info->gy = a->batch * a->kv_heads; info->gz = 1; info->threads = 32 * rows::WARPS;
+  info->smem_bytes = (int)(a->cb == 3 ? sizeof(rows::RowSmem<3, 3>) : sizeof(rows::RowSmem<4, 2>)) + 128;
+  info->regs = fa.numRegs;
+  snprintf(info->entry, sizeof info->entry, "fbla::attend_rows_item<%d, %d>", a->cb, a->fb);
+  return cudaSuccess;
 }

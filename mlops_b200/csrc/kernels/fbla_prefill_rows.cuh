@@ -1,180 +1,447 @@
-// Causal prefill attention over the compressed cache, CUDA-core version: one warp per query row.
+// Causal prefill attention of a few query rows over the compressed cache (chunks of fewer than 64 rows per KV head: drafted
+// tokens, short continuations), sm_100a.
 //
-// Semantics (the reference's DP4A prefill, attention/fbla/src/fbla_prefill.cuh:389-705): the row at position p attends
-// to 0..p -- group 0 (sink) and its own group in BF16 from the windows / the chunk, closed groups 1..own-1 through
-// their full 6-bit codes (coarse << FB | fine) with the per-(row, group) int8 qhat, 16-token integer P blocks
-// everywhere. This kernel is the simple, obviously-correct form of that definition (each lane is the record lane of
-// the same number, integer dot products by DP4A); it is the fallback the tensor-core prefill is checked against
-// and the path taken for shapes the tensor-core kernel does not cover.
+// Semantics (the reference's DP4A prefill, attention/fbla/src/fbla_prefill.cuh:389-705) -- the row at position p attends
+// to 0..p: group 0 (sink) and its own group in BF16 from the windows / the chunk, closed groups 1..own-1 through their
+// full 6-bit codes (coarse << FB | fine) with the per-(row, group) int8 qhat, 16-token integer P blocks everywhere.
+//
+// Eight rows of one KV head are the eight columns of the decode's integer tensor-core products (fbla_frag.cuh): a tile's
+// closed groups are dealt in pairs of sub-blocks to twelve warps, each streaming its run through a private two-stage ring
+// with a running (m, l, o); the BF16 blocks follow on BF16 products; the warps' rows are then merged in warp order. A long
+// cache and few tiles would leave most SMs idle, so a tile's pairs are also split into `shares`, one CTA of a thread-block
+// cluster each, whose merged rows the cluster reads from each other's shared memory: no scratch, no second launch. The
+// number of shares follows from the sizes alone (row_shares), and a CTA that has to do the whole tile (an executor's item)
+// takes the shares one after the other, so that both give the same bits.
+// Bound by instruction issue (about 2 500 warp instructions per group and tile). One warp per row walking the whole cache,
+// as this pass once did: 4 sequences x 5 drafted tokens at 12 345 tokens (32 / 8 heads) 1 670 us.
 #pragma once
-#include "fbla_device.cuh"
-#include "fbla_kernels.h"
+#include "fbla_decode.cuh"
 
 namespace fbla {
+namespace rows {
 
-template <int BITS> __device__ __forceinline__ void load_words(const uint8_t *rec, int tensor, int lane, uint32_t *W) {
-#pragma unroll
-  for (int w = 0; w < 2 * BITS; ++w) W[w] = __ldcg(reinterpret_cast<const uint32_t *>(rec + word_offset(BITS, tensor, lane, w)));
+constexpr int WARPS = 12, COLS = 8, PAIRS = SBG / 2, NST = 2;
+constexpr int MAX_SHARES = FBLA_K_ROW_SHARES;
+constexpr int SET = COLS * FBLA_K_PSTRIDE;  // floats of a tile's row set: per row o[128], m, l
+
+// How many shares a tile's closed groups are split into: the number (at most a cluster of eight) that makes waves of
+// CTAs x groups per warp smallest, the smaller one of equals. SMs: a B200's, whatever the device, so that the choice is one
+// of the sizes alone.
+__host__ __device__ inline int row_shares(long long tiles, int groups) {
+  int best = 1;
+  long long least = -1;
+  for (int c = 1; c <= MAX_SHARES; ++c) {
+    const long long cost = (tiles * c + 147) / 148 * ((groups + WARPS * c - 1) / (WARPS * c));
+    if (least < 0 || cost < least) { least = cost; best = c; }
+  }
+  return best;
 }
 
-struct RowState { float m, l, o[4]; };
+template <int CB, int FB> struct __align__(128) RowWarp {
+  uint8_t pair[NST][2 * (record_bytes(CB) + record_bytes(FB))];  // two coarse records, two fine records; later the warp's row set and BF16 staging
+  uint8_t meta[2][1024];
+  uint8_t qst[COLS * QST_ROW];
+  uint8_t pst[128];  // P bytes of a sub-block: [row][16 tokens]
+  uint64_t bar[NST], bar_meta[2];
+};
+struct __align__(16) RowStage {  // BF16 staging of a warp, in its ring
+  uint16_t v[S][D + 8];
+  uint16_t p[COLS][S];
+};
+template <int CB, int FB> struct RowSmem {
+  RowWarp<CB, FB> w[WARPS];
+  uint16_t q[COLS][D + 8];        // the tile's queries, BF16 (rows past the end: zero)
+  float share[MAX_SHARES][SET];   // the merged row sets of the shares this CTA has done
+  int failed;
+};
+static_assert(sizeof(RowSmem<3, 3>) + 128 <= 227 * 1024 && sizeof(RowSmem<4, 2>) + 128 <= 227 * 1024, "one CTA's shared memory");
+static_assert(SET * sizeof(float) + sizeof(RowStage) <= sizeof(RowWarp<4, 2>::pair) && SET * sizeof(float) + sizeof(RowStage) <= sizeof(RowWarp<3, 3>::pair), "row set and staging fit the ring");
 
-// one 16-token block given the lane's score (lanes t and t + 16 hold token t's) and a functor for sum_t p_t v[t][4 lane + cc]
-template <class PV> __device__ __forceinline__ void block_update(RowState &st, float s, uint8_t *pst, int lane, PV pv) {
-  float mb = s;
-#pragma unroll
-  for (int o = 8; o; o >>= 1) mb = fmaxf(mb, __shfl_xor_sync(FULL, mb, o));
-  if (mb == -FBLA_INF) return;  // (warp-uniform: every token masked)
-  if (lane < 16) pst[lane] = (uint8_t)__float_as_uint(fmaf(ex2(s - mb), 255.f, MAGICF));
-  __syncwarp();
-  const uint4 pw = *reinterpret_cast<const uint4 *>(pst);
-  const uint32_t P[4] = {pw.x, pw.y, pw.z, pw.w};
-  const float sp = (float)(__dp4a(P[0], 0x01010101u, 0u) + __dp4a(P[1], 0x01010101u, 0u) + __dp4a(P[2], 0x01010101u, 0u) + __dp4a(P[3], 0x01010101u, 0u));
-  float y[4];
-  pv(P, y);
-  const float mn = fmaxf(st.m, mb), al = ex2(st.m - mn), w = ex2(mb - mn);
-  st.m = mn;
-  st.l = fmaf(al, st.l, w * sp);
-#pragma unroll
-  for (int cc = 0; cc < 4; ++cc) st.o[cc] = fmaf(al, st.o[cc], w * y[cc]);
-  __syncwarp();
+// ---- thread-block cluster (stream launches only) --------------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the float(s) at this CTA's shared address p, in the cluster's CTA `rank`
+__device__ __forceinline__ uint32_t remote(const void *p, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 ld_remote4(uint32_t p) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_remote2(uint32_t p) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_remote1(uint32_t p) {
+  int v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+  return v;
 }
 
+// scores of one sub-block under both planes: code units = 2^FB h + f; thread (gid, tig): tokens gid (x[0]), gid + 8 (x[1]) of rows 2 tig, 2 tig + 1
+template <int CB, int FB>
+__device__ __forceinline__ void qk_full(const uint8_t *crec, const uint8_t *frec, int gid, int tig, const uint32_t (&B)[8], float2 (&x)[2]) {
+  float h[4], f[4];
+  qk_tile<CB>(crec, gid, tig, B, h);
+  qk_tile<FB>(frec, gid, tig, B, f);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) x[i] = __ffma2_rn(splat((float)(1 << FB)), make_float2(h[2 * i], h[2 * i + 1]), make_float2(f[2 * i], f[2 * i + 1]));
+}
+
+// the sums of a warp: rows 2 tig + e, e = 0, 1, in (.x, .y); channels 4 (8 u + gid) + cc
+struct State { float m[2]; float2 l, o[4][4]; };
+
+// ---- the warp's run of pairs [lo, hi) of the closed groups (pair p: sub-blocks 2 (p % 4), + 1 of group 1 + p / 4) ----------------
+// own[e]: the group of row 2 tig + e (it attends to the closed groups before it). false: a bounded wait gave up.
+template <int CB, int FB>
+__device__ __forceinline__ bool closed_run(const fbla_k_prefill &a, RowWarp<CB, FB> &w, const uint16_t (&q)[COLS][D + 8], size_t head, int lo, int hi,
+                                           const int (&own)[2], uint32_t &uses, State &st, int lane) {
+  constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
+  const int gid = lane >> 2, tig = lane & 3;
+  const uint32_t base = uses;  // ring uses before this run (the barriers live through all of a CTA's shares)
+  auto issue = [&](int p) {    // lane 0
+    const int s = (base + (p - lo)) % NST, J = p % PAIRS, ms = (p / PAIRS) & 1;
+    const size_t unit = head + (size_t)(1 + p / PAIRS) * a.gs;
+    const bool meta = p == lo || J == 0;
+    mbar_expect_tx(&w.bar[s], 2 * (RC + RF) + (meta ? 1024 : 0));
+    bulk_g2s(w.pair[s], a.c.coarse + (unit * SBG + 2 * J) * RC, 2 * RC, &w.bar[s]);
+    bulk_g2s(w.pair[s] + 2 * RC, a.c.fine + (unit * SBG + 2 * J) * RF, 2 * RF, &w.bar[s]);
+    if (meta) bulk_g2s(w.meta[ms], reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024, 1024, &w.bar[s]);
+  };
+  if (lane == 0) {
+    fence_async_smem();  // (the ring may have held a row set)
+#pragma unroll
+    for (int s = 0; s < NST; ++s)
+      if (lo + s < hi) issue(lo + s);
+  }
+  int p = lo;
+  while (p < hi) {
+    const int g = 1 + p / PAIRS, end = min(hi, (p / PAIRS + 1) * PAIRS);
+    const uint8_t *meta = w.meta[(p / PAIRS) & 1];
+    float2 sq2 = make_float2(0.f, 0.f), qb2 = sq2, A[4][4], L = sq2;
+    uint32_t B[8];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) A[u][cc] = make_float2(0.f, 0.f);
+    const bool on[2] = {g < own[0], g < own[1]};
+    for (bool first = true; p < end; ++p, first = false) {
+      const uint32_t use = base + (p - lo);
+      if (!__all_sync(FULL, mbar_wait_bounded(&w.bar[use % NST], (use / NST) & 1))) return false;
+      if (first) {  // the rows' qhat for this group
+        const uint4 km = lds128(meta + 16 * lane);
+#pragma unroll
+        for (int r = 0; r < COLS; ++r) {
+          const uint2 qw = *reinterpret_cast<const uint2 *>(&q[r][4 * lane]);
+          float sq, qb, qsum;
+          reinterpret_cast<uint32_t *>(w.qst + QST_ROW * r)[lane] = quantize_query_word(km, make_float4(bf_lo(qw.x), bf_hi(qw.x), bf_lo(qw.y), bf_hi(qw.y)), a.sl, sq, qb, qsum);
+          if (r == 2 * tig) { sq2.x = sq; qb2.x = qb; }
+          if (r == 2 * tig + 1) { sq2.y = sq; qb2.y = qb; }
+        }
+        __syncwarp();
+        qhat_frag<CB>(w.qst, gid, tig, B);
+      }
+#pragma unroll 1
+      for (int par = 0; par < 2; ++par) {
+        const uint8_t *crec = w.pair[use % NST] + par * RC, *frec = w.pair[use % NST] + 2 * RC + par * RF;
+        float2 x[2];
+        qk_full<CB, FB>(crec, frec, gid, tig, B, x);
+        const float2 s0 = __ffma2_rn(sq2, x[0], qb2), s1 = __ffma2_rn(sq2, x[1], qb2);
+        float mb[2] = {fmaxf(s0.x, s1.x), fmaxf(s0.y, s1.y)};
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) mb[e] = fmaxf(mb[e], __shfl_xor_sync(FULL, mb[e], o));
+        // the running maximum moves only when a block exceeds it by more than 2^8
+        const bool grow0 = on[0] && mb[0] > st.m[0] + 8.f, grow1 = on[1] && mb[1] > st.m[1] + 8.f;
+        if (__any_sync(FULL, grow0 || grow1)) {
+          const float al0 = grow0 ? ex2(st.m[0] - mb[0]) : 1.f, al1 = grow1 ? ex2(st.m[1] - mb[1]) : 1.f;
+          if (grow0) st.m[0] = mb[0];
+          if (grow1) st.m[1] = mb[1];
+          const float2 al = make_float2(al0, al1);
+          st.l = __fmul2_rn(st.l, al);
+          L = __fmul2_rn(L, al);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) { st.o[u][cc] = __fmul2_rn(st.o[u][cc], al); A[u][cc] = __fmul2_rn(A[u][cc], al); }
+        }
+        const float2 nm = make_float2(-mb[0], -mb[1]), d0 = __fadd2_rn(s0, nm), d1 = __fadd2_rn(s1, nm);
+        const float2 p0 = __ffma2_rn(make_float2(ex2(d0.x), ex2(d0.y)), splat(255.f), splat(MAGICF));
+        const float2 p1 = __ffma2_rn(make_float2(ex2(d1.x), ex2(d1.y)), splat(255.f), splat(MAGICF));
+        w.pst[32 * tig + gid] = (uint8_t)__float_as_uint(p0.x); w.pst[32 * tig + gid + 8] = (uint8_t)__float_as_uint(p1.x);
+        w.pst[32 * tig + 16 + gid] = (uint8_t)__float_as_uint(p0.y); w.pst[32 * tig + 16 + gid + 8] = (uint8_t)__float_as_uint(p1.y);
+        const float2 wt = make_float2(on[0] ? ex2(mb[0] - st.m[0]) : 0.f, on[1] ? ex2(mb[1] - st.m[1]) : 0.f);
+        __syncwarp();
+        const uint32_t b0 = lds32(w.pst + 4 * lane);  // row gid, tokens 4 tig ..
+        {
+          uint32_t d[4];
+          mma_u8u8_k16_from(d, 0x01010101u, 0x01010101u, b0, MAGIC);
+          L = __ffma2_rn(wt, isum2(d[0], d[1]), L);
+        }
+        float2 wc[4], wf[4];
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+          wc[cc] = __fmul2_rn(wt, splat((float)(1 << FB) * v_unscale<CB>(cc)));
+          wf[cc] = __fmul2_rn(wt, splat(v_unscale<FB>(cc)));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          uint32_t vh[4], vl[4], h01[4], h23[4], l01[4], l23[4];
+          v_slots<CB>(crec, 8 * u + gid, tig, vh);
+          v_slots<FB>(frec, 8 * u + gid, tig, vl);
+          mma_u8u8_k16_from(h01, vh[0], vh[1], b0, MAGIC);
+          mma_u8u8_k16_from(h23, vh[2], vh[3], b0, MAGIC);
+          mma_u8u8_k16_from(l01, vl[0], vl[1], b0, MAGIC);
+          mma_u8u8_k16_from(l23, vl[2], vl[3], b0, MAGIC);
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) {
+            const uint32_t *hh = cc < 2 ? h01 : h23, *ll = cc < 2 ? l01 : l23;
+            A[u][cc] = __ffma2_rn(wc[cc], isum2(hh[2 * (cc & 1)], hh[2 * (cc & 1) + 1]), __ffma2_rn(wf[cc], isum2(ll[2 * (cc & 1)], ll[2 * (cc & 1) + 1]), A[u][cc]));
+          }
+        }
+        __syncwarp();  // pst -- and behind the second sub-block the slot -- has been read
+      }
+      if (lane == 0 && p + NST < hi) issue(p + NST);
+    }
+    st.l = __fadd2_rn(st.l, L);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint4 vm = lds128(meta + 512 + 16 * (8 * u + gid));
+      const float vb[4] = {bf_lo(vm.x), bf_hi(vm.x), bf_lo(vm.y), bf_hi(vm.y)}, vs[4] = {bf_lo(vm.z), bf_hi(vm.z), bf_lo(vm.w), bf_hi(vm.w)};
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) st.o[u][cc] = __fadd2_rn(st.o[u][cc], __ffma2_rn(splat(vs[cc]), A[u][cc], __fmul2_rn(splat(vb[cc]), L)));
+    }
+    __syncwarp();
+  }
+  uses = base + (uint32_t)max(hi - lo, 0);
+  return true;
+}
+
+// the warp's row set in shared memory: per row o[128], m, l
+__device__ __forceinline__ void write_state(float *set, const State &st, int lane) {
+  const int gid = lane >> 2, tig = lane & 3;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    float *row = set + (2 * tig + e) * FBLA_K_PSTRIDE;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      *reinterpret_cast<float4 *>(row + 4 * (8 * u + gid)) = e ? make_float4(st.o[u][0].y, st.o[u][1].y, st.o[u][2].y, st.o[u][3].y)
+                                                                : make_float4(st.o[u][0].x, st.o[u][1].x, st.o[u][2].x, st.o[u][3].x);
+    if (gid == 0) { row[D] = st.m[e]; row[D + 1] = e ? st.l.y : st.l.x; }
+  }
+}
+
+// BF16 sub-blocks first, first + step, ... < total of the tile's list, added to the warp's row set. Block n < sink: n-th of group
+// 0; else (n - sink) % 8 of group own_lo + (n - sink) / 8. Row 2 tig + e stands at pos[e] (-1: no such row) in group own[e].
+template <class RowOf>
+__device__ __forceinline__ void exact_blocks(const fbla_k_prefill &a, const uint16_t (&q)[COLS][D + 8], RowStage &sm, float *set, int first, int step, int total,
+                                             int sink, int own_lo, int n1, const int (&pos)[2], const int (&own)[2], int lane, RowOf row_of) {
+  if (first >= total) return;
+  const int gid = lane >> 2, tig = lane & 3;
+  float m[2] = {-FBLA_INF, -FBLA_INF}, l[2] = {0.f, 0.f}, o[8][4];
+#pragma unroll
+  for (int mt = 0; mt < 8; ++mt) o[mt][0] = o[mt][1] = o[mt][2] = o[mt][3] = 0.f;
+#pragma unroll 1
+  for (int n = first; n < total; n += step) {
+    const int g = n < sink ? 0 : own_lo + (n - sink) / SBG, t0 = g * G + S * (n < sink ? n : (n - sink) % SBG);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {  // V rows
+      const int r = 2 * i + (lane >> 4);
+      const uint4 v = t0 + r < n1 ? __ldcg(reinterpret_cast<const uint4 *>(row_of(t0 + r, 1)) + (lane & 15)) : make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4 *>(&sm.v[r][8 * (lane & 15)]) = v;
+    }
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int r4 = 0; r4 < 4; ++r4) {  // channels 32 r4 + 8 tig .. of tokens gid, gid + 8
+      const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+      const uint4 ka = t0 + gid < n1 ? __ldcg(reinterpret_cast<const uint4 *>(row_of(t0 + gid, 0) + 32 * r4 + 8 * tig)) : zero;
+      const uint4 kb = t0 + gid + 8 < n1 ? __ldcg(reinterpret_cast<const uint4 *>(row_of(t0 + gid + 8, 0) + 32 * r4 + 8 * tig)) : zero;
+      const uint4 qq = *reinterpret_cast<const uint4 *>(&q[gid][32 * r4 + 8 * tig]);
+      mma_bf16_k16(x, ka.x, kb.x, ka.y, kb.y, qq.x, qq.y);
+      mma_bf16_k16(x, ka.z, kb.z, ka.w, kb.w, qq.z, qq.w);
+    }
+    float al[2], wt[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const bool here = g == 0 || own[e] == g;
+      const float s0 = here && t0 + gid <= pos[e] ? __fmul_rn(x[e], a.sl) : -FBLA_INF, s1 = here && t0 + gid + 8 <= pos[e] ? __fmul_rn(x[2 + e], a.sl) : -FBLA_INF;
+      float mb = fmaxf(s0, s1);
+#pragma unroll
+      for (int off = 4; off <= 16; off <<= 1) mb = fmaxf(mb, __shfl_xor_sync(FULL, mb, off));
+      const bool any = mb > -FBLA_INF;  // (a row that attends to nothing here keeps its sums)
+      const float mn = any ? fmaxf(m[e], mb) : m[e], mr = any ? mb : 0.f;
+      al[e] = any ? ex2(m[e] - mn) : 1.f;
+      wt[e] = any ? ex2(mb - mn) : 0.f;
+      m[e] = mn;
+      const float p0 = fmaf(ex2(s0 - mr), 255.f, MAGICF) - MAGICF, p1 = fmaf(ex2(s1 - mr), 255.f, MAGICF) - MAGICF;
+      sm.p[2 * tig + e][gid] = (uint16_t)(__float_as_uint(p0) >> 16);
+      sm.p[2 * tig + e][gid + 8] = (uint16_t)(__float_as_uint(p1) >> 16);
+      float sp = p0 + p1;
+#pragma unroll
+      for (int off = 4; off <= 16; off <<= 1) sp += __shfl_xor_sync(FULL, sp, off);
+      l[e] = fmaf(al[e], l[e], wt[e] * sp);
+    }
+    __syncwarp();
+    const uint32_t pb0 = *reinterpret_cast<const uint32_t *>(&sm.p[gid][2 * tig]), pb1 = *reinterpret_cast<const uint32_t *>(&sm.p[gid][2 * tig + 8]);
+#pragma unroll
+    for (int mt = 0; mt < 8; ++mt) {
+      uint32_t va[4];
+      ldmatrix_x4_trans(va, &sm.v[8 * (lane >> 4) + (lane & 7)][16 * mt + 8 * ((lane >> 3) & 1)]);
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_bf16_k16(y, va[0], va[1], va[2], va[3], pb0, pb1);
+      o[mt][0] = fmaf(al[0], o[mt][0], wt[0] * y[0]); o[mt][1] = fmaf(al[1], o[mt][1], wt[1] * y[1]);
+      o[mt][2] = fmaf(al[0], o[mt][2], wt[0] * y[2]); o[mt][3] = fmaf(al[1], o[mt][3], wt[1] * y[3]);
+    }
+  }
+  // into the row set
+  float sa[2], sb[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    float *row = set + (2 * tig + e) * FBLA_K_PSTRIDE;
+    const float ms = row[D], ls = row[D + 1], mn = fmaxf(ms, m[e]);
+    sa[e] = ms == -FBLA_INF ? 0.f : ex2(ms - mn);
+    sb[e] = m[e] == -FBLA_INF ? 0.f : ex2(m[e] - mn);
+#pragma unroll
+    for (int mt = 0; mt < 8; ++mt) {
+      row[16 * mt + gid] = fmaf(sa[e], row[16 * mt + gid], sb[e] * o[mt][e]);
+      row[16 * mt + gid + 8] = fmaf(sa[e], row[16 * mt + gid + 8], sb[e] * o[mt][2 + e]);
+    }
+    __syncwarp();
+    if (gid == 0) { row[D] = mn; row[D + 1] = fmaf(sa[e], ls, sb[e] * l[e]); }
+  }
+}
+}  // namespace rows
+
+// CTA x of head y: tile x / cluster of eight rows, share x % cluster (cluster 1: every share of the tile, one after the other)
 template <int CB, int FB>
 __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
-  __shared__ __align__(16) float qs[8][D];
-  __shared__ __align__(16) uint32_t qh[8][32];
-  __shared__ __align__(16) uint8_t pst[8][16];
-  const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5;
+  using namespace rows;
+  smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;
+  RowSmem<CB, FB> &sm = *reinterpret_cast<RowSmem<CB, FB> *>(smem_raw);
+  const int tid = FBLA_POS::tid(), lane = tid & 31, warp = tid >> 5, tig = lane & 3;
   const int bh = FBLA_POS::y(), b = bh / a.kv_heads, kh = bh - b * a.kv_heads, qg = a.q_heads / a.kv_heads;
   const int n0 = (a.length ? FBLA_POS::ro(a.length + (a.lstride ? b : 0)) : 0) + a.n0;
-  const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, n1 = n0 + count;
-  const int r = FBLA_POS::x() * 8 + warp;
-  if (r >= count * qg || (a.tc_min_rows && count * qg >= a.tc_min_rows)) return;  // (a long device count is the tensor-core pass's work)
-  const int i = r / qg, hq = kh * qg + (r - i * qg), pos = n0 + i, own = pos / G;
+  const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, n1 = n0 + count, rows = count * qg;
+  const int cluster = a.cluster, r0 = FBLA_POS::x() / cluster * COLS, rank = FBLA_POS::x() % cluster;
+  if (r0 >= rows || (a.tc_min_rows && rows >= a.tc_min_rows)) return;  // (cluster-uniform; a long device count is the tensor-core pass's work)
+  const int last = min(r0 + COLS, rows) - 1, max_pos = n0 + last / qg, own_min = (n0 + r0 / qg) / G, own_max = max_pos / G;
+  const int pairs = PAIRS * max(own_max - 1, 0);
+  const int shares = row_shares((long long)((rows + COLS - 1) / COLS) * a.batch * a.kv_heads, (n1 - 1) / G);
+  // the BF16 blocks: group 0, then the rows' own groups
+  const int sink = min(SBG, max_pos / S + 1), own_lo = max(own_min, 1), exact = sink + (own_max >= own_lo ? SBG * (own_max - own_lo) + (max_pos - own_max * G) / S + 1 : 0);
+  int pos[2], own[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int r = r0 + 2 * tig + e;
+    pos[e] = r < rows ? n0 + r / qg : -1;
+    own[e] = r < rows ? pos[e] / G : 0;
+  }
   const size_t eh = (size_t)bh * G * D, ih = (size_t)bh * a.count * D;
-  {
-    const uint2 w = __ldg(reinterpret_cast<const uint2 *>(a.q + ((size_t)(b * a.q_heads + hq) * a.count + i) * D) + lane);
-    *reinterpret_cast<float4 *>(&qs[warp][4 * lane]) = make_float4(bf_lo(w.x), bf_hi(w.x), bf_lo(w.y), bf_hi(w.y));
-  }
-  __syncwarp();
-  RowState st{-FBLA_INF, 0.f, {0.f, 0.f, 0.f, 0.f}};
-  const int t = lane & 15, h = lane >> 4;
-
   // the BF16 row of position tp: the chunk, the sink window, or the window of the group that was open before the chunk
-  auto row_of = [&](int tp, const uint16_t *in, const uint16_t *sink, const uint16_t *open) -> const uint16_t * {
-    return tp >= n0 ? in + ih + (size_t)(tp - n0) * D : tp < G ? sink + eh + (size_t)tp * D : open + eh + (size_t)(tp - (n0 - 1) / G * G) * D;
+  auto token_row = [&](int tp, int x) -> const uint16_t * {
+    return tp >= n0 ? (x ? a.v : a.k) + ih + (size_t)(tp - n0) * D : tp < G ? (x ? a.c.sink_v : a.c.sink_k) + eh + (size_t)tp * D
+                                                                         : (x ? a.c.open_v : a.c.open_k) + eh + (size_t)(tp - (n0 - 1) / G * G) * D;
   };
-  auto exact_group = [&](int g) {
-    for (int j = 0; j < SBG; ++j) {
-      const int t0 = g * G + j * S;
-      if (t0 > pos || t0 >= n1) break;
-      const int tp = t0 + t;
-      float x = 0.f;
-      if (tp <= pos) {
-        const uint4 *kp = reinterpret_cast<const uint4 *>(row_of(tp, a.k, a.c.sink_k, a.c.open_k) + 64 * h);
-#pragma unroll
-        for (int e8 = 0; e8 < 8; ++e8) {
-          const uint4 w = __ldcg(kp + e8);
-          const float kv[8] = {bf_lo(w.x), bf_hi(w.x), bf_lo(w.y), bf_hi(w.y), bf_lo(w.z), bf_hi(w.z), bf_lo(w.w), bf_hi(w.w)};
-#pragma unroll
-          for (int e = 0; e < 8; ++e) x = fmaf(qs[warp][64 * h + 8 * e8 + e], kv[e], x);
-        }
-      }
-      x += __shfl_xor_sync(FULL, x, 16);
-      const float s = tp <= pos ? __fmul_rn(x, a.sl) : -FBLA_INF;
-      block_update(st, s, pst[warp], lane, [&](const uint32_t (&P)[4], float (&y)[4]) {
-        y[0] = y[1] = y[2] = y[3] = 0.f;
-        for (int tt = 0; tt < S; ++tt) {
-          if (t0 + tt > pos) break;
-          const uint2 vw = __ldcg(reinterpret_cast<const uint2 *>(row_of(t0 + tt, a.v, a.c.sink_v, a.c.open_v)) + lane);
-          const float p = (float)((P[tt >> 2] >> (8 * (tt & 3))) & 255u);
-          y[0] = fmaf(p, bf_lo(vw.x), y[0]); y[1] = fmaf(p, bf_hi(vw.x), y[1]);
-          y[2] = fmaf(p, bf_lo(vw.y), y[2]); y[3] = fmaf(p, bf_hi(vw.y), y[3]);
-        }
-      });
-    }
-  };
-
-  exact_group(0);
-  if (own > 0) exact_group(own);
-  for (int g = own - 1; g >= 1; --g) {  // closed groups, newest first
-    const size_t unit = (size_t)bh * a.hs + (size_t)g * a.gs;
-    const uint8_t *meta = reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024;
-    const uint4 km = __ldcg(reinterpret_cast<const uint4 *>(meta) + lane);
-    const uint4 vm = __ldcg(reinterpret_cast<const uint4 *>(meta + 512) + lane);
-    // qhat of the row for this group (lane: channels 4 lane ..)
-    float sq, qb;
-    {
-      const float4 q4 = *reinterpret_cast<const float4 *>(&qs[warp][4 * lane]);
-      const float kb[4] = {bf_lo(km.x), bf_hi(km.x), bf_lo(km.y), bf_hi(km.y)}, ks[4] = {bf_lo(km.z), bf_hi(km.z), bf_lo(km.w), bf_hi(km.w)};
-      const float qf[4] = {q4.x, q4.y, q4.z, q4.w};
-      float z[4], amax = 0.f, dot = 0.f;
-#pragma unroll
-      for (int x = 0; x < 4; ++x) { z[x] = __fmul_rn(qf[x], ks[x]); amax = fmaxf(amax, fabsf(z[x])); dot = fmaf(qf[x], kb[x], dot); }
-      amax = warp_max(amax);
-      const float rr = quotient_127(amax);
-      uint32_t word = 0;
-#pragma unroll
-      for (int x = 0; x < 4; ++x) word |= (__float_as_uint(fmaf(z[x], rr, MAGICF)) & 255u) << (8 * x);
-      __syncwarp();
-      qh[warp][lane] = word;
-      sq = __fmul_rn(amax, __fmul_rn(a.sl, 1.f / 127.f));
-      qb = __fmul_rn(warp_sum(dot), a.sl);
-      __syncwarp();
-    }
-    const float vb[4] = {bf_lo(vm.x), bf_hi(vm.x), bf_lo(vm.y), bf_hi(vm.y)}, vs[4] = {bf_lo(vm.z), bf_hi(vm.z), bf_lo(vm.w), bf_hi(vm.w)};
-    float Ag[4] = {0.f, 0.f, 0.f, 0.f}, Bg = 0.f;  // the group's sum w y (code units) and sum w sum p, relative to mg
-    float mg = -FBLA_INF;
-    for (int j = 0; j < SBG; ++j) {
-      const uint8_t *rc_ = a.c.coarse + (unit * SBG + j) * record_bytes(CB), *rf_ = a.c.fine + (unit * SBG + j) * record_bytes(FB);
-      uint32_t Wc[2 * CB], Wf[2 * FB];
-      load_words<CB>(rc_, 0, lane, Wc);
-      load_words<FB>(rf_, 0, lane, Wf);
-      int acc = 0;
-#pragma unroll
-      for (int s = 0; s < 16; ++s) acc = __dp4a((int)((slot_value<CB>(Wc, s) << FB) | slot_value<FB>(Wf, s)), (int)qh[warp][16 * h + s], acc);
-      float x = (float)acc;
-      x += __shfl_xor_sync(FULL, x, 16);
-      const float s = fmaf(sq, x, qb);
-      float mb = s;
-#pragma unroll
-      for (int o = 8; o; o >>= 1) mb = fmaxf(mb, __shfl_xor_sync(FULL, mb, o));
-      if (lane < 16) pst[warp][lane] = (uint8_t)__float_as_uint(fmaf(ex2(s - mb), 255.f, MAGICF));
-      __syncwarp();
-      const uint4 pw = *reinterpret_cast<const uint4 *>(pst[warp]);
-      const uint32_t P[4] = {pw.x, pw.y, pw.z, pw.w};
-      const float sp = (float)(__dp4a(P[0], 0x01010101u, 0u) + __dp4a(P[1], 0x01010101u, 0u) + __dp4a(P[2], 0x01010101u, 0u) + __dp4a(P[3], 0x01010101u, 0u));
-      load_words<CB>(rc_, 1, lane, Wc);
-      load_words<FB>(rf_, 1, lane, Wf);
-      float y[4];
-#pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
-        uint32_t sum = 0;
-#pragma unroll
-        for (int quad = 0; quad < 4; ++quad)
-          sum = __dp4a((slot_value<CB>(Wc, v_slot_of(CB, cc, quad)) << FB) | slot_value<FB>(Wf, v_slot_of(FB, cc, quad)), P[quad], sum);
-        y[cc] = (float)sum;
-      }
-      const float mn = fmaxf(mg, mb), al = ex2(mg - mn), w = ex2(mb - mn);
-      mg = mn;
-      Bg = fmaf(al, Bg, w * sp);
-#pragma unroll
-      for (int cc = 0; cc < 4; ++cc) Ag[cc] = fmaf(al, Ag[cc], w * y[cc]);
-      __syncwarp();
-    }
-    const float mn = fmaxf(st.m, mg), al = ex2(st.m - mn), be = ex2(mg - mn);
-    st.m = mn;
-    st.l = fmaf(al, st.l, be * Bg);
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc) st.o[cc] = fmaf(al, st.o[cc], be * fmaf(vs[cc], Ag[cc], vb[cc] * Bg));
+  if (tid == 0) sm.failed = 0;
+  for (int e = tid; e < COLS * (D / 8); e += 32 * WARPS) {
+    const int c = e / (D / 8), r = r0 + c, i = r / qg;
+    *reinterpret_cast<uint4 *>(&sm.q[c][8 * (e % (D / 8))]) =
+        r < rows ? __ldg(reinterpret_cast<const uint4 *>(a.q + ((size_t)(b * a.q_heads + kh * qg + (r - i * qg)) * a.count + i) * D) + e % (D / 8)) : make_uint4(0u, 0u, 0u, 0u);
   }
-  const float inv = 1.f / st.l;
-  const uint32_t w0 = f32_to_bf16(st.o[0] * inv) | (uint32_t)f32_to_bf16(st.o[1] * inv) << 16;
-  const uint32_t w1 = f32_to_bf16(st.o[2] * inv) | (uint32_t)f32_to_bf16(st.o[3] * inv) << 16;
-  uint16_t *orow = a.out + (size_t)(b * a.q_heads + hq) * a.out_hs + (size_t)i * a.out_ts;
-  reinterpret_cast<uint2 *>(orow)[lane] = make_uint2(w0, w1);
+  RowWarp<CB, FB> &w = sm.w[warp];
+  if (lane == 0) {
+#pragma unroll
+    for (int s = 0; s < NST; ++s) mbar_init(&w.bar[s], 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  uint32_t uses = 0;
+  bool ok = true;
+  for (int s = cluster == 1 ? 0 : rank; s < shares; s += cluster) {
+    const int p0 = (int)((long long)pairs * s / shares), p1 = (int)((long long)pairs * (s + 1) / shares), per = (p1 - p0 + WARPS - 1) / WARPS;
+    State st;
+    st.m[0] = st.m[1] = -FBLA_INF;
+    st.l = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) st.o[u][cc] = make_float2(0.f, 0.f);
+    const int lo = min(p1, p0 + warp * per), hi = min(p1, lo + per);
+    if (ok && lo < hi) ok = closed_run<CB, FB>(a, w, sm.q, (size_t)bh * a.hs, lo, hi, own, uses, st, lane);
+    float *const set = reinterpret_cast<float *>(w.pair[0]);
+    if (ok) {
+      write_state(set, st, lane);
+      __syncwarp();
+      exact_blocks(a, sm.q, *reinterpret_cast<RowStage *>(w.pair[0] + SET * sizeof(float)), set, s * WARPS + warp, WARPS * shares, exact, sink, own_lo, n1, pos, own, lane, token_row);
+    } else if (lane == 0) {
+      sm.failed = 1;
+    }
+    __syncthreads();
+    if (warp < COLS && !sm.failed) {  // row `warp` over the warps, in their order
+      float M = -FBLA_INF;
+#pragma unroll
+      for (int x = 0; x < WARPS; ++x) M = fmaxf(M, reinterpret_cast<const float *>(sm.w[x].pair[0])[warp * FBLA_K_PSTRIDE + D]);
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+      float l = 0.f;
+#pragma unroll
+      for (int x = 0; x < WARPS; ++x) {
+        const float *row = reinterpret_cast<const float *>(sm.w[x].pair[0]) + warp * FBLA_K_PSTRIDE;
+        const float e = row[D] == -FBLA_INF ? 0.f : ex2(row[D] - M);
+        const float4 y = *reinterpret_cast<const float4 *>(row + 4 * lane);
+        l = fmaf(e, row[D + 1], l);
+        o.x = fmaf(e, y.x, o.x); o.y = fmaf(e, y.y, o.y); o.z = fmaf(e, y.z, o.z); o.w = fmaf(e, y.w, o.w);
+      }
+      float *dst = sm.share[s] + warp * FBLA_K_PSTRIDE;
+      *reinterpret_cast<float4 *>(dst + 4 * lane) = o;
+      if (lane == 0) { dst[D] = M; dst[D + 1] = l; }
+    }
+    __syncthreads();
+  }
+  if (FBLA_STREAM_LAUNCH && cluster > 1) cluster_meet();
+  // row c over the shares, in their order; a cluster's CTAs take rows rank, rank + cluster, ...
+  const int c = rank + warp * cluster;
+  if (warp < COLS && c < COLS && r0 + c < rows) {
+    bool failed = false;
+    float M = -FBLA_INF, l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < shares; ++s) {
+      const float *row = sm.share[s] + c * FBLA_K_PSTRIDE;
+      float4 y;
+      float2 ml;
+      if (FBLA_STREAM_LAUNCH && cluster > 1) {
+        const uint32_t p = remote(row, s);
+        y = ld_remote4(p + 16 * lane);
+        ml = ld_remote2(p + 4 * D);
+        failed |= ld_remote1(remote(&sm.failed, s)) != 0;
+      } else {
+        y = *reinterpret_cast<const float4 *>(row + 4 * lane);
+        ml = *reinterpret_cast<const float2 *>(row + D);
+        failed |= sm.failed != 0;
+      }
+      const float mn = fmaxf(M, ml.x), sa = M == -FBLA_INF ? 0.f : ex2(M - mn), sb = ml.x == -FBLA_INF ? 0.f : ex2(ml.x - mn);
+      M = mn;
+      l = fmaf(sa, l, sb * ml.y);
+      o.x = fmaf(sa, o.x, sb * y.x); o.y = fmaf(sa, o.y, sb * y.y); o.z = fmaf(sa, o.z, sb * y.z); o.w = fmaf(sa, o.w, sb * y.w);
+    }
+    const float inv = failed ? __int_as_float(0x7fc00000) : 1.f / l;
+    const int r = r0 + c, i = r / qg, hq = kh * qg + (r - i * qg);
+    uint16_t *orow = a.out + (size_t)(b * a.q_heads + hq) * a.out_hs + (size_t)i * a.out_ts;
+    const uint32_t w0 = f32_to_bf16(o.x * inv) | (uint32_t)f32_to_bf16(o.y * inv) << 16, w1 = f32_to_bf16(o.z * inv) | (uint32_t)f32_to_bf16(o.w * inv) << 16;
+    reinterpret_cast<uint2 *>(orow)[lane] = make_uint2(w0, w1);
+  }
+  if (FBLA_STREAM_LAUNCH && cluster > 1) cluster_meet();  // (nobody leaves while its shared memory is being read)
+  __syncthreads();
+  if (ok && lane == 0) {
+#pragma unroll
+    for (int s = 0; s < NST; ++s) mbar_inval(&w.bar[s]);
+  }
 }
 
 }  // namespace fbla
-
