@@ -3,8 +3,11 @@
 checks and exceptions -- scratch_bytes, images_bytes, decode, prefill. PyTorch supplies device memory and the current
 stream only; every computation happens inside libmlops_attention.so. There is no CPU fallback: importing this module
 without the built library raises."""
+import collections
 import ctypes
+import functools
 import os
+import threading
 
 import torch
 
@@ -106,6 +109,111 @@ def scratch_bytes(batch, q_heads, kv_heads, tokens, format, capacity):
     if n <= 0:
         raise ValueError(f"invalid FBLA configuration: batch {batch}, heads {q_heads} / {kv_heads}, tokens {tokens}, capacity {capacity}")
     return n
+
+
+# ---- calls on a whole cache object: what does not change from call to call is looked at once ---------------------------------
+class _Bound:
+    """A cache's arrays, checked, and the structure that names them to the library."""
+    __slots__ = ("arrays", "pointers", "struct", "device", "index", "batch", "kv_heads")
+
+    def __init__(self, c):
+        self.arrays = c.coarse, c.fine, c.meta, c.sink_k, c.sink_v, c.open_k, c.open_v
+        self.device = c.coarse.device
+        for x in self.arrays[:2]:
+            _tensor(x, self.device, torch.uint8, "packed cache records")
+        for x in self.arrays[2:]:
+            _tensor(x, self.device, torch.bfloat16, "cache metadata / exact group")
+        self.pointers = tuple(x.data_ptr() for x in self.arrays)
+        self.struct = ctypes.byref(Cache(*self.pointers, c.images.data_ptr() if c.images is not None else None))
+        self.index = self.device.index
+        self.batch, self.kv_heads = c.meta.size(0), c.meta.size(1)
+
+
+def bind(c):
+    """The cache's _Bound, made anew whenever one of its arrays is another tensor or lies elsewhere."""
+    b = c.__dict__.get("_bound")
+    if b is not None:
+        k, f, m, sk, sv, ok, ov = b.arrays
+        if (k is c.coarse and f is c.fine and m is c.meta and sk is c.sink_k and sv is c.sink_v and ok is c.open_k and ov is c.open_v
+                and b.pointers == (k.data_ptr(), f.data_ptr(), m.data_ptr(), sk.data_ptr(), sv.data_ptr(), ok.data_ptr(), ov.data_ptr())):
+            return b
+    b = c._bound = _Bound(c)
+    return b
+
+
+_scratch_bytes = functools.lru_cache(maxsize=256)(lambda device, *shape: scratch_bytes(*shape))
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
+class _ScratchPool:
+    """Decode scratch, one buffer per (device, stream, batch x KV heads), grown on demand and kept for later calls -- at most
+    BUFFERS of them, the least recently used one given back first. Calls of one stream run in order, so they may share one;
+    calls of different streams never do."""
+    BUFFERS = 16
+
+    def __init__(self):
+        self._buffers, self._lock = collections.OrderedDict(), threading.Lock()
+
+    def get(self, device, stream, heads, nbytes):
+        key = device.index, stream, heads
+        with self._lock:
+            held = self._buffers.get(key)
+            if held is not None and held[0] >= nbytes:
+                self._buffers.move_to_end(key)
+                return held
+        fresh = torch.empty((nbytes,), dtype=torch.uint8, device=device)  # the library needs no initial contents
+        held = nbytes, fresh.data_ptr(), fresh
+        with self._lock:
+            self._buffers[key] = held
+            self._buffers.move_to_end(key)
+            while len(self._buffers) > self.BUFFERS:
+                self._buffers.popitem(last=False)
+        return held
+
+
+_pool = _ScratchPool()
+
+
+def decode_cache(q, c, scale, tau):
+    """decode of a whole cache object with the pool's scratch"""
+    b = bind(c)
+    if q.dim() != 3 or q.size(2) != 128:
+        raise ValueError(f"q must be [batch, q_heads, 128], got {tuple(q.shape)}")
+    if not q.is_contiguous():
+        q = q.contiguous()
+    if q.device != b.device:
+        raise ValueError(f"q: expected a CUDA tensor on {b.device}")
+    if torch._C._cuda_getDevice() != b.index:
+        with torch.cuda.device(b.index):
+            return decode_cache(q, c, scale, tau)
+    batch, q_heads = q.size(0), q.size(1)
+    need = _scratch_bytes(b.index, batch, q_heads, b.kv_heads, c.capacity, c.format, c.capacity)
+    stream = _raw_stream(b.index)
+    size, scratch, keep = _pool.get(b.device, stream, batch * b.kv_heads, need)
+    out = torch.empty_like(q)
+    cfg = Config(batch, q_heads, b.kv_heads, int(c.tokens), float(scale), float(tau), int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
+    _raise(_lib.mlops_fbla_decode(ctypes.byref(cfg), q.data_ptr(), b.struct, out.data_ptr(), scratch, size, stream), "mlops_fbla_decode")
+    return out
+
+
+def prefill_cache(q, k, v, c, scale):
+    """prefill (append for q None) on a whole cache object; k and v contiguous BF16 of the cache's batch and KV heads"""
+    b = bind(c)
+    _tensor(k, b.device, torch.bfloat16, "k")
+    _tensor(v, b.device, torch.bfloat16, "v")
+    if torch._C._cuda_getDevice() != b.index:
+        with torch.cuda.device(b.index):
+            return prefill_cache(q, k, v, c, scale)
+    n, q_heads, out = k.size(2), b.kv_heads, None
+    if q is not None:
+        if q.dim() != 4 or q.size(0) != b.batch or q.size(2) != n or q.size(3) != 128:
+            raise ValueError(f"q must be [batch, q_heads, n, 128] matching k, got {tuple(q.shape)}")
+        _tensor(q, b.device, torch.bfloat16, "q")
+        q_heads, out = q.size(1), torch.empty_like(q)
+    cfg = Config(b.batch, q_heads, b.kv_heads, int(c.tokens), float(scale), 0.0, int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
+    _raise(_lib.mlops_fbla_prefill(ctypes.byref(cfg), n, q.data_ptr() if q is not None else None, k.data_ptr(), v.data_ptr(), b.struct,
+                                   out.data_ptr() if out is not None else None, _raw_stream(b.index)), "mlops_fbla_prefill")
+    return out
 
 
 def images_bytes(batch, kv_heads, capacity):

@@ -77,10 +77,7 @@ def _extend(cache, k, v, q=None, scale=0.0):
     added = int(k.shape[2])
     if cache.tokens + added > cache.capacity:
         raise ValueError(f"{added} more tokens do not fit: the cache holds {cache.tokens} of {cache.capacity}")
-    q_heads = int(q.shape[1]) if q is not None else int(k.shape[1])
-    result = _C.prefill(q, k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous(),
-                        cache.coarse, cache.fine, cache.meta, cache.sink_k, cache.sink_v, cache.open_k, cache.open_v,
-                        cache.tokens, cache.capacity, q_heads, cache.format, scale, cache.images)
+    result = _C.prefill_cache(q, k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous(), cache, scale)
     cache.tokens += added
     return result
 
@@ -125,33 +122,9 @@ def prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: FBLACache,
     return _extend(cache, k, v, q.contiguous(), scale)
 
 
-class _ScratchPool:
-    """Decode scratch, one buffer per (device, batch x KV heads), grown on demand and kept for later calls."""
-
-    def __init__(self):
-        self._buffers = {}
-
-    def get(self, device, heads, nbytes):
-        held = self._buffers.get((device, heads))
-        if held is not None and held.numel() >= nbytes:
-            return held
-        fresh = torch.empty((nbytes,), dtype=torch.uint8, device=device)  # the library needs no initial contents
-        self._buffers[(device, heads)] = fresh
-        return fresh
-
-
-_pool = _ScratchPool()
-
-
 def decode(q: torch.Tensor, cache: FBLACache, *, scale: float = 0.0, tau: float = 0.0) -> torch.Tensor:
     """Attention of one new query per head, ``q [B, Hq, 128]`` BF16, over everything in ``cache``.
     ``scale`` 0 selects 1/sqrt(128); ``tau`` 0 selects the format's refinement threshold."""
     if q.dtype != torch.bfloat16:
         raise TypeError(f"decode takes bfloat16 queries, not {q.dtype}")
-    batch, q_heads = int(q.shape[0]), int(q.shape[1])
-    kv_heads = int(cache.meta.shape[1])
-    with torch.cuda.device(q.device):
-        need = _C.scratch_bytes(batch, q_heads, kv_heads, cache.tokens, cache.format, cache.capacity)
-    scratch = _pool.get(q.device, batch * kv_heads, need)
-    return _C.decode(q.contiguous(), cache.coarse, cache.fine, cache.meta, cache.sink_k, cache.sink_v, cache.open_k,
-                     cache.open_v, scratch, cache.tokens, cache.capacity, kv_heads, cache.format, scale, tau)
+    return _C.decode_cache(q, cache, scale, tau)

@@ -455,8 +455,7 @@ mlops_fbla_status mlops_fbla_qkv_at(const mlops_fbla_config *c, const int *lengt
   fbla_k_token a;
   const mlops_fbla_status st = make_token_step(c, length, t, cache, closing, a);
   if (st != MLOPS_FBLA_OK) return st;
-  cudaError_t e = fbla_k_close_launch(&closing, 1, stream);
-  if (e == cudaSuccess) e = fbla_k_qkv_token_launch(&a, stream);
+  const cudaError_t e = fbla_k_qkv_step_launch(&closing, &a, stream);
   return e == cudaSuccess ? accepted() : device_failure("mlops_fbla_qkv_at", e);
 }
 

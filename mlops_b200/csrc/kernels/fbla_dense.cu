@@ -62,9 +62,10 @@ template <int CB, int FB, int QG> struct Kernels {
   }
   static cudaError_t all(const fbla_k_decode &a, cudaStream_t stream) {
     cudaError_t e = configure();
-    if (a.phase != 2 && e == cudaSuccess) e = pass(a, 0, false, stream);
-    if (a.phase == 1) return e == cudaSuccess ? pass(a, 1, true, stream) : e;
-    if (e == cudaSuccess) e = pass(a, 2, a.phase != 2, stream);
+    if (a.phase != 2 && e == cudaSuccess) e = pass(a, 0, true, stream);
+    if (e != cudaSuccess) return e;
+    if (a.phase == 1) return pass(a, 1, true, stream);
+    e = pass(a, 2, true, stream);
     return e == cudaSuccess ? pass(a, 3, true, stream) : e;
   }
   template <class K> static cudaError_t describe(K kernel, int items, int threads, size_t smem, fbla_k_pass *p) {

@@ -219,8 +219,9 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
   ScoreSmem &sm = *reinterpret_cast<ScoreSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
   const int hpr = a.kv_heads * a.vg;
-  allow_next_pass();
-  if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status && a.phase != 2) { a.status[0] = 0; a.status[1] = 0; }
+  wait_previous_pass();  // (lengths, queries and the cache may come from the kernel before)
+  allow_next_pass();     // (behind the wait: the value pass then finds everything before this call complete)
+  if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status) { a.status[0] = 0; a.status[1] = 0; }
   build_table(a, sm.table, 32 * SCORE_WARPS);
   if (FBLA_POS::x() == 0 && a.lstride)
     for (int i = FBLA_POS::tid(); i <= a.batch; i += 32 * SCORE_WARPS) { table_of(a)[i] = sm.table.closed[i]; table_of(a)[a.batch + 1 + i] = sm.table.exact[i]; }
@@ -561,7 +562,9 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     float R = 0.f;  // lane l: of query l % QG of the head the issuing side stands on
     auto mass_of = [&](int vh) {
       if (a.mass_given) return __ldcg(a.row_r + vh * QG + lane % QG);
-      return row_mass<QG>(a, rows_of<QG>(a, sm.table.closed, sm.table.exact, hpr, vh), vh, lane);
+      const float r = row_mass<QG>(a, rows_of<QG>(a, sm.table.closed, sm.table.exact, hpr, vh), vh, lane);
+      if (lane < QG) a.row_r[vh * QG + lane] = r;  // for the merge (every warp of the head writes the same)
+      return r;
     };
     auto lse_of = [&](const Cursor &x) {  // lane l: (sub-block l / QG, query l % QG) of the group
       return lane < SBG * QG ? __ldcg(a.lse + ((size_t)(x.b * hpr + x.hir) * a.nblocks + (size_t)group_of(a, x) * SBG) * QG + lane) : -FBLA_INF;
@@ -801,7 +804,8 @@ __device__ __forceinline__ void gather_item(const fbla_k_decode &a, uint8_t *sme
   wait_previous_pass();
   const int *t = table_of(a);
   const Rows r = rows_of<QG>(a, t, t + a.batch + 1, hpr, vh);
-  const float R = a.mass_given ? __ldcg(a.row_r + vh * QG + qi) : __shfl_sync(FULL, row_mass<QG>(a, r, vh, lane), qi);
+  // (a head without closed groups was nobody's in the value pass)
+  const float R = a.mass_given || r.v1 >= r.v0 ? __ldcg(a.row_r + vh * QG + qi) : __shfl_sync(FULL, row_mass<QG>(a, r, vh, lane), qi);
   const int status = a.status ? __ldcg(a.status) : 0;
   const int nx = r.x1 - r.x0 + 1, n = nx + r.v1 - r.v0 + 1;
   float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -835,7 +839,6 @@ __device__ __forceinline__ void gather_item(const fbla_k_decode &a, uint8_t *sme
   const size_t row = (size_t)q_row(a, b, hir, qi);
   const bool failed = status != 0;  // (a wait gave up somewhere: not a plausible number)
   const float nan = __int_as_float(0x7fc00000);
-  if (!a.mass_given && ch == 0) a.row_r[vh * QG + qi] = R;  // (for measurements: which sub-blocks were selected)
   if (a.out_partial) {
     a.out_partial[row * PSTRIDE + ch] = failed ? nan : Os;
     if (ch == 0) a.out_partial[row * PSTRIDE + D] = failed ? nan : Ls;

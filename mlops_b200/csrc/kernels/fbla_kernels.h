@@ -53,7 +53,7 @@ typedef struct {
   // the given (global) row_r, refine, and the rows' unnormalised sums (o[128], l, relative to row_r) into out_partial.
   int sh_first, sh_count;
   short shard_on, sh_windows, phase;
-  short mass_given;    // dense: the rows' masses are in row_r (a pass before, or a shard's caller) instead of formed by the passes that need them
+  short mass_given;    // dense: the rows' masses are in row_r (a pass before, or a shard's caller) instead of formed by the value pass
   float *out_partial;  // [rows][FBLA_K_PSTRIDE] floats (phase 2)
   short status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
   short fold;          // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
@@ -182,7 +182,8 @@ typedef struct {
   int batch, q_heads, kv_heads;
   uint16_t *q_out, *k_out, *v_out;
 } fbla_k_token;
-FBLA_HOST_API(cudaError_t fbla_k_qkv_token_launch(const fbla_k_token *a, cudaStream_t stream);)
+// the one-token step: the group the position closes, then the token, in one launch
+FBLA_HOST_API(cudaError_t fbla_k_qkv_step_launch(const fbla_k_prefill *closing, const fbla_k_token *a, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_qkv_chunk_launch(const fbla_k_token *a, cudaStream_t stream);)
 
 // ---- what an executor needs to run a pass from kernels of its own (include/mlops_fbla_items.h) ---------------------------

@@ -1,5 +1,7 @@
 // Launchers of the fused QKV step (bodies: fbla_qkv.cuh).
 #include "fbla_qkv.cuh"
+#include "fbla_close.cuh"
+#include "fbla_decode.cuh"
 #include <stdio.h>
 
 namespace {
@@ -19,17 +21,46 @@ __global__ void __launch_bounds__(256) qkv_token_kernel(const fbla_k_token a) {
   qkv_token_item<NORM>(a, nullptr);
 }
 
+// The whole one-token step of a (batch row, KV head): the group that the position closes is quantised from the open window,
+// then the token takes its place. One launch: the close pass alone is a launch that finds nothing to do 127 times of 128.
+template <int CB, int FB, bool NORM>
+__global__ void __launch_bounds__(CLOSE_THREADS) qkv_step_kernel(const fbla_k_prefill closing, const fbla_k_token a) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  wait_previous_pass();
+  allow_next_pass();
+  const int bh = blockIdx.x;
+  const Chunk ch = chunk_of(closing, bh / closing.kv_heads);
+  const int g = closing_group(ch, 0);
+  if (g >= 0) close_group<CB, FB>(closing, *reinterpret_cast<CloseSmem *>(smem_raw), bh, g, ch.n0);
+  qkv_token_item<NORM>(a, nullptr);
+}
+
 template <bool NORM>
 __global__ void __launch_bounds__(256) qkv_chunk_kernel(const fbla_k_token a) {
   qkv_chunk_item<NORM>(a, nullptr);
 }
 }  // namespace fbla
 
-extern "C" cudaError_t fbla_k_qkv_token_launch(const fbla_k_token *a, cudaStream_t stream) {
-  const int heads = a->batch * a->kv_heads;
-  if (a->q_norm) fbla::qkv_token_kernel<true><<<heads, 256, 0, stream>>>(*a);
-  else fbla::qkv_token_kernel<false><<<heads, 256, 0, stream>>>(*a);
-  return cudaGetLastError();
+template <int CB, int FB, bool NORM> static cudaError_t launch_step(const fbla_k_prefill &closing, const fbla_k_token &a, cudaStream_t stream) {
+  static thread_local int configured[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(fbla::qkv_step_kernel<CB, FB, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(fbla::CloseSmem));
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.batch * a.kv_heads); cfg.blockDim = dim3(fbla::CLOSE_THREADS); cfg.dynamicSmemBytes = sizeof(fbla::CloseSmem); cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fbla::qkv_step_kernel<CB, FB, NORM>, closing, a);
+}
+extern "C" cudaError_t fbla_k_qkv_step_launch(const fbla_k_prefill *closing, const fbla_k_token *a, cudaStream_t stream) {
+  if (closing->cb == 3) return a->q_norm ? launch_step<3, 3, true>(*closing, *a, stream) : launch_step<3, 3, false>(*closing, *a, stream);
+  return a->q_norm ? launch_step<4, 2, true>(*closing, *a, stream) : launch_step<4, 2, false>(*closing, *a, stream);
 }
 
 extern "C" cudaError_t fbla_k_qkv_chunk_launch(const fbla_k_token *a, cudaStream_t stream) {

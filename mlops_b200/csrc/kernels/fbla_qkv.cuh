@@ -61,8 +61,8 @@ __device__ __forceinline__ uint2 norm_rotate(const uint16_t *x, const uint16_t *
   return make_uint2(ra0 | ra1 << 16, rb0 | rb1 << 16);
 }
 
-// ---- one token per sequence: q to q_out, k and v into the windows (the group the position closes has been quantized by
-// the close pass launched before this kernel) -----------------------------------------------------------------------------
+// ---- one token per sequence: q to q_out, k and v into the windows (the group the position closes has been quantized before;
+// threads beyond the 256 that this needs repeat some of their work) -----------------------------------------------------------------------------
 template <bool NORM>
 __device__ __forceinline__ void qkv_token_item(const fbla_k_token &a, uint8_t *smem_raw) {
   __shared__ float2 cs[64];
