@@ -260,6 +260,9 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void *
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(row)) : "memory");
 }
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void *row) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(row)) : "memory");
+}
 // one window sub-block's rows in registers: 16 bytes of the K rows of tokens gid and gid + 8 per 32-channel round, and the
 // lane's share of the 16 V rows (256 x 16 bytes over the warp)
 struct WindowTile {

@@ -16,17 +16,25 @@
 // once, at the end. The two FP16 roundings (relative 2^-11, zero mean) are the only deviations from the reference's
 // arithmetic; they stay far inside the 2e-3 output tolerance.
 //
-// Warps 0-15: the rows. Softmax: two threads per row (warps w and w + 8 share a tensor-memory lane quadrant; warps 0-3,
-// 8-11: tile 0); qhat: lane-per-channel-chunk over the tile's rows. Warps 16-19: operands, shared by both tiles: unpack the
-// group's records (bulk-copied raw into shared memory) into the Kop / V' tiles. Warp 20: allocates tensor memory; its
-// lane 0 issues the bulk copies and the products, which complete on mbarriers. P' is written over qhat (dead once S is complete). Operand tiles are K-major with the 128-byte swizzle
-// (8-row x 128-byte atoms, 16-byte chunk c of row r at c ^ (r % 8)).
-// What bounds it: per (row, group) the reference's semantics need ~130 exp2 and the requantisation of the row's 128
-// query channels on the CUDA cores; the tensor-core share of a pass is about as long as its exp2 share alone.
+// Warps 0-15 (softmax), 16-23 (quantiser), 24-27 (operands), 28 (issuer). Softmax: two threads per row (warps w and w + 8
+// share a tensor-memory lane quadrant; warps 0-3, 8-11: tile 0). Quantiser: qhat of the next pass as soon as a tile's S
+// product has read the current one, while that tile's rows are in their softmax: lane-per-channel-chunk over the tile's
+// rows; the score biases of eight groups at a time are BF16 products on the side. Operand warps, shared by both tiles: they
+// take the group's records from global memory straight into registers, one operand ahead, and unpack them into the Kop /
+// V' tiles. Warp 28 allocates tensor memory; its lane 0 issues the products, which complete on mbarriers. Operand tiles are
+// K-major with the 128-byte swizzle (8-row x 128-byte atoms, 16-byte chunk c of row r at c ^ (r % 8)).
+// What bounds it: instruction issue of the CUDA cores -- per (row, group) the reference's semantics need 128 exp2 with
+// integer rounding and the requantisation of the row's 128 query channels (about 17 000 warp instructions per pass at 0.6
+// per cycle and scheduler); the tensor-core share of a pass is about as long as its exp2 share alone. Measured at batch 4 x
+// 8192 (32 / 8 heads, 4+2): sixteen warps doing softmax and requantisation in turn 5.66 ms = 388 TFLOP/s; roles of their
+// own 5.35; BF16 operands with all loads in flight 5.21; biases on tensor cores 4.75; two sweeps over eight rows of a lane
+// with one reduction 4.59 = 479 TFLOP/s. (64 registers per thread: 29 warps. Halving the softmax warps so that the tiles
+// alternate, or one copy of the unpacking code for both records of an operand warp, measured slower.)
 // Every wait is bounded: on a timeout the thread raises a flag, everybody drains, tensor memory is freed, the kernel
 // returns and the host sees fbla_k_attend_tc_status() != 0.
 #pragma once
 #include "fbla_tc.cuh"
+#include "fbla_decode.cuh"
 #include "fbla_kernels.h"
 #include <cuda_fp16.h>
 
@@ -39,11 +47,10 @@ constexpr int CTA_ROWS = 2 * ROWS;
 #define FBLA_PF_PRODUCERS 4  /* operand warps. Measured: 4 (21 warps, 80 registers, 28 bytes of spills) 336.5 TFLOP/s; 3 (96 registers, none) 324.8 */
 #endif
 constexpr int PRODUCERS = FBLA_PF_PRODUCERS, PT = 32 * PRODUCERS;  // operand warps and threads
-constexpr int PRODUCER_WARP0 = 16, ISSUER_WARP = 16 + PRODUCERS;  // warps 0-15: rows
-constexpr int THREADS = (17 + PRODUCERS) * 32;
+constexpr int QUANT_WARP0 = 16, PRODUCER_WARP0 = 24, ISSUER_WARP = 24 + PRODUCERS;
+constexpr int THREADS = (25 + PRODUCERS) * 32;
 constexpr int SLAB = ROWS * 128;          // bytes of one K slab (128 rows x 128 bytes): 64 FP16 / BF16 of the K extent
 constexpr int TILE = 2 * SLAB;            // a [128 x 128] 16-bit operand tile: 32 KiB
-constexpr int RAW = 8 * 3072;              // a raw group: 8 coarse + 8 fine records, 3072 bytes per pair in both formats
 constexpr uint32_t WAIT_LIMIT = 1u << 18;
 
 __device__ int g_status = 0;  // nonzero: a bounded wait gave up in some launch since the last read
@@ -53,11 +60,10 @@ struct __align__(1024) Smem {
   uint8_t qp[2][TILE];  // Qop of closed passes: qhat as FP16 (at the very end: staging of the output rows)
   uint8_t k[TILE];      // Kop
   uint8_t v[TILE];      // V'
-  uint8_t raw[RAW];     // the group's coarse records, then its fine records
-  uint8_t meta[2][1024];  // the metadata of closed pass c in buffer c % 2, fetched two passes ahead
-  float qscale[2][2][128], qbias[2][2][128];  // [pass parity][tile][row]: the pass's score scale and bias (from the quantising lanes to the row's threads)
+  float qscale[2][2][128];   // [pass parity][tile][row]: the pass's score scale (from the quantiser to the row's threads)
+  float qbias[2][8][2][128];  // [eight passes, alternating][pass][tile][row]: the score bias sl q . base, formed for eight groups at once
   float ex2[2][128][2];  // exchange between the two threads of a row: pass maximum, final sum
-  uint64_t bar_raw, bar_meta[2], bar_k, bar_v, bar_q[2], bar_s[2], bar_p[2], bar_o[2];
+  uint64_t bar_k, bar_v, bar_q[2], bar_s[2], bar_p[2], bar_o[2];
   uint32_t tmem_base;
   int abort;
 };
@@ -87,10 +93,27 @@ __device__ __forceinline__ uint8_t *chunk_at(uint8_t *tile, int r, int k0) {
 }
 
 // ---- record unpacking (the slot maps of include/mlops_fbla.h) --------------------------------------------------------------
-template <int BITS> __device__ __forceinline__ void lane_words(const uint8_t *rec, int tensor, int lane, uint32_t *W) {
-#pragma unroll
-  for (int w = 0; w < 2 * BITS; ++w) W[w] = lds32(rec + word_offset(BITS, tensor, lane, w));
+// one record lane's words of a tensor in a BITS plane, from global memory
+template <int BITS> __device__ __forceinline__ void load_lane(const uint8_t *rec, int tensor, int lane, uint32_t (&W)[2 * BITS]) {
+  const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(rec + word_offset(BITS, tensor, lane, 0)));
+  W[0] = x.x; W[1] = x.y; W[2] = x.z; W[3] = x.w;
+  if constexpr (BITS == 4) {
+    const uint4 y = __ldcg(reinterpret_cast<const uint4 *>(rec + word_offset(BITS, tensor, lane, 4)));
+    W[4] = y.x; W[5] = y.y; W[6] = y.z; W[7] = y.w;
+  }
+  if constexpr (BITS == 3) {
+    const uint2 y = __ldcg(reinterpret_cast<const uint2 *>(rec + word_offset(BITS, tensor, lane, 4)));
+    W[4] = y.x; W[5] = y.y;
+  }
 }
+// maxima of three (one instruction where the compiler's PTX has it: CUDA 12.9 on)
+#if __CUDACC_VER_MAJOR__ * 100 + __CUDACC_VER_MINOR__ >= 1209
+__device__ __forceinline__ float max3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+__device__ __forceinline__ float max3_abs(float a, float b, float c) { float d; asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+#else
+__device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+__device__ __forceinline__ float max3_abs(float a, float b, float c) { return fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c)); }
+#endif
 // four small unsigned integers (bytes of x, each < 1024) as two packed FP16 pairs: 0x6400 | b is 1024 + b
 __device__ __forceinline__ uint2 bytes_to_half4(uint32_t x) {
   const uint32_t lo = __byte_perm(x, 0x64646464u, 0x7170), hi = __byte_perm(x, 0x64646464u, 0x7372);  // (b1 | 0x64 << 8) << 16 | b0 | 0x64 << 8
@@ -114,6 +137,47 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// ---- operands of the BF16 groups -------------------------------------------------------------------------------------------------
+struct TokenRows {
+  const uint16_t *chunk, *sink, *open;
+  int n0;
+  __device__ __forceinline__ const uint16_t *at(int tp) const {
+    return tp >= n0 ? chunk + (size_t)(tp - n0) * D : tp < G ? sink + (size_t)tp * D : open + (size_t)(tp - (n0 - 1) / G * G) * D;
+  }
+};
+// K rows of tokens t0 .. t0 + 127 as they are (zeros from n1 on), eight 16-byte pieces of the thread in flight
+__device__ __forceinline__ void exact_k(uint8_t *tile, const TokenRows rows, int t0, int n1, int pt) {
+#pragma unroll 1
+  for (int e0 = pt; e0 < G * 16; e0 += 8 * PT) {
+    uint4 w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = e0 + PT * i, tp = t0 + (e >> 4);
+      w[i] = tp < n1 ? __ldcg(reinterpret_cast<const uint4 *>(rows.at(tp)) + (e & 15)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4 *>(chunk_at(tile, (e0 + PT * i) >> 4, 8 * (e0 & 15))) = w[i];
+  }
+}
+// V rows converted to FP16 and transposed (tokens along the K extent): a thread takes 8 channels of 8 tokens
+__device__ __forceinline__ void exact_v(uint8_t *tile, const TokenRows rows, int t0, int n1, int pt) {
+#pragma unroll 1
+  for (int e = pt; e < G * 2; e += PT) {
+    const int c = e & 15, t8 = 8 * (e >> 4);
+    uint4 w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = t0 + t8 + i < n1 ? __ldcg(reinterpret_cast<const uint4 *>(rows.at(t0 + t8 + i)) + c) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      auto at = [&](int i) {
+        const uint32_t v = x < 2 ? w[i].x : x < 4 ? w[i].y : x < 6 ? w[i].z : w[i].w;
+        return (x & 1) ? bf_hi(v) : bf_lo(v);
+      };
+      *reinterpret_cast<uint4 *>(chunk_at(tile, vrow(8 * c + x), t8)) = make_uint4(pack_half2(at(0), at(1)), pack_half2(at(2), at(3)), pack_half2(at(4), at(5)), pack_half2(at(6), at(7)));
+    }
+  }
+}
+
 template <int CB, int FB>
 __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
   smem_raw += (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // (an offset, not a rebuilt pointer: the address space stays known)
@@ -125,7 +189,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
   const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, n1 = n0 + count;
   // the last tiles attend to the most groups: they are taken first, so that the grid's tail is made of short CTAs
   const int rows = count * qg, r0 = (FBLA_POS::nx() - 1 - FBLA_POS::x()) * CTA_ROWS;
-  if (r0 >= rows || rows < a.tc_min_rows) return;  // (CTA-uniform; a short device count is the warp-per-row pass's work)
+  if (r0 >= rows || rows < a.tc_min_rows) return;  // (CTA-uniform; a short device count is the few-row pass's work)
   const int last_row = min(r0 + CTA_ROWS, rows) - 1;
   const int own_min = (n0 + r0 / qg) / G, own_max = (n0 + last_row / qg) / G;
   // passes: closed groups 1 .. own_max - 1, then the BF16 groups: 0 and the rows' own groups
@@ -137,7 +201,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
   };
 
   if (tid == 0) {
-    mbar_init(&sm.bar_raw, 1); mbar_init(&sm.bar_meta[0], 1); mbar_init(&sm.bar_meta[1], 1); mbar_init(&sm.bar_k, PT); mbar_init(&sm.bar_v, PT);
+    mbar_init(&sm.bar_k, PT); mbar_init(&sm.bar_v, PT);
     for (int x = 0; x < 2; ++x) { mbar_init(&sm.bar_q[x], 256); mbar_init(&sm.bar_s[x], 1); mbar_init(&sm.bar_p[x], 256); mbar_init(&sm.bar_o[x], 1); }
     sm.abort = 0;
     mbar_init_fence();
@@ -152,313 +216,329 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   const size_t head = (size_t)bh * a.hs, eh = (size_t)bh * G * D, ih = (size_t)bh * a.count * D;
-  // the BF16 row of position tp: the chunk, the sink window, or the window of the group that was open before the chunk
-  auto token_row = [&](int tp, const uint16_t *in, const uint16_t *sink, const uint16_t *open) -> const uint16_t * {
-    return tp >= n0 ? in + ih + (size_t)(tp - n0) * D : tp < G ? sink + eh + (size_t)tp * D : open + eh + (size_t)(tp - (n0 - 1) / G * G) * D;
-  };
+  // the BF16 rows of K and of V: the chunk, the sink window, the window of the group that was open before the chunk
+  const TokenRows rows_k{a.k + ih, a.c.sink_k + eh, a.c.open_k + eh, n0}, rows_v{a.v + ih, a.c.sink_v + eh, a.c.open_v + eh, n0};
 
   if (warp == ISSUER_WARP) {
-    // ================= issuer: bulk copies of the raw groups, the products =================
+    // ================= issuer: the products =================
+    // Per pass S(n, 0), O(n - 1, 1), S(n, 1), O(n, 0): the order in which the half passes make their operands ready. Products
+    // execute in the order they are issued, so S(n + 1, x) overwrites P'(n, x) only after O(n, x) has read it.
     if (lane == 0) {
-      auto fetch = [&](int g) {
-        const size_t unit = head + (size_t)g * a.gs;
-        mbar_expect_tx(&sm.bar_raw, SBG * (RC + RF));
-        bulk_g2s(sm.raw, a.c.coarse + unit * SBG * RC, SBG * RC, &sm.bar_raw);
-        bulk_g2s(sm.raw + SBG * RC, a.c.fine + unit * SBG * RF, SBG * RF, &sm.bar_raw);
-      };
-      auto fetch_meta = [&](int c) {  // closed pass c = group 1 + c: 1 KiB, two passes ahead of its use
-        mbar_expect_tx(&sm.bar_meta[c & 1], 1024);
-        bulk_g2s(sm.meta[c & 1], reinterpret_cast<const uint8_t *>(a.c.meta) + (head + (size_t)(1 + c) * a.gs) * 1024, 1024, &sm.bar_meta[c & 1]);
-      };
-      if (n_closed > 0) { fetch(1); fetch_meta(0); }
-      if (n_closed > 1) fetch_meta(1);
-      for (int n = 0; n < n_pass; ++n) {
-        bool closed;
-        pass_group(n, closed);
-        const uint32_t ph = n & 1, idesc = closed ? IDESC_F16 : IDESC_BF16;
-        // Both tiles' S first, then both tiles' O: the tiles run in step (holding tile 1 back by half a pass, so that one
-        // tile quantises while the other exponentiates, measured slower: each tile then waits for the other's operands)
-        bool ok = wait(sm, &sm.bar_k, ph);
-        for (int x = 0; x < 2 && ok; ++x) {
-          if (!(ok = wait(sm, &sm.bar_q[x], ph))) break;
-          tc_fence_after();
-          const uint8_t *qop = closed ? sm.qp[x] : sm.q[x];
+      auto scores = [&](int n, int x) -> bool {
+        if (!wait(sm, &sm.bar_q[x], n & 1)) return false;
+        tc_fence_after();
+        const bool closed = n < n_closed;
+        const uint8_t *qop = closed ? sm.qp[x] : sm.q[x];
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) mma_f16(tmem + 128 * x, smem_desc(qop, kk >> 2, kk & 3), smem_desc(sm.k, kk >> 2, kk & 3), idesc, kk > 0);
-          mma_commit(&sm.bar_s[x]);
-        }
-        if (!ok || !wait(sm, &sm.bar_v, ph)) break;
-        if (n + 1 < n_closed) fetch(2 + n);  // the raw buffer has been consumed: the next closed group's records
-        if (n + 2 < n_closed) fetch_meta(n + 2);  // (this pass's metadata has been consumed too)
-        for (int x = 0; x < 2 && ok; ++x) {
-          if (!(ok = wait(sm, &sm.bar_p[x], ph))) break;
-          tc_fence_after();
+        for (int kk = 0; kk < 8; ++kk)
+          mma_f16(tmem + 128 * x, smem_desc(qop, kk >> 2, kk & 3), smem_desc(sm.k, kk >> 2, kk & 3), closed ? IDESC_F16 : IDESC_BF16, kk > 0);
+        mma_commit(&sm.bar_s[x]);
+        return true;
+      };
+      auto values = [&](int n, int x) -> bool {
+        if (!wait(sm, &sm.bar_p[x], n & 1)) return false;
+        tc_fence_after();
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)  // P' of token block kk: eight columns inside the tile's S columns (see the row threads)
-            mma_f16_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (kk >> 2) + 8 * (kk & 3), smem_desc(sm.v, kk >> 2, kk & 3), IDESC_F16, n > 0 || kk > 0);
-          mma_commit(&sm.bar_o[x]);
-        }
-        if (!ok) break;
-      }
+        for (int kk = 0; kk < 8; ++kk)  // P' of token block kk: eight columns inside the tile's S columns (see the softmax threads)
+          mma_f16_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (kk >> 2) + 8 * (kk & 3), smem_desc(sm.v, kk >> 2, kk & 3), IDESC_F16, n > 0 || kk > 0);
+        mma_commit(&sm.bar_o[x]);
+        return true;
+      };
+      bool ok = true;
+      for (int n = 0; n < n_pass && ok; ++n)
+        ok = wait(sm, &sm.bar_k, n & 1) && scores(n, 0) && (n == 0 || values(n - 1, 1)) && scores(n, 1) && wait(sm, &sm.bar_v, n & 1) && values(n, 0);
+      if (ok) values(n_pass - 1, 1);
     }
   } else if (warp >= PRODUCER_WARP0) {
     // ================= operand producers =================
     const int pt = tid - 32 * PRODUCER_WARP0;  // 0 .. PT - 1
-    const int l = pt & 31;
-    int raw_uses = 0;
-    for (int n = 0; n < n_pass; ++n) {
+    const int l = pt & 31, j0 = pt >> 5;
+    constexpr int NJ = SBG / PRODUCERS;        // records per warp
+    uint32_t Wc[NJ][2 * CB], Wf[NJ][2 * FB];   // K's words of the next closed group, then V's of the current one
+    auto load = [&](int g, int tensor) {
+      const size_t unit = head + (size_t)g * a.gs;
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) {
+        load_lane<CB>(a.c.coarse + (unit * SBG + j0 + PRODUCERS * i) * RC, tensor, l, Wc[i]);
+        load_lane<FB>(a.c.fine + (unit * SBG + j0 + PRODUCERS * i) * RF, tensor, l, Wf[i]);
+      }
+    };
+    if (n_closed > 0) load(1, 0);
+    bool ok = true;
+    // Kop is free once both tiles' S of the previous pass are complete, V' once both tiles' O products are
+    auto free_k = [&](int n) { return n == 0 || (wait(sm, &sm.bar_s[0], (n - 1) & 1) && wait(sm, &sm.bar_s[1], (n - 1) & 1)); };
+    auto free_v = [&](int n) { return n == 0 || (wait(sm, &sm.bar_o[0], (n - 1) & 1) && wait(sm, &sm.bar_o[1], (n - 1) & 1)); };
+    auto done = [&](uint64_t *bar) { fence_async_smem(); mbar_arrive(bar); };
+#pragma unroll 1
+    for (int n = 0; n < n_closed; ++n) {
+      const int g = 1 + n;
+      if (!(ok = free_k(n))) break;
+      const uint4 vm = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(a.c.meta) + (head + (size_t)g * a.gs) * 1024 + 512) + l);
+      // (record j, lane l): token 16 j + l % 16, channels 64 (l / 16) + 4 s + byte: one 128-byte row of slab l / 16
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) {
+        const int tok = 16 * (j0 + PRODUCERS * i) + (l & 15);
+#pragma unroll
+        for (int s2 = 0; s2 < 8; ++s2) {
+          const uint2 x = bytes_to_half4((slot_value<CB>(Wc[i], 2 * s2) << FB) | slot_value<FB>(Wf[i], 2 * s2));
+          const uint2 y = bytes_to_half4((slot_value<CB>(Wc[i], 2 * s2 + 1) << FB) | slot_value<FB>(Wf[i], 2 * s2 + 1));
+          *reinterpret_cast<uint4 *>(chunk_at(sm.k, tok, 64 * (l >> 4) + 8 * s2)) = make_uint4(x.x, x.y, y.x, y.y);
+        }
+      }
+      load(g, 1);
+      done(&sm.bar_k);
+      if (!(ok = free_v(n))) break;
+      // (record j, lane l): channels 4 l + cc, tokens 16 j + 4 quad + byte, value base + step * code in FP16 arithmetic
+      const __half2 vb[4] = {__float2half2_rn(bf_lo(vm.x)), __float2half2_rn(bf_hi(vm.x)), __float2half2_rn(bf_lo(vm.y)), __float2half2_rn(bf_hi(vm.y))};
+      const __half2 vs[4] = {__float2half2_rn(bf_lo(vm.z)), __float2half2_rn(bf_hi(vm.z)), __float2half2_rn(bf_lo(vm.w)), __float2half2_rn(bf_hi(vm.w))};
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) {
+        const int j = j0 + PRODUCERS * i;
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+          uint32_t h[8];
+#pragma unroll
+          for (int quad = 0; quad < 4; ++quad) {
+            const uint2 c4 = bytes_to_half4((slot_value<CB>(Wc[i], v_slot_of(CB, cc, quad)) << FB) | slot_value<FB>(Wf[i], v_slot_of(FB, cc, quad)));
+            h[2 * quad] = hfma2_bits(c4.x, vs[cc], vb[cc]);
+            h[2 * quad + 1] = hfma2_bits(c4.y, vs[cc], vb[cc]);
+          }
+          *reinterpret_cast<uint4 *>(chunk_at(sm.v, 32 * cc + l, 16 * j)) = make_uint4(h[0], h[1], h[2], h[3]);
+          *reinterpret_cast<uint4 *>(chunk_at(sm.v, 32 * cc + l, 16 * j + 8)) = make_uint4(h[4], h[5], h[6], h[7]);
+        }
+      }
+      if (n + 1 < n_closed) load(g + 1, 0);
+      done(&sm.bar_v);
+    }
+#pragma unroll 1
+    for (int n = n_closed; n < n_pass && ok; ++n) {
       bool closed;
-      const int g = pass_group(n, closed);
-      const uint32_t prev = (n - 1) & 1;
-      // ---- Kop (free once both tiles' S of the previous pass are complete) ----
-      if (n > 0 && (!wait(sm, &sm.bar_s[0], prev) || !wait(sm, &sm.bar_s[1], prev))) break;
-      if (closed) {
-        if (!wait(sm, &sm.bar_meta[n & 1], (uint32_t)(n >> 1) & 1u)) break;
-        if (!wait(sm, &sm.bar_raw, raw_uses++ & 1)) break;
-      }
-      if (closed) {
-        // (record j, lane l): token 16 j + l % 16, channels 64 (l / 16) + 4 s + byte: one 128-byte row of slab l / 16
-#pragma unroll 1
-        for (int j = pt >> 5; j < SBG; j += PRODUCERS) {
-          uint32_t Wc[2 * CB], Wf[2 * FB];
-          lane_words<CB>(sm.raw + j * RC, 0, l, Wc);
-          lane_words<FB>(sm.raw + SBG * RC + j * RF, 0, l, Wf);
-          const int tok = 16 * j + (l & 15);
-#pragma unroll
-          for (int s2 = 0; s2 < 8; ++s2) {
-            const uint2 x = bytes_to_half4((slot_value<CB>(Wc, 2 * s2) << FB) | slot_value<FB>(Wf, 2 * s2));
-            const uint2 y = bytes_to_half4((slot_value<CB>(Wc, 2 * s2 + 1) << FB) | slot_value<FB>(Wf, 2 * s2 + 1));
-            *reinterpret_cast<uint4 *>(chunk_at(sm.k, tok, 64 * (l >> 4) + 8 * s2)) = make_uint4(x.x, x.y, y.x, y.y);
-          }
-        }
-      } else {
-        for (int e = pt; e < G * 16; e += PT) {  // BF16 group g: K rows as they are
-          const int tk = e >> 4, c = e & 15, tp = g * G + tk;
-          const uint4 kw = tp < n1 ? __ldcg(reinterpret_cast<const uint4 *>(token_row(tp, a.k, a.c.sink_k, a.c.open_k)) + c) : make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4 *>(chunk_at(sm.k, tk, 8 * c)) = kw;
-        }
-      }
-      fence_async_smem();
-      mbar_arrive(&sm.bar_k);
-      // ---- V' (free once both tiles' O products of the previous pass are complete) ----
-      if (n > 0 && (!wait(sm, &sm.bar_o[0], prev) || !wait(sm, &sm.bar_o[1], prev))) break;
-      if (closed) {
-        // (record j, lane l): channels 4 l + cc, tokens 16 j + 4 quad + byte, value base + step * code in FP16 arithmetic
-        const uint4 vm = lds128(sm.meta[n & 1] + 512 + 16 * l);
-        const __half2 vb[4] = {__float2half2_rn(bf_lo(vm.x)), __float2half2_rn(bf_hi(vm.x)), __float2half2_rn(bf_lo(vm.y)), __float2half2_rn(bf_hi(vm.y))};
-        const __half2 vs[4] = {__float2half2_rn(bf_lo(vm.z)), __float2half2_rn(bf_hi(vm.z)), __float2half2_rn(bf_lo(vm.w)), __float2half2_rn(bf_hi(vm.w))};
-#pragma unroll 1
-        for (int j = pt >> 5; j < SBG; j += PRODUCERS) {
-          uint32_t Wc[2 * CB], Wf[2 * FB];
-          lane_words<CB>(sm.raw + j * RC, 1, l, Wc);
-          lane_words<FB>(sm.raw + SBG * RC + j * RF, 1, l, Wf);
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            uint32_t h[8];
-#pragma unroll
-            for (int quad = 0; quad < 4; ++quad) {
-              const uint2 c4 = bytes_to_half4((slot_value<CB>(Wc, v_slot_of(CB, cc, quad)) << FB) | slot_value<FB>(Wf, v_slot_of(FB, cc, quad)));
-              h[2 * quad] = hfma2_bits(c4.x, vs[cc], vb[cc]);
-              h[2 * quad + 1] = hfma2_bits(c4.y, vs[cc], vb[cc]);
-            }
-            *reinterpret_cast<uint4 *>(chunk_at(sm.v, 32 * cc + l, 16 * j)) = make_uint4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<uint4 *>(chunk_at(sm.v, 32 * cc + l, 16 * j + 8)) = make_uint4(h[4], h[5], h[6], h[7]);
-          }
-        }
-      } else {
-        for (int e = pt; e < G * 16; e += PT) {  // V rows converted to FP16 and transposed (tokens along the K extent)
-          const int tk = e >> 4, c = e & 15, tp = g * G + tk;
-          const uint4 vw = tp < n1 ? __ldcg(reinterpret_cast<const uint4 *>(token_row(tp, a.v, a.c.sink_v, a.c.open_v)) + c) : make_uint4(0u, 0u, 0u, 0u);
-          const uint32_t w4[4] = {vw.x, vw.y, vw.z, vw.w};
-#pragma unroll
-          for (int x = 0; x < 8; ++x) {
-            const float f = (x & 1) ? bf_hi(w4[x >> 1]) : bf_lo(w4[x >> 1]);
-            *reinterpret_cast<__half *>(chunk_at(sm.v, vrow(8 * c + x), tk & ~7) + 2 * (tk & 7)) = __float2half_rn(f);
-          }
-        }
-      }
-      fence_async_smem();
-      mbar_arrive(&sm.bar_v);
+      const int t0 = pass_group(n, closed) * G;
+      if (!(ok = free_k(n))) break;
+      exact_k(sm.k, rows_k, t0, n1, pt);
+      done(&sm.bar_k);
+      if (!(ok = free_v(n))) break;
+      exact_v(sm.v, rows_v, t0, n1, pt);
+      done(&sm.bar_v);
     }
-  } else {
-    // ================= row threads: qhat, softmax, P', output =================
-    // Softmax: two threads per row (warps w and w + 8 share a tensor-memory lane quadrant): thread hf owns tokens
-    // 64 hf .. + 63 of S and P' (slab hf of the P' tile) and O columns 64 hf .. + 63; the pair meets on a named barrier to
-    // exchange the pass maximum. qhat: a different map -- a warp takes 16 rows of its tile, two rows at a time: lane
-    // (c = lane % 16, lane / 16) holds channels 8 c .. + 7 of one row, with the group's steps and bases of those channels
-    // in registers for the whole pass; max |z| and the bias dot product are reduced over the 16 lanes of a row. That
-    // keeps shared-memory traffic (the limiter of a thread-per-row quantiser, which re-reads steps and bases per row)
-    // at one load and one store per row chunk. A thread never leaves the pass loop early: after an abort every wait
-    // returns at once, so both threads of a pair still reach every named barrier.
-    const int hf = warp >> 3, X = (warp >> 2) & 1, r = 32 * (warp & 3) + lane, R = r0 + ROWS * X + r;
-    const int pair_bar = 1 + (warp & 7);
-    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory"); };
-    const bool valid = R < rows;
-    const int i = valid ? R / qg : 0, hq = kh * qg + (valid ? R - i * qg : 0), pos = n0 + i, own = pos / G;
-    const int tile_last = min(r0 + ROWS * X + ROWS, rows) - 1;                 // the tile's last row, if it has any
-    const int tile_own = tile_last >= r0 + ROWS * X ? (n0 + tile_last / qg) / G : -1;  // closed group g concerns the tile iff g < tile_own
-    // quantiser lane: chunk qc of rows qrow0 + 2 it, it = 0 .. 7 (qrow0 % 8 is 0 or 1, so (row % 8) = (2 it) | (qrow0 & 1))
-    const int qc = lane & 15, qrow0 = 16 * ((warp & 3) + 4 * hf) + (lane >> 4);
+  } else if (warp >= QUANT_WARP0) {
+    // ================= quantiser: Qop of every pass, tile 0 then tile 1 =================
+    // A warp takes 16 rows of a tile, two rows at a time: lane (c = lane % 16, lane / 16) holds channels 8 c .. + 7 of one
+    // row, with the group's steps of those channels in registers; max |z| is reduced over the 16 lanes of a row. The bias
+    // dot products q . base of eight groups at a time are one BF16 tensor-core product per 16 rows (exact products, FP32 sums).
+    const int qw = warp - QUANT_WARP0, qc = lane & 15, qrow0 = 16 * qw + (lane >> 4);  // (row % 8) of row qrow0 + 2 it = (2 it) | (qrow0 & 1)
     const uint32_t qoff = (qc >> 3) * SLAB + qrow0 * 128, qcx = (uint32_t)((qc & 7) ^ (qrow0 & 1)) << 4;
-    const uint32_t qmask = (lane & 16) ? 0xffff0000u : 0x0000ffffu;
-    // the rows' q into the BF16 Q tile (rows past the end: zeros), by the same map
+    // the rows' q into the BF16 Q tiles (rows past the end: zeros), by the same map
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int rowq = qrow0 + 2 * it, Rq = r0 + ROWS * X + rowq;
-      uint4 w = make_uint4(0u, 0u, 0u, 0u);
-      if (Rq < rows) {
-        const int iq = Rq / qg;
-        w = __ldg(reinterpret_cast<const uint4 *>(a.q + ((size_t)(b * a.q_heads + kh * qg + (Rq - iq * qg)) * a.count + iq) * D) + qc);
+    for (int X = 0; X < 2; ++X)
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int Rq = r0 + ROWS * X + qrow0 + 2 * it;
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (Rq < rows) {
+          const int iq = Rq / qg;
+          w = __ldg(reinterpret_cast<const uint4 *>(a.q + ((size_t)(b * a.q_heads + kh * qg + (Rq - iq * qg)) * a.count + iq) * D) + qc);
+        }
+        *reinterpret_cast<uint4 *>(sm.q[X] + qoff + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4))) = w;
       }
-      *reinterpret_cast<uint4 *>(sm.q[X] + qoff + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4))) = w;
+    int tile_own[2];  // closed group g concerns the tile iff g < tile_own
+#pragma unroll
+    for (int X = 0; X < 2; ++X) {
+      const int tile_last = min(r0 + ROWS * X + ROWS, rows) - 1;  // the tile's last row, if it has any
+      tile_own[X] = tile_last >= r0 + ROWS * X ? (n0 + tile_last / qg) / G : -1;
     }
-    float m_run = -FBLA_INF, l_run = 0.f;  // l_run: this thread's tokens only
+    const float2 mg = splat(MAGICF), ng = splat(-MAGICF);
+    const float sl127 = __fmul_rn(a.sl, 1.f / 127.f);
+    const uint8_t *const meta = reinterpret_cast<const uint8_t *>(a.c.meta) + head * 1024 + 32 * qc;
+    uint4 ma = make_uint4(0u, 0u, 0u, 0u), mb = ma;  // K metadata of channels 8 qc .. + 7: per four channels, four BF16 bases (unused here) then four BF16 steps
+    auto load_meta = [&](int g) {
+      ma = __ldcg(reinterpret_cast<const uint4 *>(meta + (size_t)g * a.gs * 1024));
+      mb = __ldcg(reinterpret_cast<const uint4 *>(meta + (size_t)g * a.gs * 1024 + 16));
+    };
+    if (n_closed > 0) load_meta(1);
+    __syncwarp();  // (the warp's own rows of the q tiles are in place)
+#pragma unroll 1
+    for (int n = 0; n < n_closed; ++n) {
+      const int g = 1 + n;
+      if (!(n & 7)) {  // the biases of groups g .. g + 7 (those past the last: repeated, unused)
+        const uint8_t *base = reinterpret_cast<const uint8_t *>(a.c.meta) + (head + (size_t)min(g + (lane >> 2), n_closed) * a.gs) * 1024 + 16 * ((lane & 3) >> 1) + 4 * (lane & 1);
+#pragma unroll 1
+        for (int X = 0; X < 2; ++X) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          const int row = 16 * qw + (lane & 15);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {  // channels 16 kk ..
+            uint32_t q4[4];
+            ldmatrix_x4(q4, sm.q[X] + (kk >> 2) * SLAB + row * 128 + (((2 * (kk & 3) + (lane >> 4)) ^ (row & 7)) << 4));
+            mma_bf16_k16(d, q4[0], q4[1], q4[2], q4[3], __ldcg(reinterpret_cast<const uint32_t *>(base + 64 * kk)), __ldcg(reinterpret_cast<const uint32_t *>(base + 64 * kk + 32)));
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sm.qbias[(n >> 3) & 1][2 * (lane & 3) + (i & 1)][X][16 * qw + (lane >> 2) + 8 * (i >> 1)] = __fmul_rn(d[i], a.sl);
+        }
+      }
+      const float4 s0 = make_float4(bf_lo(ma.z), bf_hi(ma.z), bf_lo(ma.w), bf_hi(ma.w));
+      const float4 s1 = make_float4(bf_lo(mb.z), bf_hi(mb.z), bf_lo(mb.w), bf_hi(mb.w));
+      if (n + 1 < n_closed) load_meta(g + 1);
+#pragma unroll 1
+      for (int X = 0; X < 2; ++X) {
+        // the tile's qhat buffer is free once the S product of the pass before is complete
+        if (n > 0) wait(sm, &sm.bar_s[X], (n - 1) & 1);
+        if (g < tile_own[X]) {
+          // z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16. First sweep: the lane's shares of max |z| for
+          // its eight rows; a butterfly over a row's 16 lanes that hands half of the rows on in
+          // every step leaves row `it` = 4 b3 + 2 b2 + b1 in the lanes with those bits, which form its r once.
+          auto z_of = [&](int it, int h, float2 (&z)[4]) -> uint32_t {  // row it + 4 h of the lane's eight
+            const uint32_t off = qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4));
+            const uint4 qv = *reinterpret_cast<const uint4 *>(sm.q[X] + off);
+            z[0] = mul2(bf2(qv.x), make_float2(s0.x, s0.y)); z[1] = mul2(bf2(qv.y), make_float2(s0.z, s0.w));
+            z[2] = mul2(bf2(qv.z), make_float2(s1.x, s1.y)); z[3] = mul2(bf2(qv.w), make_float2(s1.z, s1.w));
+            return off;
+          };
+          float amax[4] = {0.f, 0.f, 0.f, 0.f}, before[4];
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              float2 z[4];
+              z_of(it, h, z);
+              before[it] = amax[it];
+              amax[it] = max3_abs(max3_abs(z[0].x, z[0].y, z[1].x), max3_abs(z[1].y, z[2].x, z[2].y), fmaxf(fabsf(z[3].x), fabsf(z[3].y)));
+            }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {  // lane bit 3 decides which four rows are kept, bits 2 and 1 which half of what is left
+            const bool up = lane & 8;
+            const float keep = up ? amax[i] : before[i], send = up ? before[i] : amax[i];
+            amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 8));
+          }
+#pragma unroll
+          for (int w = 2; w; w >>= 1) {
+            const bool up = lane & (2 * w);
+#pragma unroll
+            for (int i = 0; i < w; ++i) {
+              const float keep = up ? amax[i + w] : amax[i], send = up ? amax[i] : amax[i + w];
+              amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 2 * w));
+            }
+          }
+          const float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 1));
+          const float rq = quotient_127(am);
+          if (!(lane & 1)) sm.qscale[n & 1][X][qrow0 + (lane & 14)] = __fmul_rn(am, sl127);  // (row qrow0 + 2 it)
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              float2 z[4];
+              const uint32_t off = z_of(it, h, z);
+              // rint(z r) as the exact float (t - 1.5 * 2^23), then FP16 (an integer of magnitude <= 127: exact)
+              const float2 rr2 = splat(__shfl_sync(FULL, rq, (lane & 16) | (8 * h + 2 * it)));
+              const float2 t0 = add2(fma2(z[0], rr2, mg), ng), t1 = add2(fma2(z[1], rr2, mg), ng);
+              const float2 t2 = add2(fma2(z[2], rr2, mg), ng), t3 = add2(fma2(z[3], rr2, mg), ng);
+              *reinterpret_cast<uint4 *>(sm.qp[X] + off) = make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
+            }
+        }
+        fence_async_smem();
+        mbar_arrive(&sm.bar_q[X]);
+      }
+    }
+    if (n_closed == 0) fence_async_smem();  // (the q tiles, otherwise covered by the first pass's)
+#pragma unroll 1
+    for (int n = n_closed; n < n_pass; ++n)  // BF16 passes take the q tiles as they are
+      for (int X = 0; X < 2; ++X) {
+        if (n > 0) wait(sm, &sm.bar_s[X], (n - 1) & 1);
+        mbar_arrive(&sm.bar_q[X]);
+      }
+  } else {
+    // ================= softmax, P', output: tile 0 then tile 1 of every pass =================
+    // Two threads per row: warps w and w + 4 share a tensor-memory lane quadrant; thread hf owns tokens 64 hf .. + 63 of S and
+    // P' and O columns 64 hf .. + 63; the pair meets on a named barrier to exchange the pass maximum. A thread never leaves
+    // the pass loop early: after an abort every wait returns at once, so both threads of a pair still reach every named barrier.
+    const int hf = warp >> 3, X = (warp >> 2) & 1, r = 32 * (warp & 3) + lane, pair_bar = 1 + (warp & 7);
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory"); };
     const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t tmem_s = tmem + 128 * X + 64 * hf + lane_base, tmem_o = tmem + 256 + 128 * X + 64 * hf + lane_base;
+    float m_run = -FBLA_INF, l_run = 0.f;  // l_run: this thread's tokens only
+    const int R = r0 + ROWS * X + r, pos = R < rows ? n0 + R / qg : -1, own = pos / G;  // pos -1: the tile has no such row
     bool ok = true;
-    // Qop of pass np into the qhat tile (free once the S product of pass np - 1 is complete), then the tile's arrival for it
-    auto prepare = [&](int np) {
-      bool closed;
-      const int g = pass_group(np, closed);
-      if (closed) {
-        // the group's metadata (fetched two passes ahead; it is replaced only after both tiles have arrived for this pass)
-        ok &= __all_sync(FULL, wait(sm, &sm.bar_meta[np & 1], (uint32_t)(np >> 1) & 1u));
-        if (g < tile_own) {
-      // qhat for this group: z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16; four rows per batch, with
-      // every load ahead of the arithmetic and every store behind it, so that the rows' dependency chains overlap
-      // K bases and steps of channels 8 qc .. 8 qc + 7: per four channels, four BF16 bases then four BF16 steps
-      const uint4 ma = lds128(sm.meta[np & 1] + 32 * qc), mb = lds128(sm.meta[np & 1] + 32 * qc + 16);
-      const float4 b0 = make_float4(bf_lo(ma.x), bf_hi(ma.x), bf_lo(ma.y), bf_hi(ma.y)), s0 = make_float4(bf_lo(ma.z), bf_hi(ma.z), bf_lo(ma.w), bf_hi(ma.w));
-      const float4 b1 = make_float4(bf_lo(mb.x), bf_hi(mb.x), bf_lo(mb.y), bf_hi(mb.y)), s1 = make_float4(bf_lo(mb.z), bf_hi(mb.z), bf_lo(mb.w), bf_hi(mb.w));
-      const float2 mg = splat(MAGICF), ng = splat(-MAGICF);
-      const float sl127 = __fmul_rn(a.sl, 1.f / 127.f);
-      const bool h3 = lane & 8;
-#pragma unroll
-      for (int bt = 0; bt < 4; ++bt) {  // two rows per batch; their z = q * step stay in registers for the second sweep
-        float2 z[2][4];
-        uint32_t off[2];
-        float amax[2], dot[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {  // the lane's share of max |z| and of the bias dot product
-          const int it = 2 * bt + k;
-          off[k] = qoff + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4));
-          const uint4 qv = *reinterpret_cast<const uint4 *>(sm.q[X] + off[k]);
-          const float2 q0 = bf2(qv.x), q1 = bf2(qv.y), q2 = bf2(qv.z), q3 = bf2(qv.w);
-          z[k][0] = mul2(q0, make_float2(s0.x, s0.y)); z[k][1] = mul2(q1, make_float2(s0.z, s0.w));
-          z[k][2] = mul2(q2, make_float2(s1.x, s1.y)); z[k][3] = mul2(q3, make_float2(s1.z, s1.w));
-          amax[k] = fmaxf(fmaxf(fmaxf(fabsf(z[k][0].x), fabsf(z[k][0].y)), fmaxf(fabsf(z[k][1].x), fabsf(z[k][1].y))),
-                          fmaxf(fmaxf(fabsf(z[k][2].x), fabsf(z[k][2].y)), fmaxf(fabsf(z[k][3].x), fabsf(z[k][3].y))));
-          float2 d2 = fma2(q0, make_float2(b0.x, b0.y), mul2(q1, make_float2(b0.z, b0.w)));
-          d2 = fma2(q2, make_float2(b1.x, b1.y), fma2(q3, make_float2(b1.z, b1.w), d2));
-          dot[k] = d2.x + d2.y;
-        }
-        // over the 16 lanes of a row: the maxima by reductions (nonnegative floats order as integers), the dot products by
-        // a merging butterfly that leaves row b3 of the batch in the lanes with bit 3 = b3
-#pragma unroll
-        for (int k = 0; k < 2; ++k) amax[k] = __uint_as_float(__reduce_max_sync(qmask, __float_as_uint(amax[k])));
-        float dsum = (h3 ? dot[1] : dot[0]) + __shfl_xor_sync(FULL, h3 ? dot[0] : dot[1], 8);
-        dsum += __shfl_xor_sync(FULL, dsum, 4);
-        dsum += __shfl_xor_sync(FULL, dsum, 2);
-        dsum += __shfl_xor_sync(FULL, dsum, 1);
-        if (!(lane & 7)) sm.qbias[np & 1][X][qrow0 + 2 * (2 * bt + ((lane >> 3) & 1))] = __fmul_rn(dsum, a.sl);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const float am = amax[k];
-          // rint(z r) as the exact float (t - 1.5 * 2^23), then FP16 (an integer of magnitude <= 127: exact)
-          const float2 rr2 = splat(quotient_127(am));
-          const float2 t0 = add2(fma2(z[k][0], rr2, mg), ng), t1 = add2(fma2(z[k][1], rr2, mg), ng);
-          const float2 t2 = add2(fma2(z[k][2], rr2, mg), ng), t3 = add2(fma2(z[k][3], rr2, mg), ng);
-          *reinterpret_cast<uint4 *>(sm.qp[X] + off[k]) = make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
-          if (qc == 0) sm.qscale[np & 1][X][qrow0 + 2 * (2 * bt + k)] = __fmul_rn(am, sl127);
-        }
-      }
-        }
-      }
-      fence_async_smem();
-      mbar_arrive(&sm.bar_q[X]);
-    };
-    prepare(0);
-    // Per pass: the softmax of S(n), whose P' goes back into tensor memory over the S columns it came from -- row r in lane
-    // r, tokens 2 c and 2 c + 1 of this thread's 64 in column c of its 64 S columns, so the O product takes P' as its
-    // tensor-memory operand and no shared memory is written -- then Qop of pass n + 1, while the O product of pass n runs.
-    // Products execute in the order they were issued: S(n + 1) overwrites P'(n) only after O(n) has read it.
     for (int n = 0; n < n_pass; ++n) {
       bool closed;
       const int g = pass_group(n, closed);
-      const bool include = valid && (closed ? g < own : (g == 0 || g == own));
-      const bool any = __any_sync(FULL, include);
-      // S(n) is complete, and with it every product issued before: O of pass n - 1 is stable
-      ok &= __all_sync(FULL, wait(sm, &sm.bar_s[X], n & 1));
-      tc_fence_after();
-      // softmax of the row over the pass's 128 tokens, by 16-token blocks; P' = fp16(2^(m_block - m_row) p)
-      const int lim = (include ? (closed ? G : pos - g * G) : -1) - 64 * hf;  // this thread's tokens 0 .. lim are attended
-      const float mul1 = closed ? sm.qscale[n & 1][X][r] : a.sl, add1 = closed ? sm.qbias[n & 1][X][r] : 0.f;  // score = mul x + add, monotonic in x (mul >= 0)
-      // sweep 1: the block maxima, from the raw sums
-      float mbk[4];
-      if (any) {
+      {
+        const bool include = pos >= 0 && (closed ? g < own : (g == 0 || g == own));
+        const bool any = __any_sync(FULL, include);
+        // S(n) is complete, and with it every product issued before: O of the tile's pass n - 1 is stable
+        ok &= __all_sync(FULL, wait(sm, &sm.bar_s[X], n & 1));
+        tc_fence_after();
+        // softmax of the row over the pass's 128 tokens, by 16-token blocks; P' = fp16(2^(m_block - m_row) p)
+        const int lim = (include ? (closed ? G : pos - g * G) : -1) - 64 * hf;  // this thread's tokens 0 .. lim are attended
+        const float mul1 = closed ? sm.qscale[n & 1][X][r] : a.sl, add1 = closed ? sm.qbias[(n >> 3) & 1][n & 7][X][r] : 0.f;  // score = mul x + add, monotonic in x (mul >= 0)
+        // sweep 1: the block maxima, from the raw sums (each block's columns are asked for while the one before is worked on)
+        float mbk[4];
+        uint32_t xa[16], xb[16];
+        if (any) {
+          tmem_ld16(tmem_s, xa);
 #pragma unroll
-        for (int cq = 0; cq < 2; ++cq) {
-          uint32_t x[32];
-          tmem_ld32(tmem_s + 32 * cq, x);
-#pragma unroll
-          for (int hb = 0; hb < 2; ++hb) {
-            const int t0 = 32 * cq + 16 * hb;
+          for (int blk = 0; blk < 4; ++blk) {
+            uint32_t (&x)[16] = blk & 1 ? xb : xa;
+            tmem_ld_wait(x);
+            if (blk < 3) tmem_ld16(tmem_s + 16 * (blk + 1), blk & 1 ? xa : xb);
+            const int t0 = 16 * blk;
             float xm = -FBLA_INF;
             if (lim >= t0 + 15) {
+              float y[4];
 #pragma unroll
-              for (int t = 0; t < 16; t += 2) xm = fmaxf(xm, fmaxf(__uint_as_float(x[16 * hb + t]), __uint_as_float(x[16 * hb + t + 1])));
+              for (int t = 0; t < 4; ++t) y[t] = max3(__uint_as_float(x[4 * t]), __uint_as_float(x[4 * t + 1]), __uint_as_float(x[4 * t + 2]));
+              xm = max3(max3(y[0], y[1], __uint_as_float(x[3])), max3(y[2], y[3], __uint_as_float(x[7])), fmaxf(__uint_as_float(x[11]), __uint_as_float(x[15])));
             } else {
 #pragma unroll
-              for (int t = 0; t < 16; ++t) if (t0 + t <= lim) xm = fmaxf(xm, __uint_as_float(x[16 * hb + t]));
+              for (int t = 0; t < 16; ++t) if (t0 + t <= lim) xm = fmaxf(xm, __uint_as_float(x[t]));
             }
-            mbk[2 * cq + hb] = xm == -FBLA_INF ? -FBLA_INF : fmaf(mul1, xm, add1);  // -inf: a block without attended tokens
+            mbk[blk] = xm == -FBLA_INF ? -FBLA_INF : fmaf(mul1, xm, add1);  // -inf: a block without attended tokens
           }
+          sm.ex2[X][r][hf] = fmaxf(fmaxf(mbk[0], mbk[1]), fmaxf(mbk[2], mbk[3]));
         }
-        sm.ex2[X][r][hf] = fmaxf(fmaxf(mbk[0], mbk[1]), fmaxf(mbk[2], mbk[3]));
-      }
-      pair_sync();
-      if (!any) {  // (warp-uniform, and the same in both warps of the pair) nothing to attend: P' = 0
-        const uint32_t zero[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        pair_sync();
+        if (!any) {  // (warp-uniform, and the same in both warps of the pair) nothing to attend: P' = 0
+          const uint32_t zero[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_st8(tmem_s + 8 * c, zero);
-      } else {
-        const float2 e = *reinterpret_cast<const float2 *>(&sm.ex2[X][r][0]);
-        const float mp = fmaxf(e.x, e.y);
-        // the row's running maximum moves only when a block exceeds it by more than 2^8 (rare): its sums and its O row in
-        // tensor memory are rescaled. Tensor-memory accesses are warp-wide, so the whole warp takes part (rows that do
-        // not move scale by 1); both threads of a row decide alike and each rescales its own 64 columns.
-        const bool need = mp > m_run + 8.f;
-        if (__any_sync(FULL, need)) {
-          const float al = need ? ex2(m_run - mp) : 1.f;  // 0 on the row's first attended block
-          if (n > 0) {
+          for (int c = 0; c < 4; ++c) tmem_st8(tmem_s + 8 * c, zero);
+        } else {
+          const float2 e = *reinterpret_cast<const float2 *>(&sm.ex2[X][r][0]);
+          const float mp = fmaxf(e.x, e.y);
+          // the row's running maximum moves only when a block exceeds it by more than 2^8 (rare): its sums and its O row in
+          // tensor memory are rescaled. Tensor-memory accesses are warp-wide, so the whole warp takes part (rows that do
+          // not move scale by 1); both threads of a row decide alike and each rescales its own 64 columns.
+          const bool need = mp > m_run + 8.f;
+          if (__any_sync(FULL, need)) {
+            const float al = need ? ex2(m_run - mp) : 1.f;  // 0 on the row's first attended block
+            if (n > 0) {
 #pragma unroll 1
-            for (int oc = 0; oc < 2; ++oc) {
-              uint32_t o[32];
-              tmem_ld32(tmem_o + 32 * oc, o);
+              for (int oc = 0; oc < 2; ++oc) {
+                uint32_t o[32];
+                tmem_ld32(tmem_o + 32 * oc, o);
 #pragma unroll
-              for (int z = 0; z < 32; ++z) o[z] = __float_as_uint(__uint_as_float(o[z]) * al);
-              tmem_st32(tmem_o + 32 * oc, o);
+                for (int z = 0; z < 32; ++z) o[z] = __float_as_uint(__uint_as_float(o[z]) * al);
+                tmem_st32(tmem_o + 32 * oc, o);
+              }
             }
+            if (need) { l_run *= al; m_run = mp; }
           }
-          if (need) { l_run *= al; m_run = mp; }
-        }
-        // sweep 2: the integer P blocks times their weights
-        const float2 mul = splat(mul1), c255 = splat(255.f), mg = splat(MAGICF), ng = splat(-MAGICF);
-        float2 lacc = make_float2(0.f, 0.f);
+          // sweep 2: the integer P blocks times their weights. With a weight of 22 bits 1.5 * 2^23 w is a float, so that
+          // (1.5 * 2^23 + p) w - 1.5 * 2^23 w is p w in one rounding (the integer p needs no instruction of its own).
+          const float2 mul = splat(mul1), c255 = splat(255.f), mg = splat(MAGICF);
+          float2 lacc = make_float2(0.f, 0.f);
+          tmem_ld16(tmem_s, xa);
 #pragma unroll
-        for (int cq = 0; cq < 2; ++cq) {
-          uint32_t x[32];
-          tmem_ld32(tmem_s + 32 * cq, x);
-#pragma unroll
-          for (int hb = 0; hb < 2; ++hb) {
-            const int t0 = 32 * cq + 16 * hb;
-            const float mb = mbk[2 * cq + hb];
+          for (int blk = 0; blk < 4; ++blk) {
+            uint32_t (&x)[16] = blk & 1 ? xb : xa;
+            tmem_ld_wait(x);
+            if (blk < 3) tmem_ld16(tmem_s + 16 * (blk + 1), blk & 1 ? xa : xb);
+            const int t0 = 16 * blk;
+            const float mb = mbk[blk];
             // score - block maximum in one step: mul x + (add - m_block)
-            const float2 addm = splat(mb == -FBLA_INF ? add1 : add1 - mb), w2 = splat(mb == -FBLA_INF ? 0.f : ex2(mb - m_run));
+            const float w1 = mb == -FBLA_INF ? 0.f : __uint_as_float(__float_as_uint(ex2(mb - m_run)) & ~3u);
+            const float2 addm = splat(mb == -FBLA_INF ? add1 : add1 - mb), w2 = splat(w1), mw = splat(-MAGICF * w1);
             float2 sc[8];
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
-              sc[t] = fma2(make_float2(__uint_as_float(x[16 * hb + 2 * t]), __uint_as_float(x[16 * hb + 2 * t + 1])), mul, addm);
+            for (int t = 0; t < 8; ++t) sc[t] = fma2(make_float2(__uint_as_float(x[2 * t]), __uint_as_float(x[2 * t + 1])), mul, addm);
             if (lim < t0 + 15) {  // the causal edge (or a row that does not attend to this group)
 #pragma unroll
               for (int t = 0; t < 8; ++t) {
@@ -467,32 +547,28 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
               }
             }
             uint32_t h[8];
-            float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
-              const float2 pf = add2(fma2(make_float2(ex2(sc[t].x), ex2(sc[t].y)), c255, mg), ng);
-              acc = add2(acc, pf);
-              const float2 pw = mul2(pf, w2);
+              const float2 pw = fma2(fma2(make_float2(ex2(sc[t].x), ex2(sc[t].y)), c255, mg), w2, mw);
+              lacc = add2(lacc, pw);
               h[t] = pack_half2(pw.x, pw.y);
             }
-            lacc = fma2(acc, w2, lacc);
-            tmem_st8(tmem_s + 16 * cq + 8 * hb, h);  // (over S columns this thread has already taken into registers)
+            tmem_st8(tmem_s + 8 * blk, h);  // (over S columns this thread has already taken into registers)
           }
+          l_run += lacc.x + lacc.y;
         }
-        l_run += lacc.x + lacc.y;
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&sm.bar_p[X]);
       }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&sm.bar_p[X]);
-      if (n + 1 < n_pass) prepare(n + 1);
     }
-    ok &= __all_sync(FULL, wait(sm, &sm.bar_o[X], (n_pass - 1) & 1));
-    tc_fence_after();
-    pair_sync();  // (the partner has read the last pass's exchange)
-    sm.ex2[X][r][hf] = l_run;
-    pair_sync();
     {
-      // O column 32 cc + l is channel 4 l + cc: through the row's (now free) P' row as BF16 in channel order, then out.
+      ok &= __all_sync(FULL, wait(sm, &sm.bar_o[X], (n_pass - 1) & 1));
+      tc_fence_after();
+      pair_sync();  // (the partner has read the last pass's exchange)
+      sm.ex2[X][r][hf] = l_run;
+      pair_sync();
+      // O column 32 cc + l is channel 4 l + cc: through the row's (now free) qhat row as BF16 in channel order, then out.
       // This thread: O columns 64 hf .. + 63 (cc = 2 hf, 2 hf + 1); then it copies chunks 8 hf .. + 7 of the row.
       const float inv = 1.f / (sm.ex2[X][r][0] + sm.ex2[X][r][1]);
       uint16_t *stage = reinterpret_cast<uint16_t *>(sm.qp[X] + r * 256);  // 256 bytes per row, private to the pair
@@ -500,13 +576,14 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
       for (int cu = 0; cu < 2; ++cu) {
         const int cc = 2 * hf + cu;
         uint32_t o[32];
-        tmem_ld32(tmem_o + 32 * cu, o);
+        tmem_ld32(tmem + 256 + 128 * X + 64 * hf + lane_base + 32 * cu, o);
 #pragma unroll
         for (int l = 0; l < 32; ++l)  // channel 4 l + cc: 16-byte chunk l / 2 of the row, stored at chunk (l / 2) ^ (r % 16)
           stage[8 * ((l >> 1) ^ (r & 15)) + 4 * (l & 1) + cc] = f32_to_bf16(__uint_as_float(o[l]) * inv);
       }
       pair_sync();
-      if (valid) {  // (after a wait that gave up: NaN, so that the failure shows in the caller's data)
+      if (R < rows) {  // (after a wait that gave up: NaN, so that the failure shows in the caller's data)
+        const int i = R / qg, hq = kh * qg + (R - i * qg);
         uint16_t *orow = a.out + (size_t)(b * a.q_heads + hq) * a.out_hs + (size_t)i * a.out_ts;
         const uint4 nan4 = make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
 #pragma unroll
@@ -521,7 +598,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
   if (tid == 0) {  // no live barrier object is left behind: an executor may run another item on this CTA next
-    mbar_inval(&sm.bar_raw); mbar_inval(&sm.bar_meta[0]); mbar_inval(&sm.bar_meta[1]); mbar_inval(&sm.bar_k); mbar_inval(&sm.bar_v);
+    mbar_inval(&sm.bar_k); mbar_inval(&sm.bar_v);
     for (int x = 0; x < 2; ++x) { mbar_inval(&sm.bar_q[x]); mbar_inval(&sm.bar_s[x]); mbar_inval(&sm.bar_p[x]); mbar_inval(&sm.bar_o[x]); }
   }
 }
