@@ -255,14 +255,15 @@ void fill_chunk(const mlops_fbla_config *c, int count, long long room, const uin
 }
 // The passes in the order that keeps them correct: closing groups reads the windows as they were, the attention reads
 // them too, and only then are the windows rewritten. Without queries one launch does both (fbla_close.cuh: write_item).
-mlops_fbla_status enqueue_chunk(const char *fn, const fbla_k_prefill &a, int closable_groups, cudaStream_t stream) {
+mlops_fbla_status enqueue_chunk(const char *fn, fbla_k_prefill &a, int closable_groups, cudaStream_t stream) {
+  a.early = closable_groups > 0;
   if (!a.q) {
     const cudaError_t e = fbla_k_write_launch(&a, closable_groups, stream);
     return e == cudaSuccess ? accepted() : device_failure(fn, e);
   }
   cudaError_t e = fbla_k_close_launch(&a, closable_groups, stream);
   if (e == cudaSuccess) e = fbla_k_attend_launch(&a, stream);
-  if (e == cudaSuccess) e = fbla_k_finish_launch(&a, stream);
+  if (e == cudaSuccess && !(a.early && !a.length && a.n0 == 0)) e = fbla_k_finish_launch(&a, stream);
   return e == cudaSuccess ? accepted() : device_failure(fn, e);
 }
 // device-length chunk (prefill_at, append_at and their plans)

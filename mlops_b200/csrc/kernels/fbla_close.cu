@@ -1,5 +1,6 @@
 // Launchers of the close / finish passes and of the chunk without queries (bodies: fbla_close.cuh).
 #include "fbla_close.cuh"
+#include "fbla_launch.h"
 #include <stdio.h>
 
 namespace {
@@ -17,16 +18,22 @@ namespace fbla {
 template <int CB, int FB>
 __global__ void __launch_bounds__(CLOSE_THREADS, 2) close_kernel(const fbla_k_prefill a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
+  wait_previous_pass();
+  allow_next_pass();
   close_item<CB, FB>(a, smem_raw);
 }
 
 template <int CB, int FB>
 __global__ void __launch_bounds__(CLOSE_THREADS, 2) write_kernel(const fbla_k_prefill a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
+  wait_previous_pass();
+  allow_next_pass();
   write_item<CB, FB>(a, smem_raw);
 }
 
 __global__ void __launch_bounds__(CLOSE_THREADS) finish_kernel(const fbla_k_prefill a) {
+  wait_previous_pass();
+  allow_next_pass();
   finish_item(a, nullptr);
 }
 
@@ -49,23 +56,18 @@ extern "C" cudaError_t fbla_k_close_launch(const fbla_k_prefill *a, int close_bl
   const cudaError_t e = fbla::configure();
   if (e != cudaSuccess) return e;
   const dim3 grid(close_blocks, a->batch * a->kv_heads);
-  if (a->cb == 3) fbla::close_kernel<3, 3><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
-  else fbla::close_kernel<4, 2><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
-  return cudaGetLastError();
+  return fbla::launch(true, 1, a->cb == 3 ? fbla::close_kernel<3, 3> : fbla::close_kernel<4, 2>, grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream, *a);
 }
 
 extern "C" cudaError_t fbla_k_write_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream) {
   const cudaError_t e = fbla::configure();
   if (e != cudaSuccess) return e;
   const dim3 grid(close_blocks > 0 ? close_blocks : 1, a->batch * a->kv_heads);
-  if (a->cb == 3) fbla::write_kernel<3, 3><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
-  else fbla::write_kernel<4, 2><<<grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream>>>(*a);
-  return cudaGetLastError();
+  return fbla::launch(true, 1, a->cb == 3 ? fbla::write_kernel<3, 3> : fbla::write_kernel<4, 2>, grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream, *a);
 }
 
 extern "C" cudaError_t fbla_k_finish_launch(const fbla_k_prefill *a, cudaStream_t stream) {
-  fbla::finish_kernel<<<a->batch * a->kv_heads, fbla::CLOSE_THREADS, 0, stream>>>(*a);
-  return cudaGetLastError();
+  return fbla::launch(true, 1, fbla::finish_kernel, dim3(a->batch * a->kv_heads), fbla::CLOSE_THREADS, 0, stream, *a);
 }
 
 extern "C" cudaError_t fbla_k_close_pass(const fbla_k_prefill *a, int close_blocks, fbla_k_pass *info) {

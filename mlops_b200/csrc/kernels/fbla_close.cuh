@@ -198,14 +198,6 @@ __device__ __forceinline__ int closing_group(const Chunk &ch, int x) {
   return g < (ch.n0 + ch.count - 1) / G ? g : -1;
 }
 
-template <int CB, int FB>
-__device__ __forceinline__ void close_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
-  const int bh = FBLA_POS::y();
-  const Chunk ch = chunk_of(a, bh / a.kv_heads);
-  const int g = closing_group(ch, FBLA_POS::x());
-  if (g >= 0) close_group<CB, FB>(a, *reinterpret_cast<CloseSmem *>(smem_raw), bh, g, ch.n0);
-}
-
 // finish: the sink window takes the chunk's positions < 128, the open window the tokens of the newest group; a fresh
 // open group's unused rows are cleared. One CTA of 512 threads per KV head, four 16-byte pieces per thread in flight.
 __device__ __forceinline__ void finish_windows(const fbla_k_prefill &a, int bh, const Chunk &ch) {
@@ -234,8 +226,17 @@ __device__ __forceinline__ void finish_windows(const fbla_k_prefill &a, int bh, 
     }
   }
 }
+template <int CB, int FB>
+__device__ __forceinline__ void close_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
+  const int bh = FBLA_POS::y();
+  const Chunk ch = chunk_of(a, bh / a.kv_heads);
+  const int g = closing_group(ch, FBLA_POS::x());
+  if (g >= 0) close_group<CB, FB>(a, *reinterpret_cast<CloseSmem *>(smem_raw), bh, g, ch.n0);
+  if (a.early && ch.n0 == 0 && FBLA_POS::x() == 0) finish_windows(a, bh, ch);
+}
 __device__ __forceinline__ void finish_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
-  finish_windows(a, FBLA_POS::x(), chunk_of(a, FBLA_POS::x() / a.kv_heads));
+  const Chunk ch = chunk_of(a, FBLA_POS::x() / a.kv_heads);
+  if (!a.early || ch.n0 > 0) finish_windows(a, FBLA_POS::x(), ch);
 }
 
 // A chunk without queries in one launch: CTA (x, bh) closes its group; CTA (0, bh) also updates the windows -- it is the

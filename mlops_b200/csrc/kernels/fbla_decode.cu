@@ -1,5 +1,6 @@
 // Launchers of the decode passes (bodies: fbla_decode.cuh).
 #include "fbla_decode.cuh"
+#include "fbla_launch.h"
 #include <stdio.h>
 
 namespace fbla {
@@ -23,18 +24,6 @@ __global__ void __launch_bounds__(32 * RefineShape<CB, FB>::WARPS, 1) refine_ker
 template <int QG>
 __global__ void __launch_bounds__(512, 2) merge_kernel(const fbla_k_decode a) {
   merge_item<QG>(a, nullptr);
-}
-
-// a launch that may begin while the previous kernel of the stream still runs (the kernel calls wait_previous_pass)
-template <class... P, class... A>
-cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 namespace {
@@ -77,14 +66,14 @@ template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a,
     else if (a.deal == FBLA_K_DEAL_FIXED) coarse_kernel<CB, FB, QG, FBLA_K_DEAL_FIXED><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
     else coarse_kernel<CB, FB, QG, FBLA_K_DEAL_COST><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = launch_dependent(select_kernel<QG>, dim3(a.phase == 1 ? 1 : a.nslices, vheads), dim3(256), 0, stream, a);
+    if (e == cudaSuccess) e = launch(true, 1, select_kernel<QG>, dim3(a.phase == 1 ? 1 : a.nslices, vheads), 256, 0, stream, a);
     if (a.phase == 1) return e;
   } else {
     select_kernel<QG><<<dim3(a.nslices, vheads), 256, 0, stream>>>(a);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = launch_dependent(refine_kernel<CB, FB, QG>, dim3(a.refine_ctas), dim3(32 * RefineShape<CB, FB>::WARPS), rsm, stream, a);
-  if (e == cudaSuccess) e = launch_dependent(merge_kernel<QG>, dim3(vheads * QG), dim3(512), 0, stream, a);
+  if (e == cudaSuccess) e = launch(true, 1, refine_kernel<CB, FB, QG>, dim3(a.refine_ctas), 32 * RefineShape<CB, FB>::WARPS, rsm, stream, a);
+  if (e == cudaSuccess) e = launch(true, 1, merge_kernel<QG>, dim3(vheads * QG), 512, 0, stream, a);
   return e;
 }
 

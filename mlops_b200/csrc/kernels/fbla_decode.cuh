@@ -235,11 +235,6 @@ __device__ __forceinline__ Split split_of(const fbla_k_decode &a, int hpr) {
   return Split{total - xw, xw};
 }
 
-// Programmatic dependent launch: the next pass of a decode is launched while this one still runs (hiding its launch
-// latency) and waits here until the previous pass has completed and its writes are visible.
-__device__ __forceinline__ void wait_previous_pass() { if (FBLA_STREAM_LAUNCH) asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allow_next_pass() { if (FBLA_STREAM_LAUNCH) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 __device__ __forceinline__ void report(const fbla_k_decode &a, int pass) {
   if (a.status) { atomicCAS(a.status, 0, pass); a.status[1] = FBLA_POS::x(); }
 }

@@ -1,5 +1,6 @@
 // Launchers of the dense decode (bodies: fbla_dense.cuh).
 #include "fbla_dense.cuh"
+#include "fbla_launch.h"
 #include <stdio.h>
 
 namespace fbla {
@@ -26,18 +27,6 @@ __global__ void __launch_bounds__(128) gather_kernel(const fbla_k_decode a) {
   gather_item<QG>(a, nullptr);
 }
 
-// a launch that may begin while the previous kernel of the stream still runs (the kernel calls wait_previous_pass)
-template <class... P, class... A>
-cudaError_t launch(bool dependent, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int CB, int FB, int QG> struct Kernels {
   static constexpr size_t SCORE_SMEM = sizeof(ScoreSmem), VALUE_SMEM = sizeof(ValueSmem<CB, FB>);
   static cudaError_t configure() {  // once per device and host thread
@@ -53,10 +42,10 @@ template <int CB, int FB, int QG> struct Kernels {
   static cudaError_t pass(const fbla_k_decode &a, int which, bool dependent, cudaStream_t stream) {
     const int vheads = a.batch * a.kv_heads * a.vg;
     switch (which) {
-      case 0: return launch(dependent, score_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * SCORE_WARPS, SCORE_SMEM, stream, a);
-      case 1: return launch(dependent, mass_kernel<QG>, dim3((vheads + 7) / 8), 256, 0, stream, a);
-      case 2: return launch(dependent, value_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * VALUE_WARPS, VALUE_SMEM, stream, a);
-      case 3: return launch(dependent, gather_kernel<QG>, dim3(vheads * QG), 128, 0, stream, a);
+      case 0: return launch(dependent, 1, score_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * SCORE_WARPS, SCORE_SMEM, stream, a);
+      case 1: return launch(dependent, 1, mass_kernel<QG>, dim3((vheads + 7) / 8), 256, 0, stream, a);
+      case 2: return launch(dependent, 1, value_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * VALUE_WARPS, VALUE_SMEM, stream, a);
+      case 3: return launch(dependent, 1, gather_kernel<QG>, dim3(vheads * QG), 128, 0, stream, a);
     }
     return cudaErrorInvalidValue;
   }

@@ -53,6 +53,11 @@ constexpr float MAGICF = 12582912.f;
 
 __host__ __device__ constexpr int record_bytes(int bits) { return 2 * bits * 256; }
 
+// Programmatic dependent launch: the next kernel of a call is launched while this one still runs (hiding its launch
+// latency) and waits here until the previous pass has completed and its writes are visible.
+__device__ __forceinline__ void wait_previous_pass() { if (FBLA_STREAM_LAUNCH) asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_pass() { if (FBLA_STREAM_LAUNCH) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- scalar helpers -------------------------------------------------------------------------------------------
 __device__ __forceinline__ float bf16_to_f32(uint16_t x) { return __uint_as_float((uint32_t)x << 16); }
 __device__ __forceinline__ uint16_t f32_to_bf16(float x) {  // round to nearest even, NaN canonical
@@ -155,6 +160,33 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(dst_smem)), "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+// ---- thread-block cluster (stream launches only) --------------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_meet() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the float(s) at this CTA's shared address p, in the cluster's CTA `rank`
+__device__ __forceinline__ uint32_t remote(const void *p, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 ld_remote4(uint32_t p) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_remote2(uint32_t p) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_remote1(uint32_t p) {
+  int v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+  return v;
 }
 
 __device__ __forceinline__ uint32_t lds32(const uint8_t *p) { return *reinterpret_cast<const uint32_t *>(p); }

@@ -146,8 +146,9 @@ typedef struct {
   // > 0 (a chunk that starts a cache whose arrays have no initial contents): the groups per KV head that the layout has
   // room for; what the chunk does not write of their units and of the sink window is zeroed (fbla_k_write_launch)
   int clear_groups;
+  int early;    // 1: the close pass also updates the windows of a chunk that starts its cache (nothing reads them then), the finish pass leaves that to it
   int room;     // tokens the cache is laid out for
-  int cluster;  // few-row pass: CTAs per tile, one per share of its groups (fbla_prefill_rows.cuh); 1: a CTA takes all shares
+  int cluster;  // attention passes: CTAs of a tile's cluster, one per share of its groups (1: one CTA does the tile)
 } fbla_k_prefill;
 
 // close_blocks: grid x of the close pass (groups the chunk can close); 0 skips it
@@ -167,6 +168,7 @@ FBLA_HOST_API(cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaS
 // error. A CTA whose wait gave up also writes NaN to every output row it owns, so the failure shows in the data.
 FBLA_HOST_API(int fbla_k_attend_tc_status(void);)
 #define FBLA_K_TC_MIN_ROWS 64
+#define FBLA_K_TILE_SHARES 8  /* CTAs of a tensor-core tile's cluster at most */
 #define FBLA_K_ROW_SHARES 8  /* CTAs of a few-row tile's cluster at most */
 
 // ---- fused QKV step: RMSNorm + rotary embedding of new tokens (+ the window stores of the one-token step) ------------------
@@ -199,7 +201,7 @@ FBLA_HOST_API(cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pas
 FBLA_HOST_API(cudaError_t fbla_k_close_pass(const fbla_k_prefill *a, int close_blocks, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_finish_pass(const fbla_k_prefill *a, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_attend_rows_pass(fbla_k_prefill *a, fbla_k_pass *info);)  // (sets a->cluster)
-FBLA_HOST_API(cudaError_t fbla_k_attend_tc_pass(const fbla_k_prefill *a, fbla_k_pass *info);)
+FBLA_HOST_API(cudaError_t fbla_k_attend_tc_pass(fbla_k_prefill *a, fbla_k_pass *info);)    // (sets a->cluster)
 FBLA_HOST_API(cudaError_t fbla_k_qkv_token_pass(const fbla_k_token *a, fbla_k_pass *info);)
 FBLA_HOST_API(cudaError_t fbla_k_qkv_chunk_pass(const fbla_k_token *a, fbla_k_pass *info);)
 

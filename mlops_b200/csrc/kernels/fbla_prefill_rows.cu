@@ -1,11 +1,14 @@
 // Launcher of the few-row prefill attention (body: fbla_prefill_rows.cuh).
 #include "fbla_prefill_rows.cuh"
+#include "fbla_launch.h"
 #include <stdio.h>
 
 namespace fbla {
 template <int CB, int FB>
 __global__ void __launch_bounds__(32 * rows::WARPS, 1) attend_rows_kernel(const fbla_k_prefill a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
+  wait_previous_pass();
+  allow_next_pass();
   attend_rows_item<CB, FB>(a, smem_raw);
 }
 
@@ -19,13 +22,7 @@ template <int CB, int FB> static cudaError_t launch_rows(const fbla_k_prefill &a
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * a.cluster, a.batch * a.kv_heads); cfg.blockDim = dim3(32 * rows::WARPS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = a.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = a.cluster > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, attend_rows_kernel<CB, FB>, a);
+  return launch(true, a.cluster, attend_rows_kernel<CB, FB>, dim3(tiles * a.cluster, a.batch * a.kv_heads), 32 * rows::WARPS, smem, stream, a);
 }
 
 // tiles of the launch: with a device count that goes to the tensor-core pass from tc_min_rows rows on, no more than it leaves here

@@ -57,32 +57,6 @@ template <int CB, int FB> struct RowSmem {
 static_assert(sizeof(RowSmem<3, 3>) + 128 <= 227 * 1024 && sizeof(RowSmem<4, 2>) + 128 <= 227 * 1024, "one CTA's shared memory");
 static_assert(SET * sizeof(float) + sizeof(RowStage) <= sizeof(RowWarp<4, 2>::pair) && SET * sizeof(float) + sizeof(RowStage) <= sizeof(RowWarp<3, 3>::pair), "row set and staging fit the ring");
 
-// ---- thread-block cluster (stream launches only) --------------------------------------------------------------------------------
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the float(s) at this CTA's shared address p, in the cluster's CTA `rank`
-__device__ __forceinline__ uint32_t remote(const void *p, int rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ float4 ld_remote4(uint32_t p) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float2 ld_remote2(uint32_t p) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ int ld_remote1(uint32_t p) {
-  int v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
-  return v;
-}
-
 // scores of one sub-block under both planes: code units = 2^FB h + f; thread (gid, tig): tokens gid (x[0]), gid + 8 (x[1]) of rows 2 tig, 2 tig + 1
 template <int CB, int FB>
 __device__ __forceinline__ void qk_full(const uint8_t *crec, const uint8_t *frec, int gid, int tig, const uint32_t (&B)[8], float2 (&x)[2]) {

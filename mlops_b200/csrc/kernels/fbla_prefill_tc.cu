@@ -1,5 +1,6 @@
 // Launchers of the tensor-core prefill attention (body: fbla_prefill_tc.cuh).
 #include "fbla_prefill_tc.cuh"
+#include "fbla_launch.h"
 #include <stdlib.h>
 #include <string.h>
 #include <stdio.h>
@@ -17,10 +18,12 @@ template <class K> cudaError_t pass_of(K kernel, int gx, int gy, int threads, si
 
 namespace fbla {
 namespace tc {
-template <int CB, int FB>
+template <int CB, int FB, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) attend_tc_kernel(const fbla_k_prefill a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  attend_tc_item<CB, FB>(a, smem_raw);
+  wait_previous_pass();
+  allow_next_pass();
+  attend_tc_item<CB, FB, SPLIT>(a, smem_raw);
 }
 }  // namespace tc
 }  // namespace fbla
@@ -34,21 +37,26 @@ extern "C" int fbla_k_attend_tc_status(void) {
 
 extern "C" cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaStream_t stream) {
   using namespace fbla::tc;
-  const int qg = a->q_heads / a->kv_heads;
-  const dim3 grid((a->count * qg + CTA_ROWS - 1) / CTA_ROWS, a->batch * a->kv_heads);
+  const int tiles = (a->count * (a->q_heads / a->kv_heads) + CTA_ROWS - 1) / CTA_ROWS, heads = a->batch * a->kv_heads;
   const size_t smem = sizeof(Smem) + 1024;
   static thread_local int configured[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attend_tc_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attend_tc_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    for (auto kernel : {attend_tc_kernel<3, 3, false>, attend_tc_kernel<3, 3, true>, attend_tc_kernel<4, 2, false>, attend_tc_kernel<4, 2, true>}) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  if (a->cb == 3) attend_tc_kernel<3, 3><<<grid, THREADS, smem, stream>>>(*a);
-  else attend_tc_kernel<4, 2><<<grid, THREADS, smem, stream>>>(*a);
-  return cudaGetLastError();
+  fbla_k_prefill args = *a;
+  // (device lengths: room for as many shares as a chunk of the ceiling's size can have at the end of the cache)
+  args.cluster = tile_shares((long long)tiles * heads, ((a->length ? a->room : a->n0 + a->count) - 1) / fbla::G + 1, FBLA_K_TILE_SHARES);
+  const bool split = args.cluster > 1;
+  const auto kernel = a->cb == 3 ? split ? attend_tc_kernel<3, 3, true> : attend_tc_kernel<3, 3, false> : split ? attend_tc_kernel<4, 2, true> : attend_tc_kernel<4, 2, false>;
+  // launched dependent where one wave holds the grid (a 777-token prompt 69.5 -> 67.8 us); several waves that began among the
+  // CTAs of the kernel before measured 3 % slower (batch 4 x 8192 4.55 -> 4.69 ms)
+  return fbla::launch(tiles * args.cluster * heads <= 148, args.cluster, kernel, dim3(tiles * args.cluster, heads), THREADS, smem, stream, args);
 }
 
 extern "C" int fbla_k_attend_plan(const fbla_k_prefill *a, fbla_k_prefill args[2], int tensor[2]) {
@@ -74,10 +82,11 @@ extern "C" cudaError_t fbla_k_attend_launch(const fbla_k_prefill *a, cudaStream_
   return e;
 }
 
-extern "C" cudaError_t fbla_k_attend_tc_pass(const fbla_k_prefill *a, fbla_k_pass *info) {
+extern "C" cudaError_t fbla_k_attend_tc_pass(fbla_k_prefill *a, fbla_k_pass *info) {
   using namespace fbla::tc;
+  a->cluster = 1;
   const int qg = a->q_heads / a->kv_heads, rows = a->count * qg, heads = a->batch * a->kv_heads;
   const size_t smem = sizeof(Smem) + 1024;
-  if (a->cb == 3) return pass_of(attend_tc_kernel<3, 3>, (rows + CTA_ROWS - 1) / CTA_ROWS, heads, THREADS, smem, "fbla::tc::attend_tc_item<3, 3>", info);
-  return pass_of(attend_tc_kernel<4, 2>, (rows + CTA_ROWS - 1) / CTA_ROWS, heads, THREADS, smem, "fbla::tc::attend_tc_item<4, 2>", info);
+  if (a->cb == 3) return pass_of(attend_tc_kernel<3, 3, false>, (rows + CTA_ROWS - 1) / CTA_ROWS, heads, THREADS, smem, "fbla::tc::attend_tc_item<3, 3>", info);
+  return pass_of(attend_tc_kernel<4, 2, false>, (rows + CTA_ROWS - 1) / CTA_ROWS, heads, THREADS, smem, "fbla::tc::attend_tc_item<4, 2>", info);
 }

@@ -64,6 +64,7 @@ struct __align__(1024) Smem {
   float qbias[2][8][2][128];  // [eight passes, alternating][pass][tile][row]: the score bias sl q . base, formed for eight groups at once
   float ex2[2][128][2];  // exchange between the two threads of a row: pass maximum, final sum
   uint64_t bar_k, bar_v, bar_q[2], bar_s[2], bar_p[2], bar_o[2];
+  float2 part[2 * ROWS];   // (m, l) of this CTA's share of every row
   uint32_t tmem_base;
   int abort;
 };
@@ -81,6 +82,18 @@ __device__ __forceinline__ bool wait(Smem &sm, uint64_t *bar, uint32_t parity) {
   *reinterpret_cast<volatile int *>(&sm.abort) = 1;
   atomicExch(&g_status, 1);
   return false;
+}
+
+// ---- splitting a tile's passes over a thread-block cluster -----------------------------------------------------------------
+// Few tiles over a long cache leave most SMs idle, and a CTA walks its groups one after the other. Then the passes of a tile
+// are split into equal runs, one CTA of a cluster each, whose (m, l, O) are merged over distributed shared memory. As many
+// as keep a run at twelve passes or more (the merge costs about three) while all clusters still fit the SMs at once -- 148,
+// less what clusters of that size waste of them. 500 tokens at 30 000 (4 / 2 heads, 3+3): 999 -> 158 us.
+__host__ __device__ inline int tile_shares(long long tiles, int passes, int most) {
+  int c = passes / 12;
+  c = c > most ? most : c;
+  while (c > 1 && tiles * c > 148 - 8 * (c - 1)) --c;
+  return c < 1 ? 1 : c;
 }
 
 // V' tile row (= O column) of channel ch: 32 (ch % 4) + ch / 4, so that the 32 lanes of a record (4 channels each) write
@@ -178,7 +191,9 @@ __device__ __forceinline__ void exact_v(uint8_t *tile, const TokenRows rows, int
   }
 }
 
-template <int CB, int FB>
+// SPLIT: a cluster per tile (one build per way: the loops of the other one would carry the share's bounds in registers they lack,
+// 9 % of the time at batch 4 x 8192)
+template <int CB, int FB, bool SPLIT = false>
 __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
   smem_raw += (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // (an offset, not a rebuilt pointer: the address space stays known)
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
@@ -188,13 +203,20 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
   const int n0 = (a.length ? FBLA_POS::ro(a.length + (a.lstride ? b : 0)) : 0) + a.n0;
   const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, n1 = n0 + count;
   // the last tiles attend to the most groups: they are taken first, so that the grid's tail is made of short CTAs
-  const int rows = count * qg, r0 = (FBLA_POS::nx() - 1 - FBLA_POS::x()) * CTA_ROWS;
+  const int cluster = SPLIT ? a.cluster : 1, rank = SPLIT ? FBLA_POS::x() % cluster : 0;
+  const int rows = count * qg, r0 = (FBLA_POS::nx() / cluster - 1 - FBLA_POS::x() / cluster) * CTA_ROWS;
   if (r0 >= rows || rows < a.tc_min_rows) return;  // (CTA-uniform; a short device count is the few-row pass's work)
   const int last_row = min(r0 + CTA_ROWS, rows) - 1;
   const int own_min = (n0 + r0 / qg) / G, own_max = (n0 + last_row / qg) / G;
   // passes: closed groups 1 .. own_max - 1, then the BF16 groups: 0 and the rows' own groups
   const int n_closed = max(own_max - 1, 0), own_lo = max(own_min, 1);
   const int n_pass = n_closed + 1 + max(own_max - own_lo + 1, 0);
+  // this CTA's share of them: passes [p_lo, p_hi), of which [p_lo, c_hi) closed, [x_lo, p_hi) BF16
+  const int shares = SPLIT ? tile_shares((long long)((rows + CTA_ROWS - 1) / CTA_ROWS) * a.batch * a.kv_heads, (n1 - 1) / G + 1, cluster) : 1;
+  if (shares == 1 && rank > 0) return;  // (the same for every CTA of the grid: nobody then meets its cluster)
+  const int p_lo = !SPLIT ? 0 : rank < shares ? (int)((long long)n_pass * rank / shares) : n_pass;
+  const int p_hi = !SPLIT || rank >= shares ? n_pass : (int)((long long)n_pass * (rank + 1) / shares);
+  const int c_hi = SPLIT ? min(n_closed, p_hi) : n_closed, x_lo = SPLIT ? max(n_closed, p_lo) : n_closed;
   auto pass_group = [&](int n, bool &closed) {
     closed = n < n_closed;
     return closed ? 1 + n : n == n_closed ? 0 : own_lo + (n - n_closed - 1);
@@ -225,7 +247,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
     // execute in the order they are issued, so S(n + 1, x) overwrites P'(n, x) only after O(n, x) has read it.
     if (lane == 0) {
       auto scores = [&](int n, int x) -> bool {
-        if (!wait(sm, &sm.bar_q[x], n & 1)) return false;
+        if (!wait(sm, &sm.bar_q[x], (n - p_lo) & 1)) return false;
         tc_fence_after();
         const bool closed = n < n_closed;
         const uint8_t *qop = closed ? sm.qp[x] : sm.q[x];
@@ -236,18 +258,18 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
         return true;
       };
       auto values = [&](int n, int x) -> bool {
-        if (!wait(sm, &sm.bar_p[x], n & 1)) return false;
+        if (!wait(sm, &sm.bar_p[x], (n - p_lo) & 1)) return false;
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // P' of token block kk: eight columns inside the tile's S columns (see the softmax threads)
-          mma_f16_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (kk >> 2) + 8 * (kk & 3), smem_desc(sm.v, kk >> 2, kk & 3), IDESC_F16, n > 0 || kk > 0);
+          mma_f16_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (kk >> 2) + 8 * (kk & 3), smem_desc(sm.v, kk >> 2, kk & 3), IDESC_F16, n > p_lo || kk > 0);
         mma_commit(&sm.bar_o[x]);
         return true;
       };
       bool ok = true;
-      for (int n = 0; n < n_pass && ok; ++n)
-        ok = wait(sm, &sm.bar_k, n & 1) && scores(n, 0) && (n == 0 || values(n - 1, 1)) && scores(n, 1) && wait(sm, &sm.bar_v, n & 1) && values(n, 0);
-      if (ok) values(n_pass - 1, 1);
+      for (int n = p_lo; n < p_hi && ok; ++n)
+        ok = wait(sm, &sm.bar_k, (n - p_lo) & 1) && scores(n, 0) && (n == p_lo || values(n - 1, 1)) && scores(n, 1) && wait(sm, &sm.bar_v, (n - p_lo) & 1) && values(n, 0);
+      if (ok && (!SPLIT || p_lo < p_hi)) values(p_hi - 1, 1);
     }
   } else if (warp >= PRODUCER_WARP0) {
     // ================= operand producers =================
@@ -263,14 +285,14 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
         load_lane<FB>(a.c.fine + (unit * SBG + j0 + PRODUCERS * i) * RF, tensor, l, Wf[i]);
       }
     };
-    if (n_closed > 0) load(1, 0);
+    if (p_lo < c_hi) load(1 + p_lo, 0);
     bool ok = true;
     // Kop is free once both tiles' S of the previous pass are complete, V' once both tiles' O products are
-    auto free_k = [&](int n) { return n == 0 || (wait(sm, &sm.bar_s[0], (n - 1) & 1) && wait(sm, &sm.bar_s[1], (n - 1) & 1)); };
-    auto free_v = [&](int n) { return n == 0 || (wait(sm, &sm.bar_o[0], (n - 1) & 1) && wait(sm, &sm.bar_o[1], (n - 1) & 1)); };
+    auto free_k = [&](int n) { return n == p_lo || (wait(sm, &sm.bar_s[0], (n - 1 - p_lo) & 1) && wait(sm, &sm.bar_s[1], (n - 1 - p_lo) & 1)); };
+    auto free_v = [&](int n) { return n == p_lo || (wait(sm, &sm.bar_o[0], (n - 1 - p_lo) & 1) && wait(sm, &sm.bar_o[1], (n - 1 - p_lo) & 1)); };
     auto done = [&](uint64_t *bar) { fence_async_smem(); mbar_arrive(bar); };
 #pragma unroll 1
-    for (int n = 0; n < n_closed; ++n) {
+    for (int n = p_lo; n < c_hi; ++n) {
       const int g = 1 + n;
       if (!(ok = free_k(n))) break;
       const uint4 vm = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(a.c.meta) + (head + (size_t)g * a.gs) * 1024 + 512) + l);
@@ -307,11 +329,11 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
           *reinterpret_cast<uint4 *>(chunk_at(sm.v, 32 * cc + l, 16 * j + 8)) = make_uint4(h[4], h[5], h[6], h[7]);
         }
       }
-      if (n + 1 < n_closed) load(g + 1, 0);
+      if (n + 1 < c_hi) load(g + 1, 0);
       done(&sm.bar_v);
     }
 #pragma unroll 1
-    for (int n = n_closed; n < n_pass && ok; ++n) {
+    for (int n = x_lo; n < p_hi && ok; ++n) {
       bool closed;
       const int t0 = pass_group(n, closed) * G;
       if (!(ok = free_k(n))) break;
@@ -334,6 +356,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
 #pragma unroll
       for (int it = 0; it < 8; ++it) {
         const int Rq = r0 + ROWS * X + qrow0 + 2 * it;
+        if (SPLIT && p_lo >= p_hi) continue;  // (a share without passes: the memory takes its row sums)
         uint4 w = make_uint4(0u, 0u, 0u, 0u);
         if (Rq < rows) {
           const int iq = Rq / qg;
@@ -355,12 +378,12 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
       ma = __ldcg(reinterpret_cast<const uint4 *>(meta + (size_t)g * a.gs * 1024));
       mb = __ldcg(reinterpret_cast<const uint4 *>(meta + (size_t)g * a.gs * 1024 + 16));
     };
-    if (n_closed > 0) load_meta(1);
+    if (p_lo < c_hi) load_meta(1 + p_lo);
     __syncwarp();  // (the warp's own rows of the q tiles are in place)
 #pragma unroll 1
-    for (int n = 0; n < n_closed; ++n) {
-      const int g = 1 + n;
-      if (!(n & 7)) {  // the biases of groups g .. g + 7 (those past the last: repeated, unused)
+    for (int n = p_lo; n < c_hi; ++n) {
+      const int g = 1 + n, k = n - p_lo;
+      if (!(k & 7)) {  // the biases of groups g .. g + 7 (those past the last: repeated, unused)
         const uint8_t *base = reinterpret_cast<const uint8_t *>(a.c.meta) + (head + (size_t)min(g + (lane >> 2), n_closed) * a.gs) * 1024 + 16 * ((lane & 3) >> 1) + 4 * (lane & 1);
 #pragma unroll 1
         for (int X = 0; X < 2; ++X) {
@@ -373,16 +396,16 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
             mma_bf16_k16(d, q4[0], q4[1], q4[2], q4[3], __ldcg(reinterpret_cast<const uint32_t *>(base + 64 * kk)), __ldcg(reinterpret_cast<const uint32_t *>(base + 64 * kk + 32)));
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) sm.qbias[(n >> 3) & 1][2 * (lane & 3) + (i & 1)][X][16 * qw + (lane >> 2) + 8 * (i >> 1)] = __fmul_rn(d[i], a.sl);
+          for (int i = 0; i < 4; ++i) sm.qbias[(k >> 3) & 1][2 * (lane & 3) + (i & 1)][X][16 * qw + (lane >> 2) + 8 * (i >> 1)] = __fmul_rn(d[i], a.sl);
         }
       }
       const float4 s0 = make_float4(bf_lo(ma.z), bf_hi(ma.z), bf_lo(ma.w), bf_hi(ma.w));
       const float4 s1 = make_float4(bf_lo(mb.z), bf_hi(mb.z), bf_lo(mb.w), bf_hi(mb.w));
-      if (n + 1 < n_closed) load_meta(g + 1);
+      if (n + 1 < c_hi) load_meta(g + 1);
 #pragma unroll 1
       for (int X = 0; X < 2; ++X) {
         // the tile's qhat buffer is free once the S product of the pass before is complete
-        if (n > 0) wait(sm, &sm.bar_s[X], (n - 1) & 1);
+        if (k > 0) wait(sm, &sm.bar_s[X], (k - 1) & 1);
         if (g < tile_own[X]) {
           // z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16. First sweep: the lane's shares of max |z| for
           // its eight rows; a butterfly over a row's 16 lanes that hands half of the rows on in
@@ -421,7 +444,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
           }
           const float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 1));
           const float rq = quotient_127(am);
-          if (!(lane & 1)) sm.qscale[n & 1][X][qrow0 + (lane & 14)] = __fmul_rn(am, sl127);  // (row qrow0 + 2 it)
+          if (!(lane & 1)) sm.qscale[k & 1][X][qrow0 + (lane & 14)] = __fmul_rn(am, sl127);  // (row qrow0 + 2 it)
 #pragma unroll 1
           for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -439,11 +462,11 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
         mbar_arrive(&sm.bar_q[X]);
       }
     }
-    if (n_closed == 0) fence_async_smem();  // (the q tiles, otherwise covered by the first pass's)
+    if (p_lo >= c_hi) fence_async_smem();  // (the q tiles, otherwise covered by the first pass's)
 #pragma unroll 1
-    for (int n = n_closed; n < n_pass; ++n)  // BF16 passes take the q tiles as they are
+    for (int n = x_lo; n < p_hi; ++n)  // BF16 passes take the q tiles as they are
       for (int X = 0; X < 2; ++X) {
-        if (n > 0) wait(sm, &sm.bar_s[X], (n - 1) & 1);
+        if (n > p_lo) wait(sm, &sm.bar_s[X], (n - 1 - p_lo) & 1);
         mbar_arrive(&sm.bar_q[X]);
       }
   } else {
@@ -458,18 +481,18 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
     float m_run = -FBLA_INF, l_run = 0.f;  // l_run: this thread's tokens only
     const int R = r0 + ROWS * X + r, pos = R < rows ? n0 + R / qg : -1, own = pos / G;  // pos -1: the tile has no such row
     bool ok = true;
-    for (int n = 0; n < n_pass; ++n) {
+    for (int n = p_lo; n < p_hi; ++n) {
       bool closed;
-      const int g = pass_group(n, closed);
+      const int g = pass_group(n, closed), k = n - p_lo;
       {
         const bool include = pos >= 0 && (closed ? g < own : (g == 0 || g == own));
         const bool any = __any_sync(FULL, include);
         // S(n) is complete, and with it every product issued before: O of the tile's pass n - 1 is stable
-        ok &= __all_sync(FULL, wait(sm, &sm.bar_s[X], n & 1));
+        ok &= __all_sync(FULL, wait(sm, &sm.bar_s[X], k & 1));
         tc_fence_after();
         // softmax of the row over the pass's 128 tokens, by 16-token blocks; P' = fp16(2^(m_block - m_row) p)
         const int lim = (include ? (closed ? G : pos - g * G) : -1) - 64 * hf;  // this thread's tokens 0 .. lim are attended
-        const float mul1 = closed ? sm.qscale[n & 1][X][r] : a.sl, add1 = closed ? sm.qbias[(n >> 3) & 1][n & 7][X][r] : 0.f;  // score = mul x + add, monotonic in x (mul >= 0)
+        const float mul1 = closed ? sm.qscale[k & 1][X][r] : a.sl, add1 = closed ? sm.qbias[(k >> 3) & 1][k & 7][X][r] : 0.f;  // score = mul x + add, monotonic in x (mul >= 0)
         // sweep 1: the block maxima, from the raw sums (each block's columns are asked for while the one before is worked on)
         float mbk[4];
         uint32_t xa[16], xb[16];
@@ -509,7 +532,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
           const bool need = mp > m_run + 8.f;
           if (__any_sync(FULL, need)) {
             const float al = need ? ex2(m_run - mp) : 1.f;  // 0 on the row's first attended block
-            if (n > 0) {
+            if (k > 0) {
 #pragma unroll 1
               for (int oc = 0; oc < 2; ++oc) {
                 uint32_t o[32];
@@ -563,14 +586,31 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
       }
     }
     {
-      ok &= __all_sync(FULL, wait(sm, &sm.bar_o[X], (n_pass - 1) & 1));
+      if (!SPLIT || p_lo < p_hi) ok &= __all_sync(FULL, wait(sm, &sm.bar_o[X], (p_hi - 1 - p_lo) & 1));
       tc_fence_after();
       pair_sync();  // (the partner has read the last pass's exchange)
       sm.ex2[X][r][hf] = l_run;
       pair_sync();
+      const float l_row = sm.ex2[X][r][0] + sm.ex2[X][r][1];
+      if (SPLIT && shares > 1) {
+        // This share's sums for the cluster: O as it lies in tensor memory, 16-byte piece c of row r at c ^ (r % 32), over the
+        // query tiles (every product has read them: the O products were issued last); (m, l) beside them.
+        float *const row = reinterpret_cast<float *>(sm.q[0]) + (size_t)(ROWS * X + r) * D;
+        if (hf == 0) sm.part[ROWS * X + r] = make_float2(m_run, l_row);
+#pragma unroll 1
+        for (int cu = 0; cu < 2; ++cu) {
+          uint32_t o[32];
+          if (p_lo < p_hi) tmem_ld32(tmem_o + 32 * cu, o);
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<uint4 *>(row + 4 * ((16 * hf + 8 * cu + c) ^ (r & 31))) =
+                p_lo < p_hi ? make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (!ok) *reinterpret_cast<volatile int *>(&sm.abort) = 1;
+      } else {
       // O column 32 cc + l is channel 4 l + cc: through the row's (now free) qhat row as BF16 in channel order, then out.
       // This thread: O columns 64 hf .. + 63 (cc = 2 hf, 2 hf + 1); then it copies chunks 8 hf .. + 7 of the row.
-      const float inv = 1.f / (sm.ex2[X][r][0] + sm.ex2[X][r][1]);
+      const float inv = 1.f / l_row;
       uint16_t *stage = reinterpret_cast<uint16_t *>(sm.qp[X] + r * 256);  // 256 bytes per row, private to the pair
 #pragma unroll 1
       for (int cu = 0; cu < 2; ++cu) {
@@ -590,6 +630,39 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
         for (int c = 8 * hf; c < 8 * hf + 8; ++c) reinterpret_cast<uint4 *>(orow)[c] = ok ? reinterpret_cast<const uint4 *>(stage)[c ^ (r & 15)] : nan4;
       }
     }
+    }
+  }
+  if (SPLIT && shares > 1) {
+    // the cluster's CTAs merge the tiles' rows: this one rows rank, rank + shares, ... in 16-byte pieces of the output
+    cluster_meet();
+    if (rank < shares) {
+      for (int e = tid; e < (2 * ROWS / shares + 1) * (D / 8); e += THREADS) {
+        const int rr = rank + shares * (e / (D / 8)), c8 = e % (D / 8), R = r0 + rr;  // channels 8 c8 ..: columns 32 cc + 2 c8, + 1
+        if (rr >= 2 * ROWS || R >= rows) continue;
+        float M = -FBLA_INF, L = 0.f;
+        float2 o[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // [cc]: channels 8 c8 + cc, + 4
+        bool failed = false;
+        for (int s = 0; s < shares; ++s) {
+          const float2 ml = ld_remote2(remote(&sm.part[rr], s));
+          const float mn = fmaxf(M, ml.x), sa = M == -FBLA_INF ? 0.f : ex2(M - mn), sb = ml.x == -FBLA_INF ? 0.f : ex2(ml.x - mn);
+          M = mn;
+          L = fmaf(sa, L, sb * ml.y);
+          failed |= ld_remote1(remote(&sm.abort, s)) != 0;
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) {
+            const int col = 32 * cc + 2 * c8;
+            const float2 y = ld_remote2(remote(reinterpret_cast<float *>(sm.q[0]) + (size_t)rr * D + 4 * ((col >> 2) ^ (rr & 31)) + (col & 3), s));
+            o[cc] = make_float2(fmaf(sa, o[cc].x, sb * y.x), fmaf(sa, o[cc].y, sb * y.y));
+          }
+        }
+        const float inv = failed ? __int_as_float(0x7fc00000) : 1.f / L;
+        const int i = R / qg, hq = kh * qg + (R - i * qg);
+        auto pack = [&](float x, float y) { return f32_to_bf16(x * inv) | (uint32_t)f32_to_bf16(y * inv) << 16; };
+        reinterpret_cast<uint4 *>(a.out + (size_t)(b * a.q_heads + hq) * a.out_hs + (size_t)i * a.out_ts)[c8] =
+            make_uint4(pack(o[0].x, o[1].x), pack(o[2].x, o[3].x), pack(o[0].y, o[1].y), pack(o[2].y, o[3].y));
+      }
+    }
+    cluster_meet();  // (nobody leaves while its shared memory is being read)
   }
   tc_fence_before();
   __syncthreads();

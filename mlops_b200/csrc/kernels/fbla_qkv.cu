@@ -1,7 +1,7 @@
 // Launchers of the fused QKV step (bodies: fbla_qkv.cuh).
 #include "fbla_qkv.cuh"
 #include "fbla_close.cuh"
-#include "fbla_decode.cuh"
+#include "fbla_launch.h"
 #include <stdio.h>
 
 namespace {
@@ -37,6 +37,8 @@ __global__ void __launch_bounds__(CLOSE_THREADS) qkv_step_kernel(const fbla_k_pr
 
 template <bool NORM>
 __global__ void __launch_bounds__(256) qkv_chunk_kernel(const fbla_k_token a) {
+  wait_previous_pass();
+  allow_next_pass();
   qkv_chunk_item<NORM>(a, nullptr);
 }
 }  // namespace fbla
@@ -50,13 +52,7 @@ template <int CB, int FB, bool NORM> static cudaError_t launch_step(const fbla_k
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a.batch * a.kv_heads); cfg.blockDim = dim3(fbla::CLOSE_THREADS); cfg.dynamicSmemBytes = sizeof(fbla::CloseSmem); cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fbla::qkv_step_kernel<CB, FB, NORM>, closing, a);
+  return fbla::launch(true, 1, fbla::qkv_step_kernel<CB, FB, NORM>, dim3(a.batch * a.kv_heads), fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream, closing, a);
 }
 extern "C" cudaError_t fbla_k_qkv_step_launch(const fbla_k_prefill *closing, const fbla_k_token *a, cudaStream_t stream) {
   if (closing->cb == 3) return a->q_norm ? launch_step<3, 3, true>(*closing, *a, stream) : launch_step<3, 3, false>(*closing, *a, stream);
@@ -65,9 +61,7 @@ extern "C" cudaError_t fbla_k_qkv_step_launch(const fbla_k_prefill *closing, con
 
 extern "C" cudaError_t fbla_k_qkv_chunk_launch(const fbla_k_token *a, cudaStream_t stream) {
   const dim3 grid((a->max_count + fbla::TOK - 1) / fbla::TOK, a->kv_heads);
-  if (a->q_norm) fbla::qkv_chunk_kernel<true><<<grid, 256, 0, stream>>>(*a);
-  else fbla::qkv_chunk_kernel<false><<<grid, 256, 0, stream>>>(*a);
-  return cudaGetLastError();
+  return fbla::launch(true, 1, a->q_norm ? fbla::qkv_chunk_kernel<true> : fbla::qkv_chunk_kernel<false>, grid, 256, 0, stream, *a);
 }
 
 extern "C" cudaError_t fbla_k_qkv_token_pass(const fbla_k_token *a, fbla_k_pass *info) {
