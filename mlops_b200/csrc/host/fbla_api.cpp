@@ -93,13 +93,15 @@ long long groups_of(long long tokens) { return (tokens + kGroup - 1) / kGroup; }
 // Byte offsets of the arrays fbla_kernels.h describes, in this order, inside the caller's scratch.
 struct ScratchMap {
   size_t lse, part, dpart, row_r, counts, items, item_off, status, bytes;
-  int nblocks, nslices;
+  int nblocks, nslices, sets;
 };
 // `shape`: the launch shape on the current device; `tokens`: what the layout has room for; extra_rows: partial rows per
 // virtual head beyond the shape's own (the per_head of the size query)
-ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_k_decode &shape, int extra_rows) {
+// two_sweeps false: the layout of the decode that needs no weights between its passes, for a scratch too small for the other one
+ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_k_decode &shape, int extra_rows, bool two_sweeps) {
   ScratchMap m{};
   const int ratio = c->q_heads / c->kv_heads, qg = queries_per_virtual_head(ratio);
+  m.sets = two_sweeps ? fbla_k_two_sets(c->batch, c->batch * c->kv_heads * (ratio / qg), shape.cb, c->capacity ? c->capacity : tokens) : 0;
   const size_t vheads = (size_t)c->batch * c->kv_heads * (ratio / qg);
   m.nblocks = (int)(groups_of(tokens) * kBlocksPerGroup);
   m.nslices = (m.nblocks + FBLA_K_SLICE - 1) / FBLA_K_SLICE;
@@ -111,7 +113,7 @@ ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_
   const size_t refine_rows = (size_t)shape.refine_ctas * shape.refine_warps + vheads;
   size_t at = 0;
   auto take = [&at](size_t bytes) { const size_t here = at; at += padded(bytes); return here; };
-  m.lse = take(vheads * m.nblocks * qg * sizeof(float));
+  m.lse = take(fbla_k_two_floats(vheads, m.nblocks, qg, m.sets) * sizeof(float));
   m.part = take(coarse_rows * row_bytes);
   m.dpart = take(refine_rows * row_bytes);
   m.row_r = take(vheads * qg * sizeof(float));
@@ -122,17 +124,19 @@ ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_
   m.bytes = at;
   return m;
 }
+// set while mlops_fbla_decode_static runs a decode: its scratch may be one that only the smaller layout fits
+thread_local bool g_small_scratch = false;
 // c->tokens here is the token count the LAYOUT is made for
 bool decode_shape_acceptable(const mlops_fbla_config *c) {
   if (!c || !heads_consistent(c) || !unit_strides_consistent(c)) return false;
   if (c->tokens <= 0 || c->tokens > kTokenLimit) return false;
   return c->capacity == 0 || c->capacity >= c->tokens;
 }
-size_t scratch_size(const mlops_fbla_config *layout, int extra_rows) {
+size_t scratch_size(const mlops_fbla_config *layout, int extra_rows, bool two_sweeps = true) {
   fbla_k_decode shape{};
   shape.cb = coarse_bits(layout);
   if (fbla_k_decode_shape(&shape) != cudaSuccess) return 0;
-  return map_scratch(layout, layout->tokens, shape, extra_rows).bytes;
+  return map_scratch(layout, layout->tokens, shape, extra_rows, two_sweeps).bytes;
 }
 
 // Checks a decode and fills the kernels' arguments. `length` non-null: a device-length call, laid out by cfg->capacity.
@@ -161,7 +165,8 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   a.fb = fine_bits(c);
   const cudaError_t shape_error = fbla_k_decode_shape(&a);
   if (shape_error != cudaSuccess) return device_failure(fn, shape_error);
-  const ScratchMap m = map_scratch(&layout, layout.tokens, a, 0);
+  ScratchMap m = map_scratch(&layout, layout.tokens, a, 0, true);
+  if (scratch_bytes < m.bytes && g_small_scratch) m = map_scratch(&layout, layout.tokens, a, 0, false);
   if (scratch_bytes < m.bytes) return refuse(fn, "the scratch is %zu bytes but this decode takes %zu", scratch_bytes, m.bytes);
   const int ratio = c->q_heads / c->kv_heads;
   a.qg = queries_per_virtual_head(ratio);
@@ -201,7 +206,7 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   const float usual = c->format == MLOPS_FBLA_3P3 ? 3e-4f : 1e-3f, threshold = c->tau != 0.f ? c->tau : usual;
   a.log2_tau = log2f(threshold);
   // (a shard's two phases share the scratch but only the second one uses tau: they decide by the format's own)
-  a.dense = (short)fbla_k_decode_dense(&a, room, wants_output ? threshold : usual);
+  a.dense = (short)fbla_k_two_mode(m.sets, room, wants_output ? threshold : usual);
   return MLOPS_FBLA_OK;
 }
 mlops_fbla_status enqueue_decode(const char *fn, fbla_k_decode &a, cudaStream_t stream) {
@@ -318,6 +323,16 @@ size_t mlops_fbla_decode_scratch_bytes_for(const mlops_fbla_config *c, int per_h
 mlops_fbla_status mlops_fbla_decode(const mlops_fbla_config *c, const uint16_t *q, const mlops_fbla_cache *k, uint16_t *out,
                                     void *scratch, size_t scratch_bytes, cudaStream_t stream) {
   return run_decode("mlops_fbla_decode", c, nullptr, q, k, out, scratch, scratch_bytes, stream);
+}
+
+// (for fbla_static.cu) the least scratch a decode runs with, and a decode in that much or more
+size_t fbla_host_least_scratch(const mlops_fbla_config *c) { return decode_shape_acceptable(c) && known_format(c) ? scratch_size(c, 0, false) : 0; }
+mlops_fbla_status fbla_host_decode_within(const mlops_fbla_config *c, const uint16_t *q, const mlops_fbla_cache *k, uint16_t *out, void *scratch,
+                                          size_t scratch_bytes, cudaStream_t stream) {
+  g_small_scratch = true;
+  const mlops_fbla_status st = mlops_fbla_decode(c, q, k, out, scratch, scratch_bytes, stream);
+  g_small_scratch = false;
+  return st;
 }
 
 mlops_fbla_status mlops_fbla_decode_at(const mlops_fbla_config *c, const int *length, const uint16_t *q, const mlops_fbla_cache *k,

@@ -27,6 +27,11 @@
 #include <cstdio>
 #include <mutex>
 
+// host/fbla_api.cpp
+extern "C" size_t fbla_host_least_scratch(const mlops_fbla_config *cfg);
+extern "C" mlops_fbla_status fbla_host_decode_within(const mlops_fbla_config *cfg, const uint16_t *q, const mlops_fbla_cache *cache, uint16_t *output,
+                                                     void *scratch, size_t scratch_bytes, cudaStream_t stream);
+
 #define FBLA_STATIC_SCRATCH_BYTES (32u << 20)
 
 static __device__ __align__(256) unsigned char fbla_static_scratch[FBLA_STATIC_SCRATCH_BYTES];
@@ -71,7 +76,7 @@ extern "C" const char *mlops_fbla_decode_static_error(void) { return g_error; }
 extern "C" mlops_fbla_status mlops_fbla_decode_static(const mlops_fbla_config *cfg, const uint16_t *q, const mlops_fbla_cache *cache,
                                                        uint16_t *output, cudaStream_t stream) {
   g_error[0] = 0;
-  const size_t need = mlops_fbla_decode_scratch_bytes(cfg);
+  const size_t need = fbla_host_least_scratch(cfg);
   if (need == 0) {
     snprintf(g_error, sizeof g_error, "mlops_fbla_decode_static: invalid configuration");
     return MLOPS_FBLA_INVALID_VALUE;
@@ -83,7 +88,7 @@ extern "C" mlops_fbla_status mlops_fbla_decode_static(const mlops_fbla_config *c
   }
   void *scratch = static_scratch();
   if (!scratch) return MLOPS_FBLA_CUDA_ERROR;
-  const mlops_fbla_status st = mlops_fbla_decode(cfg, q, cache, output, scratch, FBLA_STATIC_SCRATCH_BYTES, stream);
+  const mlops_fbla_status st = fbla_host_decode_within(cfg, q, cache, output, scratch, FBLA_STATIC_SCRATCH_BYTES, stream);
   if (st != MLOPS_FBLA_OK) snprintf(g_error, sizeof g_error, "%s", mlops_fbla_last_error());
   return st;
 }

@@ -1,26 +1,28 @@
-// FBLA compressed-KV decode for sm_100a where most sub-blocks are refined ("dense"): scores, then every block's value once.
+// FBLA compressed-KV decode for sm_100a in two sweeps: every sub-block's scores, then every sub-block's values once.
 //
-// The decode of fbla_decode.cuh streams all coarse planes once and corrects the selected sub-blocks afterwards by
-// full - coarse; where most are selected (contexts up to about 16 / tau tokens: the average 16-token block then holds more
-// than tau of the mass) it computes their coarse scores and values twice and throws them away. Here
-//   * the score pass reads only the K half of the coarse plane (straight into registers, no staging), forms every
-//     sub-block's log2 mass and the rows' running (m, l), and serves the BF16 windows;
-//   * the value pass knows every row's mass R before it starts, so it knows which (query, sub-block) pairs are selected: it
-//     scores each sub-block again, with its fine bits where selected, and accumulates its values once, in units of 2^-R
-//     -- no running maximum, no correction, no item list. Fine records nobody selected are not read.
-// Both passes put the score columns of several sub-blocks into one product's eight columns (queries of sub-block b in
-// columns b QG ..; its A fragments meet a B operand that is zero elsewhere, and all add into the same accumulators), so the
-// softmax arithmetic runs once per eight (sub-block, query) columns on full warps. Semantics, formats and the definition of
-// every number are fbla_decode.cuh's; only the order of the sums differs.
+//   * The score pass reads only the K half of the records (straight into registers, no staging), forms every sub-block's log2
+//     mass and its integer weights p = round(255 * 2^(s - max)), which it leaves in the scratch (16 bytes per sub-block and
+//     query, beside the block maximum), and the rows' running (m, l); it also serves the BF16 windows.
+//   * The value pass knows every row's mass R before it starts, so it knows which (query, sub-block) pairs are selected. It
+//     reads the V half of the coarse records, of the fine records where some query selected the sub-block, and accumulates
+//     each sub-block once, in units of 2^-R -- no scores, no running maximum, no correction of a coarse sum, no item list.
+// FBLA_K_TWO_BOTH: the score pass reads K's fine half too and leaves both the coarse and the full weights, of which the value
+// pass takes the one its selection asks for: for rows whose sub-blocks are mostly selected. FBLA_K_TWO_COARSE: it leaves the coarse
+// weights only and the value pass scores the few selected sub-blocks again.
+// Both passes put the columns of several sub-blocks into one product's eight columns (queries of sub-block b in columns
+// b QG ..; its A fragments meet a B operand that is zero elsewhere, and all add into the same accumulators), so the softmax
+// arithmetic runs once per eight (sub-block, query) columns on full warps. Semantics, formats and the definition of every
+// number are fbla_decode.cuh's; only the order of the sums differs.
 // Work is dealt in contiguous runs of the flattened (virtual head, group, piece of a group) list: first to CTAs, then to
 // the CTA's warps, so that a head's partial rows are one per CTA, folded in warp order (reproducible bit for bit).
+// Bound by instruction issue: see the figures at the two passes.
 #pragma once
 #include "fbla_decode.cuh"
 
 namespace fbla {
 namespace dense {
 
-constexpr int SCORE_WARPS = 16, VALUE_WARPS = FBLA_K_DENSE_VALUE_WARPS;
+constexpr int SCORE_WARPS = FBLA_K_TWO_SCORE_WARPS, VALUE_WARPS = FBLA_K_TWO_VALUE_WARPS;
 constexpr int MAX_BATCH = FBLA_K_DENSE_MAX_BATCH;
 constexpr int PAIRS = SBG / 2;   // pairs of sub-blocks per group: the value pass's unit
 // a window sub-block's time in the score pass, in pieces of a group (8 / QG sub-blocks: 1 / QG of the group)
@@ -91,7 +93,7 @@ template <bool EXACT> __device__ __forceinline__ Cursor find(const fbla_k_decode
   return c;
 }
 
-// ---- scratch (inside the decode's `part` and `dpart` arrays) -----------------------------------------------------------------
+// ---- scratch (`lse`; the rest inside the decode's `part` and `dpart` arrays) -----------------------------------------------------------------
 // Window chunks: the flattened window sub-blocks in runs of `run`; chunk c leaves one (m, l, o) row per virtual head it meets, at
 // slot c + vh. Value rows (o, l in units of 2^-R) and the score pass's (m, l) pairs: one per (CTA, virtual head), slot cta + vh.
 __device__ __forceinline__ int window_run(const fbla_k_decode &a, int total) { return max(1, (total + a.coarse_ctas * SCORE_WARPS - 1) / (a.coarse_ctas * SCORE_WARPS)); }
@@ -105,43 +107,72 @@ __device__ __forceinline__ float2 *mass_pair(const fbla_k_decode &a, int slot) {
 // prefix sums for the later passes: closed [batch + 1], exact [batch + 1]
 __device__ __forceinline__ int *table_of(const fbla_k_decode &a) { return reinterpret_cast<int *>(mass_pair(a, a.coarse_ctas + a.batch * a.kv_heads * a.vg)); }
 
-// ---- quantisation of the virtual head's queries for one group (quantize_query_word), into QG rows of qst --------------------
-// q: the queries in global memory; rows of qst are QST_ROW bytes apart. Per query the caller gets sq, qb, qsum through `take`.
-template <int QG, class Take>
-__device__ __forceinline__ void quantize_rows(uint4 km, const uint2 (&q)[QG], float sl, uint8_t *qst, int lane, Take take) {
+// lse: per cell (virtual head, sub-block, query) the log2 mass; behind it, per set of weights (0 coarse, 1 full), the block maxima,
+// and then the sets' weights, 16 bytes per cell. (fbla_k_two_cells: cells, padded.)
+__device__ __forceinline__ size_t cells_of(const fbla_k_decode &a) { return fbla_k_two_cells((size_t)a.batch * a.kv_heads * a.vg, a.nblocks, a.qg); }
+__device__ __forceinline__ float *block_max(const fbla_k_decode &a, int set) { return a.lse + (size_t)(1 + set) * cells_of(a); }
+__device__ __forceinline__ uint32_t *weights(const fbla_k_decode &a, int set) {
+  const size_t n = cells_of(a);
+  return reinterpret_cast<uint32_t *>(a.lse) + (size_t)(1 + a.dense + 4 * set) * n;  // (a.dense: the number of sets)
+}
+
+// ---- quantisation of the virtual head's queries for one group (as quantize_query_word), into QG rows of qst, QST_ROW bytes apart ----
+// am: the queries' max |z| (the same in every lane); dot: the lane's share of the result of a butterfly that hands half of the
+// queries on in each of its first steps: q . base of query dot_query(lane).
+template <int QG> __device__ __forceinline__ int dot_lane(int q) { return QG == 4 ? ((q >> 1) << 4) | ((q & 1) << 3) : QG == 2 ? q << 4 : 0; }
+template <int QG>
+__device__ __forceinline__ void quantize_group(uint4 km, const uint2 (&q)[QG], uint8_t *qst, int lane, float (&am)[QG], float &dot) {
+  const float2 b0 = make_float2(bf_lo(km.x), bf_hi(km.x)), b1 = make_float2(bf_lo(km.y), bf_hi(km.y));
+  const float2 s0 = make_float2(bf_lo(km.z), bf_hi(km.z)), s1 = make_float2(bf_lo(km.w), bf_hi(km.w));
+  float d[QG];
 #pragma unroll
-  for (int qi = 0; qi < QG; ++qi) {
-    float sq, qb, qsum;
-    const float4 q4 = make_float4(bf_lo(q[qi].x), bf_hi(q[qi].x), bf_lo(q[qi].y), bf_hi(q[qi].y));
-    reinterpret_cast<uint32_t *>(qst + QST_ROW * qi)[lane] = quantize_query_word(km, q4, sl, sq, qb, qsum);
-    take(qi, sq, qb, qsum);
+  for (int i = 0; i < QG; ++i) {
+    const float2 x0 = make_float2(bf_lo(q[i].x), bf_hi(q[i].x)), x1 = make_float2(bf_lo(q[i].y), bf_hi(q[i].y));
+    const float2 z0 = __fmul2_rn(x0, s0), z1 = __fmul2_rn(x1, s1), t = __ffma2_rn(x1, b1, __fmul2_rn(x0, b0));
+    d[i] = t.x + t.y;
+    am[i] = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(max3_abs(max3_abs(z0.x, z0.y, z1.x), z1.y, z1.y))));
+    const float2 r = splat(quotient_127(am[i])), mg = splat(MAGICF);
+    const float2 c0 = __ffma2_rn(z0, r, mg), c1 = __ffma2_rn(z1, r, mg);
+    reinterpret_cast<uint32_t *>(qst + QST_ROW * i)[lane] =
+        __byte_perm(__byte_perm(__float_as_uint(c0.x), __float_as_uint(c0.y), 0x0040), __byte_perm(__float_as_uint(c1.x), __float_as_uint(c1.y), 0x0040), 0x5410);
   }
+  int o = 16;
+#pragma unroll
+  for (int w = QG / 2; w; w >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < w; ++i) d[i] = (up ? d[i + w] : d[i]) + __shfl_xor_sync(FULL, up ? d[i] : d[i + w], o);
+  }
+#pragma unroll
+  for (; o; o >>= 1) d[0] += __shfl_xor_sync(FULL, d[0], o);
+  dot = d[0];
 }
 
 // ---- score pass -----------------------------------------------------------------------------------------------------------------
 // K words of one sub-block in registers: what thread (gid, tig) supplies to the products, for tokens gid and gid + 8.
-// 4 bits: the thread takes the 16-byte piece `tig` of a token's four (words 0-3 / 4-7 of the two channel halves), whose four
-// words serve two products; 3 bits: the words of qk_tile<3>.
-template <int CB> struct KWords;
-template <> struct KWords<4> {
+// 4 and 2 bits: the thread's slots are 4 t + i and 8 + 4 t + i (i = 0..3, t = tig % 2) of channel half tig / 2, so that a token's words
+// come in 16-byte pieces (2 bits: both t read the same piece); 3 bits: the words of qk_tile<3>.
+template <int BITS> struct KWords {
   uint4 a, a8;
-  __device__ __forceinline__ void load(const uint8_t *rec, int gid, int tig) {
-    const uint8_t *p = rec + 512 * (tig & 1) + 256 * (tig >> 1) + 16 * gid;
+  static __device__ __forceinline__ int offset(int gid, int tig) { return (BITS == 4 ? 512 * (tig & 1) : 0) + 256 * (tig >> 1) + 16 * gid; }
+  __device__ __forceinline__ void load(const uint8_t *p, int) {  // p: the record + offset
     a = __ldg(reinterpret_cast<const uint4 *>(p));
     a8 = __ldg(reinterpret_cast<const uint4 *>(p + 128));
   }
 };
 template <> struct KWords<3> {
   uint32_t a, a8, c, c8, e, e8, f, f8;
-  __device__ __forceinline__ void load(const uint8_t *rec, int gid, int tig) {
-    const uint32_t *p = reinterpret_cast<const uint32_t *>(rec + 16 * gid + 4 * tig), *q = reinterpret_cast<const uint32_t *>(rec + 1024 + 16 * gid + 4 * (tig >> 1));
+  static __device__ __forceinline__ int offset(int gid, int tig) { return 16 * gid + 4 * tig; }
+  static __device__ __forceinline__ int tail(int tig) { return 1024 + 4 * (tig >> 1) - 4 * tig; }  // from there to the words 4 + tig / 2
+  __device__ __forceinline__ void load(const uint8_t *p8, int tail) {
+    const uint32_t *p = reinterpret_cast<const uint32_t *>(p8), *q = reinterpret_cast<const uint32_t *>(p8 + tail);
     a = __ldg(p); a8 = __ldg(p + 32); c = __ldg(p + 64); c8 = __ldg(p + 96);
     e = __ldg(q); e8 = __ldg(q + 32); f = __ldg(q + 2); f8 = __ldg(q + 34);
   }
 };
 // the qhat words matching KWords
 template <int CB> __device__ __forceinline__ void score_frag(const uint8_t *qst, int row, int tig, uint32_t (&B)[8]) {
-  if (CB == 4) {  // low nibbles: slots 4 (tig % 2) + i of half tig / 2; high nibbles: 8 further
+  if (CB == 4) {  // slots 4 t + i, then 8 + 4 t + i, of half tig / 2
     const uint8_t *p = qst + QST_ROW * row + 64 * (tig >> 1) + 16 * (tig & 1);
     const uint4 lo = lds128(p), hi = lds128(p + 32);
     B[0] = lo.x; B[1] = lo.y; B[2] = lo.z; B[3] = lo.w; B[4] = hi.x; B[5] = hi.y; B[6] = hi.z; B[7] = hi.w;
@@ -149,22 +180,27 @@ template <int CB> __device__ __forceinline__ void score_frag(const uint8_t *qst,
     qhat_frag<3>(qst, row, tig, B);
   }
 }
-// adds the sub-block's products to the accumulators (low and high class); B is zero in other sub-blocks' columns
-template <int CB> __device__ __forceinline__ void score_products(const KWords<CB> &k, const uint32_t (&B)[8], uint32_t mask, int tig, uint32_t (&lo)[4], uint32_t (&hi)[4]) {
-  uint32_t b[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) b[i] = B[i] & mask;
-  if constexpr (CB == 4) {
-    constexpr uint32_t L = 0x0f0f0f0fu, H = 0xf0f0f0f0u;
-    mma_u8s8_k32(lo, k.a.x & L, k.a8.x & L, k.a.y & L, k.a8.y & L, b[0], b[1]);
-    mma_u8s8_k32(hi, k.a.x & H, k.a8.x & H, k.a.y & H, k.a8.y & H, b[4], b[5]);
-    mma_u8s8_k32(lo, k.a.z & L, k.a8.z & L, k.a.w & L, k.a8.w & L, b[2], b[3]);
-    mma_u8s8_k32(hi, k.a.z & H, k.a8.z & H, k.a.w & H, k.a8.w & H, b[6], b[7]);
+// The sub-block's products, in accumulators of the low and of the high class (times 16, 3 bits: 8): set (FIRST) or added to.
+template <bool FIRST> __device__ __forceinline__ void mma_step(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if (FIRST) mma_u8s8_k32_from(d, a0, a1, a2, a3, b0, b1, MAGIC);
+  else mma_u8s8_k32(d, a0, a1, a2, a3, b0, b1);
+}
+template <int BITS, bool FIRST>
+__device__ __forceinline__ void score_products(const KWords<BITS> &k, const uint32_t (&b)[8], int tig, uint32_t (&lo)[4], uint32_t (&hi)[4]) {
+  if constexpr (BITS != 3) {
+    constexpr uint32_t L = BITS == 4 ? 0x0f0f0f0fu : 0x03030303u, H = L << 4;
+    const int sh = BITS == 2 ? 2 * (tig & 1) : 0;
+    const uint4 a = BITS == 2 ? make_uint4(k.a.x >> sh, k.a.y >> sh, k.a.z >> sh, k.a.w >> sh) : k.a;
+    const uint4 a8 = BITS == 2 ? make_uint4(k.a8.x >> sh, k.a8.y >> sh, k.a8.z >> sh, k.a8.w >> sh) : k.a8;
+    mma_step<FIRST>(lo, a.x & L, a8.x & L, a.y & L, a8.y & L, b[0], b[1]);
+    mma_step<FIRST>(hi, a.x & H, a8.x & H, a.y & H, a8.y & H, b[4], b[5]);
+    mma_u8s8_k32(lo, a.z & L, a8.z & L, a.w & L, a8.w & L, b[2], b[3]);
+    mma_u8s8_k32(hi, a.z & H, a8.z & H, a.w & H, a8.w & H, b[6], b[7]);
   } else {
     const int sh = 4 + (tig & 1), se = 3 * (tig & 1);
     constexpr uint32_t L = 0x07070707u, M = 0x38383838u, T2 = 0x03030303u, T1 = 0x04040404u;
-    mma_u8s8_k32(lo, k.a & L, k.a8 & L, k.c & L, k.c8 & L, b[0], b[1]);
-    mma_u8s8_k32(hi, k.a & M, k.a8 & M, k.c & M, k.c8 & M, b[2], b[3]);
+    mma_step<FIRST>(lo, k.a & L, k.a8 & L, k.c & L, k.c8 & L, b[0], b[1]);
+    mma_step<FIRST>(hi, k.a & M, k.a8 & M, k.c & M, k.c8 & M, b[2], b[3]);
     mma_u8s8_k32(lo, ((k.a >> 6) & T2) | ((k.e >> sh) & T1), ((k.a8 >> 6) & T2) | ((k.e8 >> sh) & T1),
                  ((k.c >> 6) & T2) | ((k.f >> sh) & T1), ((k.c8 >> 6) & T2) | ((k.f8 >> sh) & T1), b[4], b[5]);
     mma_u8s8_k32(lo, (k.e >> se) & L, (k.e8 >> se) & L, (k.f >> se) & L, (k.f8 >> se) & L, b[6], b[7]);
@@ -174,7 +210,10 @@ template <int CB> __device__ __forceinline__ void score_products(const KWords<CB
 struct ScoreWarp {
   union {
     ExactWarp exact;
-    uint8_t qst[4 * QST_ROW];
+    struct {
+      uint8_t qst[4 * QST_ROW];
+      uint8_t pst[2][128];  // P bytes of a unit, coarse and full: [column][16 tokens]
+    } s;
   };
 };
 struct __align__(16) ScoreSmem {
@@ -211,11 +250,12 @@ __device__ __forceinline__ void score_item_units(const fbla_k_decode &a, int tot
   hi = first + min(count, at + (warp < nc ? with : without));
 }
 
-template <int CB, int FB, int QG>
+template <int CB, int FB, int QG, int MODE>
 __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   constexpr int NB = 8 / QG, UPG = QG;  // sub-blocks per unit, units per group
   constexpr float HOFF = .5f * ((1 << FB) - 1);
-  constexpr int RB = record_bytes(CB);
+  constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
+  constexpr bool BOTH = MODE == FBLA_K_TWO_BOTH;
   ScoreSmem &sm = *reinterpret_cast<ScoreSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
   const int hpr = a.kv_heads * a.vg;
@@ -230,9 +270,8 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
   score_item_units<QG>(a, total, x_total, run, warp, chunk, lo, hi);
   if (chunk >= 0) exact_range<QG, false>(a, sm.w[warp].exact, lane, chunk * run, min(x_total, (chunk + 1) * run), find<true>(a, sm.table.exact, hpr, chunk * run), window_row(a, chunk));
   __syncwarp();
-  uint8_t *const qst = sm.w[warp].qst;
-  for (int i = lane; i < 4 * QST_ROW / 4; i += 32) reinterpret_cast<uint32_t *>(qst)[i] = 0u;
-  __syncwarp();
+  uint8_t *const qst = sm.w[warp].s.qst;
+  uint8_t (*const pst)[128] = sm.w[warp].s.pst;
 
   const int cta = FBLA_POS::x();
   int first_vh = -1, cur_vh = -1;
@@ -257,21 +296,36 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
   if (lo < hi) {
     Cursor c = find<false>(a, sm.table.closed, hpr, lo / UPG);
     int piece = lo % UPG;
-    // the group a cursor stands on: its first record and its metadata
-    auto records = [&](const Cursor &x, const uint8_t *&rec, const uint8_t *&meta) {
+    // Where the next unit's words lie, and the cells of the unit in work: pointers that run on, set anew with every head only.
+    const uint8_t *kp, *fp, *mp;
+    float *lp;
+    uint32_t *wp;
+    const size_t n_cells = cells_of(a);
+    const long long k_skip = (long long)(a.gs - 1) * SBG * RC, f_skip = (long long)(a.gs - 1) * SBG * RF, m_step = (long long)a.gs * 1024;
+    const int k_tail = KWords<3>::tail(tig);
+    auto place_records = [&](const Cursor &x, int pc) {
       const size_t unit = (size_t)((x.b * hpr + x.hir) / a.vg) * a.hs + (size_t)group_of(a, x) * a.gs;
-      rec = a.c.coarse + unit * SBG * RB;
-      meta = reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024;
+      kp = a.c.coarse + (unit * SBG + pc * NB) * RC + KWords<CB>::offset(gid, tig);
+      fp = a.c.fine + (unit * SBG + pc * NB) * RF + KWords<FB>::offset(gid, tig);
+      mp = reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024 + 16 * lane;
     };
-    const uint8_t *rec, *meta;
-    records(c, rec, meta);
-    uint4 km = __ldg(reinterpret_cast<const uint4 *>(meta) + lane);
+    place_records(c, piece);
+    uint4 km = __ldg(reinterpret_cast<const uint4 *>(mp));
     KWords<CB> kw[NB];  // the next unit's words
+    KWords<FB> kf[NB];
+    auto load = [&] {
 #pragma unroll
-    for (int b = 0; b < NB; ++b) kw[b].load(rec + (piece * NB + b) * RB, gid, tig);
+      for (int b = 0; b < NB; ++b) {
+        kw[b].load(kp + b * RC, k_tail);
+        if (BOTH) kf[b].load(fp + b * RF, k_tail);
+      }
+      kp += NB * RC; fp += NB * RF;
+    };
+    load();
     uint2 q[QG];
-    uint32_t B[8];
-    float c0[2] = {0.f, 0.f}, sqc[2] = {0.f, 0.f};
+    constexpr int SETS = QG == 4 ? 2 : 1;  // (with four queries the two sub-blocks' operands are kept, else formed per sub-block)
+    uint32_t B[SETS][8];
+    float2 c0 = make_float2(0.f, 0.f), sqc = c0, sqf = c0, qb2 = c0;
     bool fresh = true;  // the group's queries have not been quantised yet
     for (int u = lo; u < hi; ++u) {
       const int vh = c.b * hpr + c.hir;
@@ -280,63 +334,104 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
         else first_vh = vh;
         cur_vh = vh;
         m[0] = m[1] = -FBLA_INF; l[0] = l[1] = 0.f;
+        const size_t cell = ((size_t)vh * a.nblocks + (size_t)group_of(a, c) * SBG) * QG + 8 * piece;
+        lp = a.lse + cell + 2 * tig;
+        wp = weights(a, 0) + cell * 4 + lane;
 #pragma unroll
         for (int qi = 0; qi < QG; ++qi) q[qi] = __ldg(reinterpret_cast<const uint2 *>(a.q + (size_t)q_row(a, c.b, c.hir, qi) * D) + lane);
       }
       if (fresh) {
         fresh = false;
         __syncwarp();
-        quantize_rows<QG>(km, q, a.sl, qst, lane, [&](int qi, float sq, float qb, float qsum) {
-          const float cc = fmaf(__fmul_rn(sq, HOFF), qsum, qb), s2 = __fmul_rn(sq, (float)(1 << FB));
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-            if (qi == (2 * tig + e) % QG) { c0[e] = cc; sqc[e] = s2; }
-        });
+        float am[QG], dot;
+        quantize_group<QG>(km, q, qst, lane, am, dot);
         __syncwarp();
-        score_frag<CB>(qst, gid % QG, tig, B);
-      }
-      uint32_t dl[4] = {MAGIC, MAGIC, MAGIC, MAGIC}, dh[4] = {MAGIC, MAGIC, MAGIC, MAGIC};
+        uint32_t b[8], d[4];
+        score_frag<CB>(qst, gid % QG, tig, b);
+        // the sums of the codes of the thread's columns: products with an all-ones A
+        mma_u8s8_k32_from(d, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, b[0], b[1], MAGIC);
 #pragma unroll
-      for (int b = 0; b < NB; ++b) score_products<CB>(kw[b], B, gid / QG == b ? FULL : 0u, tig, dl, dh);
-      float *const lse = a.lse + ((size_t)vh * a.nblocks + (size_t)group_of(a, c) * SBG) * QG + 8 * piece + 2 * tig;
+        for (int i = 2; i < 8; i += 2) mma_u8s8_k32(d, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, b[i], b[i + 1]);
+        const int qa = (2 * tig) % QG, qz = (2 * tig + 1) % QG;  // the columns' queries
+        const float2 amax = make_float2(QG == 4 && (tig & 1) ? am[2 % QG] : am[0], QG == 4 && (tig & 1) ? am[3 % QG] : am[1 % QG]);
+        sqf = __fmul2_rn(amax, splat(__fmul_rn(a.sl, 1.f / 127.f)));
+        qb2 = __fmul2_rn(make_float2(__shfl_sync(FULL, dot, dot_lane<QG>(qa)), __shfl_sync(FULL, dot, dot_lane<QG>(qz))), splat(a.sl));
+        sqc = __fmul2_rn(sqf, splat((float)(1 << FB)));
+        c0 = __ffma2_rn(__fmul2_rn(sqf, splat(HOFF)), isum2(d[0], d[1]), qb2);
+#pragma unroll
+        for (int x = 0; x < SETS; ++x)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) B[x][i] = SETS == 1 || gid / QG == x ? b[i] : 0u;
+      }
+      constexpr float UC = CB == 4 ? 1.f / 16 : 1.f / 8, UF = FB == 2 ? 1.f / 16 : 1.f / 8;
+      uint32_t dl[4], dh[4], fl[4], fh[4];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        uint32_t mb[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mb[i] = SETS == 2 ? B[b % SETS][i] : gid / QG == b ? B[0][i] : 0u;
+        if (b == 0) score_products<CB, true>(kw[b], mb, tig, dl, dh); else score_products<CB, false>(kw[b], mb, tig, dl, dh);
+        if (BOTH) { if (b == 0) score_products<FB, true>(kf[b], mb, tig, fl, fh); else score_products<FB, false>(kf[b], mb, tig, fl, fh); }
+      }
       // the next unit's words, and the next group's metadata with the group's first
       if (++piece == UPG) {
         piece = 0;
         fresh = true;
         if (u + 1 < hi) {
-          advance<false>(a, hpr, c);
-          records(c, rec, meta);
-          km = __ldg(reinterpret_cast<const uint4 *>(meta) + lane);
+          if (c.i + 1 < c.n) {
+            ++c.i;
+            kp += k_skip; fp += f_skip; mp += m_step;
+          } else {
+            advance<false>(a, hpr, c);
+            place_records(c, 0);
+          }
+          km = __ldg(reinterpret_cast<const uint4 *>(mp));
         }
       }
-      if (u + 1 < hi) {
+      if (u + 1 < hi) load();
+      // code sums of tokens gid (x[0]), gid + 8 (x[1]) of the thread's columns, and from them scores, maxima, weights
+      auto softmax = [&](float2 sA, float2 sB, float2 &mb, float2 &pA, float2 &pB, uint8_t *p) {
+        mb = make_float2(fmaxf(sA.x, sB.x), fmaxf(sA.y, sB.y));
 #pragma unroll
-        for (int b = 0; b < NB; ++b) kw[b].load(rec + (piece * NB + b) * RB, gid, tig);
+        for (int o = 4; o <= 16; o <<= 1) {
+          mb.x = fmaxf(mb.x, __shfl_xor_sync(FULL, mb.x, o));
+          mb.y = fmaxf(mb.y, __shfl_xor_sync(FULL, mb.y, o));
+        }
+        const float2 nm = make_float2(-mb.x, -mb.y), dA = __fadd2_rn(sA, nm), dB = __fadd2_rn(sB, nm);
+        pA = __ffma2_rn(make_float2(ex2(dA.x), ex2(dA.y)), splat(255.f), splat(MAGICF));
+        pB = __ffma2_rn(make_float2(ex2(dB.x), ex2(dB.y)), splat(255.f), splat(MAGICF));
+        p += 32 * tig + gid;  // columns 2 tig, 2 tig + 1: 16 bytes apart
+        p[0] = (uint8_t)__float_as_uint(pA.x); p[16] = (uint8_t)__float_as_uint(pA.y);
+        p[8] = (uint8_t)__float_as_uint(pB.x); p[24] = (uint8_t)__float_as_uint(pB.y);
+      };
+      const float2 xA = __ffma2_rn(isum2(dh[0], dh[1]), splat(UC), isum2(dl[0], dl[1])), xB = __ffma2_rn(isum2(dh[2], dh[3]), splat(UC), isum2(dl[2], dl[3]));
+      float2 mb, pA, pB;
+      __syncwarp();  // (the previous unit's bytes have been read)
+      softmax(__ffma2_rn(sqc, xA, c0), __ffma2_rn(sqc, xB, c0), mb, pA, pB, pst[0]);
+      if (BOTH) {
+        const float2 fA = __ffma2_rn(isum2(fh[0], fh[1]), splat(UF), isum2(fl[0], fl[1])), fB = __ffma2_rn(isum2(fh[2], fh[3]), splat(UF), isum2(fl[2], fl[3]));
+        float2 mf, qA, qB;
+        softmax(__ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), xA, fA), qb2), __ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), xB, fB), qb2), mf, qA, qB, pst[1]);
+        if (gid == 0) *reinterpret_cast<float2 *>(lp + 2 * n_cells) = mf;
       }
-      constexpr float UN = CB == 4 ? 1.f / 16 : 1.f / 8;
-      const float2 x01 = __ffma2_rn(isum2(dh[0], dh[1]), splat(UN), isum2(dl[0], dl[1])), x23 = __ffma2_rn(isum2(dh[2], dh[3]), splat(UN), isum2(dl[2], dl[3]));
-      const float2 sq2 = make_float2(sqc[0], sqc[1]), cc2 = make_float2(c0[0], c0[1]);
-      const float2 s01 = __ffma2_rn(sq2, x01, cc2), s23 = __ffma2_rn(sq2, x23, cc2);  // tokens gid, gid + 8 of the thread's columns
-      float mb[2] = {fmaxf(s01.x, s23.x), fmaxf(s01.y, s23.y)};
-#pragma unroll
-      for (int o = 4; o <= 16; o <<= 1)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) mb[e] = fmaxf(mb[e], __shfl_xor_sync(FULL, mb[e], o));
-      const float2 nm = make_float2(-mb[0], -mb[1]), d01 = __fadd2_rn(s01, nm), d23 = __fadd2_rn(s23, nm);
-      const float2 p01 = __ffma2_rn(make_float2(ex2(d01.x), ex2(d01.y)), splat(255.f), splat(MAGICF));
-      const float2 p23 = __ffma2_rn(make_float2(ex2(d23.x), ex2(d23.y)), splat(255.f), splat(MAGICF));
       // both columns' sums of p in one word (each below 2^13): low half column 0, high half column 1
-      uint32_t ps = (__float_as_uint(p01.x) + __float_as_uint(p23.x)) + ((__float_as_uint(p01.y) + __float_as_uint(p23.y)) << 16) - 2u * MAGIC;
+      uint32_t ps = (__float_as_uint(pA.x) + __float_as_uint(pB.x)) + ((__float_as_uint(pA.y) + __float_as_uint(pB.y)) << 16) - 2u * MAGIC;
 #pragma unroll
       for (int o = 4; o <= 16; o <<= 1) ps += __shfl_xor_sync(FULL, ps, o);
       const float2 sp = isum2((ps & 0xffffu) | MAGIC, (ps >> 16) | MAGIC);
-      if (gid == 0) *reinterpret_cast<float2 *>(lse) = make_float2(mb[0] + lg2(sp.x), mb[1] + lg2(sp.y));
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float mn = fmaxf(m[e], mb[e]);
-        l[e] = fmaf(l[e], ex2(m[e] - mn), (e ? sp.y : sp.x) * ex2(mb[e] - mn));
-        m[e] = mn;
+      if (gid == 0) {
+        *reinterpret_cast<float2 *>(lp) = make_float2(mb.x + lg2(sp.x), mb.y + lg2(sp.y));
+        *reinterpret_cast<float2 *>(lp + n_cells) = mb;
       }
+      // the running maximum moves only when a block exceeds it by more than 2^8
+      if (mb.x > m[0] + 8.f) { l[0] *= ex2(m[0] - mb.x); m[0] = mb.x; }
+      if (mb.y > m[1] + 8.f) { l[1] *= ex2(m[1] - mb.y); m[1] = mb.y; }
+      l[0] = fmaf(sp.x, ex2(mb.x - m[0]), l[0]);
+      l[1] = fmaf(sp.y, ex2(mb.y - m[1]), l[1]);
+      __syncwarp();
+      *wp = lds32(pst[0] + 4 * lane);
+      if (BOTH) wp[4 * n_cells] = lds32(pst[1] + 4 * lane);
+      lp += 8; wp += 32;
     }
     leave(sm.stage[warp][cur_vh == first_vh ? 0 : 1]);
   }
@@ -422,21 +517,58 @@ __device__ __forceinline__ void mass_item(const fbla_k_decode &a, uint8_t *smem_
 }
 
 // ---- value pass -------------------------------------------------------------------------------------------------------------------
-template <int CB, int FB> struct __align__(128) ValueWarp {
-  static constexpr int NST = 2;
-  uint8_t pair[NST][2 * (record_bytes(CB) + record_bytes(FB))];  // two coarse records, two fine records
-  uint8_t meta[2][1024];
-  uint8_t qst[4 * QST_ROW];
-  uint8_t pst[128];  // P bytes: [sub-block of the pair][query 0..3][16 tokens]
-  float stage[4][PSTRIDE];  // the row set of the first virtual head of the warp's run (the last one's lies in `pair`)
-  uint64_t bar[NST], bar_meta[2];
+// V words of a record in registers: what thread (gid, tig) supplies to the products for record lanes 8 u + gid, u = 0..3, and its
+// slots (as v_slots of fbla_frag.cuh).
+template <int BITS> struct VWords {
+  uint32_t w[4][BITS == 2 ? 1 : BITS == 4 ? 2 : 3];
+  static __device__ __forceinline__ int offset(int gid, int tig) { return BITS == 4 ? 1024 + 512 * (tig >> 1) + 16 * gid + 8 * (tig & 1) : 512 + 16 * gid + 4 * tig; }
+  // p: the record + offset; 3 bits: d1, d2 from there to W[4 + tig / 2] (the top bit of slot 12 + tig) and W[4 + tig % 2] (slot 4 + tig
+  // for tig < 2, 10 + tig - 2 beyond)
+  __device__ __forceinline__ void load(const uint8_t *p, int d1, int d2) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if constexpr (BITS == 4) {
+        const uint2 y = __ldg(reinterpret_cast<const uint2 *>(p + 128 * u));
+        w[u][0] = y.x; w[u][1] = y.y;
+      } else {
+        w[u][0] = __ldg(reinterpret_cast<const uint32_t *>(p + 128 * u));
+        if constexpr (BITS == 3) {
+          w[u][1] = __ldg(reinterpret_cast<const uint32_t *>(p + d1 + 64 * u));
+          w[u][2] = __ldg(reinterpret_cast<const uint32_t *>(p + d2 + 64 * u));
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void slots(int u, int tig, uint32_t (&v)[4]) const {
+    const uint32_t a = w[u][0];
+    if constexpr (BITS == 4) {
+      const uint32_t b = w[u][1];
+      v[0] = a & 0x0f0f0f0fu; v[1] = b & 0x0f0f0f0fu; v[2] = a & 0xf0f0f0f0u; v[3] = b & 0xf0f0f0f0u;
+    } else if constexpr (BITS == 2) {
+      v[0] = a & 0x03030303u; v[1] = a & 0x0c0c0c0cu; v[2] = a & 0x30303030u; v[3] = a & 0xc0c0c0c0u;
+    } else {
+      v[0] = a & 0x07070707u;
+      v[1] = a & 0x38383838u;
+      v[2] = (w[u][2] >> (3 * (tig >> 1))) & 0x07070707u;
+      v[3] = ((a >> 6) & 0x03030303u) | ((w[u][1] >> (4 + (tig & 1))) & 0x04040404u);
+    }
+  }
+};
+struct __align__(16) ValueWarp {
+  uint8_t meta[2][512];        // V's metadata of the group in work and of the next
+  uint8_t qst[4 * QST_ROW];    // (scoring again: FBLA_K_TWO_COARSE)
+  uint8_t pst[128];
+  float stage[4][PSTRIDE];     // the row set of the first virtual head of the warp's run
+  // The current head's sums (Sums, [word][lane]): in registers they would halve the warps that an SM holds. At the end: the last
+  // head's row set.
+  float2 run[17][32];
   int stage_vh[2];
 };
-template <int CB, int FB> struct ValueSmem {
-  ValueWarp<CB, FB> w[VALUE_WARPS];
+struct ValueSmem {
+  ValueWarp w[VALUE_WARPS];
   Table table;
 };
-static_assert(sizeof(ValueSmem<3, 3>) + 128 <= 227 * 1024 && sizeof(ValueSmem<4, 2>) + 128 <= 227 * 1024, "one CTA's shared memory");
+static_assert(sizeof(ValueSmem) + 128 <= 227 * 1024, "one CTA's shared memory");
 
 // scores of a record pair of a BITS plane: columns 0-3 the first record's queries, 4-7 the second's. Thread (gid, tig): tokens
 // gid, gid + 8 of columns 2 tig, 2 tig + 1. m0 / m1: all ones in the threads whose B column belongs to the first / second record.
@@ -499,13 +631,6 @@ __device__ __forceinline__ void qk_pair(const uint8_t *ra, const uint8_t *rb, in
 struct Sums {
   float2 l, o[4][4];
 };
-__device__ __forceinline__ void clear(Sums &s) {
-  s.l = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc) s.o[u][cc] = make_float2(0.f, 0.f);
-}
 template <int QG> __device__ __forceinline__ void write_sums(float *p, const Sums &s, int lane) {
   const int gid = lane >> 2, tig = lane & 3;
 #pragma unroll
@@ -527,244 +652,254 @@ template <int QG> __device__ __forceinline__ void write_sums(float *p, const Sum
   }
 }
 
+// The full scores of a pair of sub-blocks, from both planes: {block maximum of the thread's columns 2 tig, 2 tig + 1 (sub-block
+// tig / 2, queries 2 (tig % 2) + e), the lane's word of P (column gid, tokens 4 tig ..)}. Rare: a function of its own.
+struct Again { float m0, m1; uint32_t p; };
 template <int CB, int FB, int QG>
+__device__ __noinline__ Again score_again(const uint8_t *ra, const uint8_t *fa, const uint8_t *meta, const uint16_t *q0, float sl, uint8_t *qst, uint8_t *pst, int lane) {
+  const int gid = lane >> 2, tig = lane & 3;
+  uint2 q[QG];
+#pragma unroll
+  for (int qi = 0; qi < QG; ++qi) q[qi] = __ldg(reinterpret_cast<const uint2 *>(q0 + qi * D) + lane);
+  float am[QG], dot;
+  __syncwarp();
+  if (QG < 4)
+    for (int i = lane; i < 4 * QST_ROW / 4; i += 32) reinterpret_cast<uint32_t *>(qst)[i] = 0u;
+  __syncwarp();
+  quantize_group<QG>(__ldg(reinterpret_cast<const uint4 *>(meta) + lane), q, qst, lane, am, dot);
+  __syncwarp();
+  uint32_t B[8];
+  qhat_frag<CB>(qst, gid & 3, tig, B);
+  const int qa = (2 * (tig & 1)) % QG, qz = (2 * (tig & 1) + 1) % QG;
+  const float2 amax = make_float2(QG == 4 && (tig & 1) ? am[2 % QG] : am[0], QG == 4 && (tig & 1) ? am[3 % QG] : am[1 % QG]);
+  const float2 sqf = __fmul2_rn(amax, splat(__fmul_rn(sl, 1.f / 127.f)));
+  const float2 qb = __fmul2_rn(make_float2(__shfl_sync(FULL, dot, dot_lane<QG>(qa)), __shfl_sync(FULL, dot, dot_lane<QG>(qz))), splat(sl));
+  const uint32_t m0 = gid < 4 ? FULL : 0u;
+  float2 x[2], y[2];
+  qk_pair<CB>(ra, ra + record_bytes(CB), gid, tig, B, m0, ~m0, x);
+  qk_pair<FB>(fa, fa + record_bytes(FB), gid, tig, B, m0, ~m0, y);
+  const float2 s0 = __ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), x[0], y[0]), qb), s1 = __ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), x[1], y[1]), qb);
+  float2 mb = make_float2(fmaxf(s0.x, s1.x), fmaxf(s0.y, s1.y));
+#pragma unroll
+  for (int o = 4; o <= 16; o <<= 1) {
+    mb.x = fmaxf(mb.x, __shfl_xor_sync(FULL, mb.x, o));
+    mb.y = fmaxf(mb.y, __shfl_xor_sync(FULL, mb.y, o));
+  }
+  uint8_t *p = pst + 32 * tig + gid;
+  p[0] = (uint8_t)__float_as_uint(fmaf(ex2(s0.x - mb.x), 255.f, MAGICF)); p[16] = (uint8_t)__float_as_uint(fmaf(ex2(s0.y - mb.y), 255.f, MAGICF));
+  p[8] = (uint8_t)__float_as_uint(fmaf(ex2(s1.x - mb.x), 255.f, MAGICF)); p[24] = (uint8_t)__float_as_uint(fmaf(ex2(s1.y - mb.y), 255.f, MAGICF));
+  __syncwarp();
+  return Again{mb.x, mb.y, lds32(pst + 4 * lane)};
+}
+
+template <int CB, int FB, int QG, int MODE>
 __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem_raw) {
-  constexpr int RC = record_bytes(CB), RF = record_bytes(FB), NST = ValueWarp<CB, FB>::NST;
+  constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
   constexpr float HOFF = .5f * ((1 << FB) - 1);
-  smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;
-  ValueSmem<CB, FB> &sm = *reinterpret_cast<ValueSmem<CB, FB> *>(smem_raw);
+  constexpr bool BOTH = MODE == FBLA_K_TWO_BOTH;
+  ValueSmem &sm = *reinterpret_cast<ValueSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
   const int hpr = a.kv_heads * a.vg, cta = FBLA_POS::x();
-  ValueWarp<CB, FB> &w = sm.w[warp];
+  ValueWarp &w = sm.w[warp];
   allow_next_pass();
   build_table(a, sm.table, 32 * VALUE_WARPS);
   const int total = PAIRS * total_of<false>(a, sm.table.closed, hpr), per = (total + (int)FBLA_POS::nx() - 1) / (int)FBLA_POS::nx();
   const int c_lo = min(total, cta * per), c_n = min(total, c_lo + per) - c_lo, wper = (c_n + VALUE_WARPS - 1) / VALUE_WARPS;
   const int lo = c_lo + min(c_n, warp * wper), hi = c_lo + min(c_n, (warp + 1) * wper);
-  for (int i = lane; i < 4 * QST_ROW / 4; i += 32) reinterpret_cast<uint32_t *>(w.qst)[i] = 0u;
-  reinterpret_cast<uint32_t *>(w.pst)[lane] = 0u;
-  if (lane == 0) {
-#pragma unroll
-    for (int s = 0; s < NST; ++s) mbar_init(&w.bar[s], 1);
-    mbar_init(&w.bar_meta[0], 1);
-    mbar_init(&w.bar_meta[1], 1);
-    mbar_init_fence();
-  }
-  __syncwarp();
   wait_previous_pass();
   int first_vh = -1, cur_vh = -1;
-  bool ok = true;
   if (lo < hi) {
-    // The stream of pairs. A cursor stands on a group; `mask` of a group: bit (sub-block QG + query) selected.
     Cursor c = find<false>(a, sm.table.closed, hpr, lo / PAIRS);
-    const int J0 = lo % PAIRS;
     const int groups = (hi - 1) / PAIRS - lo / PAIRS + 1;
-    float R = 0.f;  // lane l: of query l % QG of the head the issuing side stands on
-    auto mass_of = [&](int vh) {
-      if (a.mass_given) return __ldcg(a.row_r + vh * QG + lane % QG);
-      const float r = row_mass<QG>(a, rows_of<QG>(a, sm.table.closed, sm.table.exact, hpr, vh), vh, lane);
-      if (lane < QG) a.row_r[vh * QG + lane] = r;  // for the merge (every warp of the head writes the same)
+    int left = hi - lo;  // pairs
+    // The sums of integer products are taken as they are: a nonnegative s32 below 2^23 read as FP32 is the subnormal s 2^-149, and a
+    // weight times 2^75 brings the product back into range; the group's sums come out times 2^-74.
+    constexpr float UP = 37778931862957161709568.f /* 2^75 */, BACK = 18889465931478580854784.f /* 2^74 */;
+    // a group's place: its unit, and its first cell
+    auto unit_of = [&](const Cursor &x) { return (size_t)((x.b * hpr + x.hir) / a.vg) * a.hs + (size_t)group_of(a, x) * a.gs; };
+    auto cell_of = [&](const Cursor &x) { return ((size_t)(x.b * hpr + x.hir) * a.nblocks + (size_t)group_of(a, x) * SBG) * QG; };
+    const float *const mx0 = block_max(a, 0), *const mx1 = block_max(a, 1);
+    const int pcol = (gid >> 2) * QG + (gid & 3);  // the lane's column of a pair's P words: sub-block gid / 4, query gid % 4
+    const bool has = (gid & 3) < QG;
+    const uint32_t *const w0 = weights(a, 0) + 4 * pcol + tig, *const w1 = weights(a, 1) + 4 * pcol + tig;
+    // what a group's cells hold, lane l: cell l = (sub-block l / QG, query l % QG)
+    float lse_n, mc_n, mf_n = 0.f;
+    size_t cell = cell_of(c), cell_n;
+    auto ask = [&](size_t at) {
+      lse_n = -FBLA_INF; mc_n = 0.f;
+      if (lane < SBG * QG) { lse_n = __ldcg(a.lse + at + lane); mc_n = __ldcg(mx0 + at + lane); if (BOTH) mf_n = __ldcg(mx1 + at + lane); }
+    };
+    uint32_t pc = 0u, pf = 0u;  // the next pair's words
+    auto ask_p = [&](size_t at, int J) {
+      if (has) { pc = __ldcg(w0 + (at + 2 * QG * J) * 4); if (BOTH) pf = __ldcg(w1 + (at + 2 * QG * J) * 4); }
+    };
+    size_t unit = unit_of(c);
+    auto fetch_meta = [&](size_t un, int buf) {  // V's 512 bytes of metadata
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n\tcp.async.commit_group;"
+                   ::"r"(smem_u32(w.meta[buf] + 16 * lane)), "l"(reinterpret_cast<const uint8_t *>(a.c.meta) + un * 1024 + 512 + 16 * lane) : "memory");
+    };
+    int J = lo % PAIRS;
+    ask(cell);
+    ask_p(cell, J);
+    fetch_meta(unit, 0);
+    // where the words of the next pair (coarse) and of the pair in work (fine) lie: pointers that run on within a head
+    const uint8_t *cp = a.c.coarse + (unit * SBG + 2 * J) * RC + VWords<CB>::offset(gid, tig), *fp = a.c.fine + (unit * SBG + 2 * J) * RF + VWords<FB>::offset(gid, tig);
+    const long long c_skip = (long long)(a.gs - 1) * SBG * RC, f_skip = (long long)(a.gs - 1) * SBG * RF;
+    const int d1 = 1280 - 512 - 8 * gid - 4 * tig + 4 * (tig >> 1), d2 = 1280 - 512 - 8 * gid - 4 * tig + 4 * (tig & 1);
+    VWords<CB> va, vb;
+    auto load_coarse = [&] {
+      va.load(cp, d1, d2);
+      vb.load(cp + RC, d1, d2);
+      cp += 2 * RC;
+    };
+    load_coarse();
+    float R = 0.f;  // lane l: of query l % QG of the current head
+    auto sums = [&] {
+      Sums r;
+      r.l = w.run[16][lane];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) r.o[u][cc] = w.run[4 * u + cc][lane];
       return r;
     };
-    auto lse_of = [&](const Cursor &x) {  // lane l: (sub-block l / QG, query l % QG) of the group
-      return lane < SBG * QG ? __ldcg(a.lse + ((size_t)(x.b * hpr + x.hir) * a.nblocks + (size_t)group_of(a, x) * SBG) * QG + lane) : -FBLA_INF;
-    };
-    auto issue = [&](const Cursor &x, uint32_t mask, int J, int s, bool with_meta, int ms) {  // lane 0
-      const size_t unit = (size_t)((x.b * hpr + x.hir) / a.vg) * a.hs + (size_t)group_of(a, x) * a.gs;
-      const bool fine = (mask >> (2 * QG * J)) & ((1u << (2 * QG)) - 1u);
-      if (with_meta) {
-        mbar_expect_tx(&w.bar_meta[ms], 1024);
-        bulk_g2s(w.meta[ms], reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024, 1024, &w.bar_meta[ms]);
-      }
-      mbar_expect_tx(&w.bar[s], 2 * RC + (fine ? 2 * RF : 0));
-      bulk_g2s(w.pair[s], a.c.coarse + (unit * SBG + 2 * J) * RC, 2 * RC, &w.bar[s]);
-      if (fine) bulk_g2s(w.pair[s] + 2 * RC, a.c.fine + (unit * SBG + 2 * J) * RF, 2 * RF, &w.bar[s]);
-    };
-    int r_vh = c.b * hpr + c.hir;  // the head R belongs to
-    R = mass_of(r_vh);
-    uint32_t mask = __ballot_sync(FULL, lse_of(c) - R > a.log2_tau), next_mask = 0;
-    float Rc = R;        // R of the group in work
-    Cursor n = c;        // the next group
-    // group k covers pairs [k ? 0 : J0, ..); chunk number = pair number - lo
-    int issued = 0;      // chunks issued
-    const int chunks = hi - lo;
-    // issues the next chunk; it belongs to group k or, from its pair `cross` on, to group k + 1
-    auto issue_next = [&](int pair_in_group, const Cursor &x, uint32_t mk, int ms) {
-      if (lane == 0) issue(x, mk, pair_in_group, issued % NST, issued == 0 || pair_in_group == 0, ms);
-      ++issued;
-    };
-    Sums run;
-    uint2 q[QG];
-    float2 Rq = make_float2(0.f, 0.f);
-    int done = 0;        // chunks consumed
-    bool have_next = groups > 1;
-    if (have_next) {
-      advance<false>(a, hpr, n);
-      const int nv = n.b * hpr + n.hir;
-      if (nv != r_vh) { R = mass_of(nv); r_vh = nv; }
-      next_mask = __ballot_sync(FULL, lse_of(n) - R > a.log2_tau);
-    }
-    // prologue: the first NST chunks
-#pragma unroll
-    for (int s = 0; s < NST; ++s)
-      if (issued < chunks) {
-        const int pg = J0 + issued;
-        if (pg < PAIRS) issue_next(pg, c, mask, 0); else issue_next(pg - PAIRS, n, next_mask, 1);
-      }
-    for (int k = 0; k < groups && ok; ++k) {
-      const int j0 = k ? 0 : J0, j1 = min(PAIRS, j0 + chunks - done);
-      const int vh = c.b * hpr + c.hir;
-      float Rn = R;      // R of the next group
+#pragma unroll 1
+    for (int k = 0; k < groups; ++k) {
+      const int vh = c.b * hpr + c.hir, j1 = min(PAIRS, J + left);
       if (vh != cur_vh) {
-        if (cur_vh >= 0) { if (cur_vh == first_vh) write_sums<QG>(&w.stage[0][0], run, lane); else write_sums<QG>(value_row(a, cta + cur_vh), run, lane); }
+        if (cur_vh >= 0) write_sums<QG>(cur_vh == first_vh ? &w.stage[0][0] : value_row(a, cta + cur_vh), sums(), lane);
         else first_vh = vh;
         cur_vh = vh;
-        clear(run);
-        Rq = make_float2(__shfl_sync(FULL, Rc, (2 * (tig & 1)) % QG), __shfl_sync(FULL, Rc, (2 * (tig & 1) + 1) % QG));
 #pragma unroll
-        for (int qi = 0; qi < QG; ++qi) q[qi] = __ldg(reinterpret_cast<const uint2 *>(a.q + (size_t)q_row(a, c.b, c.hir, qi) * D) + lane);
+        for (int x = 0; x < 17; ++x) w.run[x][lane] = make_float2(0.f, 0.f);
+        if (a.mass_given) R = __ldcg(a.row_r + vh * QG + lane % QG);
+        else {
+          R = row_mass<QG>(a, rows_of<QG>(a, sm.table.closed, sm.table.exact, hpr, vh), vh, lane);
+          if (lane < QG) a.row_r[vh * QG + lane] = R;  // for the merge (every warp of the head writes the same)
+        }
       }
-      // the group after the next: its masses are asked for now and looked at when its first chunk is issued
-      Cursor nn = n;
-      float nn_lse = -FBLA_INF;
-      const bool have_nn = k + 2 < groups;
-      if (have_nn) { advance<false>(a, hpr, nn); nn_lse = lse_of(nn); }
-      if (!__all_sync(FULL, mbar_wait_bounded(&w.bar_meta[k & 1], (uint32_t)((k >> 1) & 1)))) { ok = false; break; }
-      const uint8_t *meta = w.meta[k & 1];
-      float2 sq2 = make_float2(0.f, 0.f), qb2 = sq2, c02 = sq2;
-      __syncwarp();
-      quantize_rows<QG>(lds128(meta + 16 * lane), q, a.sl, w.qst, lane, [&](int qi, float sq, float qb, float qsum) {
-        const float cc = fmaf(__fmul_rn(sq, HOFF), qsum, qb);
-        if (qi == 2 * (tig & 1)) { sq2.x = sq; qb2.x = qb; c02.x = cc; }
-        if (qi == 2 * (tig & 1) + 1) { sq2.y = sq; qb2.y = qb; c02.y = cc; }
-      });
-      __syncwarp();
-      uint32_t B[8];
-      qhat_frag<CB>(w.qst, gid & 3, tig, B);
-      const uint32_t m0 = gid < 4 ? FULL : 0u, m1 = ~m0;
+      const uint32_t mask = __ballot_sync(FULL, lse_n - R > a.log2_tau);  // bit cell: selected
+      float wl = ex2((BOTH && ((mask >> lane) & 1) ? mf_n : mc_n) - R) * UP;  // lane: the weight of its cell
+      if (lane >= SBG * QG) wl = 0.f;
+      // the next group: its cells, its metadata
+      Cursor n = c;
+      size_t unit_n = unit;
+      const bool more = k + 1 < groups, stay = c.i + 1 < c.n;  // stay: the next group is the head's next
+      if (more) {
+        if (stay) { ++n.i; unit_n += a.gs; cell_n = cell + SBG * QG; }
+        else { advance<false>(a, hpr, n); unit_n = unit_of(n); cell_n = cell_of(n); }
+        ask(cell_n);
+        fetch_meta(unit_n, (k + 1) & 1);
+      }
       float2 A[4][4], L = make_float2(0.f, 0.f), Hc = L;  // the group's sums in code units; sum w sum p, and its unselected part
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) A[u][cc] = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int J = j0; J < j1; ++J) {
-        const int s = done % NST;
-        if (!__all_sync(FULL, mbar_wait_bounded(&w.bar[s], (uint32_t)((done / NST) & 1)))) { ok = false; break; }
-        ++done;
-        const uint8_t *ra = w.pair[s], *rb = ra + RC, *fa = ra + 2 * RC, *fb = fa + RF;
+      for (; J < j1; ++J, --left) {
         const uint32_t pm = (mask >> (2 * QG * J)) & ((1u << (2 * QG)) - 1u);  // the pair's selections
-        const bool fine = pm != 0;
-        // the thread's two columns: sub-block tig >> 1, queries 2 (tig & 1) + e
-        const uint32_t mine = pm >> (QG * (tig >> 1) + 2 * (tig & 1));
-        const float2 sel = make_float2(mine & 1u && query_valid<QG>(tig, 0) ? 1.f : 0.f, mine & 2u && query_valid<QG>(tig, 1) ? 1.f : 0.f);
-        float2 x[2], y[2];
-        qk_pair<CB>(ra, rb, gid, tig, B, m0, m1, x);
-        float2 cst = c02;
-        if (fine) {
-          qk_pair<FB>(fa, fb, gid, tig, B, m0, m1, y);
-          cst = make_float2(sel.x != 0.f ? qb2.x : c02.x, sel.y != 0.f ? qb2.y : c02.y);
-#pragma unroll
-          for (int i = 0; i < 2; ++i) x[i] = __ffma2_rn(splat((float)(1 << FB)), x[i], __fmul2_rn(sel, y[i]));  // whole numbers, exact
-        } else {
-#pragma unroll
-          for (int i = 0; i < 2; ++i) x[i] = __fmul2_rn(splat((float)(1 << FB)), x[i]);
+        VWords<FB> fa, fb;
+        if (pm) {
+          fa.load(fp, d1, d2);
+          fb.load(fp + RF, d1, d2);
         }
-        const float2 s0 = __ffma2_rn(sq2, x[0], cst), s1 = __ffma2_rn(sq2, x[1], cst);
-        float mb[2] = {fmaxf(s0.x, s1.x), fmaxf(s0.y, s1.y)};
-#pragma unroll
-        for (int o = 4; o <= 16; o <<= 1)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) mb[e] = fmaxf(mb[e], __shfl_xor_sync(FULL, mb[e], o));
-        const float2 nm = make_float2(-mb[0], -mb[1]), d0 = __fadd2_rn(s0, nm), d1 = __fadd2_rn(s1, nm);
-        const float2 p0 = __ffma2_rn(make_float2(ex2(d0.x), ex2(d0.y)), splat(255.f), splat(MAGICF));
-        const float2 p1 = __ffma2_rn(make_float2(ex2(d1.x), ex2(d1.y)), splat(255.f), splat(MAGICF));
-        if (query_valid<QG>(tig, 0)) { w.pst[32 * tig + gid] = (uint8_t)__float_as_uint(p0.x); w.pst[32 * tig + gid + 8] = (uint8_t)__float_as_uint(p1.x); }
-        if (query_valid<QG>(tig, 1)) { w.pst[32 * tig + 16 + gid] = (uint8_t)__float_as_uint(p0.y); w.pst[32 * tig + 16 + gid + 8] = (uint8_t)__float_as_uint(p1.y); }
-        const float2 wt = make_float2(query_valid<QG>(tig, 0) ? ex2(mb[0] - Rq.x) : 0.f, query_valid<QG>(tig, 1) ? ex2(mb[1] - Rq.y) : 0.f);
-        const float2 ws = __fmul2_rn(wt, sel);
-        __syncwarp();
-        const uint32_t pw = lds32(w.pst + 4 * lane), b0 = pw & m0, b1 = pw & m1;
+        fp += 2 * RF;
+        uint32_t pw = BOTH && ((pm >> pcol) & 1) ? pf : pc;
+        if (!has) pw = 0u;
+        if (!BOTH && pm) {  // full scores of the pair, for the selected cells
+          const Again g = score_again<CB, FB, QG>(a.c.coarse + (unit * SBG + 2 * J) * RC, a.c.fine + (unit * SBG + 2 * J) * RF, reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024,
+                                                  a.q + (size_t)q_row(a, c.b, c.hir, 0) * D, a.sl, w.qst, w.pst, lane);
+          if (has && ((pm >> pcol) & 1)) pw = g.p;
+          const int mine = lane - 2 * QG * J, col = mine < 0 ? 0 : (mine / QG) * 4 + mine % QG;  // the lane's cell as a column of the pair
+          const float f0 = __shfl_sync(FULL, g.m0, col >> 1), f1 = __shfl_sync(FULL, g.m1, col >> 1);
+          if (mine >= 0 && mine < 2 * QG && ((mask >> lane) & 1)) wl = ex2(((col & 1) ? f1 : f0) - R) * UP;
+        }
+        const bool last = J + 1 >= PAIRS;
+        if (left > 1) ask_p(last ? cell_n : cell, last ? 0 : J + 1);
+        // the thread's two columns: sub-block tig >> 1, queries 2 (tig & 1) + e
+        const int own = QG * (tig >> 1) + 2 * (tig & 1);
+        float2 wt = make_float2(__shfl_sync(FULL, wl, 2 * QG * J + own), __shfl_sync(FULL, wl, (2 * QG * J + own + 1) & 31));
+        if (QG < 4) { if (!query_valid<QG>(tig, 0)) wt.x = 0.f; if (!query_valid<QG>(tig, 1)) wt.y = 0.f; }
+        const float2 ws = make_float2((pm >> own) & 1 ? wt.x : 0.f, (pm >> own) & 2 ? wt.y : 0.f);
+        const uint32_t b0 = gid < 4 ? pw : 0u, b1 = gid < 4 ? 0u : pw;
         {
           uint32_t d[4];
-          mma_u8u8_k32_from(d, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, b0, b1, MAGIC);
-          const float2 sp = isum2(d[0], d[1]);
+          mma_u8u8_k32_zero(d, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, b0, b1);
+          const float2 sp = tiny2(d[0], d[1]);
           L = __ffma2_rn(wt, sp, L);
           Hc = __ffma2_rn(__fadd2_rn(wt, make_float2(-ws.x, -ws.y)), sp, Hc);
         }
         // the weights times the planes' class factors: code units = 2^FB h + f
-        float2 wc[4], wf[4];
+        auto add = [&](const uint32_t (&x)[4], const uint32_t (&y)[4], const float2 (&f)[4], float2 (&to)[4]) {
+          uint32_t d01[4], d23[4];
+          mma_u8u8_k32_zero(d01, x[0], x[1], y[0], y[1], b0, b1);
+          mma_u8u8_k32_zero(d23, x[2], x[3], y[2], y[3], b0, b1);
+          to[0] = __ffma2_rn(f[0], tiny2(d01[0], d01[1]), to[0]);
+          to[1] = __ffma2_rn(f[1], tiny2(d01[2], d01[3]), to[1]);
+          to[2] = __ffma2_rn(f[2], tiny2(d23[0], d23[1]), to[2]);
+          to[3] = __ffma2_rn(f[3], tiny2(d23[2], d23[3]), to[3]);
+        };
+        {
+          float2 f[4];
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          wc[cc] = __fmul2_rn(wt, splat((float)(1 << FB) * v_unscale<CB>(cc)));
-          wf[cc] = __fmul2_rn(ws, splat(v_unscale<FB>(cc)));
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          uint32_t va[4], vb[4], d01[4], d23[4];
-          v_slots<CB>(ra, 8 * u + gid, tig, va);
-          v_slots<CB>(rb, 8 * u + gid, tig, vb);
-          mma_u8u8_k32_from(d01, va[0], va[1], vb[0], vb[1], b0, b1, MAGIC);
-          mma_u8u8_k32_from(d23, va[2], va[3], vb[2], vb[3], b0, b1, MAGIC);
-          A[u][0] = __ffma2_rn(wc[0], isum2(d01[0], d01[1]), A[u][0]);
-          A[u][1] = __ffma2_rn(wc[1], isum2(d01[2], d01[3]), A[u][1]);
-          A[u][2] = __ffma2_rn(wc[2], isum2(d23[0], d23[1]), A[u][2]);
-          A[u][3] = __ffma2_rn(wc[3], isum2(d23[2], d23[3]), A[u][3]);
-        }
-        if (fine) {
+          for (int cc = 0; cc < 4; ++cc) f[cc] = __fmul2_rn(wt, splat((float)(1 << FB) * v_unscale<CB>(cc)));
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            uint32_t va[4], vb[4], d01[4], d23[4];
-            v_slots<FB>(fa, 8 * u + gid, tig, va);
-            v_slots<FB>(fb, 8 * u + gid, tig, vb);
-            mma_u8u8_k32_from(d01, va[0], va[1], vb[0], vb[1], b0, b1, MAGIC);
-            mma_u8u8_k32_from(d23, va[2], va[3], vb[2], vb[3], b0, b1, MAGIC);
-            A[u][0] = __ffma2_rn(wf[0], isum2(d01[0], d01[1]), A[u][0]);
-            A[u][1] = __ffma2_rn(wf[1], isum2(d01[2], d01[3]), A[u][1]);
-            A[u][2] = __ffma2_rn(wf[2], isum2(d23[0], d23[1]), A[u][2]);
-            A[u][3] = __ffma2_rn(wf[3], isum2(d23[2], d23[3]), A[u][3]);
+            uint32_t x[4], y[4];
+            va.slots(u, tig, x);
+            vb.slots(u, tig, y);
+            add(x, y, f, A[u]);
           }
         }
-        __syncwarp();  // the slot and pst have been read
-        if (issued < chunks) {
-          const int pg = J + NST;
-          if (pg < PAIRS) issue_next(pg, c, mask, k & 1); else issue_next(pg - PAIRS, n, next_mask, (k + 1) & 1);
+        if (left > 1) {
+          if (last) {
+            if (stay) { cp += c_skip; fp += f_skip; }
+            else {
+              cp = a.c.coarse + unit_n * SBG * RC + VWords<CB>::offset(gid, tig);
+              fp = a.c.fine + unit_n * SBG * RF + VWords<FB>::offset(gid, tig);
+            }
+          }
+          load_coarse();
+        }
+        if (pm) {
+          float2 f[4];
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) f[cc] = __fmul2_rn(ws, splat(v_unscale<FB>(cc)));
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            uint32_t x[4], y[4];
+            fa.slots(u, tig, x);
+            fb.slots(u, tig, y);
+            add(x, y, f, A[u]);
+          }
         }
       }
-      if (!ok) break;
-      run.l = __fadd2_rn(run.l, L);
+      J = 0;
+      if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      const uint8_t *meta = w.meta[k & 1];
+      L = __fmul2_rn(L, splat(BACK)); Hc = __fmul2_rn(Hc, splat(HOFF * BACK));
+      w.run[16][lane] = __fadd2_rn(w.run[16][lane], L);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const uint4 vm = lds128(meta + 512 + 16 * (8 * u + gid));
-        const float vb[4] = {bf_lo(vm.x), bf_hi(vm.x), bf_lo(vm.y), bf_hi(vm.y)}, vs[4] = {bf_lo(vm.z), bf_hi(vm.z), bf_lo(vm.w), bf_hi(vm.w)};
+        const uint4 vm = lds128(meta + 16 * (8 * u + gid));
+        const float vbs[4] = {bf_lo(vm.x), bf_hi(vm.x), bf_lo(vm.y), bf_hi(vm.y)}, vs[4] = {bf_lo(vm.z), bf_hi(vm.z), bf_lo(vm.w), bf_hi(vm.w)};
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc)
-          run.o[u][cc] = __fadd2_rn(run.o[u][cc], __ffma2_rn(splat(vs[cc]), __ffma2_rn(splat(HOFF), Hc, A[u][cc]), __fmul2_rn(splat(vb[cc]), L)));
+          w.run[4 * u + cc][lane] = __fadd2_rn(w.run[4 * u + cc][lane], __ffma2_rn(splat(vs[cc]), __ffma2_rn(splat(BACK), A[u][cc], Hc), __fmul2_rn(splat(vbs[cc]), L)));
       }
-      // on to the next group
-      c = n; mask = next_mask; Rc = Rn;
-      if (have_nn) {
-        const int nv = nn.b * hpr + nn.hir;
-        if (nv != r_vh) { R = mass_of(nv); r_vh = nv; }
-        next_mask = __ballot_sync(FULL, nn_lse - R > a.log2_tau);
-        n = nn;
-      }
+      __syncwarp();  // (the metadata buffer has been read)
+      c = n; unit = unit_n; cell = cell_n;
     }
-    if (ok) {
-      __syncwarp();
-      write_sums<QG>(cur_vh == first_vh ? &w.stage[0][0] : reinterpret_cast<float *>(w.pair[0]), run, lane);
-    } else if (lane == 0) report(a, 3);
-  }
-  __syncwarp();
-  if (ok && lane == 0) {
-#pragma unroll
-    for (int s = 0; s < NST; ++s) mbar_inval(&w.bar[s]);
-    mbar_inval(&w.bar_meta[0]);
-    mbar_inval(&w.bar_meta[1]);
+    const Sums r = sums();
+    __syncwarp();
+    write_sums<QG>(cur_vh == first_vh ? &w.stage[0][0] : reinterpret_cast<float *>(w.run), r, lane);
   }
   if (lane == 0) {
-    w.stage_vh[0] = ok ? first_vh : -1;
-    w.stage_vh[1] = ok && cur_vh != first_vh ? cur_vh : -1;
+    w.stage_vh[0] = first_vh;
+    w.stage_vh[1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
 #pragma unroll 1
@@ -772,14 +907,13 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     const int v = w.stage_vh[r];
     if (v < 0) continue;
     if (r == 0 && warp > 0) {
-      const ValueWarp<CB, FB> &prev = sm.w[warp - 1];
+      const ValueWarp &prev = sm.w[warp - 1];
       if ((prev.stage_vh[1] >= 0 ? prev.stage_vh[1] : prev.stage_vh[0]) == v) continue;
     }
     const bool open = r == 1 || w.stage_vh[1] < 0;
-    const float *own = r ? reinterpret_cast<const float *>(w.pair[0]) : &w.stage[0][0];
     float *dst = value_row(a, cta + v);
     for (int i = lane; i < QG * (PSTRIDE / 4); i += 32) {
-      float4 s = reinterpret_cast<const float4 *>(own)[i];
+      float4 s = reinterpret_cast<const float4 *>(r ? reinterpret_cast<const float *>(w.run) : &w.stage[0][0])[i];
       if (open)
         for (int x = warp + 1; x < VALUE_WARPS && sm.w[x].stage_vh[0] == v; ++x) {
           const float4 y = reinterpret_cast<const float4 *>(&sm.w[x].stage[0][0])[i];

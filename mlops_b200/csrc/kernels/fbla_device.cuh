@@ -73,10 +73,21 @@ __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32
 __device__ __forceinline__ float lg2(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float isum(uint32_t acc) { return __uint_as_float(acc) - MAGICF; }  // exact for |sum| < 2^22
 
+// maxima of three (one instruction where the compiler's PTX has it: CUDA 12.9 on)
+#if __CUDACC_VER_MAJOR__ * 100 + __CUDACC_VER_MINOR__ >= 1209
+__device__ __forceinline__ float max3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+__device__ __forceinline__ float max3_abs(float a, float b, float c) { float d; asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+#else
+__device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+__device__ __forceinline__ float max3_abs(float a, float b, float c) { return fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c)); }
+#endif
+
 // packed pairs of FP32 (FADD2 / FMUL2 / FFMA2 of sm_100: two lanes of arithmetic per instruction)
 __device__ __forceinline__ float2 isum2(uint32_t a, uint32_t b) {
   return __fadd2_rn(make_float2(__uint_as_float(a), __uint_as_float(b)), make_float2(-MAGICF, -MAGICF));
 }
+// two nonnegative s32 below 2^23 as the FP32 subnormals of the same bits: the numbers times 2^-149
+__device__ __forceinline__ float2 tiny2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
 __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
 
 // fl(127 / a) for a = max |q step|, both BF16, so that a has at most 16 significand bits; 0 for a = 0. One refinement step
@@ -120,6 +131,11 @@ __device__ __forceinline__ void mma_u8s8_k32_from(uint32_t (&d)[4], uint32_t a0,
 __device__ __forceinline__ void mma_u8u8_k32_from(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, uint32_t c) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
+}
+// D = A B; sums that are taken as FP32 subnormals (tiny2)
+__device__ __forceinline__ void mma_u8u8_k32_zero(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "n"(0));
 }
 __device__ __forceinline__ void mma_u8u8_k32(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
