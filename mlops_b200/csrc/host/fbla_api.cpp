@@ -73,6 +73,8 @@ int queries_per_virtual_head(int ratio) {
   if (ratio == 1 || ratio == 2 || ratio == 4) return ratio;
   return ratio % 4 == 0 ? 4 : ratio % 2 == 0 ? 2 : 1;
 }
+// the format's own selection threshold
+float usual_tau(const mlops_fbla_config *c) { return c->format == MLOPS_FBLA_3P3 ? 3e-4f : 1e-3f; }
 // softmax scale times log2(e): scores live in the log2 domain
 float log2_scale(const mlops_fbla_config *c) {
   const float natural = c->scale == 0.f ? 1.f / sqrtf((float)kHeadDim) : c->scale;
@@ -93,7 +95,8 @@ long long groups_of(long long tokens) { return (tokens + kGroup - 1) / kGroup; }
 // Byte offsets of the arrays fbla_kernels.h describes, in this order, inside the caller's scratch.
 struct ScratchMap {
   size_t lse, part, dpart, row_r, counts, items, item_off, status, bytes;
-  int nblocks, nslices, sets;
+  int nblocks, nslices;
+  bool two;  // with the weights of a decode in two sweeps behind lse
 };
 // `shape`: the launch shape on the current device; `tokens`: what the layout has room for; extra_rows: partial rows per
 // virtual head beyond the shape's own (the per_head of the size query)
@@ -101,7 +104,8 @@ struct ScratchMap {
 ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_k_decode &shape, int extra_rows, bool two_sweeps) {
   ScratchMap m{};
   const int ratio = c->q_heads / c->kv_heads, qg = queries_per_virtual_head(ratio);
-  m.sets = two_sweeps ? fbla_k_two_sets(c->batch, c->batch * c->kv_heads * (ratio / qg), shape.cb, c->capacity ? c->capacity : tokens) : 0;
+  // (the size does not depend on the call's tau: room for the weights where the format's own asks for them)
+  m.two = two_sweeps && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * (ratio / qg), c->capacity ? c->capacity : tokens, usual_tau(c));
   const size_t vheads = (size_t)c->batch * c->kv_heads * (ratio / qg);
   m.nblocks = (int)(groups_of(tokens) * kBlocksPerGroup);
   m.nslices = (m.nblocks + FBLA_K_SLICE - 1) / FBLA_K_SLICE;
@@ -113,7 +117,7 @@ ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_
   const size_t refine_rows = (size_t)shape.refine_ctas * shape.refine_warps + vheads;
   size_t at = 0;
   auto take = [&at](size_t bytes) { const size_t here = at; at += padded(bytes); return here; };
-  m.lse = take(fbla_k_two_floats(vheads, m.nblocks, qg, m.sets) * sizeof(float));
+  m.lse = take(fbla_k_two_cells(vheads, m.nblocks, qg) * (m.two ? FBLA_K_TWO_FLOATS : 1) * sizeof(float));
   m.part = take(coarse_rows * row_bytes);
   m.dpart = take(refine_rows * row_bytes);
   m.row_r = take(vheads * qg * sizeof(float));
@@ -203,10 +207,10 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   // Which coarse kernel runs is decided by the cache's room where it has one, for host and device lengths alike: both
   // calls on one cache then run the same kernels and return the same bits.
   fbla_k_decode_split(&a, room);
-  const float usual = c->format == MLOPS_FBLA_3P3 ? 3e-4f : 1e-3f, threshold = c->tau != 0.f ? c->tau : usual;
+  const float threshold = c->tau != 0.f ? c->tau : usual_tau(c);
   a.log2_tau = log2f(threshold);
   // (a shard's two phases share the scratch but only the second one uses tau: they decide by the format's own)
-  a.dense = (short)fbla_k_two_mode(m.sets, room, wants_output ? threshold : usual);
+  a.dense = m.two && (!wants_output || fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * a.vg, room, threshold));
   return MLOPS_FBLA_OK;
 }
 mlops_fbla_status enqueue_decode(const char *fn, fbla_k_decode &a, cudaStream_t stream) {

@@ -1,14 +1,14 @@
 // FBLA compressed-KV decode for sm_100a in two sweeps: every sub-block's scores, then every sub-block's values once.
 //
-//   * The score pass reads only the K half of the records (straight into registers, no staging), forms every sub-block's log2
-//     mass and its integer weights p = round(255 * 2^(s - max)), which it leaves in the scratch (16 bytes per sub-block and
-//     query, beside the block maximum), and the rows' running (m, l); it also serves the BF16 windows.
+//   * The score pass reads only the K half of the records, both planes (straight into registers, no staging), forms every
+//     sub-block's coarse and full scores, its log2 mass and its integer weights p = round(255 * 2^(s - max)) under both, which it
+//     leaves in the scratch (16 bytes per sub-block, query and set, beside the block maximum), and the rows' running (m, l); it
+//     also serves the BF16 windows.
 //   * The value pass knows every row's mass R before it starts, so it knows which (query, sub-block) pairs are selected. It
-//     reads the V half of the coarse records, of the fine records where some query selected the sub-block, and accumulates
-//     each sub-block once, in units of 2^-R -- no scores, no running maximum, no correction of a coarse sum, no item list.
-// FBLA_K_TWO_BOTH: the score pass reads K's fine half too and leaves both the coarse and the full weights, of which the value
-// pass takes the one its selection asks for: for rows whose sub-blocks are mostly selected. FBLA_K_TWO_COARSE: it leaves the coarse
-// weights only and the value pass scores the few selected sub-blocks again.
+//     reads the V half of the coarse records, of the fine records where some query selected the sub-block, takes the weights
+//     that the selection asks for and accumulates each sub-block once, in units of 2^-R -- no scores, no running maximum, no
+//     correction of a coarse sum, no item list.
+// For rows whose sub-blocks are mostly selected (fbla_k_two_sweeps); the decode of fbla_decode.cuh serves the others.
 // Both passes put the columns of several sub-blocks into one product's eight columns (queries of sub-block b in columns
 // b QG ..; its A fragments meet a B operand that is zero elsewhere, and all add into the same accumulators), so the softmax
 // arithmetic runs once per eight (sub-block, query) columns on full warps. Semantics, formats and the definition of every
@@ -110,11 +110,7 @@ __device__ __forceinline__ int *table_of(const fbla_k_decode &a) { return reinte
 // lse: per cell (virtual head, sub-block, query) the log2 mass; behind it, per set of weights (0 coarse, 1 full), the block maxima,
 // and then the sets' weights, 16 bytes per cell. (fbla_k_two_cells: cells, padded.)
 __device__ __forceinline__ size_t cells_of(const fbla_k_decode &a) { return fbla_k_two_cells((size_t)a.batch * a.kv_heads * a.vg, a.nblocks, a.qg); }
-__device__ __forceinline__ float *block_max(const fbla_k_decode &a, int set) { return a.lse + (size_t)(1 + set) * cells_of(a); }
-__device__ __forceinline__ uint32_t *weights(const fbla_k_decode &a, int set) {
-  const size_t n = cells_of(a);
-  return reinterpret_cast<uint32_t *>(a.lse) + (size_t)(1 + a.dense + 4 * set) * n;  // (a.dense: the number of sets)
-}
+__device__ __forceinline__ uint32_t *weights_of(const fbla_k_decode &a) { return reinterpret_cast<uint32_t *>(a.lse) + 3 * cells_of(a); }
 
 // ---- quantisation of the virtual head's queries for one group (as quantize_query_word), into QG rows of qst, QST_ROW bytes apart ----
 // am: the queries' max |z| (the same in every lane); dot: the lane's share of the result of a butterfly that hands half of the
@@ -250,12 +246,11 @@ __device__ __forceinline__ void score_item_units(const fbla_k_decode &a, int tot
   hi = first + min(count, at + (warp < nc ? with : without));
 }
 
-template <int CB, int FB, int QG, int MODE>
+template <int CB, int FB, int QG>
 __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   constexpr int NB = 8 / QG, UPG = QG;  // sub-blocks per unit, units per group
   constexpr float HOFF = .5f * ((1 << FB) - 1);
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
-  constexpr bool BOTH = MODE == FBLA_K_TWO_BOTH;
   ScoreSmem &sm = *reinterpret_cast<ScoreSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
   const int hpr = a.kv_heads * a.vg;
@@ -317,7 +312,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         kw[b].load(kp + b * RC, k_tail);
-        if (BOTH) kf[b].load(fp + b * RF, k_tail);
+        kf[b].load(fp + b * RF, k_tail);
       }
       kp += NB * RC; fp += NB * RF;
     };
@@ -336,7 +331,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
         m[0] = m[1] = -FBLA_INF; l[0] = l[1] = 0.f;
         const size_t cell = ((size_t)vh * a.nblocks + (size_t)group_of(a, c) * SBG) * QG + 8 * piece;
         lp = a.lse + cell + 2 * tig;
-        wp = weights(a, 0) + cell * 4 + lane;
+        wp = weights_of(a) + cell * 4 + lane;
 #pragma unroll
         for (int qi = 0; qi < QG; ++qi) q[qi] = __ldg(reinterpret_cast<const uint2 *>(a.q + (size_t)q_row(a, c.b, c.hir, qi) * D) + lane);
       }
@@ -371,7 +366,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
 #pragma unroll
         for (int i = 0; i < 8; ++i) mb[i] = SETS == 2 ? B[b % SETS][i] : gid / QG == b ? B[0][i] : 0u;
         if (b == 0) score_products<CB, true>(kw[b], mb, tig, dl, dh); else score_products<CB, false>(kw[b], mb, tig, dl, dh);
-        if (BOTH) { if (b == 0) score_products<FB, true>(kf[b], mb, tig, fl, fh); else score_products<FB, false>(kf[b], mb, tig, fl, fh); }
+        if (b == 0) score_products<FB, true>(kf[b], mb, tig, fl, fh); else score_products<FB, false>(kf[b], mb, tig, fl, fh);
       }
       // the next unit's words, and the next group's metadata with the group's first
       if (++piece == UPG) {
@@ -408,7 +403,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
       float2 mb, pA, pB;
       __syncwarp();  // (the previous unit's bytes have been read)
       softmax(__ffma2_rn(sqc, xA, c0), __ffma2_rn(sqc, xB, c0), mb, pA, pB, pst[0]);
-      if (BOTH) {
+      {
         const float2 fA = __ffma2_rn(isum2(fh[0], fh[1]), splat(UF), isum2(fl[0], fl[1])), fB = __ffma2_rn(isum2(fh[2], fh[3]), splat(UF), isum2(fl[2], fl[3]));
         float2 mf, qA, qB;
         softmax(__ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), xA, fA), qb2), __ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), xB, fB), qb2), mf, qA, qB, pst[1]);
@@ -430,7 +425,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
       l[1] = fmaf(sp.y, ex2(mb.y - m[1]), l[1]);
       __syncwarp();
       *wp = lds32(pst[0] + 4 * lane);
-      if (BOTH) wp[4 * n_cells] = lds32(pst[1] + 4 * lane);
+      wp[4 * n_cells] = lds32(pst[1] + 4 * lane);
       lp += 8; wp += 32;
     }
     leave(sm.stage[warp][cur_vh == first_vh ? 0 : 1]);
@@ -556,8 +551,6 @@ template <int BITS> struct VWords {
 };
 struct __align__(16) ValueWarp {
   uint8_t meta[2][512];        // V's metadata of the group in work and of the next
-  uint8_t qst[4 * QST_ROW];    // (scoring again: FBLA_K_TWO_COARSE)
-  uint8_t pst[128];
   float stage[4][PSTRIDE];     // the row set of the first virtual head of the warp's run
   // The current head's sums (Sums, [word][lane]): in registers they would halve the warps that an SM holds. At the end: the last
   // head's row set.
@@ -569,62 +562,6 @@ struct ValueSmem {
   Table table;
 };
 static_assert(sizeof(ValueSmem) + 128 <= 227 * 1024, "one CTA's shared memory");
-
-// scores of a record pair of a BITS plane: columns 0-3 the first record's queries, 4-7 the second's. Thread (gid, tig): tokens
-// gid, gid + 8 of columns 2 tig, 2 tig + 1. m0 / m1: all ones in the threads whose B column belongs to the first / second record.
-template <int BITS>
-__device__ __forceinline__ void qk_pair(const uint8_t *ra, const uint8_t *rb, int gid, int tig, const uint32_t (&B)[8], uint32_t m0, uint32_t m1, float2 (&x)[2]) {
-  constexpr int NC = BITS == 2 ? 4 : 2;
-  uint32_t d[NC][4];
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) d[c][i] = MAGIC;
-#pragma unroll
-  for (int par = 0; par < 2; ++par) {
-    const uint8_t *rec = par ? rb : ra, *p0 = rec + 16 * gid + 4 * tig, *p1 = p0 + 128;
-    const uint32_t m = par ? m1 : m0;
-    uint32_t b[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) b[i] = B[i] & m;
-    if (BITS == 4) {
-      const uint32_t a = lds32(p0), a8 = lds32(p1), bb = lds32(p0 + 512), bb8 = lds32(p1 + 512);
-      const uint32_t c = lds32(p0 + 256), c8 = lds32(p1 + 256), e = lds32(p0 + 768), e8 = lds32(p1 + 768);
-      constexpr uint32_t L = 0x0f0f0f0fu, H = 0xf0f0f0f0u;
-      mma_u8s8_k32(d[0], a & L, a8 & L, bb & L, bb8 & L, b[0], b[1]);
-      mma_u8s8_k32(d[1], a & H, a8 & H, bb & H, bb8 & H, b[2], b[3]);
-      mma_u8s8_k32(d[0], c & L, c8 & L, e & L, e8 & L, b[4], b[5]);
-      mma_u8s8_k32(d[1], c & H, c8 & H, e & H, e8 & H, b[6], b[7]);
-    } else if (BITS == 2) {
-      const uint32_t a = lds32(p0), a8 = lds32(p1), c = lds32(p0 + 256), c8 = lds32(p1 + 256);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t M = 0x03030303u << (2 * k);
-        mma_u8s8_k32(d[k % NC], a & M, a8 & M, c & M, c8 & M, b[k], b[4 + k]);
-      }
-    } else {
-      const int sh = 4 + (tig & 1), se = 3 * (tig & 1);
-      const uint8_t *q0 = rec + 1024 + 16 * gid + 4 * (tig >> 1), *q1 = q0 + 128;
-      const uint32_t a = lds32(p0), a8 = lds32(p1), c = lds32(p0 + 256), c8 = lds32(p1 + 256);
-      const uint32_t e = lds32(q0), e8 = lds32(q1), f = lds32(q0 + 8), f8 = lds32(q1 + 8);
-      constexpr uint32_t L = 0x07070707u, M = 0x38383838u, T2 = 0x03030303u, T1 = 0x04040404u;
-      mma_u8s8_k32(d[0], a & L, a8 & L, c & L, c8 & L, b[0], b[1]);
-      mma_u8s8_k32(d[1], a & M, a8 & M, c & M, c8 & M, b[2], b[3]);
-      mma_u8s8_k32(d[0], ((a >> 6) & T2) | ((e >> sh) & T1), ((a8 >> 6) & T2) | ((e8 >> sh) & T1),
-                   ((c >> 6) & T2) | ((f >> sh) & T1), ((c8 >> 6) & T2) | ((f8 >> sh) & T1), b[4], b[5]);
-      mma_u8s8_k32(d[0], (e >> se) & L, (e8 >> se) & L, (f >> se) & L, (f8 >> se) & L, b[6], b[7]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    if (BITS == 2)
-      x[i] = __ffma2_rn(isum2(d[3 % NC][2 * i], d[3 % NC][2 * i + 1]), splat(1.f / 64),
-                        __ffma2_rn(isum2(d[2 % NC][2 * i], d[2 % NC][2 * i + 1]), splat(1.f / 16),
-                                   __ffma2_rn(isum2(d[1][2 * i], d[1][2 * i + 1]), splat(1.f / 4), isum2(d[0][2 * i], d[0][2 * i + 1]))));
-    else
-      x[i] = __ffma2_rn(isum2(d[1][2 * i], d[1][2 * i + 1]), splat(BITS == 4 ? 1.f / 16 : 1.f / 8), isum2(d[0][2 * i], d[0][2 * i + 1]));
-  }
-}
 
 // the sums of one virtual head over the warp's pairs, in units of 2^-R: thread (gid, tig) holds channels 4 (8 u + gid) + cc of
 // queries 2 (tig & 1) + e, summed over the sub-blocks of parity tig >> 1
@@ -652,51 +589,10 @@ template <int QG> __device__ __forceinline__ void write_sums(float *p, const Sum
   }
 }
 
-// The full scores of a pair of sub-blocks, from both planes: {block maximum of the thread's columns 2 tig, 2 tig + 1 (sub-block
-// tig / 2, queries 2 (tig % 2) + e), the lane's word of P (column gid, tokens 4 tig ..)}. Rare: a function of its own.
-struct Again { float m0, m1; uint32_t p; };
 template <int CB, int FB, int QG>
-__device__ __noinline__ Again score_again(const uint8_t *ra, const uint8_t *fa, const uint8_t *meta, const uint16_t *q0, float sl, uint8_t *qst, uint8_t *pst, int lane) {
-  const int gid = lane >> 2, tig = lane & 3;
-  uint2 q[QG];
-#pragma unroll
-  for (int qi = 0; qi < QG; ++qi) q[qi] = __ldg(reinterpret_cast<const uint2 *>(q0 + qi * D) + lane);
-  float am[QG], dot;
-  __syncwarp();
-  if (QG < 4)
-    for (int i = lane; i < 4 * QST_ROW / 4; i += 32) reinterpret_cast<uint32_t *>(qst)[i] = 0u;
-  __syncwarp();
-  quantize_group<QG>(__ldg(reinterpret_cast<const uint4 *>(meta) + lane), q, qst, lane, am, dot);
-  __syncwarp();
-  uint32_t B[8];
-  qhat_frag<CB>(qst, gid & 3, tig, B);
-  const int qa = (2 * (tig & 1)) % QG, qz = (2 * (tig & 1) + 1) % QG;
-  const float2 amax = make_float2(QG == 4 && (tig & 1) ? am[2 % QG] : am[0], QG == 4 && (tig & 1) ? am[3 % QG] : am[1 % QG]);
-  const float2 sqf = __fmul2_rn(amax, splat(__fmul_rn(sl, 1.f / 127.f)));
-  const float2 qb = __fmul2_rn(make_float2(__shfl_sync(FULL, dot, dot_lane<QG>(qa)), __shfl_sync(FULL, dot, dot_lane<QG>(qz))), splat(sl));
-  const uint32_t m0 = gid < 4 ? FULL : 0u;
-  float2 x[2], y[2];
-  qk_pair<CB>(ra, ra + record_bytes(CB), gid, tig, B, m0, ~m0, x);
-  qk_pair<FB>(fa, fa + record_bytes(FB), gid, tig, B, m0, ~m0, y);
-  const float2 s0 = __ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), x[0], y[0]), qb), s1 = __ffma2_rn(sqf, __ffma2_rn(splat((float)(1 << FB)), x[1], y[1]), qb);
-  float2 mb = make_float2(fmaxf(s0.x, s1.x), fmaxf(s0.y, s1.y));
-#pragma unroll
-  for (int o = 4; o <= 16; o <<= 1) {
-    mb.x = fmaxf(mb.x, __shfl_xor_sync(FULL, mb.x, o));
-    mb.y = fmaxf(mb.y, __shfl_xor_sync(FULL, mb.y, o));
-  }
-  uint8_t *p = pst + 32 * tig + gid;
-  p[0] = (uint8_t)__float_as_uint(fmaf(ex2(s0.x - mb.x), 255.f, MAGICF)); p[16] = (uint8_t)__float_as_uint(fmaf(ex2(s0.y - mb.y), 255.f, MAGICF));
-  p[8] = (uint8_t)__float_as_uint(fmaf(ex2(s1.x - mb.x), 255.f, MAGICF)); p[24] = (uint8_t)__float_as_uint(fmaf(ex2(s1.y - mb.y), 255.f, MAGICF));
-  __syncwarp();
-  return Again{mb.x, mb.y, lds32(pst + 4 * lane)};
-}
-
-template <int CB, int FB, int QG, int MODE>
 __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
   constexpr float HOFF = .5f * ((1 << FB) - 1);
-  constexpr bool BOTH = MODE == FBLA_K_TWO_BOTH;
   ValueSmem &sm = *reinterpret_cast<ValueSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
   const int hpr = a.kv_heads * a.vg, cta = FBLA_POS::x();
@@ -718,20 +614,20 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     // a group's place: its unit, and its first cell
     auto unit_of = [&](const Cursor &x) { return (size_t)((x.b * hpr + x.hir) / a.vg) * a.hs + (size_t)group_of(a, x) * a.gs; };
     auto cell_of = [&](const Cursor &x) { return ((size_t)(x.b * hpr + x.hir) * a.nblocks + (size_t)group_of(a, x) * SBG) * QG; };
-    const float *const mx0 = block_max(a, 0), *const mx1 = block_max(a, 1);
+    const size_t n_cells = cells_of(a);
     const int pcol = (gid >> 2) * QG + (gid & 3);  // the lane's column of a pair's P words: sub-block gid / 4, query gid % 4
     const bool has = (gid & 3) < QG;
-    const uint32_t *const w0 = weights(a, 0) + 4 * pcol + tig, *const w1 = weights(a, 1) + 4 * pcol + tig;
+    const uint32_t *const w0 = weights_of(a) + 4 * pcol + tig, *const w1 = w0 + 4 * n_cells;
     // what a group's cells hold, lane l: cell l = (sub-block l / QG, query l % QG)
     float lse_n, mc_n, mf_n = 0.f;
     size_t cell = cell_of(c), cell_n;
     auto ask = [&](size_t at) {
       lse_n = -FBLA_INF; mc_n = 0.f;
-      if (lane < SBG * QG) { lse_n = __ldcg(a.lse + at + lane); mc_n = __ldcg(mx0 + at + lane); if (BOTH) mf_n = __ldcg(mx1 + at + lane); }
+      if (lane < SBG * QG) { const float *p = a.lse + at + lane; lse_n = __ldcg(p); mc_n = __ldcg(p + n_cells); mf_n = __ldcg(p + 2 * n_cells); }
     };
     uint32_t pc = 0u, pf = 0u;  // the next pair's words
     auto ask_p = [&](size_t at, int J) {
-      if (has) { pc = __ldcg(w0 + (at + 2 * QG * J) * 4); if (BOTH) pf = __ldcg(w1 + (at + 2 * QG * J) * 4); }
+      if (has) { pc = __ldcg(w0 + (at + 2 * QG * J) * 4); pf = __ldcg(w1 + (at + 2 * QG * J) * 4); }
     };
     size_t unit = unit_of(c);
     auto fetch_meta = [&](size_t un, int buf) {  // V's 512 bytes of metadata
@@ -779,7 +675,7 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
         }
       }
       const uint32_t mask = __ballot_sync(FULL, lse_n - R > a.log2_tau);  // bit cell: selected
-      float wl = ex2((BOTH && ((mask >> lane) & 1) ? mf_n : mc_n) - R) * UP;  // lane: the weight of its cell
+      float wl = ex2(((mask >> lane) & 1 ? mf_n : mc_n) - R) * UP;          // lane: the weight of its cell
       if (lane >= SBG * QG) wl = 0.f;
       // the next group: its cells, its metadata
       Cursor n = c;
@@ -805,16 +701,8 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
           fb.load(fp + RF, d1, d2);
         }
         fp += 2 * RF;
-        uint32_t pw = BOTH && ((pm >> pcol) & 1) ? pf : pc;
+        uint32_t pw = (pm >> pcol) & 1 ? pf : pc;
         if (!has) pw = 0u;
-        if (!BOTH && pm) {  // full scores of the pair, for the selected cells
-          const Again g = score_again<CB, FB, QG>(a.c.coarse + (unit * SBG + 2 * J) * RC, a.c.fine + (unit * SBG + 2 * J) * RF, reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024,
-                                                  a.q + (size_t)q_row(a, c.b, c.hir, 0) * D, a.sl, w.qst, w.pst, lane);
-          if (has && ((pm >> pcol) & 1)) pw = g.p;
-          const int mine = lane - 2 * QG * J, col = mine < 0 ? 0 : (mine / QG) * 4 + mine % QG;  // the lane's cell as a column of the pair
-          const float f0 = __shfl_sync(FULL, g.m0, col >> 1), f1 = __shfl_sync(FULL, g.m1, col >> 1);
-          if (mine >= 0 && mine < 2 * QG && ((mask >> lane) & 1)) wl = ex2(((col & 1) ? f1 : f0) - R) * UP;
-        }
         const bool last = J + 1 >= PAIRS;
         if (left > 1) ask_p(last ? cell_n : cell, last ? 0 : J + 1);
         // the thread's two columns: sub-block tig >> 1, queries 2 (tig & 1) + e

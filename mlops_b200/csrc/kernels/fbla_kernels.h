@@ -57,7 +57,7 @@ typedef struct {
   float *out_partial;  // [rows][FBLA_K_PSTRIDE] floats (phase 2)
   short status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
   short fold;          // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
-  short dense;         // 0: coarse sums, then corrections (fbla_decode.cuh); else two sweeps (fbla_dense.cuh), FBLA_K_TWO_*
+  short dense;         // 1: two sweeps, weights kept between them (fbla_dense.cuh); 0: coarse sums, then corrections (fbla_decode.cuh)
   short deal;          // how the coarse pass's warps share the work, FBLA_K_DEAL_*
 } fbla_k_decode;
 #define FBLA_K_DEAL_LENGTHS 0 /* a CTA's warps are split between windows and groups by the rows' lengths (short contexts) */
@@ -65,8 +65,6 @@ typedef struct {
 #define FBLA_K_DEAL_COST 2    /* every warp takes an equal cost share of windows and groups (long contexts) */
 
 #define FBLA_K_DENSE_MAX_BATCH 1024  /* batch rows of a dense decode: their prefix sums lie in shared memory */
-#define FBLA_K_TWO_COARSE 1 /* two sweeps, one set of weights kept between them: the coarse ones */
-#define FBLA_K_TWO_BOTH 2   /* two sweeps, two sets: coarse and full */
 #define FBLA_K_TWO_SCORE_WARPS 16
 #define FBLA_K_TWO_VALUE_WARPS 16
 #define FBLA_K_PSTRIDE 132 /* floats of one partial row: o[128], then (m, l) or (dl) and padding */
@@ -79,14 +77,12 @@ FBLA_HOST_API(cudaError_t fbla_k_decode_launch(const fbla_k_decode *a, cudaStrea
 FBLA_HOST_API(cudaError_t fbla_k_decode_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)
 // chooses the split of the coarse CTAs' warps for rows of about `tokens` tokens (after fbla_k_decode_shape; the scratch layout holds either)
 FBLA_HOST_API(void fbla_k_decode_split(fbla_k_decode *a, long long tokens);)
-// (virtual head, sub-block, query) cells of a decode, padded to 256 bytes of floats; and the floats of the `lse` array with
-// `sets` sets of weights behind it (fbla_dense.cuh)
+// (virtual head, sub-block, query) cells of a decode, padded to 256 bytes of floats. The `lse` array of a decode in two sweeps is
+// followed by 2 x cells block maxima and 2 x cells x 16 bytes of weights: FBLA_K_TWO_FLOATS floats per cell in all.
 static inline __host__ __device__ size_t fbla_k_two_cells(size_t vheads, int nblocks, int qg) { return (vheads * nblocks * qg + 63) / 64 * 64; }
-static inline __host__ __device__ size_t fbla_k_two_floats(size_t vheads, int nblocks, int qg, int sets) { return fbla_k_two_cells(vheads, nblocks, qg) * (1 + 5 * (size_t)sets); }
-// the sets of weights that a decode of rows of about `tokens` tokens keeps at most (0: it does not run in two sweeps), and how many it
-// keeps with selection threshold tau
-FBLA_HOST_API(int fbla_k_two_sets(int batch, int vheads, int cb, long long tokens);)
-FBLA_HOST_API(int fbla_k_two_mode(int sets, long long tokens, float tau);)
+#define FBLA_K_TWO_FLOATS 11
+// whether a decode of rows of about `tokens` tokens with selection threshold tau runs in two sweeps
+FBLA_HOST_API(int fbla_k_two_sweeps(int batch, int vheads, long long tokens, float tau);)
 // the dense passes (0 scores, 1 rows' masses, 2 values, 3 merge): a whole decode or shard phase; one pass
 FBLA_HOST_API(cudaError_t fbla_k_dense_launch(const fbla_k_decode *a, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_dense_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)
