@@ -38,7 +38,7 @@ extern "C" {
  * tcgen05 tensor cores; no split pieces, no TC_MERGE pass, no TRANSCODE: this library keeps no images; a prefill plan whose
  * count lives on the device and may reach 64 rows has a TC and a STREAM pass, of which the count activates one), FINISH (one KV
  * head's windows), COARSE / REFINE (CTA x of the persistent pass), SELECT (slice x of virtual head y), MERGE (one output
- * row), QKV (one (batch, KV head)), QKV_CHUNK (8 positions x of KV head y). */
+ * row); a decode in two sweeps: COARSE (scores), SELECT (the masses of 8 virtual heads), REFINE (values), MERGE, QKV (one (batch, KV head)), QKV_CHUNK (8 positions x of KV head y). */
 enum { MLOPS_FBLA_ITEM_CLOSE = 1, MLOPS_FBLA_ITEM_TRANSCODE, MLOPS_FBLA_ITEM_STREAM, MLOPS_FBLA_ITEM_TC,
        MLOPS_FBLA_ITEM_TC_MERGE, MLOPS_FBLA_ITEM_FINISH, MLOPS_FBLA_ITEM_COARSE, MLOPS_FBLA_ITEM_SELECT,
        MLOPS_FBLA_ITEM_REFINE, MLOPS_FBLA_ITEM_MERGE, MLOPS_FBLA_ITEM_QKV, MLOPS_FBLA_ITEM_QKV_CHUNK };
