@@ -12,7 +12,7 @@ __global__ void __launch_bounds__(32 * rows::WARPS, 1) attend_rows_kernel(const 
   attend_rows_item<CB, FB>(a, smem_raw);
 }
 
-template <int CB, int FB> static cudaError_t launch_rows(const fbla_k_prefill &a, int tiles, cudaStream_t stream) {
+template <int CB, int FB> static cudaError_t launch_rows(const fbla_k_prefill &a, int bundles, cudaStream_t stream) {
   constexpr int smem = (int)sizeof(rows::RowSmem<CB, FB>);
   static thread_local int configured[64] = {0};
   int dev = 0;
@@ -22,7 +22,7 @@ template <int CB, int FB> static cudaError_t launch_rows(const fbla_k_prefill &a
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  return launch(true, a.cluster, attend_rows_kernel<CB, FB>, dim3(tiles * a.cluster, a.batch * a.kv_heads), 32 * rows::WARPS, smem, stream, a);
+  return launch(true, a.cluster, attend_rows_kernel<CB, FB>, dim3(bundles * a.cluster, a.batch * a.kv_heads), 32 * rows::WARPS, smem, stream, a);
 }
 
 // tiles of the launch: with a device count that goes to the tensor-core pass from tc_min_rows rows on, no more than it leaves here
@@ -33,15 +33,17 @@ static int row_tiles(const fbla_k_prefill &a) {
 }  // namespace fbla
 
 extern "C" cudaError_t fbla_k_attend_rows_launch(const fbla_k_prefill *a, cudaStream_t stream) {
-  const int tiles = fbla::row_tiles(*a);
+  int bundles = fbla::row_tiles(*a);
   fbla_k_prefill args = *a;
-  if (a->length) {  // the shares follow from the device's length and count: the cluster has room for as many as they can become
+  if (a->length || a->dcount) {  // the deal follows from the device's length and count: the launch has room for what they can become
     const long long most = (a->room / fbla::G + fbla::rows::WARPS - 1) / fbla::rows::WARPS;
     args.cluster = most < 1 ? 1 : most > FBLA_K_ROW_SHARES ? FBLA_K_ROW_SHARES : (int)most;
   } else {
-    args.cluster = fbla::rows::row_shares((long long)tiles * a->batch * a->kv_heads, (a->n0 + a->count - 1) / fbla::G);
+    const fbla::rows::RowDeal deal = fbla::rows::row_deal(bundles, a->batch * a->kv_heads, (a->n0 + a->count - 1) / fbla::G);
+    bundles = (bundles + deal.tiles - 1) / deal.tiles;
+    args.cluster = deal.shares;
   }
-  return a->cb == 3 ? fbla::launch_rows<3, 3>(args, tiles, stream) : fbla::launch_rows<4, 2>(args, tiles, stream);
+  return a->cb == 3 ? fbla::launch_rows<3, 3>(args, bundles, stream) : fbla::launch_rows<4, 2>(args, bundles, stream);
 }
 
 extern "C" cudaError_t fbla_k_attend_rows_pass(fbla_k_prefill *a, fbla_k_pass *info) {

@@ -21,20 +21,36 @@ namespace fbla {
 namespace rows {
 
 constexpr int WARPS = 12, COLS = 8, PAIRS = SBG / 2, NST = 2;
-constexpr int MAX_SHARES = FBLA_K_ROW_SHARES;
+constexpr int MAX_SHARES = FBLA_K_ROW_SHARES, MAX_TILES = 4;
 constexpr int SET = COLS * FBLA_K_PSTRIDE;  // floats of a tile's row set: per row o[128], m, l
 
-// How many shares a tile's closed groups are split into: the number (at most a cluster of eight) that makes waves of
-// CTAs x groups per warp smallest, the smaller one of equals. SMs: a B200's, whatever the device, so that the choice is one
-// of the sizes alone.
-__host__ __device__ inline int row_shares(long long tiles, int groups) {
-  int best = 1;
-  long long least = -1;
-  for (int c = 1; c <= MAX_SHARES; ++c) {
-    const long long cost = (tiles * c + 147) / 148 * ((groups + WARPS * c - 1) / (WARPS * c));
-    if (least < 0 || cost < least) { least = cost; best = c; }
+// How the rows of `heads` KV heads are dealt: `tiles` row tiles to a CTA, `shares` CTAs (a cluster) to those tiles' groups.
+struct RowDeal { int tiles, shares; };
+// The deal whose longest SM has least to do: waves of CTAs x (a CTA's fixed cost + pairs of a warp). The fixed cost -- queries,
+// BF16 blocks, merges -- measured as that of five pairs. SMs: a B200's 148, whatever the device, so that the choice is one of
+// the sizes alone; clusters: what fits GPCs of 16, as every GPC has at least that many (96 clusters of three took three waves).
+// No more shares than give a CTA twelve groups, so that a launch whose length is on the device need not make larger clusters
+// than the cache's room asks for.
+__host__ __device__ inline int deal_cost(int t, int c, int row_tiles, int heads, int groups) {  // (what is no deal: the largest cost)
+  if (t > MAX_TILES || (t > 1 && t > row_tiles) || (c > 1 && WARPS * (c - 1) >= groups)) return (1 << 26) - 1;
+  const int room = c == 1 ? 148 : 8 * (16 / c) * c, warps = WARPS / t * c;
+  const long long cost = (long long)(((row_tiles + t - 1) / t * heads * c + room - 1) / room) * (5 + (PAIRS * groups + warps - 1) / warps);
+  return cost < (1 << 26) - 2 ? (int)cost : (1 << 26) - 2;
+}
+__host__ __device__ inline RowDeal row_deal(int row_tiles, int heads, int groups) {
+#ifdef __CUDA_ARCH__  // a lane per deal (every thread of the warp is here)
+  static_assert(MAX_TILES * MAX_SHARES == 32, "a deal per lane");
+  const unsigned lane = FBLA_POS::tid() & 31, n = __reduce_min_sync(FULL, (unsigned)deal_cost(1 + lane / MAX_SHARES, 1 + lane % MAX_SHARES, row_tiles, heads, groups) << 5 | lane) & 31;
+#else
+  int n = 0;
+  for (int x = 0, least = 1 << 26; x < MAX_TILES * MAX_SHARES; ++x) {
+    const int cost = deal_cost(1 + x / MAX_SHARES, 1 + x % MAX_SHARES, row_tiles, heads, groups);
+    if (cost < least) { least = cost; n = x; }
   }
-  return best;
+#endif
+  RowDeal d;
+  d.tiles = 1 + n / MAX_SHARES; d.shares = 1 + n % MAX_SHARES;
+  return d;
 }
 
 template <int CB, int FB> struct __align__(128) RowWarp {
@@ -50,8 +66,8 @@ struct __align__(16) RowStage {  // BF16 staging of a warp, in its ring
 };
 template <int CB, int FB> struct RowSmem {
   RowWarp<CB, FB> w[WARPS];
-  uint16_t q[COLS][D + 8];        // the tile's queries, BF16 (rows past the end: zero)
-  float share[MAX_SHARES][SET];   // the merged row sets of the shares this CTA has done
+  uint16_t q[MAX_TILES][COLS][D + 8];  // the tiles' queries, BF16 (rows past the end: zero)
+  float share[MAX_TILES][SET];         // the merged row sets of the shares this CTA has done
   int failed;
 };
 static_assert(sizeof(RowSmem<3, 3>) + 128 <= 227 * 1024 && sizeof(RowSmem<4, 2>) + 128 <= 227 * 1024, "one CTA's shared memory");
@@ -291,9 +307,16 @@ __device__ __forceinline__ void exact_blocks(const fbla_k_prefill &a, const uint
     if (gid == 0) { row[D] = mn; row[D + 1] = fmaf(sa[e], ls, sb[e] * l[e]); }
   }
 }
+// another share's sums (m, l, y) added to the sums (M, L, o) of the shares before it
+__device__ __forceinline__ void add_share(float &M, float &L, float4 &o, float m, float l, float4 y) {
+  const float mn = fmaxf(M, m), sa = M == -FBLA_INF ? 0.f : ex2(M - mn), sb = m == -FBLA_INF ? 0.f : ex2(m - mn);
+  M = mn;
+  L = fmaf(sa, L, sb * l);
+  o.x = fmaf(sa, o.x, sb * y.x); o.y = fmaf(sa, o.y, sb * y.y); o.z = fmaf(sa, o.z, sb * y.z); o.w = fmaf(sa, o.w, sb * y.w);
+}
 }  // namespace rows
 
-// CTA x of head y: tile x / cluster of eight rows, share x % cluster (cluster 1: every share of the tile, one after the other)
+// CTA x of head y: bundle x / cluster of the deal's tiles, share x % cluster (cluster 1: every share of the bundle, one after the other)
 template <int CB, int FB>
 __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
   using namespace rows;
@@ -303,13 +326,20 @@ __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_
   const int bh = FBLA_POS::y(), b = bh / a.kv_heads, kh = bh - b * a.kv_heads, qg = a.q_heads / a.kv_heads;
   const int n0 = (a.length ? FBLA_POS::ro(a.length + (a.lstride ? b : 0)) : 0) + a.n0;
   const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, n1 = n0 + count, rows = count * qg;
-  const int cluster = a.cluster, r0 = FBLA_POS::x() / cluster * COLS, rank = FBLA_POS::x() % cluster;
-  if (r0 >= rows || (a.tc_min_rows && rows >= a.tc_min_rows)) return;  // (cluster-uniform; a long device count is the tensor-core pass's work)
+  const int cluster = a.cluster, rank = FBLA_POS::x() % cluster;
+  if (a.tc_min_rows && rows >= a.tc_min_rows) return;  // (a long device count is the tensor-core pass's work)
+  const RowDeal deal = row_deal((rows + COLS - 1) / COLS, a.batch * a.kv_heads, (n1 - 1) / G);
+  const int shares = deal.shares, first_row = FBLA_POS::x() / cluster * deal.tiles * COLS, held = deal.tiles * COLS;
+  if (first_row >= rows) return;  // (cluster-uniform)
+  // the warp's tile, and its place among the tile's warps
+  const int per_tile = WARPS / deal.tiles, tile = min(warp / per_tile, deal.tiles - 1), place = warp - tile * per_tile;
+  const int r0 = first_row + tile * COLS;
+  const bool live = r0 < rows && place < per_tile;
   const int last = min(r0 + COLS, rows) - 1, max_pos = n0 + last / qg, own_min = (n0 + r0 / qg) / G, own_max = max_pos / G;
-  const int pairs = PAIRS * max(own_max - 1, 0);
-  const int shares = row_shares((long long)((rows + COLS - 1) / COLS) * a.batch * a.kv_heads, (n1 - 1) / G);
+  const int pairs = live ? PAIRS * max(own_max - 1, 0) : 0;
   // the BF16 blocks: group 0, then the rows' own groups
-  const int sink = min(SBG, max_pos / S + 1), own_lo = max(own_min, 1), exact = sink + (own_max >= own_lo ? SBG * (own_max - own_lo) + (max_pos - own_max * G) / S + 1 : 0);
+  const int sink = min(SBG, max_pos / S + 1), own_lo = max(own_min, 1);
+  const int exact = live ? sink + (own_max >= own_lo ? SBG * (own_max - own_lo) + (max_pos - own_max * G) / S + 1 : 0) : 0;
   int pos[2], own[2];
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
@@ -324,9 +354,9 @@ __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_
                                                                          : (x ? a.c.open_v : a.c.open_k) + eh + (size_t)(tp - (n0 - 1) / G * G) * D;
   };
   if (tid == 0) sm.failed = 0;
-  for (int e = tid; e < COLS * (D / 8); e += 32 * WARPS) {
-    const int c = e / (D / 8), r = r0 + c, i = r / qg;
-    *reinterpret_cast<uint4 *>(&sm.q[c][8 * (e % (D / 8))]) =
+  for (int e = tid; e < held * (D / 8); e += 32 * WARPS) {
+    const int c = e / (D / 8), r = first_row + c, i = r / qg;
+    *reinterpret_cast<uint4 *>(&sm.q[0][c][8 * (e % (D / 8))]) =
         r < rows ? __ldg(reinterpret_cast<const uint4 *>(a.q + ((size_t)(b * a.q_heads + kh * qg + (r - i * qg)) * a.count + i) * D) + e % (D / 8)) : make_uint4(0u, 0u, 0u, 0u);
   }
   RowWarp<CB, FB> &w = sm.w[warp];
@@ -339,7 +369,7 @@ __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_
   uint32_t uses = 0;
   bool ok = true;
   for (int s = cluster == 1 ? 0 : rank; s < shares; s += cluster) {
-    const int p0 = (int)((long long)pairs * s / shares), p1 = (int)((long long)pairs * (s + 1) / shares), per = (p1 - p0 + WARPS - 1) / WARPS;
+    const int p0 = (int)((long long)pairs * s / shares), p1 = (int)((long long)pairs * (s + 1) / shares), per = (p1 - p0 + per_tile - 1) / per_tile;
     State st;
     st.m[0] = st.m[1] = -FBLA_INF;
     st.l = make_float2(0.f, 0.f);
@@ -347,32 +377,39 @@ __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_
     for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc) st.o[u][cc] = make_float2(0.f, 0.f);
-    const int lo = min(p1, p0 + warp * per), hi = min(p1, lo + per);
-    if (ok && lo < hi) ok = closed_run<CB, FB>(a, w, sm.q, (size_t)bh * a.hs, lo, hi, own, uses, st, lane);
+    const int lo = min(p1, p0 + place * per), hi = min(p1, lo + per);
+    if (ok && lo < hi) ok = closed_run<CB, FB>(a, w, sm.q[tile], (size_t)bh * a.hs, lo, hi, own, uses, st, lane);
     float *const set = reinterpret_cast<float *>(w.pair[0]);
     if (ok) {
       write_state(set, st, lane);
       __syncwarp();
-      exact_blocks(a, sm.q, *reinterpret_cast<RowStage *>(w.pair[0] + SET * sizeof(float)), set, s * WARPS + warp, WARPS * shares, exact, sink, own_lo, n1, pos, own, lane, token_row);
+      exact_blocks(a, sm.q[tile], *reinterpret_cast<RowStage *>(w.pair[0] + SET * sizeof(float)), set, s * per_tile + place, per_tile * shares, exact, sink, own_lo, n1, pos, own, lane, token_row);
     } else if (lane == 0) {
       sm.failed = 1;
     }
     __syncthreads();
-    if (warp < COLS && !sm.failed) {  // row `warp` over the warps, in their order
+    for (int c = warp; c < held && !sm.failed; c += WARPS) {  // row c over its tile's warps, in their order, then behind the earlier shares
+      const RowWarp<CB, FB> *tw = sm.w + c / COLS * per_tile;
+      const int at = c % COLS * FBLA_K_PSTRIDE;
       float M = -FBLA_INF;
-#pragma unroll
-      for (int x = 0; x < WARPS; ++x) M = fmaxf(M, reinterpret_cast<const float *>(sm.w[x].pair[0])[warp * FBLA_K_PSTRIDE + D]);
+      for (int x = 0; x < per_tile; ++x) M = fmaxf(M, reinterpret_cast<const float *>(tw[x].pair[0])[at + D]);
       float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
       float l = 0.f;
-#pragma unroll
-      for (int x = 0; x < WARPS; ++x) {
-        const float *row = reinterpret_cast<const float *>(sm.w[x].pair[0]) + warp * FBLA_K_PSTRIDE;
+      for (int x = 0; x < per_tile; ++x) {
+        const float *row = reinterpret_cast<const float *>(tw[x].pair[0]) + at;
         const float e = row[D] == -FBLA_INF ? 0.f : ex2(row[D] - M);
         const float4 y = *reinterpret_cast<const float4 *>(row + 4 * lane);
         l = fmaf(e, row[D + 1], l);
         o.x = fmaf(e, y.x, o.x); o.y = fmaf(e, y.y, o.y); o.z = fmaf(e, y.z, o.z); o.w = fmaf(e, y.w, o.w);
       }
-      float *dst = sm.share[s] + warp * FBLA_K_PSTRIDE;
+      float *dst = sm.share[c / COLS] + at;
+      if (cluster == 1 && s > 0) {
+        float4 before = *reinterpret_cast<const float4 *>(dst + 4 * lane);
+        float m0 = dst[D], l0 = dst[D + 1];
+        __syncwarp();
+        add_share(m0, l0, before, M, l, o);
+        M = m0; l = l0; o = before;
+      }
       *reinterpret_cast<float4 *>(dst + 4 * lane) = o;
       if (lane == 0) { dst[D] = M; dst[D + 1] = l; }
     }
@@ -380,32 +417,24 @@ __device__ __forceinline__ void attend_rows_item(const fbla_k_prefill &a, uint8_
   }
   if (FBLA_STREAM_LAUNCH && cluster > 1) cluster_meet();
   // row c over the shares, in their order; a cluster's CTAs take rows rank, rank + cluster, ...
-  const int c = rank + warp * cluster;
-  if (warp < COLS && c < COLS && r0 + c < rows) {
-    bool failed = false;
+  for (int c = rank + warp * cluster; c < held && first_row + c < rows; c += WARPS * cluster) {
+    bool failed = sm.failed != 0;
+    const float *row = sm.share[c / COLS] + c % COLS * FBLA_K_PSTRIDE;
     float M = -FBLA_INF, l = 0.f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < shares; ++s) {
-      const float *row = sm.share[s] + c * FBLA_K_PSTRIDE;
-      float4 y;
-      float2 ml;
-      if (FBLA_STREAM_LAUNCH && cluster > 1) {
+    if (FBLA_STREAM_LAUNCH && cluster > 1) {
+      for (int s = 0; s < shares; ++s) {
         const uint32_t p = remote(row, s);
-        y = ld_remote4(p + 16 * lane);
-        ml = ld_remote2(p + 4 * D);
+        const float2 ml = ld_remote2(p + 4 * D);
         failed |= ld_remote1(remote(&sm.failed, s)) != 0;
-      } else {
-        y = *reinterpret_cast<const float4 *>(row + 4 * lane);
-        ml = *reinterpret_cast<const float2 *>(row + D);
-        failed |= sm.failed != 0;
+        add_share(M, l, o, ml.x, ml.y, ld_remote4(p + 16 * lane));
       }
-      const float mn = fmaxf(M, ml.x), sa = M == -FBLA_INF ? 0.f : ex2(M - mn), sb = ml.x == -FBLA_INF ? 0.f : ex2(ml.x - mn);
-      M = mn;
-      l = fmaf(sa, l, sb * ml.y);
-      o.x = fmaf(sa, o.x, sb * y.x); o.y = fmaf(sa, o.y, sb * y.y); o.z = fmaf(sa, o.z, sb * y.z); o.w = fmaf(sa, o.w, sb * y.w);
+    } else {
+      o = *reinterpret_cast<const float4 *>(row + 4 * lane);
+      l = row[D + 1];
     }
     const float inv = failed ? __int_as_float(0x7fc00000) : 1.f / l;
-    const int r = r0 + c, i = r / qg, hq = kh * qg + (r - i * qg);
+    const int r = first_row + c, i = r / qg, hq = kh * qg + (r - i * qg);
     uint16_t *orow = a.out + (size_t)(b * a.q_heads + hq) * a.out_hs + (size_t)i * a.out_ts;
     const uint32_t w0 = f32_to_bf16(o.x * inv) | (uint32_t)f32_to_bf16(o.y * inv) << 16, w1 = f32_to_bf16(o.z * inv) | (uint32_t)f32_to_bf16(o.w * inv) << 16;
     reinterpret_cast<uint2 *>(orow)[lane] = make_uint2(w0, w1);
