@@ -19,6 +19,11 @@ __device__ __forceinline__ void mma_u8u8_k16_from(uint32_t (&d)[4], uint32_t a0,
   asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(b0), "r"(c));
 }
+// D = A B; sums that are taken as FP32 subnormals (tiny2)
+__device__ __forceinline__ void mma_u8u8_k16_zero(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(b0), "n"(0));
+}
 __device__ __forceinline__ void mma_u8u8_k16(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
   asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
@@ -113,5 +118,67 @@ template <int BITS> __host__ __device__ constexpr float v_unscale(int cc) {
   return BITS == 4 ? (cc < 2 ? 1.f : 1.f / 16) : BITS == 2 ? (cc == 0 ? 1.f : cc == 1 ? 1.f / 4 : cc == 2 ? 1.f / 16 : 1.f / 64)
                                                             : (cc == 1 ? 1.f / 8 : 1.f);
 }
+
+// ---- full codes -------------------------------------------------------------------------------------------------------
+// Both planes of a slot joined to its code 2^FB h + f, four of them in the bytes of a word, times a class factor of their own
+// (4 + 2 bits: 4 but for the slots whose fine bits are the lowest; 3 + 3 bits: 1). One product and one sum then do for both
+// planes: half the matrix instructions, and a quarter of the FP32 work behind them, for one shift more per slot.
+__device__ __forceinline__ uint32_t join_4p2(int m, uint32_t h, uint32_t f) {  // m: place of the fine bits; h: the coarse word, low nibble m < 2, else high
+  return m == 0   ? ((h << 2) & 0x3c3c3c3cu) | (f & 0x03030303u)
+         : m == 1 ? ((h << 4) & 0xf0f0f0f0u) | (f & 0x0c0c0c0cu)
+                  : (h & 0xf0f0f0f0u) | ((f >> (2 * m - 2)) & 0x0c0c0c0cu);
+}
+// 3 + 3 bits: bits 0-2, bits 3-5, bits 3 hi .. of the words, and the slot that is split over two words (its top bit is bit sh of e)
+__device__ __forceinline__ uint32_t join_low(uint32_t h, uint32_t f) { return ((h << 3) & 0x38383838u) | (f & 0x07070707u); }
+__device__ __forceinline__ uint32_t join_mid(uint32_t h, uint32_t f) { return (h & 0x38383838u) | ((f >> 3) & 0x07070707u); }
+__device__ __forceinline__ uint32_t join_at(uint32_t h, uint32_t f, int hi) { return ((h << (3 - 3 * hi)) & 0x38383838u) | ((f >> (3 * hi)) & 0x07070707u); }
+__device__ __forceinline__ uint32_t join_split(uint32_t h, uint32_t eh, uint32_t f, uint32_t ef, int sh) {
+  return ((h >> 3) & 0x18181818u) | ((eh >> (sh - 3)) & 0x20202020u) | ((f >> 6) & 0x03030303u) | ((ef >> sh) & 0x04040404u);
+}
+
+// scores under the full codes: thread (gid, tig): tokens gid (x[0]) and gid + 8 (x[1]) of columns 2 tig, 2 tig + 1; B: qhat_frag<CB>
+template <int CB, int FB>
+__device__ __forceinline__ void qk_full(const uint8_t *crec, const uint8_t *frec, int gid, int tig, const uint32_t (&B)[8], float2 (&x)[2]) {
+  const uint8_t *p = crec + 16 * gid + 4 * tig, *r = frec + 16 * gid + 4 * tig;
+  uint32_t one[4], two[4];
+  if (CB == 4) {
+    const uint32_t a = lds32(p), a8 = lds32(p + 128), b = lds32(p + 512), b8 = lds32(p + 640);
+    const uint32_t c = lds32(p + 256), c8 = lds32(p + 384), d = lds32(p + 768), d8 = lds32(p + 896);
+    const uint32_t f = lds32(r), f8 = lds32(r + 128), g = lds32(r + 256), g8 = lds32(r + 384);
+    mma_u8s8_k32_from(two, join_4p2(1, b, f), join_4p2(1, b8, f8), join_4p2(2, a, f), join_4p2(2, a8, f8), B[1], B[2], MAGIC);
+    mma_u8s8_k32_from(one, join_4p2(0, a, f), join_4p2(0, a8, f8), join_4p2(0, c, g), join_4p2(0, c8, g8), B[0], B[4], MAGIC);
+    mma_u8s8_k32(two, join_4p2(3, b, f), join_4p2(3, b8, f8), join_4p2(1, d, g), join_4p2(1, d8, g8), B[3], B[5]);
+    mma_u8s8_k32(two, join_4p2(2, c, g), join_4p2(2, c8, g8), join_4p2(3, d, g), join_4p2(3, d8, g8), B[6], B[7]);
+  } else {
+    const int sh = 4 + (tig & 1), hi = tig & 1, t = 1024 + 16 * gid + 4 * (tig >> 1);
+    const uint32_t a = lds32(p), a8 = lds32(p + 128), c = lds32(p + 256), c8 = lds32(p + 384);
+    const uint32_t e = lds32(crec + t), e8 = lds32(crec + t + 128), g = lds32(crec + t + 8), g8 = lds32(crec + t + 136);
+    const uint32_t fa = lds32(r), fa8 = lds32(r + 128), fc = lds32(r + 256), fc8 = lds32(r + 384);
+    const uint32_t fe = lds32(frec + t), fe8 = lds32(frec + t + 128), fg = lds32(frec + t + 8), fg8 = lds32(frec + t + 136);
+    mma_u8s8_k32_from(one, join_low(a, fa), join_low(a8, fa8), join_low(c, fc), join_low(c8, fc8), B[0], B[1], MAGIC);
+    mma_u8s8_k32_from(two, join_mid(a, fa), join_mid(a8, fa8), join_mid(c, fc), join_mid(c8, fc8), B[2], B[3], MAGIC);
+    mma_u8s8_k32(one, join_split(a, e, fa, fe, sh), join_split(a8, e8, fa8, fe8, sh), join_split(c, g, fc, fg, sh), join_split(c8, g8, fc8, fg8, sh), B[4], B[5]);
+    mma_u8s8_k32(two, join_at(e, fe, hi), join_at(e8, fe8, hi), join_at(g, fg, hi), join_at(g8, fg8, hi), B[6], B[7]);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) x[i] = __ffma2_rn(isum2(two[2 * i], two[2 * i + 1]), splat(CB == 4 ? .25f : 1.f), isum2(one[2 * i], one[2 * i + 1]));
+}
+
+// the values' joined words, channels 4 l + 0..3 of record lane l, token quad tig; channel cc carries 1 / v_full_unscale<CB>(cc)
+template <int CB, int FB> __device__ __forceinline__ void v_full(const uint8_t *crec, const uint8_t *frec, int l, int tig, uint32_t (&v)[4]) {
+  const uint32_t f = lds32(frec + 512 + 16 * l + 4 * tig);
+  if (CB == 4) {
+    const uint2 h = lds64(crec + 1024 + 512 * (tig >> 1) + 16 * l + 8 * (tig & 1));
+    v[0] = join_4p2(0, h.x, f); v[1] = join_4p2(1, h.y, f); v[2] = join_4p2(2, h.x, f); v[3] = join_4p2(3, h.y, f);
+  } else {
+    const uint32_t h = lds32(crec + 512 + 16 * l + 4 * tig);
+    const uint2 y = lds64(crec + 1280 + 8 * l), z = lds64(frec + 1280 + 8 * l);
+    v[0] = join_low(h, f);
+    v[1] = join_mid(h, f);
+    v[2] = join_at((tig & 1) ? y.y : y.x, (tig & 1) ? z.y : z.x, tig >> 1);
+    v[3] = join_split(h, (tig >> 1) ? y.y : y.x, f, (tig >> 1) ? z.y : z.x, 4 + (tig & 1));
+  }
+}
+template <int CB> __host__ __device__ constexpr float v_full_unscale(int cc) { return CB == 4 && cc > 0 ? .25f : 1.f; }
 
 }  // namespace fbla

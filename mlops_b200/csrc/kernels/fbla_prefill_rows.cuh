@@ -73,16 +73,6 @@ template <int CB, int FB> struct RowSmem {
 static_assert(sizeof(RowSmem<3, 3>) + 128 <= 227 * 1024 && sizeof(RowSmem<4, 2>) + 128 <= 227 * 1024, "one CTA's shared memory");
 static_assert(SET * sizeof(float) + sizeof(RowStage) <= sizeof(RowWarp<4, 2>::pair) && SET * sizeof(float) + sizeof(RowStage) <= sizeof(RowWarp<3, 3>::pair), "row set and staging fit the ring");
 
-// scores of one sub-block under both planes: code units = 2^FB h + f; thread (gid, tig): tokens gid (x[0]), gid + 8 (x[1]) of rows 2 tig, 2 tig + 1
-template <int CB, int FB>
-__device__ __forceinline__ void qk_full(const uint8_t *crec, const uint8_t *frec, int gid, int tig, const uint32_t (&B)[8], float2 (&x)[2]) {
-  float h[4], f[4];
-  qk_tile<CB>(crec, gid, tig, B, h);
-  qk_tile<FB>(frec, gid, tig, B, f);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) x[i] = __ffma2_rn(splat((float)(1 << FB)), make_float2(h[2 * i], h[2 * i + 1]), make_float2(f[2 * i], f[2 * i + 1]));
-}
-
 // the sums of a warp: rows 2 tig + e, e = 0, 1, in (.x, .y); channels 4 (8 u + gid) + cc
 struct State { float m[2]; float2 l, o[4][4]; };
 
@@ -92,6 +82,8 @@ template <int CB, int FB>
 __device__ __forceinline__ bool closed_run(const fbla_k_prefill &a, RowWarp<CB, FB> &w, const uint16_t (&q)[COLS][D + 8], size_t head, int lo, int hi,
                                            const int (&own)[2], uint32_t &uses, State &st, int lane) {
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
+  // A group's integer sums are read as the FP32 subnormals of the same bits (2^-149 each); the weights carry 2^75, the group's end 2^74
+  constexpr float UP = 37778931862957161709568.f /* 2^75 */, BACK = 18889465931478580854784.f /* 2^74 */;
   const int gid = lane >> 2, tig = lane & 3;
   const uint32_t base = uses;  // ring uses before this run (the barriers live through all of a CTA's shares)
   auto issue = [&](int p) {    // lane 0
@@ -169,43 +161,35 @@ __device__ __forceinline__ bool closed_run(const fbla_k_prefill &a, RowWarp<CB, 
         const float2 wt = make_float2(on[0] ? ex2(mb[0] - st.m[0]) : 0.f, on[1] ? ex2(mb[1] - st.m[1]) : 0.f);
         __syncwarp();
         const uint32_t b0 = lds32(w.pst + 4 * lane);  // row gid, tokens 4 tig ..
+        const float2 w0 = __fmul2_rn(wt, splat(UP)), w1 = __fmul2_rn(wt, splat(UP * v_full_unscale<CB>(1)));
         {
           uint32_t d[4];
-          mma_u8u8_k16_from(d, 0x01010101u, 0x01010101u, b0, MAGIC);
-          L = __ffma2_rn(wt, isum2(d[0], d[1]), L);
-        }
-        float2 wc[4], wf[4];
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          wc[cc] = __fmul2_rn(wt, splat((float)(1 << FB) * v_unscale<CB>(cc)));
-          wf[cc] = __fmul2_rn(wt, splat(v_unscale<FB>(cc)));
+          mma_u8u8_k16_zero(d, 0x01010101u, 0x01010101u, b0);
+          L = __ffma2_rn(w0, tiny2(d[0], d[1]), L);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          uint32_t vh[4], vl[4], h01[4], h23[4], l01[4], l23[4];
-          v_slots<CB>(crec, 8 * u + gid, tig, vh);
-          v_slots<FB>(frec, 8 * u + gid, tig, vl);
-          mma_u8u8_k16_from(h01, vh[0], vh[1], b0, MAGIC);
-          mma_u8u8_k16_from(h23, vh[2], vh[3], b0, MAGIC);
-          mma_u8u8_k16_from(l01, vl[0], vl[1], b0, MAGIC);
-          mma_u8u8_k16_from(l23, vl[2], vl[3], b0, MAGIC);
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            const uint32_t *hh = cc < 2 ? h01 : h23, *ll = cc < 2 ? l01 : l23;
-            A[u][cc] = __ffma2_rn(wc[cc], isum2(hh[2 * (cc & 1)], hh[2 * (cc & 1) + 1]), __ffma2_rn(wf[cc], isum2(ll[2 * (cc & 1)], ll[2 * (cc & 1) + 1]), A[u][cc]));
-          }
+          uint32_t v[4], d01[4], d23[4];
+          v_full<CB, FB>(crec, frec, 8 * u + gid, tig, v);
+          mma_u8u8_k16_zero(d01, v[0], v[1], b0);
+          mma_u8u8_k16_zero(d23, v[2], v[3], b0);
+          A[u][0] = __ffma2_rn(w0, tiny2(d01[0], d01[1]), A[u][0]);
+          A[u][1] = __ffma2_rn(w1, tiny2(d01[2], d01[3]), A[u][1]);
+          A[u][2] = __ffma2_rn(w1, tiny2(d23[0], d23[1]), A[u][2]);
+          A[u][3] = __ffma2_rn(w1, tiny2(d23[2], d23[3]), A[u][3]);
         }
         __syncwarp();  // pst -- and behind the second sub-block the slot -- has been read
       }
       if (lane == 0 && p + NST < hi) issue(p + NST);
     }
+    L = __fmul2_rn(L, splat(BACK));
     st.l = __fadd2_rn(st.l, L);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const uint4 vm = lds128(meta + 512 + 16 * (8 * u + gid));
       const float vb[4] = {bf_lo(vm.x), bf_hi(vm.x), bf_lo(vm.y), bf_hi(vm.y)}, vs[4] = {bf_lo(vm.z), bf_hi(vm.z), bf_lo(vm.w), bf_hi(vm.w)};
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) st.o[u][cc] = __fadd2_rn(st.o[u][cc], __ffma2_rn(splat(vs[cc]), A[u][cc], __fmul2_rn(splat(vb[cc]), L)));
+      for (int cc = 0; cc < 4; ++cc) st.o[u][cc] = __ffma2_rn(splat(vs[cc]), __fmul2_rn(splat(BACK), A[u][cc]), __ffma2_rn(splat(vb[cc]), L, st.o[u][cc]));
     }
     __syncwarp();
   }
