@@ -1,6 +1,6 @@
 """The few-row prefill attention (chunks of fewer than 64 rows per KV head) where its dealing can go wrong: no cache, one
-group, a chunk that crosses a group boundary, tiles with padding rows, one and several shares of a tile's groups; host and
-device lengths and an executor's items bit for bit."""
+group, a chunk that crosses a group boundary, tiles with padding rows, one and several shares of a tile's groups, several
+tiles to a CTA (the last CTA's fewer); host and device lengths and an executor's items bit for bit."""
 import ctypes
 
 import pytest
@@ -20,7 +20,8 @@ def ours():
 
 @pytest.mark.parametrize("mode", ["3+3", "4+2"])
 @pytest.mark.parametrize("B,QH,KH,n0,n", [(1, 1, 1, 0, 1), (1, 4, 2, 0, 20), (2, 2, 2, 127, 3), (1, 8, 2, 250, 13), (3, 4, 1, 1000, 5), (1, 2, 1, 128, 31),
-                                          (1, 8, 2, 5000, 6), (1, 1, 1, 9215, 2), (4, 16, 4, 3000, 1), (1, 6, 2, 12345, 21)])
+                                          (1, 8, 2, 5000, 6), (1, 1, 1, 9215, 2), (4, 16, 4, 3000, 1), (1, 6, 2, 12345, 21),
+                                          (4, 8, 8, 1669, 36), (1, 8, 8, 6275, 43), (4, 24, 24, 2000, 25)])
 def test_few_rows(ours, oracle, mode, B, QH, KH, n0, n):
     q, k, v = datagen.uneven_case(n0 + n, B, QH, KH, n0 + n, q_rows=n0 + n)
     q = q[:, :, n0:].copy()
