@@ -5,15 +5,17 @@
 // to 0..p: group 0 (sink) and its own group in BF16 from the windows / the chunk, closed groups 1..own-1 through their
 // full 6-bit codes (coarse << FB | fine) with the per-(row, group) int8 qhat, 16-token integer P blocks everywhere.
 //
-// Eight rows of one KV head are the eight columns of the decode's integer tensor-core products (fbla_frag.cuh): a tile's
-// closed groups are dealt in pairs of sub-blocks to twelve warps, each streaming its run through a private two-stage ring
-// with a running (m, l, o); the BF16 blocks follow on BF16 products; the warps' rows are then merged in warp order. A long
-// cache and few tiles would leave most SMs idle, so a tile's pairs are also split into `shares`, one CTA of a thread-block
-// cluster each, whose merged rows the cluster reads from each other's shared memory: no scratch, no second launch. The
-// number of shares follows from the sizes alone (row_shares), and a CTA that has to do the whole tile (an executor's item)
-// takes the shares one after the other, so that both give the same bits.
-// Bound by instruction issue (about 2 500 warp instructions per group and tile). One warp per row walking the whole cache,
-// as this pass once did: 4 sequences x 5 drafted tokens at 12 345 tokens (32 / 8 heads) 1 670 us.
+// Eight rows of one KV head (a row tile) are the eight columns of the decode's integer tensor-core products, both planes joined
+// to their codes on the way into the fragments (fbla_frag.cuh). A CTA's twelve warps are dealt to one to four row tiles, and a
+// tile's closed groups, in pairs of sub-blocks, to its warps, each streaming its run through a private two-stage ring with a
+// running (m, l, o); the BF16 blocks follow on BF16 products; the warps' rows are then merged in warp order. A long cache and
+// few tiles would leave most SMs idle, so the pairs are also split into shares, one CTA of a thread-block cluster each, whose
+// merged rows the cluster reads from each other's shared memory: no scratch, no second launch. Tiles and shares follow from the
+// sizes alone (row_deal), and a CTA that has to do every share (an executor's item) takes them one after the other, so that
+// both give the same bits.
+// Bound by instruction latency: three warps per scheduler (the sums take the registers) issue about 0.5 instructions per cycle.
+// 4 sequences x 5 drafted tokens at 12 345 tokens (32 / 8 heads): one warp per row walking the whole cache 1 670 us; a tile
+// to a CTA and as many shares as even out the groups 120 (96 clusters of three: three waves); the deal 78; joined codes 65.
 #pragma once
 #include "fbla_decode.cuh"
 
