@@ -443,7 +443,7 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
   constexpr float HOFF = .5f * ((1 << FB) - 1);
   StreamWarp<CB> &sm = ring.w;
   const int gid = lane >> 2, tig = lane & 3;
-  const bool odd = tig >> 1;  // threads tig >= 2 accumulate the odd sub-block of every pair (columns 4..7 of the value products)
+  // (threads tig >= 2 hold the odd sub-block of every pair: columns 4..7 of the score and value products)
   if (!ring.wait_meta(k)) return false;
   const uint8_t *meta = sm.meta[k & 1];
   // qhat of every query; c0 / sqc of the thread's two score columns
@@ -460,58 +460,37 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
     }
   }
   __syncwarp();
-  uint32_t B[8];
-  qhat_frag<CB>(sm.qst, gid, tig, B);
-  // the group's sums in code units, relative to the running maximum run.m: A = sum w y, Bs = sum w sum p
+  uint32_t X[8], Y[8];
+  qhat_frag<CB>(sm.qst, gid & 3, tig, X);
+#pragma unroll
+  for (int m = 0; m < 8; ++m) { Y[m] = gid < 4 ? 0u : X[m]; X[m] = gid < 4 ? X[m] : 0u; }
+  // the group's sums in code units, relative to the running maximum run.m: A = sum w y, Bs = sum w sum p. A's integer sums are
+  // read as the FP32 subnormals of the same bits (2^-149 each); its weights carry 2^75, the group's end the other 2^74.
+  constexpr float UP = 37778931862957161709568.f /* 2^75 */, BACK = 18889465931478580854784.f /* 2^74 */;
   float2 A[4][4], Bs = make_float2(0.f, 0.f);
 #pragma unroll
   for (int u = 0; u < 4; ++u)
 #pragma unroll
     for (int cc = 0; cc < 4; ++cc) A[u][cc] = make_float2(0.f, 0.f);
   const float2 sqc2 = make_float2(sqc[0], sqc[1]), c02 = make_float2(c0[0], c0[1]);
-  // Software pipeline over the group's four record pairs: the scores of pair J + 1 (stage A: shared loads, score products,
-  // sub-block maxima) are issued before the softmax and value products of pair J (stage B), so that each stage's
-  // latencies are covered by the other's instructions.
-  struct Scores { float s[2][4], mb[2][2]; };
-  // stage A of pair J: scores s[par][i], i = (token gid, column 2 tig), (gid, 2 tig + 1), (gid + 8, 2 tig), (gid + 8, 2 tig + 1)
-  // (only columns < QG, i.e. threads tig < 2, are queries; the others multiply zero rows of qst), and their maxima
-  auto stage_a = [&](int J, Scores &sc) -> bool {
+#pragma unroll 1
+  for (int J = 0; J < SBG / 2; ++J) {
     const int p = CoarseShape<CB>::CPG * k + J / CoarseShape<CB>::PPC;  // the pair's chunk
     if (J % CoarseShape<CB>::PPC == 0 && !ring.wait_pair(p)) return false;
     const uint8_t *ra = sm.pair[p % CoarseShape<CB>::NP] + (J % CoarseShape<CB>::PPC) * CoarseShape<CB>::PAIR_BYTES, *rb = ra + RB;
+    // scores of the thread's own sub-block 2 J + (tig >> 1), queries 2 (tig & 1) + e in (.x, .y): tokens gid, gid + 8; their maxima
+    float2 s[2];
+    qk_pair<CB>(ra, rb, gid, tig, X, Y, s);
 #pragma unroll
-    for (int par = 0; par < 2; ++par) {
-      float x[4];
-      qk_tile<CB>(par ? rb : ra, gid, tig, B, x);
-      const float2 s01 = __ffma2_rn(sqc2, make_float2(x[0], x[1]), c02), s23 = __ffma2_rn(sqc2, make_float2(x[2], x[3]), c02);
-      sc.s[par][0] = s01.x; sc.s[par][1] = s01.y; sc.s[par][2] = s23.x; sc.s[par][3] = s23.y;
-    }
+    for (int r = 0; r < 2; ++r) s[r] = __ffma2_rn(sqc2, s[r], c02);
+    float mbj[2] = {fmaxf(s[0].x, s[1].x), fmaxf(s[0].y, s[1].y)}, mp[2];
 #pragma unroll
-    for (int par = 0; par < 2; ++par)
+    for (int o = 4; o <= 16; o <<= 1)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float v = fmaxf(sc.s[par][e], sc.s[par][2 + e]);
-        v = fmaxf(v, __shfl_xor_sync(FULL, v, 4));
-        v = fmaxf(v, __shfl_xor_sync(FULL, v, 8));
-        v = fmaxf(v, __shfl_xor_sync(FULL, v, 16));
-        sc.mb[par][e] = v;
-      }
-    return true;
-  };
-  // stage B of pair J: sub-blocks 2 J (parity 0) and 2 J + 1 (parity 1)
-  auto stage_b = [&](int J, const Scores &sc) {
-    const int p = CoarseShape<CB>::CPG * k + J / CoarseShape<CB>::PPC;
-    const uint8_t *ra = sm.pair[p % CoarseShape<CB>::NP] + (J % CoarseShape<CB>::PPC) * CoarseShape<CB>::PAIR_BYTES, *rb = ra + RB;
-    // the thread's own sub-block 2 J + (tig >> 1) of queries 2 (tig & 1) + e, and the pair's maximum (the same value in
-    // both parities' threads, so their running maxima stay equal)
-    float mbj[2], mp[2];
+      for (int e = 0; e < 2; ++e) mbj[e] = fmaxf(mbj[e], __shfl_xor_sync(FULL, mbj[e], o));
+    // the pair's maximum (the same value in both parities' threads, so their running maxima stay equal)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float other = __shfl_xor_sync(FULL, sc.mb[1][e], 2);
-      mbj[e] = odd ? other : sc.mb[0][e];
-      const float pm = fmaxf(sc.mb[0][e], sc.mb[1][e]), pmo = __shfl_xor_sync(FULL, pm, 2);
-      mp[e] = odd ? pmo : pm;
-    }
+    for (int e = 0; e < 2; ++e) mp[e] = fmaxf(mbj[e], __shfl_xor_sync(FULL, mbj[e], 2));
     // the running maximum moves only when a pair exceeds it by more than 2^8 (weights stay <= 2^8; the rescale is rare)
     const bool grow = mp[0] > run.m[0] + 8.f || mp[1] > run.m[1] + 8.f;
     if (__any_sync(FULL, grow)) {
@@ -530,22 +509,20 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) { run.o[u][cc] = __fmul2_rn(run.o[u][cc], al2); A[u][cc] = __fmul2_rn(A[u][cc], al2); }
     }
-    if (tig < 2) {  // P bytes: pst[parity][query][token]
+    // P bytes: pst[parity][query][token]
+    const float2 nm = make_float2(-mbj[0], -mbj[1]);
+    uint8_t *const pb = sm.pst + 32 * tig + gid;
 #pragma unroll
-      for (int par = 0; par < 2; ++par)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          if (query_valid<QG>(tig, e)) {
-            const int qe = 2 * tig + e;
-            sm.pst[(par * 4 + qe) * 16 + gid] = (uint8_t)__float_as_uint(fmaf(ex2(sc.s[par][e] - sc.mb[par][e]), 255.f, MAGICF));
-            sm.pst[(par * 4 + qe) * 16 + gid + 8] = (uint8_t)__float_as_uint(fmaf(ex2(sc.s[par][2 + e] - sc.mb[par][e]), 255.f, MAGICF));
-          }
+    for (int r = 0; r < 2; ++r) {
+      const float2 d = __fadd2_rn(s[r], nm), pr = __ffma2_rn(make_float2(ex2(d.x), ex2(d.y)), splat(255.f), splat(MAGICF));
+      if (query_valid<QG>(tig, 0)) pb[8 * r] = (uint8_t)__float_as_uint(pr.x);
+      if (query_valid<QG>(tig, 1)) pb[8 * r + 16] = (uint8_t)__float_as_uint(pr.y);
     }
     __syncwarp();
     // column gid of the value products: gid < 4: parity 0, query gid, k block = tokens 4 tig ..; gid >= 4: parity 1
     const uint32_t pw = lds32(sm.pst + 4 * lane);
     const uint32_t b0 = gid < 4 ? pw : 0u, b1 = gid < 4 ? 0u : pw;
-    const float2 wj = make_float2(ex2(mbj[0] - run.m[0]), ex2(mbj[1] - run.m[1]));
+    const float2 wj = make_float2(ex2(mbj[0] - run.m[0]), ex2(mbj[1] - run.m[1])), wu = __fmul2_rn(wj, splat(UP));
     {  // sum p of both sub-blocks, every column: a product with an all-ones A
       uint32_t d[4];
       mma_u8u8_k32_from(d, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, b0, b1, MAGIC);
@@ -562,21 +539,15 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
       v_slots<CB>(ra, 8 * u + gid, tig, va);
       v_slots<CB>(rb, 8 * u + gid, tig, vb);
       uint32_t d01[4], d23[4];
-      mma_u8u8_k32_from(d01, va[0], va[1], vb[0], vb[1], b0, b1, MAGIC);  // rows gid: channel cc 0, gid + 8: cc 1
-      mma_u8u8_k32_from(d23, va[2], va[3], vb[2], vb[3], b0, b1, MAGIC);  // cc 2, cc 3
-      A[u][0] = __ffma2_rn(wj, isum2(d01[0], d01[1]), A[u][0]);
-      A[u][1] = __ffma2_rn(wj, isum2(d01[2], d01[3]), A[u][1]);
-      A[u][2] = __ffma2_rn(wj, isum2(d23[0], d23[1]), A[u][2]);
-      A[u][3] = __ffma2_rn(wj, isum2(d23[2], d23[3]), A[u][3]);
+      mma_u8u8_k32_zero(d01, va[0], va[1], vb[0], vb[1], b0, b1);  // rows gid: channel cc 0, gid + 8: cc 1
+      mma_u8u8_k32_zero(d23, va[2], va[3], vb[2], vb[3], b0, b1);  // cc 2, cc 3
+      A[u][0] = __ffma2_rn(wu, tiny2(d01[0], d01[1]), A[u][0]);
+      A[u][1] = __ffma2_rn(wu, tiny2(d01[2], d01[3]), A[u][1]);
+      A[u][2] = __ffma2_rn(wu, tiny2(d23[0], d23[1]), A[u][2]);
+      A[u][3] = __ffma2_rn(wu, tiny2(d23[2], d23[3]), A[u][3]);
     }
     __syncwarp();  // pst is free; after a chunk's last pair its slot is too
     if (J % CoarseShape<CB>::PPC == CoarseShape<CB>::PPC - 1) ring.issue_next();  // refill the slot with the chunk NP ahead
-  };
-#pragma unroll 1
-  for (int J = 0; J < SBG / 2; ++J) {
-    Scores sc;
-    if (!stage_a(J, sc)) return false;
-    stage_b(J, sc);
   }
   // fold the group into the running softmax: o += vs' A + vb' B, coarse cell midpoints folded into vb'
   run.l[0] += Bs.x; run.l[1] += Bs.y;
@@ -587,7 +558,7 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
 #pragma unroll
     for (int cc = 0; cc < 4; ++cc) {
       const float vbp = fmaf(vs[cc], HOFF, vb[cc]), vsp = __fmul_rn(vs[cc], (float)(1 << FB) * v_unscale<CB>(cc));
-      run.o[u][cc] = __fadd2_rn(run.o[u][cc], __ffma2_rn(splat(vsp), A[u][cc], __fmul2_rn(splat(vbp), Bs)));
+      run.o[u][cc] = __fadd2_rn(run.o[u][cc], __ffma2_rn(splat(vsp), __fmul2_rn(splat(BACK), A[u][cc]), __fmul2_rn(splat(vbp), Bs)));
     }
   }
   return true;

@@ -93,6 +93,56 @@ template <int BITS> __device__ __forceinline__ void qk_tile(const uint8_t *rec, 
   }
 }
 
+// The same scores of two sub-blocks at once, for at most four queries: columns 0-3 are the queries under sub-block 0 (k blocks
+// 0-3 of every product), columns 4-7 under sub-block 1 (k blocks 4-7). As many products as two qk_tile, but no column multiplies
+// zeros for nothing: half the results to convert, reduce and exponentiate. X: qhat_frag's words where gid < 4, else 0; Y: the
+// words (of query gid - 4) where gid >= 4, else 0.
+template <int BITS> __device__ __forceinline__ void qk_pair(const uint8_t *r0, const uint8_t *r1, int gid, int tig, const uint32_t (&X)[8], const uint32_t (&Y)[8], float2 (&x)[2]) {
+  const uint8_t *p = r0 + 16 * gid + 4 * tig, *r = r1 + 16 * gid + 4 * tig;
+  if (BITS == 4) {
+    uint32_t lo[4], hi[4];
+    constexpr uint32_t L = 0x0f0f0f0fu, H = 0xf0f0f0f0u;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {  // words W[tig], W[4 + tig] of half 0, then of half 1
+      const int o = 512 * (w & 1) + 256 * (w >> 1), m = (w & 1) + 4 * (w >> 1);
+      const uint32_t a = lds32(p + o), a8 = lds32(p + o + 128), b = lds32(r + o), b8 = lds32(r + o + 128);
+      if (w == 0) {
+        mma_u8s8_k32_from(lo, a & L, a8 & L, b & L, b8 & L, X[m], Y[m], MAGIC);
+        mma_u8s8_k32_from(hi, a & H, a8 & H, b & H, b8 & H, X[m + 2], Y[m + 2], MAGIC);
+      } else {
+        mma_u8s8_k32(lo, a & L, a8 & L, b & L, b8 & L, X[m], Y[m]);
+        mma_u8s8_k32(hi, a & H, a8 & H, b & H, b8 & H, X[m + 2], Y[m + 2]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) x[i] = __ffma2_rn(isum2(hi[2 * i], hi[2 * i + 1]), splat(1.f / 16), isum2(lo[2 * i], lo[2 * i + 1]));
+  } else {
+    static_assert(BITS == 3 || BITS == 4, "coarse planes");
+    const int sh = 4 + (tig & 1), se = 3 * (tig & 1), t = 1024 + 16 * gid + 4 * (tig >> 1);
+    constexpr uint32_t L = 0x07070707u, M = 0x38383838u, T2 = 0x03030303u, T1 = 0x04040404u;
+    uint32_t lo[4], mid[4], ex[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // halves
+      const uint32_t a = lds32(p + 256 * h), a8 = lds32(p + 256 * h + 128), b = lds32(r + 256 * h), b8 = lds32(r + 256 * h + 128);
+      const uint32_t e = lds32(r0 + t + 8 * h), e8 = lds32(r0 + t + 8 * h + 128), f = lds32(r1 + t + 8 * h), f8 = lds32(r1 + t + 8 * h + 128);
+      if (h == 0) {
+        mma_u8s8_k32_from(lo, a & L, a8 & L, b & L, b8 & L, X[0], Y[0], MAGIC);
+        mma_u8s8_k32_from(mid, a & M, a8 & M, b & M, b8 & M, X[2], Y[2], MAGIC);
+        mma_u8s8_k32_from(ex, (e >> se) & L, (e8 >> se) & L, (f >> se) & L, (f8 >> se) & L, X[6], Y[6], MAGIC);
+      } else {
+        mma_u8s8_k32(lo, a & L, a8 & L, b & L, b8 & L, X[1], Y[1]);
+        mma_u8s8_k32(mid, a & M, a8 & M, b & M, b8 & M, X[3], Y[3]);
+        mma_u8s8_k32(ex, (e >> se) & L, (e8 >> se) & L, (f >> se) & L, (f8 >> se) & L, X[7], Y[7]);
+      }
+      mma_u8s8_k32(lo, ((a >> 6) & T2) | ((e >> sh) & T1), ((a8 >> 6) & T2) | ((e8 >> sh) & T1), ((b >> 6) & T2) | ((f >> sh) & T1),
+                   ((b8 >> 6) & T2) | ((f8 >> sh) & T1), X[4 + h], Y[4 + h]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      x[i] = __fadd2_rn(__ffma2_rn(isum2(mid[2 * i], mid[2 * i + 1]), splat(1.f / 8), isum2(lo[2 * i], lo[2 * i + 1])), isum2(ex[2 * i], ex[2 * i + 1]));
+  }
+}
+
 // ---- values ---------------------------------------------------------------------------------------------------------
 // The four masked slot words (channels 4 l + 0..3 of record lane l, token quad tig) of a BITS-plane record's V half.
 // Channel cc carries the factor 1 / v_unscale<BITS>(cc).
