@@ -165,23 +165,22 @@ extern "C" cudaError_t fbla_k_decode_shape(fbla_k_decode *a) {
 }
 
 // How the coarse CTAs' warps share the work (see split_of, deal_of), from the tokens a row has at most:
-//   by the lengths when the BF16 windows would get three or more of a CTA's eight warps (contexts up to about 4 700 tokens);
-//   else seven streaming warps and one window warp per CTA, or every warp an equal cost share of windows and groups --
-//   whichever leaves a streaming warp fewer groups, counted as the kernels deal them (whole groups per warp), with 5 %
-//   against the deal by cost: its eight streaming warps per CTA run a group that much slower than seven beside a window
-//   warp do. Measured on B200, by cost against seven + one: batch 1 x 128K tokens 80.0 -> 75.3 us per step in 3+3 and
+//   by the lengths when the BF16 windows would get three eighths of a CTA's warps or more (contexts up to about 4 700 tokens);
+//   else all warps but one stream and one serves windows, or every warp has an equal cost share of windows and groups --
+//   whichever leaves an eighth of a CTA fewer groups (whole groups), with 5 % against the deal by cost: a CTA whose every
+//   warp streams runs a group that much slower. The line was measured with eight warps per CTA and holds with twelve. Measured on B200 (eight warps), by cost against seven + one: batch 1 x 128K tokens 80.0 -> 75.3 us per step in 3+3 and
 //   65.7 -> 61.6 in 4+2 (7 groups per warp instead of 8), batch 64 x 1K..64K 2.07 -> 2.02 ms, but batch 8 x 16K 120.0 ->
 //   123.9 (8 groups per warp either way).
 extern "C" void fbla_k_decode_split(fbla_k_decode *a, long long tokens) {
-  const int total = (a->cb == 4 ? fbla::CoarseShape<4>::TOTAL : fbla::CoarseShape<3>::TOTAL);
+  constexpr int total = 8;  // (the choice is made in eighths of a CTA)
   const long long groups = (tokens + fbla::G - 1) / fbla::G, S = groups > 2 ? groups - 2 : 0;
   const long long W = groups <= 1 ? (tokens + fbla::S - 1) / fbla::S : 2 * fbla::SBG;  // (a full open window: the choice is monotone in tokens)
   const bool by_lengths = S == 0 || (2 * total * W + S + W) / (2 * (S + W)) >= 3;
   const long long heads = (long long)a->batch * a->kv_heads * a->vg, ctas = a->coarse_ctas > 0 ? a->coarse_ctas : 148;
-  // groups a streaming warp takes: seven + one; by cost (deal_of's share, a whole number of groups)
+  // groups an eighth of a CTA takes: seven eighths streaming; by cost (deal_of's share, a whole number of groups)
   const long long fixed = (heads * S + ctas * (total - 1) - 1) / (ctas * (total - 1));
   const long long cost = (fbla::GROUP_COST * heads * S + fbla::WINDOW_COST * heads * W + fbla::GROUP_COST * ctas * total - 1) / (fbla::GROUP_COST * ctas * total);
-  a->coarse_warps = total;
+  a->coarse_warps = a->cb == 4 ? fbla::CoarseShape<4>::TOTAL : fbla::CoarseShape<3>::TOTAL;
   a->deal = by_lengths ? FBLA_K_DEAL_LENGTHS : 21 * cost < 20 * fixed ? FBLA_K_DEAL_COST : FBLA_K_DEAL_FIXED;
   // Folding the warps' partial rows per CTA costs the coarse pass a barrier and a few microseconds at its very end and saves
   // the later passes their walk over the rows: it pays when a virtual head is spread over many warps, i.e. when there are

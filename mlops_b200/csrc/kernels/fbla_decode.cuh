@@ -29,21 +29,22 @@ constexpr int SLICE = FBLA_K_SLICE;      // sub-blocks per select slice
 #ifndef FBLA_RNST
 #define FBLA_RNST 2  /* refine ring stages per warp */
 #endif
-// Eight warps per CTA leave a thread 255 registers, which the coarse loop needs to run without spills. Measured on B200
-// with streaming + window warps (decode batch 8 x 16K 4+2 / batch 1 x 128K 3+3 / 4+2, us per step):
-// 10 + 2 warps (168 registers) 135.5 / 80.3 / 78.1; 8 + 2: 121.3 / 81.0 / 65.2; 7 + 1: 121.7 / 76.3 / 63.5; 6 + 2: 131.6 / 84.3 / 68.6.
-// FBLA_CW*: the streaming warps of that fixed split; a CTA has one warp more (CoarseShape::TOTAL).
+// Twelve warps per CTA leave a thread 168 registers, which hold the coarse loop but for a few spills outside it since a pair's
+// sub-blocks share the score products' columns. Measured on B200, eight warps -> twelve (us per step, one sweep): 1 x 1 M tokens
+// 4+2 240 -> 229; 1 x 512 K 3+3 158 -> 149; 8 x 16 K 4+2 72.7 -> 65.2; 2 x 64 K 66.3 -> 63.8; 1 x 128 K 66.6 -> 62.5. A ring slot
+// holds one record pair: with two, twelve warps do not fit the shared memory.
+// FBLA_CW*: the streaming warps of the fixed split at most; a CTA has one warp more (CoarseShape::TOTAL).
 #ifndef FBLA_CW4
-#define FBLA_CW4 7
+#define FBLA_CW4 11
 #endif
 #ifndef FBLA_CW3
-#define FBLA_CW3 7
+#define FBLA_CW3 11
 #endif
 #ifndef FBLA_NP
 #define FBLA_NP 2
 #endif
 #ifndef FBLA_PPC
-#define FBLA_PPC 2  // record pairs per chunk (one bulk copy, one barrier wait)
+#define FBLA_PPC 1  // record pairs per chunk (one bulk copy, one barrier wait)
 #endif
 template <int CB> struct CoarseShape {
   static constexpr int WARPS = CB == 4 ? FBLA_CW4 : FBLA_CW3, TOTAL = WARPS + 1;
@@ -171,7 +172,7 @@ template <int CB> struct __align__(128) StreamWarp {
   // The partial rows of the first and the last virtual head of the warp's run, which neighbouring warps of the CTA may
   // share: they are folded into one row per (CTA, virtual head) before they leave the CTA. stage_vh: the rows' virtual
   // heads (-1: no such row).
-  float stage[2][4][FBLA_K_PSTRIDE];
+  __align__(16) float stage[2][4][FBLA_K_PSTRIDE];
   int stage_vh[2];
 };
 struct __align__(16) ExactWarp {
@@ -229,7 +230,11 @@ __device__ __forceinline__ void deal_range(const Deal &d, long long w, long long
 struct Split { int sw, xw; };  // streaming / window warps per CTA
 __device__ __forceinline__ Split split_of(const fbla_k_decode &a, int hpr) {
   const int total = (a.cb == 4 ? FBLA_CW4 : FBLA_CW3) + 1;
-  if (a.deal == FBLA_K_DEAL_FIXED) return Split{total - 1, 1};
+  if (a.deal == FBLA_K_DEAL_FIXED) {  // no more streaming warps than the groups a warp takes at most need: every CTA then has its share of few groups
+    const long long units = total_units<false>(a, hpr), per = max(1ll, ceil_div(units, (long long)a.coarse_ctas * (total - 1)));
+    const int sw = max(1, (int)ceil_div(units, (long long)a.coarse_ctas * per));
+    return Split{sw, total - sw};
+  }
   const long long S = GROUP_COST * total_units<false>(a, hpr), W = WINDOW_COST_SHORT * total_units<true>(a, hpr);  // in eighths of a group's time
   const int xw = S == 0 ? total : max(1, min(total - 1, (int)((2 * total * W + S + W) / (2 * (S + W)))));
   return Split{total - xw, xw};
@@ -638,7 +643,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
   int sw = Sh::TOTAL;                 // streaming warps of this CTA
   long long gw, lo, hi;               // the warp's index among the grid's streaming warps and its run of the flattened groups
   if (DEAL != FBLA_K_DEAL_COST) {  // the CTA's last xw warps serve windows, the others stream
-    const Split sp = DEAL == FBLA_K_DEAL_LENGTHS ? split_of(a, hpr) : Split{Sh::WARPS, 1};
+    const Split sp = split_of(a, hpr);
     sw = sp.sw;
     if (warp >= sw) {
       exact_warp<QG>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, FBLA_POS::x() * sp.xw + (warp - sw), FBLA_POS::nx() * sp.xw);

@@ -44,7 +44,7 @@ typedef struct {
   int hs, gs;            // units between KV heads and between groups
   int qg, vg;            // queries per virtual head, virtual heads per KV head
   int cb, fb;            // plane bits
-  int coarse_ctas, coarse_warps;  // persistent coarse CTAs and their warps (8): how the work is dealt to them is `deal`
+  int coarse_ctas, coarse_warps;  // persistent coarse CTAs and their warps: how the work is dealt to them is `deal`
   int refine_ctas, refine_warps;  // RW = refine_ctas * refine_warps
   float sl, log2_tau;
   // Sequence shards (one GPU's part of a long context); shard_on 0: the whole cache. A shard processes the closed groups
@@ -61,7 +61,7 @@ typedef struct {
   short deal;          // how the coarse pass's warps share the work, FBLA_K_DEAL_*
 } fbla_k_decode;
 #define FBLA_K_DEAL_LENGTHS 0 /* a CTA's warps are split between windows and groups by the rows' lengths (short contexts) */
-#define FBLA_K_DEAL_FIXED 1   /* seven warps of a CTA stream groups, the eighth serves windows */
+#define FBLA_K_DEAL_FIXED 1   /* the last warps of a CTA (one at least) serve windows, the others stream groups */
 #define FBLA_K_DEAL_COST 2    /* every warp takes an equal cost share of windows and groups (long contexts) */
 
 #define FBLA_K_DENSE_MAX_BATCH 1024  /* batch rows of a dense decode: their prefix sums lie in shared memory */
