@@ -230,11 +230,7 @@ __device__ __forceinline__ void deal_range(const Deal &d, long long w, long long
 struct Split { int sw, xw; };  // streaming / window warps per CTA
 __device__ __forceinline__ Split split_of(const fbla_k_decode &a, int hpr) {
   const int total = (a.cb == 4 ? FBLA_CW4 : FBLA_CW3) + 1;
-  if (a.deal == FBLA_K_DEAL_FIXED) {  // no more streaming warps than the groups a warp takes at most need: every CTA then has its share of few groups
-    const long long units = total_units<false>(a, hpr), per = max(1ll, ceil_div(units, (long long)a.coarse_ctas * (total - 1)));
-    const int sw = max(1, (int)ceil_div(units, (long long)a.coarse_ctas * per));
-    return Split{sw, total - sw};
-  }
+  if (a.deal == FBLA_K_DEAL_FIXED) return Split{total - 1, 1};
   const long long S = GROUP_COST * total_units<false>(a, hpr), W = WINDOW_COST_SHORT * total_units<true>(a, hpr);  // in eighths of a group's time
   const int xw = S == 0 ? total : max(1, min(total - 1, (int)((2 * total * W + S + W) / (2 * (S + W)))));
   return Split{total - xw, xw};
@@ -643,7 +639,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
   int sw = Sh::TOTAL;                 // streaming warps of this CTA
   long long gw, lo, hi;               // the warp's index among the grid's streaming warps and its run of the flattened groups
   if (DEAL != FBLA_K_DEAL_COST) {  // the CTA's last xw warps serve windows, the others stream
-    const Split sp = split_of(a, hpr);
+    const Split sp = DEAL == FBLA_K_DEAL_LENGTHS ? split_of(a, hpr) : Split{Sh::WARPS, 1};
     sw = sp.sw;
     if (warp >= sw) {
       exact_warp<QG>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, FBLA_POS::x() * sp.xw + (warp - sw), FBLA_POS::nx() * sp.xw);
