@@ -63,30 +63,22 @@ def kernel_source(name, threads, statements, items=None):
     return head + f'  for (int item = blockIdx.x; item < {items}; item += gridDim.x) {{\n    {statements}\n    __syncthreads();\n  }}\n}}\n'
 
 
-def compile_program(source, want_cubin=True):
-    """NVRTC: returns the cubin (or PTX) bytes; raises with the log on failure"""
+def compile_program(source):
+    """NVRTC: returns the cubin's bytes; raises with the log on failure"""
     from cuda.bindings import nvrtc
     err, prog = nvrtc.nvrtcCreateProgram(source.encode(), b"executor.cu", 0, [], [])
     assert err == nvrtc.nvrtcResult.NVRTC_SUCCESS
-    opts = [b"--std=c++17", b"--gpu-architecture=sm_100a" if want_cubin else b"--gpu-architecture=compute_100a",
-            ("-I" + os.path.join(ROOT, "include")).encode(), ("-I" + CUDA_INCLUDE).encode()]
+    opts = [b"--std=c++17", b"--gpu-architecture=sm_100a", ("-I" + os.path.join(ROOT, "include")).encode(), ("-I" + CUDA_INCLUDE).encode()]
     err, = nvrtc.nvrtcCompileProgram(prog, len(opts), opts)
     _, n = nvrtc.nvrtcGetProgramLogSize(prog)
     log = b" " * (n + 8)  # (never a one-byte object: CPython shares those, and the call writes into the buffer)
     nvrtc.nvrtcGetProgramLog(prog, log)
     if err != nvrtc.nvrtcResult.NVRTC_SUCCESS:
         raise RuntimeError("NVRTC: " + log.decode(errors="replace")[-4000:])
-    if want_cubin:
-        _, size = nvrtc.nvrtcGetCUBINSize(prog)
-        out = b" " * (size + 8)
-        nvrtc.nvrtcGetCUBIN(prog, out)
-        out = out[:size]
-    else:
-        _, size = nvrtc.nvrtcGetPTXSize(prog)
-        out = b" " * (size + 8)
-        nvrtc.nvrtcGetPTX(prog, out)
-        out = out[:size]
-    return out
+    _, size = nvrtc.nvrtcGetCUBINSize(prog)
+    out = b" " * (size + 8)
+    nvrtc.nvrtcGetCUBIN(prog, out)
+    return out[:size]
 
 
 def item_call(lib, p):
