@@ -2,12 +2,12 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--workload NAME]
 
-The headline line (default workload, `decode_128k`) is the configuration BASELINE.json's metric is quoted on: one decode
+The headline line (default workload, `decode_128k`) is the one the metric is quoted on: one decode
 step -- one new token -- of batch 1, 32 query heads / 8 KV heads, head_dim 128, over 131 072 cached tokens in 3+3 mode,
 seeded BF16 N(0,1) inputs, softmax scale 1/sqrt(128), default tau; the cache was written by the library itself
 (quantize-on-write). The same JSON line carries sub-records (`sub`) for the other configurations, each with its own
-`ms_per_step`, `e2e` and `roofline`: the 4+2 format at 128K, configs[1] (batch 8 x 16 384, 4+2), configs[3] (causal
-prefill batch 4 x 8 192, TFLOP/s) and configs[4] (mixed serving decode, batch 64, ragged 1K..64K contexts).
+`ms_per_step`, `e2e` and `roofline`: the 4+2 format at 128K, batch 8 x 16 384 in 4+2, causal
+prefill of batch 4 x 8 192 (TFLOP/s) and mixed serving decode (batch 64, ragged 1K..64K contexts).
 
 Timing: after W >= 3 warm-up steps, blocks of exactly K steps between two CUDA events on the launching stream (with a
 barrier + synchronize on both sides), repeated until at least half a second has been timed; `ms_per_step` is the median
@@ -19,8 +19,8 @@ bounded sample of the oracle's port of the reference's host-side float64 model o
 
 N > 1 (torchrun, one rank per GPU): the SAME job split over the ranks (strong scaling) -- the 8 KV heads of the headline
 decode are dealt to the ranks, each with its heads' cache; no data-path collective is needed (NCCL carries the barrier
-and the max over ranks). Sub-records: configs[1] and configs[4] by KV head, configs[3] by (batch row, KV head), and
-configs[2]'s sequence split of one 262 144-token context with its two small exchanges.
+and the max over ranks). Sub-records: the batched and the serving decode by KV head, the prefill by (batch row, KV head),
+and the sequence split of one 262 144-token context with its two small exchanges.
 `--impl reference` times the reference's host-side path (the oracle port) on the host cores, same configuration.
 """
 import argparse
@@ -43,17 +43,17 @@ WORKLOADS = {
     "decode_128k_4p2": dict(kind="decode", batch=1, q_heads=32, kv_heads=8, tokens=131072, mode="4+2", seed=1003, outliers=False,
                             name="decode B1 32q/8kv ctx131072 4+2 (the metric's 128K context)"),
     "decode_4k": dict(kind="decode", batch=1, q_heads=16, kv_heads=8, tokens=4096, mode="3+3", seed=1001, outliers=True,
-                      name="decode B1 16q/8kv ctx4096 3+3 (BASELINE configs[0])"),
+                      name="decode B1 16q/8kv ctx4096 3+3"),
     "decode_b8": dict(kind="decode", batch=8, q_heads=32, kv_heads=8, tokens=16384, mode="4+2", seed=1002, outliers=True,
-                      name="decode B8 32q/8kv ctx16384 4+2 (BASELINE configs[1])"),
+                      name="decode B8 32q/8kv ctx16384 4+2"),
     "serving_b64": dict(kind="serving", batch=64, q_heads=32, kv_heads=8, lo=1024, hi=65536, mode="3+3", seed=1005,
-                        name="serving decode B64 32q/8kv 3+3, contexts U[1024, 65536], 256-token pages (BASELINE configs[4])"),
+                        name="serving decode B64 32q/8kv 3+3, contexts U[1024, 65536], 256-token pages"),
     "prefill_b4": dict(kind="prefill", batch=4, q_heads=32, kv_heads=8, tokens=8192, mode="4+2", seed=1004,
-                       name="causal prefill B4 S8192 32q/8kv 4+2 (BASELINE configs[3])"),
+                       name="causal prefill B4 S8192 32q/8kv 4+2"),
     "prefill_b1": dict(kind="prefill", batch=1, q_heads=32, kv_heads=8, tokens=8192, mode="4+2", seed=1004,
-                       name="causal prefill B1 S8192 32q/8kv 4+2 (one sequence of BASELINE configs[3]; for profiler captures)"),
-    "seqsplit_256k": dict(kind="seqsplit", tokens=262144, name="sequence-split decode B1 32q/8kv ctx262144 3+3 (BASELINE configs[2])"),
-    "seqsplit_1m": dict(kind="seqsplit", tokens=1 << 20, name="sequence-split decode B1 32q/8kv ctx1048576 3+3 (BASELINE configs[2])"),
+                       name="causal prefill B1 S8192 32q/8kv 4+2 (one of the four sequences; for profiler captures)"),
+    "seqsplit_256k": dict(kind="seqsplit", tokens=262144, name="sequence-split decode B1 32q/8kv ctx262144 3+3"),
+    "seqsplit_1m": dict(kind="seqsplit", tokens=1 << 20, name="sequence-split decode B1 32q/8kv ctx1048576 3+3"),
 }
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the workload's dominant kernel, from the ncu captures summarised
 # under profiles/ (1 GPU); reported with their source, never as a measurement of the run that prints them
@@ -388,7 +388,7 @@ def decode_record(cfg, rec, n_gpus):
     return out
 
 
-# ---- serving decode ---------------------------------------------------------------------------------------------
+# ---- serving decode ----------------------------------------------------------------------------------------------------------
 def run_serving(D, cfg, args):
     """Batch 64, ragged contexts: per-row device lengths (length_stride 1) over a cache laid out in whole 256-token pages.
     world > 1: the KV heads are dealt to the ranks. Tokens are seeded N(0,1) drawn on the device."""
@@ -465,7 +465,7 @@ def run_serving(D, cfg, args):
                 dtype="u8")
 
 
-# ---- prefill ----------------------------------------------------------------------------------------------------
+# ---- prefill -----------------------------------------------------------------------------------------------------------------
 def run_prefill(D, cfg, args):
     """Causal prefill of whole sequences into an empty cache: quantize-on-write of the chunk's groups, attention over the
     compressed cache on tensor cores, window update. world > 1: the (batch row, KV head) units are dealt to the ranks.
@@ -557,7 +557,7 @@ def run_prefill(D, cfg, args):
                 dtype="f16 x f16 -> f32", tokens_per_s=B * S / (ms * 1e-3))
 
 
-# ---- sequence split ----------------------------------------------------------------------------------------------
+# ---- sequence split -----------------------------------------------------------------------------------------------------------
 def run_seqsplit(D, cfg, args):
     """One sequence (batch 1, 32q/8kv, 3+3, plain N(0,1)) split over the ranks by whole groups; every decode step = two
     local passes + two small exchanges (row masses, partial sums)."""

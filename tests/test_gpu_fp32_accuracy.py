@@ -15,8 +15,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("mode", ["3+3", "4+2"])
-@pytest.mark.parametrize("B,QH,KH,N,seed,outliers", [(1, 16, 8, 4096, 1001, True),
-                                                     (2, 32, 8, 16384, 1002, True),     # two rows of configs[1]
+@pytest.mark.parametrize("B,QH,KH,N,seed,outliers", [(1, 16, 8, 4096, 1001, True),      # a short context
+                                                     (2, 32, 8, 16384, 1002, True),     # two rows of the batched decode
                                                      (1, 32, 8, 131072, 1003, False)])  # the metric's 128K context
 def test_unrounded_decode_output_against_float64_model(oracle, mode, B, QH, KH, N, seed, outliers):
     from mlops_b200.attention import sharded

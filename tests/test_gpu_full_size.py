@@ -1,7 +1,7 @@
-"""Parity at BASELINE's full sizes, and the layout options of the C API (strided units, strided outputs).
+"""Parity at the benchmark's full sizes, and the layout options of the C API (strided units, strided outputs).
 
-Full sizes: decode configs[1] (batch 8, 32q/8kv, ctx 16 384, 4+2) against the CPU oracle on every row and against the
-reference's CUDA library; prefill with configs[3]'s shape (one of its four sequences: 32q/8kv, 8 192 tokens, 4+2)
+Full sizes: the batched decode (batch 8, 32q/8kv, ctx 16 384, 4+2) against the CPU oracle on every row and against the
+reference's CUDA library; prefill of one of the benchmark's four sequences (32q/8kv, 8 192 tokens, 4+2)
 against the oracle on sampled positions and through a size-independent property (one 8 192-token chunk == four
 2 048-token chunks: the same cache bytes, outputs within tolerance of each other).
 Layout options follow attention/fbla/tests/test_fbla.cu:874-957 (units of several layers side by side; token-major
@@ -38,9 +38,9 @@ def test_decode_configs1_full_size(ours, ref, oracle):
     out = ours.decode(c, qd)
     torch.cuda.synchronize()
     o = oracle.encode(k, v, mode)
-    gu.assert_cache_equal(c, o, "configs[1] cache")
+    gu.assert_cache_equal(c, o, "batch 8 cache")
     want, stats = oracle.decode(q, o, stats=True)
-    gu.check_close(gu.bits_of(out), want, "configs[1] decode")
+    gu.check_close(gu.bits_of(out), want, "batch 8 decode")
     assert 0.5 < stats[3] / stats[2] < 0.95  # the refined share of this input (0.776): both passes are exercised at scale
     if ref is not None:
         a = datagen.bf16_to_f32(gu.bits_of(out)).astype(np.float64)
@@ -68,7 +68,7 @@ def test_prefill_configs3_shape(ours, oracle):
     want = oracle.prefill(q, k, v, oracle.empty(B, KH, S, mode), pos_step=step)
     idx = np.arange(0, S, step)
     for i in idx:
-        gu.check_close(gu.bits_of(out1)[:, :, i], want[:, :, i], f"configs[3] prefill position {i}")
+        gu.check_close(gu.bits_of(out1)[:, :, i], want[:, :, i], f"prefill position {i}")
 
 
 @pytest.mark.parametrize("mode", ["3+3", "4+2"])

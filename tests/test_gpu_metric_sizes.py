@@ -1,11 +1,11 @@
-"""Parity at the sizes the headline metric and the BASELINE configurations name, through the C ABI, against the CPU
+"""Parity at the sizes the headline metric and the benchmark's workloads name, through the C ABI, against the CPU
 oracle and against the reference's own CUDA library (oracle/_ref) on the same device buffers:
 
   * decode batch 1, 32q / 8kv, 131 072 tokens, both formats (the metric's "128K ctx");
   * the reference's own 262 144-token decode case (attention/fbla/tests/test_fbla.cu:1219: 4q / 2kv, tau 1e-4, seed 9);
-  * 1 048 576 tokens (configs[2]) through 8 emulated sequence shards against the single-cache decode;
-  * causal prefill batch 4 x 8 192, 32q / 8kv, 4+2 (configs[3]) at sampled positions of every sequence;
-  * mixed serving decode (configs[4]): batch 64, 32q / 8kv, 3+3, per-row device lengths drawn from [1 024, 65 536],
+  * 1 048 576 tokens through 8 emulated sequence shards against the single-cache decode;
+  * causal prefill batch 4 x 8 192, 32q / 8kv, 4+2 at sampled positions of every sequence;
+  * mixed serving decode: batch 64, 32q / 8kv, 3+3, per-row device lengths drawn from [1 024, 65 536],
     the cache laid out in whole 256-token pages (two group units per page) through head_stride / group_stride.
 
 Every case prints its measured distances, max|ours - oracle| / max|oracle| and max|ours - ref_gpu| / max|ref_gpu|."""
@@ -77,7 +77,7 @@ def test_decode_262144_reference_case(ours, ref, oracle, mode):
 
 
 def test_decode_1m_through_eight_shards(ours, ref):
-    """configs[2] at its largest: one 1 048 576-token sequence (3+3) held as 8 sequence shards -- here all on one GPU and
+    """The sequence split at its largest: one 1 048 576-token sequence (3+3) held as 8 sequence shards -- here all on one GPU and
     run one after the other, the two exchanges replaced by a concatenation and a sum -- against the decode of the same
     tokens held in one cache, and against the reference's CUDA library on that cache."""
     from mlops_b200.attention import sharded
@@ -124,12 +124,12 @@ def test_prefill_configs3_batch4(ours, ref, oracle):
     torch.cuda.synchronize()
     assert ctypes.CDLL(gu.OURS).fbla_k_attend_tc_status() == 0
     o = oracle.encode(k, v, mode)
-    gu.assert_cache_equal(c, o, "configs[3] cache after the prefill")
+    gu.assert_cache_equal(c, o, "cache after the prefill")
     step = 1171  # 7 positions per sequence through the oracle's float64 model of the reference's prefill
     want = oracle.prefill(q, k, v, oracle.empty(B, KH, S, mode), pos_step=step)
     worst = 0.0
     for i in range(0, S, step):
-        worst = max(worst, gu.check_close(gu.bits_of(out)[:, :, i], want[:, :, i], f"configs[3] prefill position {i}"))
+        worst = max(worst, gu.check_close(gu.bits_of(out)[:, :, i], want[:, :, i], f"prefill position {i}"))
     rel_ref = float("nan")
     if ref is not None:
         rc = ref.empty(B, KH, S, mode)
@@ -149,7 +149,7 @@ def serving_lengths(batch=64, seed=1005):
 
 
 def build_serving_cache(lib, lengths, KH, mode, page_tokens=256, seed=1005, keep=()):
-    """configs[4]'s cache: every row laid out for the same number of whole pages (the API addresses units affinely:
+    """The serving cache: every row laid out for the same number of whole pages (the API addresses units affinely:
     head_stride = groups per head, group_stride = 1, so a 256-token page is two consecutive group units), filled row by
     row with seeded N(0,1) tokens up to the row's own length. keep: rows whose (k, v) bit patterns are returned."""
     B = len(lengths)
@@ -205,10 +205,10 @@ def test_serving_decode_configs4(ours, ref, oracle):
 
         needed = False
         try:
-            worst = max(worst, gu.check_close(gu.bits_of(out)[b:b + 1], model, f"configs[4] row {b} ({lengths[b]} tokens)"))
+            worst = max(worst, gu.check_close(gu.bits_of(out)[b:b + 1], model, f"serving row {b} ({lengths[b]} tokens)"))
         except AssertionError:
             needed = True
-            assert inside_envelope(a[b:b + 1]), f"configs[4] row {b} ({lengths[b]} tokens) lies outside the model's envelope around tau"
+            assert inside_envelope(a[b:b + 1]), f"serving row {b} ({lengths[b]} tokens) lies outside the model's envelope around tau"
         if r is not None:
             # the reference's CUDA library, same batched call: both outputs are BF16-rounded, hence one ulp; where that
             # fails, both must be inside the model's envelope (the two libraries decided a borderline block differently)
