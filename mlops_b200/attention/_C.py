@@ -111,34 +111,22 @@ def scratch_bytes(batch, q_heads, kv_heads, tokens, format, capacity):
     return n
 
 
-# ---- calls on a whole cache object: what does not change from call to call is looked at once ---------------------------------
-class _Bound:
-    """A cache's arrays, checked, and the structure that names them to the library."""
-    __slots__ = ("arrays", "pointers", "struct", "device", "index", "batch", "kv_heads")
-
-    def __init__(self, c):
-        self.arrays = c.coarse, c.fine, c.meta, c.sink_k, c.sink_v, c.open_k, c.open_v
-        self.device = c.coarse.device
-        for x in self.arrays[:2]:
-            _tensor(x, self.device, torch.uint8, "packed cache records")
-        for x in self.arrays[2:]:
-            _tensor(x, self.device, torch.bfloat16, "cache metadata / exact group")
-        self.pointers = tuple(x.data_ptr() for x in self.arrays)
-        self.struct = ctypes.byref(Cache(*self.pointers, c.images.data_ptr() if c.images is not None else None))
-        self.index = self.device.index
-        self.batch, self.kv_heads = c.meta.size(0), c.meta.size(1)
+# ---- calls on a whole cache object --------------------------------------------------------------------------------------------
+_RECORDS, _ROWS = "packed cache records", "cache metadata / exact group"
+_KINDS = ((torch.uint8, _RECORDS),) * 2 + ((torch.bfloat16, _ROWS),) * 5
 
 
-def bind(c):
-    """The cache's _Bound, made anew whenever one of its arrays is another tensor or lies elsewhere."""
-    b = c.__dict__.get("_bound")
-    if b is not None:
-        k, f, m, sk, sv, ok, ov = b.arrays
-        if (k is c.coarse and f is c.fine and m is c.meta and sk is c.sink_k and sv is c.sink_v and ok is c.open_k and ov is c.open_v
-                and b.pointers == (k.data_ptr(), f.data_ptr(), m.data_ptr(), sk.data_ptr(), sv.data_ptr(), ok.data_ptr(), ov.data_ptr())):
-            return b
-    b = c._bound = _Bound(c)
-    return b
+def _arrays(c):
+    """A cache's arrays, checked as `decode` and `prefill` check theirs: the structure that names them to the library, their device.
+    (Looked at in every call -- 2 us of the host's time -- and nothing of it kept: a cache is a plain record that its user may change,
+    copy and save.)"""
+    arrays = c.coarse, c.fine, c.meta, c.sink_k, c.sink_v, c.open_k, c.open_v
+    device = arrays[0].device
+    index = arrays[0].get_device()
+    for x, (dtype, what) in zip(arrays, _KINDS):
+        if index < 0 or x.get_device() != index or x.dtype is not dtype or not x.is_contiguous():
+            _tensor(x, device, dtype, what)
+    return _cache(*arrays, c.images), device
 
 
 _scratch_bytes = functools.lru_cache(maxsize=256)(lambda device, *shape: scratch_bytes(*shape))
@@ -176,43 +164,44 @@ _pool = _ScratchPool()
 
 def decode_cache(q, c, scale, tau):
     """decode of a whole cache object with the pool's scratch"""
-    b = bind(c)
+    struct, device = _arrays(c)
     if q.dim() != 3 or q.size(2) != 128:
         raise ValueError(f"q must be [batch, q_heads, 128], got {tuple(q.shape)}")
     if not q.is_contiguous():
         q = q.contiguous()
-    if q.device != b.device:
-        raise ValueError(f"q: expected a CUDA tensor on {b.device}")
-    if torch._C._cuda_getDevice() != b.index:
-        with torch.cuda.device(b.index):
+    if q.device != device:
+        raise ValueError(f"q: expected a CUDA tensor on {device}")
+    if torch._C._cuda_getDevice() != device.index:
+        with torch.cuda.device(device.index):
             return decode_cache(q, c, scale, tau)
-    batch, q_heads = q.size(0), q.size(1)
-    need = _scratch_bytes(b.index, batch, q_heads, b.kv_heads, c.capacity, c.format, c.capacity)
-    stream = _raw_stream(b.index)
-    size, scratch, keep = _pool.get(b.device, stream, batch * b.kv_heads, need)
+    batch, q_heads, kv_heads = q.size(0), q.size(1), c.meta.size(1)
+    need = _scratch_bytes(device.index, batch, q_heads, kv_heads, c.capacity, c.format, c.capacity)
+    stream = _raw_stream(device.index)
+    size, scratch, keep = _pool.get(device, stream, batch * kv_heads, need)
     out = torch.empty_like(q)
-    cfg = Config(batch, q_heads, b.kv_heads, int(c.tokens), float(scale), float(tau), int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
-    _raise(_lib.mlops_fbla_decode(ctypes.byref(cfg), q.data_ptr(), b.struct, out.data_ptr(), scratch, size, stream), "mlops_fbla_decode")
+    cfg = Config(batch, q_heads, kv_heads, int(c.tokens), float(scale), float(tau), int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
+    _raise(_lib.mlops_fbla_decode(ctypes.byref(cfg), q.data_ptr(), ctypes.byref(struct), out.data_ptr(), scratch, size, stream), "mlops_fbla_decode")
     return out
 
 
 def prefill_cache(q, k, v, c, scale):
     """prefill (append for q None) on a whole cache object; k and v contiguous BF16 of the cache's batch and KV heads"""
-    b = bind(c)
-    _tensor(k, b.device, torch.bfloat16, "k")
-    _tensor(v, b.device, torch.bfloat16, "v")
-    if torch._C._cuda_getDevice() != b.index:
-        with torch.cuda.device(b.index):
+    struct, device = _arrays(c)
+    _tensor(k, device, torch.bfloat16, "k")
+    _tensor(v, device, torch.bfloat16, "v")
+    if torch._C._cuda_getDevice() != device.index:
+        with torch.cuda.device(device.index):
             return prefill_cache(q, k, v, c, scale)
-    n, q_heads, out = k.size(2), b.kv_heads, None
+    batch, kv_heads, n, out = c.meta.size(0), c.meta.size(1), k.size(2), None
+    q_heads = kv_heads
     if q is not None:
-        if q.dim() != 4 or q.size(0) != b.batch or q.size(2) != n or q.size(3) != 128:
+        if q.dim() != 4 or q.size(0) != batch or q.size(2) != n or q.size(3) != 128:
             raise ValueError(f"q must be [batch, q_heads, n, 128] matching k, got {tuple(q.shape)}")
-        _tensor(q, b.device, torch.bfloat16, "q")
+        _tensor(q, device, torch.bfloat16, "q")
         q_heads, out = q.size(1), torch.empty_like(q)
-    cfg = Config(b.batch, q_heads, b.kv_heads, int(c.tokens), float(scale), 0.0, int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
-    _raise(_lib.mlops_fbla_prefill(ctypes.byref(cfg), n, q.data_ptr() if q is not None else None, k.data_ptr(), v.data_ptr(), b.struct,
-                                   out.data_ptr() if out is not None else None, _raw_stream(b.index)), "mlops_fbla_prefill")
+    cfg = Config(batch, q_heads, kv_heads, int(c.tokens), float(scale), 0.0, int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
+    _raise(_lib.mlops_fbla_prefill(ctypes.byref(cfg), n, q.data_ptr() if q is not None else None, k.data_ptr(), v.data_ptr(), ctypes.byref(struct),
+                                   out.data_ptr() if out is not None else None, _raw_stream(device.index)), "mlops_fbla_prefill")
     return out
 
 

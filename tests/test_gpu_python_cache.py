@@ -1,0 +1,56 @@
+"""The Python cache record and what the calls on it keep: a cache that has been in use can be copied, pickled and saved; every call
+looks at the arrays it is given; the decode's scratch is nobody else's (threads on one stream, captured graphs)."""
+import copy
+import io
+import pickle
+
+import pytest
+import torch
+
+from mlops_b200 import attention
+
+pytestmark = pytest.mark.gpu
+ARRAYS = ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v")
+
+
+def _case(tokens=300, batch=1, q_heads=4, kv_heads=2, mode="3+3", capacity=1024):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(tokens)
+    k, v = (torch.randn((batch, kv_heads, tokens, 128), generator=gen, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    return torch.randn((batch, q_heads, 128), generator=gen, dtype=torch.bfloat16, device="cuda"), attention.encode(k, v, mode, capacity)
+
+
+def _saved(cache):
+    file = io.BytesIO()
+    torch.save(cache, file)
+    file.seek(0)
+    return torch.load(file, weights_only=False)
+
+
+@pytest.mark.parametrize("branch", [copy.deepcopy, lambda c: pickle.loads(pickle.dumps(c)), _saved], ids=["deepcopy", "pickle", "save"])
+def test_a_cache_in_use_can_be_branched(branch):
+    q, cache = _case()
+    want = attention.decode(q, cache)
+    attention.append(cache, *(torch.zeros((1, 2, 1, 128), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+    other = branch(cache)
+    assert other.tokens == cache.tokens == 301
+    for a in ARRAYS:
+        assert torch.equal(getattr(other, a), getattr(cache, a)) and getattr(other, a).data_ptr() != getattr(cache, a).data_ptr()
+    kept = other.open_k.clone()
+    attention.append(cache, *(torch.ones((1, 2, 1, 128), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+    assert torch.equal(other.open_k, kept)
+    other.tokens = 300
+    assert torch.equal(attention.decode(q, other), want)
+
+
+def test_every_call_looks_at_the_arrays():
+    q, cache = _case()
+    attention.decode(q, cache)
+    cache.open_k.transpose_(2, 3)  # (the same tensor at the same address, no longer the layout the library reads)
+    with pytest.raises(ValueError, match="contiguous"):
+        attention.decode(q, cache)
+    cache.open_k.transpose_(2, 3)
+    attention.decode(q, cache)
+    cache.sink_v.transpose_(2, 3)
+    with pytest.raises(ValueError, match="contiguous"):
+        attention.append(cache, *(torch.zeros((1, 2, 1, 128), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
