@@ -154,6 +154,7 @@ typedef struct {
   int early;    // 1: the close pass also updates the windows of a chunk that starts its cache (nothing reads them then), the finish pass leaves that to it
   int room;     // tokens the cache is laid out for
   int cluster;  // attention passes: CTAs of a tile's cluster, one per share of its groups (1: one CTA does the tile)
+  int above;    // tensor-core pass: this launch works where the chunk's tiles have more than `above` and at most `cluster` shares
 } fbla_k_prefill;
 
 // close_blocks: grid x of the close pass (groups the chunk can close); 0 skips it
@@ -169,6 +170,10 @@ FBLA_HOST_API(int fbla_k_attend_plan(const fbla_k_prefill *a, fbla_k_prefill arg
 FBLA_HOST_API(cudaError_t fbla_k_attend_launch(const fbla_k_prefill *a, cudaStream_t stream);)  // every pass of the plan
 FBLA_HOST_API(cudaError_t fbla_k_attend_rows_launch(const fbla_k_prefill *a, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaStream_t stream);)
+// How the tensor-core pass of `tiles` pairs of row tiles per KV head over `passes` groups is launched (pure host arithmetic): one launch
+// for a count on the host, one or two for a count on the device with that ceiling, of which the count picks one. Returns their number.
+typedef struct { int cluster, above, tiles; } fbla_k_tc_deal;
+FBLA_HOST_API(int fbla_k_attend_tc_deal(int heads, int tiles, int passes, int device_count, fbla_k_tc_deal deal[2]);)
 // 1 if a bounded wait of the tensor-core kernel gave up since the last call (and clears it), 0 if not, -1 on a CUDA
 // error. A CTA whose wait gave up also writes NaN to every output row it owns, so the failure shows in the data.
 FBLA_HOST_API(int fbla_k_attend_tc_status(void);)

@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(THREADS, 1) attend_tc_kernel(const fbla_k_pref
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   wait_previous_pass();
   allow_next_pass();
-  attend_tc_item<CB, FB, SPLIT>(a, smem_raw);
+  attend_tiles<CB, FB, SPLIT ? CLUSTER : WHOLE>(a, smem_raw);
 }
 }  // namespace tc
 }  // namespace fbla
@@ -33,6 +33,21 @@ extern "C" int fbla_k_attend_tc_status(void) {
   if (cudaMemcpyFromSymbol(&v, fbla::tc::g_status, sizeof(int)) != cudaSuccess) return -1;
   if (v) cudaMemcpyToSymbol(fbla::tc::g_status, &zero, sizeof(int));
   return v;
+}
+
+// The launches of a chunk (see fbla_kernels.h). A chunk of the ceiling's own size, at the end of the cache's room, has the fewest shares;
+// where fewer tokens can have more, the larger clusters are a launch of their own, with as many tiles as can have them: for one
+// launch with the largest cluster, a chunk of the ceiling's size would wait for SMs that its idle CTAs' clusters ask for.
+extern "C" int fbla_k_attend_tc_deal(int heads, int tiles, int passes, int device_count, fbla_k_tc_deal deal[2]) {
+  using fbla::tc::tile_shares;
+  const int own = tile_shares((long long)tiles * heads, passes, FBLA_K_TILE_SHARES), most = device_count ? tile_shares(heads, passes, FBLA_K_TILE_SHARES) : own;
+  int n = 0;
+  if (most > own) {
+    const int few = (148 - 8 * own) / ((own + 1) * heads);
+    deal[n++] = fbla_k_tc_deal{most, own, few < tiles ? few : tiles};
+  }
+  deal[n++] = fbla_k_tc_deal{own, 0, tiles};
+  return n;
 }
 
 extern "C" cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaStream_t stream) {
@@ -49,14 +64,21 @@ extern "C" cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaStre
     }
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  fbla_k_prefill args = *a;
-  // (device lengths: room for as many shares as a chunk of the ceiling's size can have at the end of the cache)
-  args.cluster = tile_shares((long long)tiles * heads, ((a->length ? a->room : a->n0 + a->count) - 1) / fbla::G + 1, FBLA_K_TILE_SHARES);
-  const bool split = args.cluster > 1;
-  const auto kernel = a->cb == 3 ? split ? attend_tc_kernel<3, 3, true> : attend_tc_kernel<3, 3, false> : split ? attend_tc_kernel<4, 2, true> : attend_tc_kernel<4, 2, false>;
-  // launched dependent where one wave holds the grid (a 777-token prompt 69.5 -> 67.8 us); several waves that began among the
-  // CTAs of the kernel before measured 3 % slower (batch 4 x 8192 4.55 -> 4.69 ms)
-  return fbla::launch(tiles * args.cluster * heads <= 148, args.cluster, kernel, dim3(tiles * args.cluster, heads), THREADS, smem, stream, args);
+  fbla_k_tc_deal deal[2];
+  const int launches = fbla_k_attend_tc_deal(heads, tiles, ((a->length ? a->room : a->n0 + a->count) - 1) / fbla::G + 1, a->dcount != nullptr, deal);
+  for (int i = 0; i < launches; ++i) {
+    fbla_k_prefill args = *a;
+    args.cluster = deal[i].cluster;
+    args.above = deal[i].above;
+    const bool split = args.cluster > 1;
+    const auto kernel = a->cb == 3 ? split ? attend_tc_kernel<3, 3, true> : attend_tc_kernel<3, 3, false> : split ? attend_tc_kernel<4, 2, true> : attend_tc_kernel<4, 2, false>;
+    const int wide = deal[i].tiles * args.cluster;
+    // launched dependent where one wave holds the grid (a 777-token prompt 69.5 -> 67.8 us); several waves that began among the
+    // CTAs of the kernel before measured 3 % slower (batch 4 x 8192 4.55 -> 4.69 ms)
+    const cudaError_t e = fbla::launch(wide * heads <= 148, args.cluster, kernel, dim3(wide, heads), THREADS, smem, stream, args);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 extern "C" int fbla_k_attend_plan(const fbla_k_prefill *a, fbla_k_prefill args[2], int tensor[2]) {
@@ -84,7 +106,7 @@ extern "C" cudaError_t fbla_k_attend_launch(const fbla_k_prefill *a, cudaStream_
 
 extern "C" cudaError_t fbla_k_attend_tc_pass(fbla_k_prefill *a, fbla_k_pass *info) {
   using namespace fbla::tc;
-  a->cluster = 1;
+  a->cluster = 1;  // (an item takes a tile's shares in turn)
   const int qg = a->q_heads / a->kv_heads, rows = a->count * qg, heads = a->batch * a->kv_heads;
   const size_t smem = sizeof(Smem) + 1024;
   if (a->cb == 3) return pass_of(attend_tc_kernel<3, 3, false>, (rows + CTA_ROWS - 1) / CTA_ROWS, heads, THREADS, smem, "fbla::tc::attend_tc_item<3, 3>", info);

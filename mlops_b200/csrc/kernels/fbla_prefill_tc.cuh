@@ -88,7 +88,11 @@ __device__ __forceinline__ bool wait(Smem &sm, uint64_t *bar, uint32_t parity) {
 // Few tiles over a long cache leave most SMs idle, and a CTA walks its groups one after the other. Then the passes of a tile
 // are split into equal runs, one CTA of a cluster each, whose (m, l, O) are merged over distributed shared memory. As many
 // as keep a run at twelve passes or more (the merge costs about three) while all clusters still fit the SMs at once -- 148,
-// less what clusters of that size waste of them. 500 tokens at 30 000 (4 / 2 heads, 3+3): 999 -> 158 us.
+// less what clusters of that size waste of them (a B200's number whatever the device: the runs decide the order of the sums, and
+// with them the result's bits). 500 tokens at 30 000 (4 / 2 heads, 3+3): 999 -> 158 us.
+// The number follows from the chunk's own size, wherever that lives: a launch for a count on the device serves the numbers
+// (above, cluster], and of the launches for one chunk the count picks one; an executor's item does a tile's shares one after the
+// other and merges them as the cluster does. So all of them give the same bits.
 __host__ __device__ inline int tile_shares(long long tiles, int passes, int most) {
   int c = passes / 12;
   c = c > most ? most : c;
@@ -183,10 +187,18 @@ __device__ __forceinline__ void exact_v(uint8_t *tile, const TokenRows rows, int
   }
 }
 
-// SPLIT: a cluster per tile (one build per way: the loops of the other one would carry the share's bounds in registers they lack,
-// 9 % of the time at batch 4 x 8192)
-template <int CB, int FB, bool SPLIT = false>
-__device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
+// How a CTA's two tiles are done: in one piece; as a share of a cluster; as one of the shares that an item does in turn. (One build
+// per way: the loops of the first would carry the share's bounds in registers they lack, 9 % of the time at batch 4 x 8192.)
+enum Way { WHOLE, CLUSTER, IN_TURN };
+// IN_TURN: what the shares so far have left for the thread's row and columns
+struct Kept { float m, l, o[64]; };
+__device__ __forceinline__ int shares_of(const fbla_k_prefill &a, int rows, int n1) {
+  return tile_shares((long long)((rows + CTA_ROWS - 1) / CTA_ROWS) * a.batch * a.kv_heads, (n1 - 1) / G + 1, FBLA_K_TILE_SHARES);
+}
+
+template <int CB, int FB, Way WAY>
+__device__ __forceinline__ void attend_tiles(const fbla_k_prefill &a, uint8_t *smem_raw, int turn = 0, Kept *kept = nullptr) {
+  constexpr bool SPLIT = WAY != WHOLE;
   smem_raw += (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // (an offset, not a rebuilt pointer: the address space stays known)
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
@@ -195,7 +207,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
   const int n0 = (a.length ? FBLA_POS::ro(a.length + (a.lstride ? b : 0)) : 0) + a.n0;
   const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, n1 = n0 + count;
   // the last tiles attend to the most groups: they are taken first, so that the grid's tail is made of short CTAs
-  const int cluster = SPLIT ? a.cluster : 1, rank = SPLIT ? FBLA_POS::x() % cluster : 0;
+  const int cluster = WAY == CLUSTER ? a.cluster : 1, rank = WAY == CLUSTER ? FBLA_POS::x() % cluster : turn;
   const int rows = count * qg, r0 = (FBLA_POS::nx() / cluster - 1 - FBLA_POS::x() / cluster) * CTA_ROWS;
   if (r0 >= rows || rows < a.tc_min_rows) return;  // (CTA-uniform; a short device count is the few-row pass's work)
   const int last_row = min(r0 + CTA_ROWS, rows) - 1;
@@ -204,10 +216,11 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
   const int n_closed = max(own_max - 1, 0), own_lo = max(own_min, 1);
   const int n_pass = n_closed + 1 + max(own_max - own_lo + 1, 0);
   // this CTA's share of them: passes [p_lo, p_hi), of which [p_lo, c_hi) closed, [x_lo, p_hi) BF16
-  const int shares = SPLIT ? tile_shares((long long)((rows + CTA_ROWS - 1) / CTA_ROWS) * a.batch * a.kv_heads, (n1 - 1) / G + 1, cluster) : 1;
-  if (shares == 1 && rank > 0) return;  // (the same for every CTA of the grid: nobody then meets its cluster)
-  const int p_lo = !SPLIT ? 0 : rank < shares ? (int)((long long)n_pass * rank / shares) : n_pass;
-  const int p_hi = !SPLIT || rank >= shares ? n_pass : (int)((long long)n_pass * (rank + 1) / shares);
+  const int shares = shares_of(a, rows, n1);
+  // (the same for every CTA of the grid, and of a cluster those leave that have no share: its barriers wait for threads that have not exited)
+  if (WAY == WHOLE ? shares > 1 : WAY == CLUSTER && (shares <= a.above || shares > cluster || rank >= shares)) return;
+  const int p_lo = !SPLIT ? 0 : (int)((long long)n_pass * rank / shares);
+  const int p_hi = !SPLIT ? n_pass : (int)((long long)n_pass * (rank + 1) / shares);
   const int c_hi = SPLIT ? min(n_closed, p_hi) : n_closed, x_lo = SPLIT ? max(n_closed, p_lo) : n_closed;
   auto pass_group = [&](int n, bool &closed) {
     closed = n < n_closed;
@@ -584,7 +597,7 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
       sm.ex2[X][r][hf] = l_run;
       pair_sync();
       const float l_row = sm.ex2[X][r][0] + sm.ex2[X][r][1];
-      if (SPLIT && shares > 1) {
+      if (WAY == CLUSTER && shares > 1) {
         // This share's sums for the cluster: O as it lies in tensor memory, 16-byte piece c of row r at c ^ (r % 32), over the
         // query tiles (every product has read them: the O products were issued last); (m, l) beside them.
         float *const row = reinterpret_cast<float *>(sm.q[0]) + (size_t)(ROWS * X + r) * D;
@@ -600,15 +613,33 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
         }
         if (!ok) *reinterpret_cast<volatile int *>(&sm.abort) = 1;
       } else {
+      float l_all = l_row;
+      if constexpr (WAY == IN_TURN) {  // this share's sums onto those of the shares before, as the cluster's CTAs add them
+        const float mn = fmaxf(kept->m, m_run), sa = kept->m == -FBLA_INF ? 0.f : ex2(kept->m - mn), sb = m_run == -FBLA_INF ? 0.f : ex2(m_run - mn);
+        kept->m = mn;
+        l_all = kept->l = fmaf(sa, kept->l, sb * l_row);
+#pragma unroll 1
+        for (int cu = 0; cu < 2; ++cu) {
+          uint32_t o[32];
+          if (p_lo < p_hi) tmem_ld32(tmem_o + 32 * cu, o);
+#pragma unroll
+          for (int z = 0; z < 32; ++z) kept->o[32 * cu + z] = fmaf(sa, kept->o[32 * cu + z], sb * (p_lo < p_hi ? __uint_as_float(o[z]) : 0.f));
+        }
+        if (!ok) kept->l = l_all = __int_as_float(0x7fc00000);
+      }
+      if (WAY != IN_TURN || rank == shares - 1) {
       // O column 32 cc + l is channel 4 l + cc: through the row's (now free) qhat row as BF16 in channel order, then out.
       // This thread: O columns 64 hf .. + 63 (cc = 2 hf, 2 hf + 1); then it copies chunks 8 hf .. + 7 of the row.
-      const float inv = 1.f / l_row;
+      const float inv = 1.f / l_all;
       uint16_t *stage = reinterpret_cast<uint16_t *>(sm.qp[X] + r * 256);  // 256 bytes per row, private to the pair
 #pragma unroll 1
       for (int cu = 0; cu < 2; ++cu) {
         const int cc = 2 * hf + cu;
         uint32_t o[32];
-        tmem_ld32(tmem + 256 + 128 * X + 64 * hf + lane_base + 32 * cu, o);
+        if constexpr (WAY == IN_TURN) {
+#pragma unroll
+          for (int l = 0; l < 32; ++l) o[l] = __float_as_uint(kept->o[32 * cu + l]);
+        } else tmem_ld32(tmem + 256 + 128 * X + 64 * hf + lane_base + 32 * cu, o);
 #pragma unroll
         for (int l = 0; l < 32; ++l)  // channel 4 l + cc: 16-byte chunk l / 2 of the row, stored at chunk (l / 2) ^ (r % 16)
           stage[8 * ((l >> 1) ^ (r & 15)) + 4 * (l & 1) + cc] = f32_to_bf16(__uint_as_float(o[l]) * inv);
@@ -621,13 +652,14 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
 #pragma unroll
         for (int c = 8 * hf; c < 8 * hf + 8; ++c) reinterpret_cast<uint4 *>(orow)[c] = ok ? reinterpret_cast<const uint4 *>(stage)[c ^ (r & 15)] : nan4;
       }
+      }
     }
     }
   }
-  if (SPLIT && shares > 1) {
+  if (WAY == CLUSTER && shares > 1) {
     // the cluster's CTAs merge the tiles' rows: this one rows rank, rank + shares, ... in 16-byte pieces of the output
     cluster_meet();
-    if (rank < shares) {
+    {
       for (int e = tid; e < (2 * ROWS / shares + 1) * (D / 8); e += THREADS) {
         const int rr = rank + shares * (e / (D / 8)), c8 = e % (D / 8), R = r0 + rr;  // channels 8 c8 ..: columns 32 cc + 2 c8, + 1
         if (rr >= 2 * ROWS || R >= rows) continue;
@@ -666,6 +698,24 @@ __device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t 
     mbar_inval(&sm.bar_k); mbar_inval(&sm.bar_v);
     for (int x = 0; x < 2; ++x) { mbar_inval(&sm.bar_q[x]); mbar_inval(&sm.bar_s[x]); mbar_inval(&sm.bar_p[x]); mbar_inval(&sm.bar_o[x]); }
   }
+}
+
+// An executor's item: two tiles, in one piece or share after share.
+template <int CB, int FB>
+__device__ __forceinline__ void attend_tc_item(const fbla_k_prefill &a, uint8_t *smem_raw) {
+  const int n0 = (a.length ? FBLA_POS::ro(a.length + (a.lstride ? FBLA_POS::y() / a.kv_heads : 0)) : 0) + a.n0;
+  const int count = a.dcount ? FBLA_POS::ro(a.dcount) : a.count, shares = shares_of(a, count * (a.q_heads / a.kv_heads), n0 + count);
+  if (shares == 1) {
+    attend_tiles<CB, FB, WHOLE>(a, smem_raw);
+    return;
+  }
+  Kept kept;
+  kept.m = -FBLA_INF;
+  kept.l = 0.f;
+#pragma unroll 1
+  for (int z = 0; z < 64; ++z) kept.o[z] = 0.f;
+#pragma unroll 1
+  for (int s = 0; s < shares; ++s) attend_tiles<CB, FB, IN_TURN>(a, smem_raw, s, &kept);
 }
 
 }  // namespace tc

@@ -54,6 +54,36 @@ def test_rows_are_folded_per_cta_for_few_heads_only(lib):
     assert split_of(lib, 4, 4, 8, 2, 65536)[1] == 0
 
 
+class Deal(ctypes.Structure):
+    _fields_ = [("cluster", ctypes.c_int), ("above", ctypes.c_int), ("tiles", ctypes.c_int)]
+
+
+def test_one_launch_of_a_device_count_serves_every_chunk(lib):
+    """The shares of a chunk's tiles follow from its own size; of the launches for a ceiling exactly one serves them, with all of the chunk's tiles."""
+    def deal_of(heads, tiles, passes, device_count):
+        d = (Deal * 2)()
+        n = lib.fbla_k_attend_tc_deal(heads, tiles, passes, device_count, d)
+        return [(x.cluster, x.above, x.tiles) for x in d[:n]]
+
+    def shares(heads, tiles, passes):
+        (cluster, above, _), = deal_of(heads, tiles, passes, 0)
+        assert above == 0
+        return cluster
+    assert shares(2, 2, 95) == 7 and shares(8, 64, 512) == 1 and shares(1, 1, 23) == 1 and shares(1, 1, 24) == 2 and shares(8, 1, 1 << 19) == 8
+    for heads in (1, 2, 8, 16, 70, 71, 512):
+        for room in (8, 24, 25, 60, 96, 1000):
+            for ceiling in (1, 2, 3, 7, 12, 36, 70, 71, 300):
+                launches = deal_of(heads, ceiling, room, 1)
+                for tiles in sorted({1, 2, 3, 5, 11, 12, 35, ceiling // 2, ceiling}):
+                    if not 1 <= tiles <= ceiling:
+                        continue
+                    for passes in (1, 12, 24, room // 2, room):
+                        if 1 <= passes <= room:
+                            n = shares(heads, tiles, passes)
+                            serving = [x for x in launches if x[1] < n <= x[0]]
+                            assert len(serving) == 1 and serving[0][2] >= tiles, (heads, room, ceiling, tiles, passes, launches)
+
+
 def test_bench_accounts_the_bytes_the_way_the_reference_bench_does():
     """Algorithmic bytes of a decode: per closed (KV head, group) 8 coarse records + 1 KiB of metadata, 512 B per BF16
     window token, 3 072 B per refined (KV head, sub-block) (attention/fbla/bench/bench_fbla.cu:136-141)."""
