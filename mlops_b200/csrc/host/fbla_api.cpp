@@ -822,7 +822,7 @@ int mlops_fbla_item_access(const mlops_fbla_items *passes, int npasses, int pass
       const bool scores = p.kind == MLOPS_FBLA_ITEM_COARSE, values = p.kind == MLOPS_FBLA_ITEM_REFINE;
       if (scores || values) {
         r.add(MLOPS_FBLA_ARG_Q, 0, 0, (long long)a.batch * a.q_heads * row);
-        for (int h = 0; h < heads; ++h) head_units(r, p, h, 0, true, values, true);
+        for (int h = 0; h < heads; ++h) head_units(r, p, h, 0, true, true, true);  // (the scores are formed under both planes)
         r.add(MLOPS_FBLA_ARG_SCRATCH, scores, lse, part - lse);
         r.add(MLOPS_FBLA_ARG_SCRATCH, 1, status, 16);
       }
@@ -839,6 +839,7 @@ int mlops_fbla_item_access(const mlops_fbla_items *passes, int npasses, int pass
       }
       if (p.kind == MLOPS_FBLA_ITEM_MERGE) {
         const int vh = item / a.qg, qi = item % a.qg, b = vh / hpr, hir = vh % hpr;
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 0, status, 16);
         r.add(MLOPS_FBLA_ARG_OUT, 1, ((long long)b * a.q_heads + (hir / a.vg) * (a.qg * a.vg) + (hir % a.vg) * a.qg + qi) * row, row);
       }
       return r.n;
@@ -874,6 +875,7 @@ int mlops_fbla_item_access(const mlops_fbla_items *passes, int npasses, int pass
       r.add(MLOPS_FBLA_ARG_SCRATCH, 0, dpart, row_r - dpart);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 0, row_r + (long long)vh * a.qg * 4, a.qg * 4);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 0, item_off, (long long)(vheads + 1) * 4);
+      r.add(MLOPS_FBLA_ARG_SCRATCH, 0, status, 16);
       r.add(MLOPS_FBLA_ARG_OUT, 1, qrow * row, row);
     }
   } else if (p.kind == MLOPS_FBLA_ITEM_QKV || p.kind == MLOPS_FBLA_ITEM_QKV_CHUNK) {

@@ -88,10 +88,12 @@ def item_call(lib, p):
     return buf.value.decode()
 
 
-def run_plan(lib, passes, n, stream, ctas=None):
+def run_plan(lib, passes, n, stream, ctas=None, around=None):
     """Compiles one kernel per pass and launches them in order on `stream` (a CUDA stream handle): an executor whose only
     dependency rule is 'every item of a pass after every item of the pass before' (stream order). ctas: run every pass
-    as a persistent loop on that many CTAs instead of one CTA per item."""
+    as a persistent loop on that many CTAs instead of one CTA per item. around(i): a context manager for pass i."""
+    import contextlib
+
     import numpy as np
     import torch
     from cuda.bindings import driver
@@ -112,7 +114,8 @@ def run_plan(lib, passes, n, stream, ctas=None):
         keep.append(blob)
         arg = np.array([blob.data_ptr()], dtype=np.uint64)
         params = np.array([arg.ctypes.data], dtype=np.uint64)
-        err, = driver.cuLaunchKernel(fn, p.items if ctas is None else min(ctas, p.items), 1, 1, p.threads, 1, 1, p.smem_bytes, stream, params.ctypes.data, 0)
+        with around(i) if around else contextlib.nullcontext():
+            err, = driver.cuLaunchKernel(fn, p.items if ctas is None else min(ctas, p.items), 1, 1, p.threads, 1, 1, p.smem_bytes, stream, params.ctypes.data, 0)
         assert err == driver.CUresult.CUDA_SUCCESS, err
     torch.cuda.synchronize()
     driver.cuModuleUnload(module)

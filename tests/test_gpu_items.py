@@ -2,6 +2,7 @@
 compiled by NVRTC, one CTA per item, passes in stream order), gives bit for bit what the equally named stream call gives;
 and every byte a call changes lies inside the write ranges that mlops_fbla_item_access declares.
 Modelled on attention/fbla/tests/test_items.cu:489-496 (items == stream API) and :300-420 (ranges)."""
+import contextlib
 import ctypes
 import os
 
@@ -89,6 +90,38 @@ def test_decode_plan_equals_decode_at(ours, mode, QH, KH, N, cap, ctas):
     changed = scratch.cpu().numpy() != before
     _covered(changed, _write_ranges(lib, passes, n, "SCRATCH"), "decode scratch")
     _covered(np.ones(out.numel() * 2, bool), _write_ranges(lib, passes, n, "OUT"), "decode output")
+
+
+@pytest.mark.parametrize("mode,N,cap", [("4+2", 3000, 4096), ("3+3", 3000, 4096), ("4+2", 3000, 49152), ("3+3", 3000, 163840)])
+def test_decode_passes_read_what_they_declare(ours, mode, N, cap):
+    """An executor may hold other bytes in an array while a pass runs that does not name it: every pass of the decode's plan (two sweeps, and
+    the coarse sweep with corrections under a large capacity) with noise in the cache arrays that none of its items reads."""
+    QH, KH = 8, 2
+    q, k, v = datagen.baseline_case(42, 1, QH, KH, N)
+    qd = gu.bf16_tensor(q)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=cap)
+    length = _i32(N)
+    want = ours.decode_at(c, qd, length)
+    lib, vp, kc, passes, out = ours.lib, ctypes.c_void_p, ours._cache(c), (iu.Items * 4)(), torch.full_like(qd, -9.0)
+    nbytes = lib.mlops_fbla_decode_scratch_bytes(ctypes.byref(gu.Config(1, QH, KH, cap, 0, 0, gu.FORMATS[mode][2], cap, 0, 0, 0, 0, 0)))
+    scratch = torch.empty((nbytes,), dtype=torch.uint8, device="cuda")
+    n = lib.mlops_fbla_decode_at_items(ctypes.byref(_cfg(c, QH)), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
+                                       vp(scratch.data_ptr()), ctypes.c_size_t(nbytes), 0, passes, 4)
+    assert n == 4, ours.error()
+    arrays = dict(COARSE=c["coarse"], FINE=c["fine"], META=c["meta"], SINK_K=c["sink_k"], SINK_V=c["sink_v"], OPEN_K=c["open_k"], OPEN_V=c["open_v"])
+
+    @contextlib.contextmanager
+    def around(i):
+        named = {iu.ARGS[r.arg] for item in range(passes[i].items) for r in iu.access(lib, passes, n, i, item)}
+        kept = {a: t.clone() for a, t in arrays.items() if a not in named}
+        for a in kept:
+            arrays[a].view(torch.uint8).random_(0, 64)  # (finite BF16 numbers)
+        yield
+        for a, t in kept.items():
+            arrays[a].copy_(t)
+
+    iu.run_plan(lib, passes, n, _stream(), around=around)
+    assert torch.equal(out, want)
 
 
 @pytest.mark.parametrize("mode,count,ctas", [("4+2", 300, None), ("3+3", 5, None), ("3+3", 700, 3)])
