@@ -131,31 +131,42 @@ def _arrays(c):
 
 _scratch_bytes = functools.lru_cache(maxsize=256)(lambda device, *shape: scratch_bytes(*shape))
 _raw_stream = torch._C._cuda_getCurrentRawStream
+_capturing = torch._C._cuda_isCurrentStreamCapturing
+
+
+class _Scratch:
+    """a decode's scratch; `lock` is held while a call's kernels are enqueued, so that threads on one stream do not mix theirs"""
+    __slots__ = ("bytes", "buffer", "pointer", "lock")
+
+    def __init__(self, nbytes, device):
+        self.bytes, self.lock = nbytes, threading.Lock()
+        self.buffer = torch.empty((nbytes,), dtype=torch.uint8, device=device)  # the library needs no initial contents
+        self.pointer = self.buffer.data_ptr()
 
 
 class _ScratchPool:
-    """Decode scratch, one buffer per (device, stream, batch x KV heads), grown on demand and kept for later calls -- at most
-    BUFFERS of them, the least recently used one given back first. Calls of one stream run in order, so they may share one;
-    calls of different streams never do."""
+    """Decode scratch, one buffer per (device, stream), grown on demand and kept for later calls -- at most BUFFERS of them, the
+    least recently used one given back first (to the stream's own free memory: the kernels that use it come before whatever takes it
+    next). Calls of one stream run in order, so they may share one; calls of different streams never do. A call that is being captured
+    has one of its own, from the graph's memory: a replay may run on any stream and at any later time."""
     BUFFERS = 16
 
     def __init__(self):
-        self._buffers, self._lock = collections.OrderedDict(), threading.Lock()
+        self._held, self._lock = collections.OrderedDict(), threading.Lock()
 
-    def get(self, device, stream, heads, nbytes):
-        key = device.index, stream, heads
+    def get(self, device, stream, nbytes):
+        if device.type == "cuda" and _capturing():
+            return _Scratch(nbytes, device)
+        key = device, stream
         with self._lock:
-            held = self._buffers.get(key)
-            if held is not None and held[0] >= nbytes:
-                self._buffers.move_to_end(key)
+            held = self._held.get(key)
+            if held is not None and held.bytes >= nbytes:
+                self._held.move_to_end(key)
                 return held
-        fresh = torch.empty((nbytes,), dtype=torch.uint8, device=device)  # the library needs no initial contents
-        held = nbytes, fresh.data_ptr(), fresh
-        with self._lock:
-            self._buffers[key] = held
-            self._buffers.move_to_end(key)
-            while len(self._buffers) > self.BUFFERS:
-                self._buffers.popitem(last=False)
+            self._held[key] = held = _Scratch(nbytes, device)
+            self._held.move_to_end(key)
+            while len(self._held) > self.BUFFERS:
+                self._held.popitem(last=False)
         return held
 
 
@@ -177,10 +188,12 @@ def decode_cache(q, c, scale, tau):
     batch, q_heads, kv_heads = q.size(0), q.size(1), c.meta.size(1)
     need = _scratch_bytes(device.index, batch, q_heads, kv_heads, c.capacity, c.format, c.capacity)
     stream = _raw_stream(device.index)
-    size, scratch, keep = _pool.get(device, stream, batch * kv_heads, need)
+    scratch = _pool.get(device, stream, need)
     out = torch.empty_like(q)
     cfg = Config(batch, q_heads, kv_heads, int(c.tokens), float(scale), float(tau), int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
-    _raise(_lib.mlops_fbla_decode(ctypes.byref(cfg), q.data_ptr(), ctypes.byref(struct), out.data_ptr(), scratch, size, stream), "mlops_fbla_decode")
+    with scratch.lock:
+        status = _lib.mlops_fbla_decode(ctypes.byref(cfg), q.data_ptr(), ctypes.byref(struct), out.data_ptr(), scratch.pointer, scratch.bytes, stream)
+    _raise(status, "mlops_fbla_decode")
     return out
 
 

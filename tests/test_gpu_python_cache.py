@@ -3,6 +3,7 @@ looks at the arrays it is given; the decode's scratch is nobody else's (threads 
 import copy
 import io
 import pickle
+import threading
 
 import pytest
 import torch
@@ -54,3 +55,51 @@ def test_every_call_looks_at_the_arrays():
     cache.sink_v.transpose_(2, 3)
     with pytest.raises(ValueError, match="contiguous"):
         attention.append(cache, *(torch.zeros((1, 2, 1, 128), dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+
+
+def test_a_captured_decode_keeps_its_scratch():
+    """A graph's kernels name the scratch of the calls it was captured from: nothing that runs later may be given that memory, however
+    many streams decode in between."""
+    q, cache = _case(3000, 2, 8, 2, capacity=4096)
+    want = attention.decode(q, cache)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        attention.decode(q, cache)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = attention.decode(q, cache)
+    others = [torch.cuda.Stream() for _ in range(20)]
+    for s in others:
+        with torch.cuda.stream(s):
+            attention.decode(q, cache)
+    torch.cuda.synchronize()
+    nbytes = attention._C.scratch_bytes(2, 8, 2, 4096, cache.format, 4096)
+    with torch.cuda.stream(stream):
+        guards = [torch.full((nbytes,), 0x5A, dtype=torch.uint8, device="cuda") for _ in range(4)]
+    stream.synchronize()
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert all(bool((g == 0x5A).all()) for g in guards)
+
+
+def test_threads_on_one_stream():
+    """Two threads that decode on the same stream share its scratch: the kernels of one call are never enqueued between another's."""
+    cases = [_case(n, 1, 8, 2, capacity=4096) for n in (3001, 3002)]
+    want = [attention.decode(*c) for c in cases]
+    torch.cuda.synchronize()
+    wrong, start = [], threading.Barrier(2)
+
+    def work(i):
+        start.wait()
+        outs = [attention.decode(*cases[i]) for _ in range(300)]
+        torch.cuda.synchronize()
+        wrong.extend(k for k, o in enumerate(outs) if not torch.equal(o, want[i]))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
