@@ -186,11 +186,13 @@ def decode_cache(q, c, scale, tau):
         with torch.cuda.device(device.index):
             return decode_cache(q, c, scale, tau)
     batch, q_heads, kv_heads = q.size(0), q.size(1), c.meta.size(1)
-    need = _scratch_bytes(device.index, batch, q_heads, kv_heads, c.capacity, c.format, c.capacity)
+    tokens, capacity = int(c.tokens), int(c.capacity)
+    room = min(capacity, -(-tokens // 16384) * 16384)  # (asked for once in 16 384 tokens; a slot may have room for far more than it holds)
+    need = _scratch_bytes(device.index, batch, q_heads, kv_heads, room, c.format, capacity)
     stream = _raw_stream(device.index)
     scratch = _pool.get(device, stream, need)
     out = torch.empty_like(q)
-    cfg = Config(batch, q_heads, kv_heads, int(c.tokens), float(scale), float(tau), int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
+    cfg = Config(batch, q_heads, kv_heads, tokens, float(scale), float(tau), int(c.format), capacity, 0, 0, 0, 0, 0)
     with scratch.lock:
         status = _lib.mlops_fbla_decode(ctypes.byref(cfg), q.data_ptr(), ctypes.byref(struct), out.data_ptr(), scratch.pointer, scratch.bytes, stream)
     _raise(status, "mlops_fbla_decode")

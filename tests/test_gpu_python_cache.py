@@ -103,3 +103,15 @@ def test_threads_on_one_stream():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_scratch_follows_the_tokens():
+    """A slot with room for more tokens than one decode takes is decoded as long as it holds no more than that."""
+    q, cache = _case(300)
+    slot = attention.empty(1, 2, (1 << 26) + 128, "3+3")
+    for a in ARRAYS:
+        held = getattr(cache, a)
+        getattr(slot, a)[:, :, :held.shape[2]].copy_(held)
+    slot.tokens = 300
+    got, want = (attention.decode(q, c).float() for c in (slot, cache))
+    assert float((got - want).abs().max()) <= 2e-3 * float(want.abs().max()) + 2.0 ** -7 * float(want.abs().max())
