@@ -24,10 +24,6 @@ __device__ __forceinline__ void mma_u8u8_k16_zero(uint32_t (&d)[4], uint32_t a0,
   asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(b0), "n"(0));
 }
-__device__ __forceinline__ void mma_u8u8_k16(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
-}
 
 // ---- qhat fragments -------------------------------------------------------------------------------------------------
 // qst: 8 rows (fragment columns: queries, rows >= QG zero) of 128 s8 codes in channel order, row stride QST_ROW bytes

@@ -16,11 +16,6 @@ template <class K> cudaError_t pass_of(K kernel, int gx, int gy, int threads, si
 }  // namespace
 
 namespace fbla {
-template <bool NORM>
-__global__ void __launch_bounds__(256) qkv_token_kernel(const fbla_k_token a) {
-  qkv_token_item<NORM>(a, nullptr);
-}
-
 // The whole one-token step of a (batch row, KV head): the group that the position closes is quantised from the open window,
 // then the token takes its place. One launch: the close pass alone is a launch that finds nothing to do 127 times of 128.
 template <int CB, int FB, bool NORM>
@@ -64,10 +59,11 @@ extern "C" cudaError_t fbla_k_qkv_chunk_launch(const fbla_k_token *a, cudaStream
   return fbla::launch(true, 1, a->q_norm ? fbla::qkv_chunk_kernel<true> : fbla::qkv_chunk_kernel<false>, grid, 256, 0, stream, *a);
 }
 
+// (the registers of the kernel that runs the item here: the whole step)
 extern "C" cudaError_t fbla_k_qkv_token_pass(const fbla_k_token *a, fbla_k_pass *info) {
   const int heads = a->batch * a->kv_heads;
-  if (a->q_norm) return pass_of(fbla::qkv_token_kernel<true>, heads, 1, 256, 0, "fbla::qkv_token_item<true>", info);
-  return pass_of(fbla::qkv_token_kernel<false>, heads, 1, 256, 0, "fbla::qkv_token_item<false>", info);
+  if (a->q_norm) return pass_of(fbla::qkv_step_kernel<3, 3, true>, heads, 1, 256, 0, "fbla::qkv_token_item<true>", info);
+  return pass_of(fbla::qkv_step_kernel<3, 3, false>, heads, 1, 256, 0, "fbla::qkv_token_item<false>", info);
 }
 
 extern "C" cudaError_t fbla_k_qkv_chunk_pass(const fbla_k_token *a, fbla_k_pass *info) {
