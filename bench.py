@@ -363,10 +363,15 @@ def decode_record(cfg, rec, n_gpus):
                 kernel="decode call, all passes", algorithmic_bytes=rec["abytes"], bytes_parts=rec["parts"])
     if rec["pass_us"]:
         us, parts = rec["pass_us"], rec["parts"]
-        if rec["dense"]:  # scores: K's half of the coarse records and of the metadata; values: everything once
+        if rec["dense"]:
+            # scores: K's half of both planes and of the metadata, the windows; written: 40 bytes per (sub-block, query). values: V's
+            # half of the coarse plane and of the metadata, of the fine one where refined, and 28 of those 40 bytes
             names = ["score_kernel", "mass_kernel", "value_kernel", "gather_kernel"]
-            fine = (3, 2)[cfg["mode"] == "4+2"] / 6  # the fine records' share of a refined sub-block's bytes
-            bytes_of = [parts["coarse_and_meta"] / 2 + parts["bf16_windows"], None, parts["coarse_and_meta"] + fine * parts["refine"], None]
+            cb, fb = (4, 2) if cfg["mode"] == "4+2" else (3, 3)
+            units = parts["coarse_and_meta"] / (8 * 512 * cb + 1024)
+            cells = units * 8 * (cfg["q_heads"] // cfg["kv_heads"])
+            bytes_of = [units * (2048 * (cb + fb) + 512) + parts["bf16_windows"] + 40 * cells, None,
+                        units * (2048 * cb + 512) + parts["refine"] * fb / 12 + 28 * cells, None]
         else:
             names = ["coarse_kernel", "select_kernel", "refine_kernel", "merge_kernel"]
             bytes_of = [parts["coarse_and_meta"] + parts["bf16_windows"], None, parts["refine"], None]
