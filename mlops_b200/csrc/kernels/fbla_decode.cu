@@ -4,10 +4,10 @@
 #include <stdio.h>
 
 namespace fbla {
-template <int CB, int FB, int QG, int DEAL>
-__global__ void __launch_bounds__(32 * CoarseShape<CB>::TOTAL, 1) coarse_kernel(const fbla_k_decode a) {
+template <int CB, int FB, int QG, int DEAL, int SHAPE>
+__global__ void __launch_bounds__(32 * CoarseShape<CB, SHAPE>::TOTAL, 1) coarse_kernel(const fbla_k_decode a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  coarse_item<CB, FB, QG, DEAL>(a, smem_raw);
+  coarse_item<CB, FB, QG, DEAL, SHAPE>(a, smem_raw);
 }
 
 template <int QG>
@@ -37,18 +37,31 @@ template <class K> cudaError_t pass_of(K kernel, int gx, int gy, int threads, si
 }
 }  // namespace
 
+// the coarse kernel of a deal and a shape (a.deal, a.deep), its threads and shared memory
+struct CoarseBuild { void (*kernel)(const fbla_k_decode); int threads; size_t smem; };
+template <int CB, int FB, int QG, int SHAPE> CoarseBuild coarse_build(int deal) {
+  return CoarseBuild{deal == FBLA_K_DEAL_LENGTHS ? coarse_kernel<CB, FB, QG, FBLA_K_DEAL_LENGTHS, SHAPE>
+                     : deal == FBLA_K_DEAL_FIXED ? coarse_kernel<CB, FB, QG, FBLA_K_DEAL_FIXED, SHAPE> : coarse_kernel<CB, FB, QG, FBLA_K_DEAL_COST, SHAPE>,
+                     32 * CoarseShape<CB, SHAPE>::TOTAL, sizeof(CoarseSmem<CB, SHAPE>)};
+}
+template <int CB, int FB, int QG> CoarseBuild coarse_build(int deal, int deep) {
+  return deep ? coarse_build<CB, FB, QG, DEEP>(deal) : coarse_build<CB, FB, QG, WIDE>(deal);
+}
+
 constexpr int REFINE_SMEM_MAX = 220 * 1024;  // dynamic shared memory of the refine pass (its ring + the slice prefix)
 template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a, cudaStream_t stream) {
   const int vheads = a.batch * a.kv_heads * a.vg;
-  const size_t csm = sizeof(CoarseSmem<CB>);
   const size_t rsm = sizeof(RefineWarp<CB, FB>) * RefineShape<CB, FB>::WARPS + sizeof(int) * ((size_t)vheads * a.nslices + 1);
   static thread_local int configured[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(coarse_kernel<CB, FB, QG, FBLA_K_DEAL_LENGTHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(coarse_kernel<CB, FB, QG, FBLA_K_DEAL_FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(coarse_kernel<CB, FB, QG, FBLA_K_DEAL_COST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
+    cudaError_t e = cudaSuccess;
+    for (const int deal : {FBLA_K_DEAL_LENGTHS, FBLA_K_DEAL_FIXED, FBLA_K_DEAL_COST})
+      for (const int deep : {0, 1}) {
+        const CoarseBuild c = coarse_build<CB, FB, QG>(deal, deep);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
+      }
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(refine_kernel<CB, FB, QG>, cudaFuncAttributeMaxDynamicSharedMemorySize, REFINE_SMEM_MAX);
     if (e != cudaSuccess) return e;
@@ -62,9 +75,8 @@ template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a,
     if (e != cudaSuccess) return e;
   }
   if (a.phase != 2) {
-    if (a.deal == FBLA_K_DEAL_LENGTHS) coarse_kernel<CB, FB, QG, FBLA_K_DEAL_LENGTHS><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
-    else if (a.deal == FBLA_K_DEAL_FIXED) coarse_kernel<CB, FB, QG, FBLA_K_DEAL_FIXED><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
-    else coarse_kernel<CB, FB, QG, FBLA_K_DEAL_COST><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
+    const CoarseBuild c = coarse_build<CB, FB, QG>(a.deal, a.deep);
+    c.kernel<<<a.coarse_ctas, c.threads, c.smem, stream>>>(a);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = launch(true, 1, select_kernel<QG>, dim3(a.phase == 1 ? 1 : a.nslices, vheads), 256, 0, stream, a);
     if (a.phase == 1) return e;
@@ -80,15 +92,14 @@ template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a,
 // one pass alone, as an ordinary launch (no overlap with its neighbours): for measurements pass by pass
 template <int CB, int FB, int QG> cudaError_t launch_one(const fbla_k_decode &a, int pass, cudaStream_t stream) {
   const int vheads = a.batch * a.kv_heads * a.vg;
-  const size_t csm = sizeof(CoarseSmem<CB>);
   const size_t rsm = sizeof(RefineWarp<CB, FB>) * RefineShape<CB, FB>::WARPS + sizeof(int) * ((size_t)vheads * a.nslices + 1);
   if (rsm > REFINE_SMEM_MAX) return cudaErrorInvalidValue;
   switch (pass) {
-    case 0:
-      if (a.deal == FBLA_K_DEAL_LENGTHS) coarse_kernel<CB, FB, QG, FBLA_K_DEAL_LENGTHS><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
-      else if (a.deal == FBLA_K_DEAL_FIXED) coarse_kernel<CB, FB, QG, FBLA_K_DEAL_FIXED><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
-      else coarse_kernel<CB, FB, QG, FBLA_K_DEAL_COST><<<a.coarse_ctas, 32 * CoarseShape<CB>::TOTAL, csm, stream>>>(a);
+    case 0: {
+      const CoarseBuild c = coarse_build<CB, FB, QG>(a.deal, a.deep);
+      c.kernel<<<a.coarse_ctas, c.threads, c.smem, stream>>>(a);
       break;
+    }
     case 1: select_kernel<QG><<<dim3(a.nslices, vheads), 256, 0, stream>>>(a); break;
     case 2: refine_kernel<CB, FB, QG><<<a.refine_ctas, 32 * RefineShape<CB, FB>::WARPS, rsm, stream>>>(a); break;
     case 3: merge_kernel<QG><<<vheads * QG, 512, 0, stream>>>(a); break;
@@ -99,14 +110,12 @@ template <int CB, int FB, int QG> cudaError_t launch_one(const fbla_k_decode &a,
 
 template <int CB, int FB, int QG> cudaError_t passes_of(const fbla_k_decode &a, fbla_k_pass *p) {
   const int vheads = a.batch * a.kv_heads * a.vg;
-  const size_t csm = sizeof(CoarseSmem<CB>) + 128;
   const size_t rsm = sizeof(RefineWarp<CB, FB>) * RefineShape<CB, FB>::WARPS + sizeof(int) * ((size_t)vheads * a.nslices + 1) + 128;
   if (rsm - 128 > REFINE_SMEM_MAX) return cudaErrorInvalidValue;
   char e[96];
-  snprintf(e, sizeof e, "fbla::coarse_item<%d, %d, %d, %d>", CB, FB, QG, (int)a.deal);
-  cudaError_t st = a.deal == FBLA_K_DEAL_LENGTHS ? pass_of(coarse_kernel<CB, FB, QG, FBLA_K_DEAL_LENGTHS>, a.coarse_ctas, 1, 32 * CoarseShape<CB>::TOTAL, csm, e, p + 0)
-                   : a.deal == FBLA_K_DEAL_FIXED ? pass_of(coarse_kernel<CB, FB, QG, FBLA_K_DEAL_FIXED>, a.coarse_ctas, 1, 32 * CoarseShape<CB>::TOTAL, csm, e, p + 0)
-                                                 : pass_of(coarse_kernel<CB, FB, QG, FBLA_K_DEAL_COST>, a.coarse_ctas, 1, 32 * CoarseShape<CB>::TOTAL, csm, e, p + 0);
+  const CoarseBuild c = coarse_build<CB, FB, QG>(a.deal, a.deep);
+  snprintf(e, sizeof e, "fbla::coarse_item<%d, %d, %d, %d, %d>", CB, FB, QG, (int)a.deal, (int)a.deep);
+  cudaError_t st = pass_of(c.kernel, a.coarse_ctas, 1, c.threads, c.smem + 128, e, p + 0);
   snprintf(e, sizeof e, "fbla::select_item<%d>", QG);
   if (st == cudaSuccess) st = pass_of(select_kernel<QG>, a.nslices, vheads, 256, 0, e, p + 1);
   snprintf(e, sizeof e, "fbla::refine_item<%d, %d, %d>", CB, FB, QG);
@@ -158,7 +167,7 @@ extern "C" cudaError_t fbla_k_decode_shape(fbla_k_decode *a) {
   e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   a->coarse_ctas = sms;
-  a->coarse_warps = fbla::CoarseShape<4>::TOTAL;  // (the larger of the two layouts: what the scratch is sized for)
+  a->coarse_warps = fbla::CoarseShape<4, fbla::WIDE>::TOTAL;  // (the larger of the two shapes: what the scratch is sized for)
   a->refine_ctas = sms;
   a->refine_warps = fbla::RefineShape<4, 2>::WARPS;
   return cudaSuccess;
@@ -168,9 +177,17 @@ extern "C" cudaError_t fbla_k_decode_shape(fbla_k_decode *a) {
 //   by the lengths when the BF16 windows would get three eighths of a CTA's warps or more (contexts up to about 4 700 tokens);
 //   else all warps but one stream and one serves windows, or every warp has an equal cost share of windows and groups --
 //   whichever leaves an eighth of a CTA fewer groups (whole groups), with 5 % against the deal by cost: a CTA whose every
-//   warp streams runs a group that much slower. The line was measured with eight warps per CTA and holds with twelve. Measured on B200 (eight warps), by cost against seven + one: batch 1 x 128K tokens 80.0 -> 75.3 us per step in 3+3 and
-//   65.7 -> 61.6 in 4+2 (7 groups per warp instead of 8), batch 64 x 1K..64K 2.07 -> 2.02 ms, but batch 8 x 16K 120.0 ->
-//   123.9 (8 groups per warp either way).
+//   warp streams runs a group that much slower. Measured on B200 with the eight warps of the deep shape, by cost against seven + one:
+//   batch 1 x 128K tokens 80.0 -> 75.3 us per step in 3+3 and 65.7 -> 61.6 in 4+2 (7 groups per warp instead of 8), batch 64 x 1K..64K
+//   2.07 -> 2.02 ms, but batch 8 x 16K 120.0 -> 123.9 (8 groups per warp either way). With the twelve warps of the wide shape, fixed
+//   split / by cost: 1 x 128K 3+3 73.8 / 62.8, 1 x 512K 149 / 138, 8 x 128K 276 / 262; where the choice falls on the slower of the two
+//   it costs up to 8 % (2 x 50 000, 4+2: 55.6 / 59.9).
+// And the shape. A group takes a warp 1.4 times as long among twelve as among eight, so the wide shape pays where it leaves a warp less
+// than three quarters of the groups (whole groups); with several queries and one or two groups per warp its shallower look-ahead costs more
+// than that. Measured wide / deep, us per step, one sweep, N(0, 1), by (groups per warp deep, wide): 4+2 1 x 60 000 (4, 3) 46.9 / 41.6;
+// 1 x 150 000 (8, 6) 71.2 / 61.3; 1 x 20 000 (2, 1) 44.2 / 41.4, with one query per head 31.2 / 32.6; 3+3 1 x 128K (7, 5) 62.5 / 63.5; 1 x 266 667
+// (15, 10) 92.3 / 100.8; 2 x 66 667 (8, 5) 104 / 114. (Eight warps as they were before the pair's sub-blocks shared the score products'
+// columns: 1 x 60 000 43.7, 1 x 150 000 63.4, 1 x 266 667 102.5.)
 extern "C" void fbla_k_decode_split(fbla_k_decode *a, long long tokens) {
   constexpr int total = 8;  // (the choice is made in eighths of a CTA)
   const long long groups = (tokens + fbla::G - 1) / fbla::G, S = groups > 2 ? groups - 2 : 0;
@@ -180,8 +197,15 @@ extern "C" void fbla_k_decode_split(fbla_k_decode *a, long long tokens) {
   // groups an eighth of a CTA takes: seven eighths streaming; by cost (deal_of's share, a whole number of groups)
   const long long fixed = (heads * S + ctas * (total - 1) - 1) / (ctas * (total - 1));
   const long long cost = (fbla::GROUP_COST * heads * S + fbla::WINDOW_COST * heads * W + fbla::GROUP_COST * ctas * total - 1) / (fbla::GROUP_COST * ctas * total);
-  a->coarse_warps = a->cb == 4 ? fbla::CoarseShape<4>::TOTAL : fbla::CoarseShape<3>::TOTAL;
   a->deal = by_lengths ? FBLA_K_DEAL_LENGTHS : 21 * cost < 20 * fixed ? FBLA_K_DEAL_COST : FBLA_K_DEAL_FIXED;
+  auto per_warp = [&](int warps) {  // groups of a streaming warp in a shape of `warps`
+    const long long share = a->deal == FBLA_K_DEAL_COST ? fbla::GROUP_COST * ctas * warps : ctas * (warps - 1);
+    const long long units = a->deal == FBLA_K_DEAL_COST ? fbla::GROUP_COST * heads * S + fbla::WINDOW_COST * heads * W : heads * S;
+    return (units + share - 1) / share;
+  };
+  constexpr int eight = fbla::CoarseShape<4, fbla::DEEP>::TOTAL, twelve = fbla::CoarseShape<4, fbla::WIDE>::TOTAL;
+  a->deep = 3 * per_warp(eight) <= 4 * per_warp(twelve) || 2 * per_warp(twelve) <= a->qg;
+  a->coarse_warps = a->deep ? eight : twelve;
   // Folding the warps' partial rows per CTA costs the coarse pass a barrier and a few microseconds at its very end and saves
   // the later passes their walk over the rows: it pays when a virtual head is spread over many warps, i.e. when there are
   // few heads (measured on B200: batch 1 x 8 KV heads at 128K tokens -4.5 us per step, batch 8 x 8 heads at 16K +3 us).
@@ -195,6 +219,14 @@ extern "C" void fbla_k_decode_split_of(int cb, int batch, int kv_heads, int vg, 
   fbla_k_decode_split(&a, tokens);
   *deal = a.deal;
   *fold = a.fold;
+}
+
+extern "C" int fbla_k_decode_deep_of(int batch, int kv_heads, int vg, int qg, long long tokens) {
+  fbla_k_decode a = {};
+  a.cb = 4; a.batch = batch; a.kv_heads = kv_heads; a.vg = vg; a.qg = qg;
+  a.coarse_ctas = 148;
+  fbla_k_decode_split(&a, tokens);
+  return a.deep;
 }
 
 extern "C" cudaError_t fbla_k_decode_launch(const fbla_k_decode *a, cudaStream_t stream) {

@@ -5,12 +5,12 @@
 // p = round(255 * 2^(s - max)), coarse cells decoded at their midpoint, blocks with 2^(lse_j - R) > tau corrected by
 // (full - coarse). The structure is new:
 //   * a persistent grid, one CTA per SM; every warp owns a contiguous range of the flattened list of closed
-//     (virtual head, group) units and a private 2-stage ring in shared memory that whole groups (8 records + 1 KiB
+//     (virtual head, group) units and a private two-slot ring in shared memory that record pairs (and a group's 1 KiB of
 //     metadata) are streamed into by 1-D bulk asynchronous copies completing on mbarriers (all waits bounded);
 //   * scores and values are integer tensor-core products taken straight from the packed records (fbla_frag.cuh):
 //     tokens on M for S^T = K_codes qhat^T, channels on M for O^T = V_codes^T P^T, both P blocks of a record pair
 //     in the 8 columns of one product; the instruction count per byte no longer grows with the GQA ratio;
-//   * one extra warp per CTA serves the BF16 sink / open windows with plain loads and FP32 FMAs.
+//   * the BF16 sink / open windows run on BF16 tensor-core products, on warps of their own or as part of every warp's share.
 // Reduction orders are fixed by (warp, unit) ranges alone, so outputs are bit-reproducible run to run.
 #pragma once
 #include "fbla_frag.cuh"
@@ -21,40 +21,25 @@ namespace fbla {
 constexpr int PSTRIDE = FBLA_K_PSTRIDE;  // floats of one partial row: o[128], m, l, 2 pad (coarse); o[128], dl, 3 pad (refine)
 constexpr int SLICE = FBLA_K_SLICE;      // sub-blocks per select slice
 
-// Streaming warps per CTA and ring slots per warp, per coarse bit width. A slot holds one record pair (32 tokens);
-// the group's metadata has two slots of its own. NP <= 4 (one group of lookahead) keeps two metadata slots enough.
 #ifndef FBLA_RW
 #define FBLA_RW 12   /* refine warps per CTA */
 #endif
 #ifndef FBLA_RNST
 #define FBLA_RNST 2  /* refine ring stages per warp */
 #endif
-// Twelve warps per CTA leave a thread 168 registers, which hold the coarse loop but for a few spills outside it since a pair's
-// sub-blocks share the score products' columns. Measured on B200, eight warps -> twelve (us per step, one sweep): 1 x 1 M tokens
-// 4+2 240 -> 229; 1 x 512 K 3+3 158 -> 149; 8 x 16 K 4+2 72.7 -> 65.2; 2 x 64 K 66.3 -> 63.8; 1 x 128 K 66.6 -> 62.5. A ring slot
-// holds one record pair: with two, twelve warps do not fit the shared memory.
-// FBLA_CW*: the streaming warps of the fixed split at most; a CTA has one warp more (CoarseShape::TOTAL).
-#ifndef FBLA_CW4
-#define FBLA_CW4 11
-#endif
-#ifndef FBLA_CW3
-#define FBLA_CW3 11
-#endif
-#ifndef FBLA_NP
-#define FBLA_NP 2
-#endif
-#ifndef FBLA_PPC
-#define FBLA_PPC 1  // record pairs per chunk (one bulk copy, one barrier wait)
-#endif
-template <int CB> struct CoarseShape {
-  static constexpr int WARPS = CB == 4 ? FBLA_CW4 : FBLA_CW3, TOTAL = WARPS + 1;
-  static constexpr int NP = FBLA_NP;
-  static constexpr int PPC = FBLA_PPC, CPG = 4 / FBLA_PPC;  // pairs per chunk, chunks per group
-  static constexpr int PAIR_BYTES = 2 * record_bytes(CB), CHUNK_BYTES = FBLA_PPC * PAIR_BYTES;
+// The coarse pass has two shapes. WIDE: twelve warps per CTA (168 registers a thread hold the loop but for a few spills outside it), two
+// record pairs in flight per warp. DEEP: eight warps, a whole group in flight (two slots of two pairs; for twelve warps these do not
+// fit the shared memory), for a warp with few groups, which waits for each of its loads.
+enum Shape { WIDE, DEEP };
+template <int CB, int SHAPE> struct CoarseShape {
+  static constexpr int TOTAL = SHAPE == DEEP ? 8 : 12, WARPS = TOTAL - 1;  // WARPS: the streaming ones of the fixed split
+  static constexpr int NP = 2;                                             // ring slots per warp
+  static constexpr int PPC = SHAPE == DEEP ? 2 : 1, CPG = 4 / PPC;         // pairs per chunk (one bulk copy, one barrier wait), chunks per group
+  static constexpr int PAIR_BYTES = 2 * record_bytes(CB), CHUNK_BYTES = PPC * PAIR_BYTES;
   static constexpr int GROUP_BYTES = SBG * record_bytes(CB);
+  static_assert(NP * PPC <= 4, "at most one group of lookahead: two metadata slots are enough");
 };
 static_assert(FBLA_RNST == 2, "the refine pass keeps the metadata of two groups");
-static_assert(FBLA_NP >= 2 && FBLA_NP * FBLA_PPC <= 4 && 4 % FBLA_PPC == 0, "ring slots per warp: at most one group of lookahead");
 
 // ---- where a batch row's tokens put its units -----------------------------------------------------------------------
 struct Row { int tokens, groups, g0, closed, na, exact; };  // g0: the first closed group processed; na: sink sub-blocks
@@ -163,12 +148,13 @@ __device__ __forceinline__ void quantize_query(uint4 km, float4 q4, float sl, ui
 }
 
 // ---- shared memory of the coarse kernel ---------------------------------------------------------------------------------
-template <int CB> struct __align__(128) StreamWarp {
-  uint8_t pair[CoarseShape<CB>::NP][CoarseShape<CB>::CHUNK_BYTES];  // ring of chunks (PPC record pairs each)
+template <int CB, int SHAPE> struct __align__(128) StreamWarp {
+  using Sh = CoarseShape<CB, SHAPE>;
+  uint8_t pair[Sh::NP][Sh::CHUNK_BYTES];  // ring of chunks (PPC record pairs each)
   uint8_t meta[2][1024];                                           // metadata of the group in progress and of the next
   uint8_t qst[8 * QST_ROW];  // qhat rows (rows >= QG stay zero)
   uint8_t pst[128];          // P bytes of a record pair: [block parity][query 0..3][16 tokens]
-  uint64_t bar_pair[CoarseShape<CB>::NP], bar_meta[2];
+  uint64_t bar_pair[Sh::NP], bar_meta[2];
   // The partial rows of the first and the last virtual head of the warp's run, which neighbouring warps of the CTA may
   // share: they are folded into one row per (CTA, virtual head) before they leave the CTA. stage_vh: the rows' virtual
   // heads (-1: no such row).
@@ -182,11 +168,11 @@ struct __align__(16) ExactWarp {
 };
 // (every warp has streaming buffers; a warp that serves windows keeps its ExactWarp in the buffers it does not stream
 // into yet, or at all)
-template <int CB> struct CoarseSmem {
-  StreamWarp<CB> w[CoarseShape<CB>::TOTAL];
+template <int CB, int SHAPE> struct CoarseSmem {
+  StreamWarp<CB, SHAPE> w[CoarseShape<CB, SHAPE>::TOTAL];
+  static_assert(sizeof(w) + 128 <= 227 * 1024, "one CTA's shared memory");
+  static_assert(sizeof(ExactWarp) <= sizeof(w[0]), "a window warp's state fits a streaming warp's");
 };
-static_assert(sizeof(CoarseSmem<3>) + 128 <= 227 * 1024 && sizeof(CoarseSmem<4>) + 128 <= 227 * 1024, "one CTA's shared memory");
-static_assert(sizeof(ExactWarp) <= sizeof(StreamWarp<3>) && sizeof(ExactWarp) <= sizeof(StreamWarp<4>), "a window warp's state fits a streaming warp's");
 
 // ---- the coarse pass's work, split over its warps --------------------------------------------------------------------------
 // Streaming units are the closed groups of all virtual heads, flattened; window units the 16-token sub-blocks of the
@@ -197,18 +183,18 @@ static_assert(sizeof(ExactWarp) <= sizeof(StreamWarp<3>) && sizeof(ExactWarp) <=
 // each kind's units are dealt in equal contiguous runs over its warps of all CTAs. xw is the windows' share of all units
 // by cost (a sub-block 3 eighths of a group at these lengths), at least one warp for the windows and one for the groups
 // if there are any. The host asks for it when the windows are a large part of the work: short contexts
-// at large batch (batch 256 x 512 tokens: 638 -> 352 us per step, batch 32 x 4096: 182 -> 166).
+// at large batch (one sweep, eight warps, batch 256 x 512 tokens: 638 -> 352 us per step, batch 32 x 4096: 182 -> 166).
 //
 // FBLA_K_DEAL_FIXED (contexts in between): the same with xw = 1, whatever the lengths.
 //
 // FBLA_K_DEAL_COST (long contexts): no warp is set aside. All units form one list, window sub-blocks first, then the groups, each
 // with a cost in eighths of a group's time: a window sub-block, on its BF16 tensor-core products, costs half a group
-// (measured, batch 1 x 128K tokens, us per step with costs 2 / 3 / 4 / 6 / 10: 3+3 67.9 / 69.8 / 66.0 / 66.3 / -, 4+2
+// (measured with eight warps per CTA, batch 1 x 128K tokens, us per step with costs 2 / 3 / 4 / 6 / 10: 3+3 67.9 / 69.8 / 66.0 / 66.3 / -, 4+2
 // 64.6 / 60.6 / 55.9 / - / 59.3; what matters most is that a share is a whole number of groups: with 57 instead of 56
 // eighths one warp in eight streams 8 groups instead of 7). Every warp of the grid takes the units whose cost interval
 // starts inside its equal share [w P, (w + 1) P) of the total, serves its window sub-blocks and then streams its
 // groups. A share is at least one unit's cost, so consecutive units lie in the same or in consecutive warps. At batch 1
-// and 128K tokens a warp then streams 7 groups instead of 8.
+// and 128K tokens one of eight warps then streams 7 groups instead of 8.
 struct Deal { long long S, X, P; int wc; };  // groups, window sub-blocks, cost share per warp, cost of a window sub-block
 constexpr int GROUP_COST = 8, WINDOW_COST = 4, WINDOW_COST_SHORT = 3;  // a warp's time for a group / a window sub-block, in eighths of a group
 __device__ __forceinline__ Deal deal_of(const fbla_k_decode &a, int hpr) {
@@ -229,7 +215,7 @@ __device__ __forceinline__ void deal_range(const Deal &d, long long w, long long
 }
 struct Split { int sw, xw; };  // streaming / window warps per CTA
 __device__ __forceinline__ Split split_of(const fbla_k_decode &a, int hpr) {
-  const int total = (a.cb == 4 ? FBLA_CW4 : FBLA_CW3) + 1;
+  const int total = a.coarse_warps;
   if (a.deal == FBLA_K_DEAL_FIXED) return Split{total - 1, 1};
   const long long S = GROUP_COST * total_units<false>(a, hpr), W = WINDOW_COST_SHORT * total_units<true>(a, hpr);  // in eighths of a group's time
   const int xw = S == 0 ? total : max(1, min(total - 1, (int)((2 * total * W + S + W) / (2 * (S + W)))));
@@ -403,9 +389,9 @@ template <int QG> __device__ __forceinline__ bool query_valid(int tig, int e) { 
 // The warp's stream of record pairs: chunk p = CPG k + i holds pairs PPC i .. of the k-th group of the warp's range, in ring
 // slot p % NP (its (p / NP)-th use); the group's metadata travels with chunk 0 into metadata slot k & 1. All lanes carry the
 // (warp-uniform) state; lane 0 issues the copies.
-template <int CB> struct Ring {
-  using Sh = CoarseShape<CB>;
-  StreamWarp<CB> &w;
+template <int CB, int SHAPE> struct Ring {
+  using Sh = CoarseShape<CB, SHAPE>;
+  StreamWarp<CB, SHAPE> &w;
   const fbla_k_decode &a;
   int hpr, lane;
   Cursor fc;                           // the group of the next chunk to issue
@@ -437,12 +423,13 @@ template <int CB> struct Ring {
 };
 
 // Group k of the warp's range. Returns false if a bounded wait gave up.
-template <int CB, int FB, int QG>
-__device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4 (&q4)[QG], float sl, int lane, Run &run,
+template <int CB, int FB, int QG, int SHAPE>
+__device__ __forceinline__ bool coarse_group(Ring<CB, SHAPE> &ring, int k, const float4 (&q4)[QG], float sl, int lane, Run &run,
                                              float *lse_group /* [8 sub-blocks][QG] of this (virtual head, group) */) {
   constexpr int RB = record_bytes(CB);
   constexpr float HOFF = .5f * ((1 << FB) - 1);
-  StreamWarp<CB> &sm = ring.w;
+  using Sh = CoarseShape<CB, SHAPE>;
+  StreamWarp<CB, SHAPE> &sm = ring.w;
   const int gid = lane >> 2, tig = lane & 3;
   // (threads tig >= 2 hold the odd sub-block of every pair: columns 4..7 of the score and value products)
   if (!ring.wait_meta(k)) return false;
@@ -476,9 +463,9 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
   const float2 sqc2 = make_float2(sqc[0], sqc[1]), c02 = make_float2(c0[0], c0[1]);
 #pragma unroll 1
   for (int J = 0; J < SBG / 2; ++J) {
-    const int p = CoarseShape<CB>::CPG * k + J / CoarseShape<CB>::PPC;  // the pair's chunk
-    if (J % CoarseShape<CB>::PPC == 0 && !ring.wait_pair(p)) return false;
-    const uint8_t *ra = sm.pair[p % CoarseShape<CB>::NP] + (J % CoarseShape<CB>::PPC) * CoarseShape<CB>::PAIR_BYTES, *rb = ra + RB;
+    const int p = Sh::CPG * k + J / Sh::PPC;  // the pair's chunk
+    if (J % Sh::PPC == 0 && !ring.wait_pair(p)) return false;
+    const uint8_t *ra = sm.pair[p % Sh::NP] + (J % Sh::PPC) * Sh::PAIR_BYTES, *rb = ra + RB;
     // scores of the thread's own sub-block 2 J + (tig >> 1), queries 2 (tig & 1) + e in (.x, .y): tokens gid, gid + 8; their maxima
     float2 s[2];
     qk_pair<CB>(ra, rb, gid, tig, X, Y, s);
@@ -548,7 +535,7 @@ __device__ __forceinline__ bool coarse_group(Ring<CB> &ring, int k, const float4
       A[u][3] = __ffma2_rn(wu, tiny2(d23[2], d23[3]), A[u][3]);
     }
     __syncwarp();  // pst is free; after a chunk's last pair its slot is too
-    if (J % CoarseShape<CB>::PPC == CoarseShape<CB>::PPC - 1) ring.issue_next();  // refill the slot with the chunk NP ahead
+    if (J % Sh::PPC == Sh::PPC - 1) ring.issue_next();  // refill the slot with the chunk NP ahead
   }
   // fold the group into the running softmax: o += vs' A + vb' B, coarse cell midpoints folded into vb'
   run.l[0] += Bs.x; run.l[1] += Bs.y;
@@ -603,7 +590,7 @@ template <int QG> __device__ __forceinline__ void write_partial(float *p, const 
 // dst (scratch) = the staged row set `own` merged with the first staged row sets of the next `more` warps (`next` points at
 // the first of them, the following ones lie one StreamWarp further each): per query the usual log-sum-exp merge of
 // (m, l, o[128]), taken in warp order. Lane l owns channels 4 l .. 4 l + 3.
-template <int QG, class W>
+template <int QG>
 __device__ __forceinline__ void fold_rows(float *dst, const float *own, const float *next, int more, int lane, size_t warp_stride_floats) {
 #pragma unroll
   for (int qi = 0; qi < QG; ++qi) {
@@ -626,13 +613,13 @@ __device__ __forceinline__ void fold_rows(float *dst, const float *own, const fl
 }
 
 // DEAL: how the work is dealt to the warps (FBLA_K_DEAL_*, the host's choice in fbla_k_decode::deal; one build per way, so
-// that none carries the others' code)
-template <int CB, int FB, int QG, int DEAL>
+// that none carries the others' code); SHAPE likewise (fbla_k_decode::deep)
+template <int CB, int FB, int QG, int DEAL, int SHAPE = WIDE>
 __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *smem_raw) {
-  using Sh = CoarseShape<CB>;
+  using Sh = CoarseShape<CB, SHAPE>;
   allow_next_pass();
   smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;  // (an executor's storage is 16-byte aligned; an offset keeps the pointer's address space known)
-  CoarseSmem<CB> &sm = *reinterpret_cast<CoarseSmem<CB> *>(smem_raw);
+  CoarseSmem<CB, SHAPE> &sm = *reinterpret_cast<CoarseSmem<CB, SHAPE> *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5;
   if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status && !a.status_cleared) { a.status[0] = 0; a.status[1] = 0; }
   const int hpr = a.kv_heads * a.vg;
@@ -657,7 +644,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
     if (xlo < xhi) exact_range<QG, true>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, xlo, xhi, locate<true>(a, hpr, xlo), window_rows(a, QG, (int)gw));
     __syncwarp();
   }
-  StreamWarp<CB> &w = sm.w[warp];
+  StreamWarp<CB, SHAPE> &w = sm.w[warp];
   for (int i = lane; i < (int)sizeof(w.qst) / 4; i += 32) reinterpret_cast<uint32_t *>(w.qst)[i] = 0u;
   reinterpret_cast<uint32_t *>(w.pst)[lane] = 0u;
   if (lane == 0) {
@@ -689,7 +676,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
   bool ok = true;
   if (lo < hi) {
     Cursor cc = locate<false>(a, hpr, lo);
-    Ring<CB> ring{w, a, hpr, lane, cc, 0, (int)(Sh::CPG * (hi - lo)), nullptr, nullptr};
+    Ring<CB, SHAPE> ring{w, a, hpr, lane, cc, 0, (int)(Sh::CPG * (hi - lo)), nullptr, nullptr};
     ring.point();
 #pragma unroll
     for (int s = 0; s < Sh::NP; ++s) ring.issue_next();
@@ -710,7 +697,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
           q4[qi] = make_float4(bf_lo(qw.x), bf_hi(qw.x), bf_lo(qw.y), bf_hi(qw.y));
         }
       }
-      if (!coarse_group<CB, FB, QG>(ring, (int)(u - lo), q4, a.sl, lane, run, a.lse + ((size_t)vh * a.nblocks + (size_t)group_of(a, cc) * SBG) * QG)) {
+      if (!coarse_group<CB, FB, QG, SHAPE>(ring, (int)(u - lo), q4, a.sl, lane, run, a.lse + ((size_t)vh * a.nblocks + (size_t)group_of(a, cc) * SBG) * QG)) {
         if (lane == 0) report(a, 1);
         ok = false;
         break;
@@ -737,12 +724,12 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
     const int v = w.stage_vh[r];
     if (v < 0) continue;
     if (r == 0 && warp > 0) {
-      const StreamWarp<CB> &prev = sm.w[warp - 1];
+      const StreamWarp<CB, SHAPE> &prev = sm.w[warp - 1];
       const int prev_last = prev.stage_vh[1] >= 0 ? prev.stage_vh[1] : prev.stage_vh[0];
       if (prev_last == v) continue;
     }
     if (r == 0 && w.stage_vh[1] >= 0) {  // the virtual head ends inside this warp's run: nothing to fold
-      fold_rows<QG, StreamWarp<CB>>(a.part + (size_t)(cta + v) * QG * PSTRIDE, &w.stage[0][0][0], nullptr, 0, lane, 0);
+      fold_rows<QG>(a.part + (size_t)(cta + v) * QG * PSTRIDE, &w.stage[0][0][0], nullptr, 0, lane, 0);
       continue;
     }
     int more = 0;
@@ -750,7 +737,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
       ++more;
       if (sm.w[x].stage_vh[1] >= 0) break;
     }
-    fold_rows<QG, StreamWarp<CB>>(a.part + (size_t)(cta + v) * QG * PSTRIDE, &w.stage[r][0][0], warp + 1 < sw ? &sm.w[warp + 1].stage[0][0][0] : nullptr, more, lane, sizeof(StreamWarp<CB>) / sizeof(float));
+    fold_rows<QG>(a.part + (size_t)(cta + v) * QG * PSTRIDE, &w.stage[r][0][0], warp + 1 < sw ? &sm.w[warp + 1].stage[0][0][0] : nullptr, more, lane, sizeof(w) / sizeof(float));
   }
 }
 

@@ -56,7 +56,8 @@ typedef struct {
   short mass_given;    // dense: the rows' masses are in row_r (a pass before, or a shard's caller) instead of formed by the value pass
   float *out_partial;  // [rows][FBLA_K_PSTRIDE] floats (phase 2)
   short status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
-  short fold;          // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
+  char fold;           // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
+  char deep;           // the coarse pass's shape: 1: few warps with a whole group in flight each; 0: more warps (fbla_decode.cuh)
   short dense;         // 1: two sweeps, weights kept between them (fbla_dense.cuh); 0: coarse sums, then corrections (fbla_decode.cuh)
   short deal;          // how the coarse pass's warps share the work, FBLA_K_DEAL_*
 } fbla_k_decode;
@@ -88,6 +89,8 @@ FBLA_HOST_API(cudaError_t fbla_k_dense_launch(const fbla_k_decode *a, cudaStream
 FBLA_HOST_API(cudaError_t fbla_k_dense_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)
 // the same choice for a shape given by its numbers (pure host arithmetic: no device is touched): deal and fold as fbla_k_decode_split sets them
 FBLA_HOST_API(void fbla_k_decode_split_of(int cb, int batch, int kv_heads, int vg, long long tokens, int *deal, int *fold);)
+// and its shape for qg queries per virtual head
+FBLA_HOST_API(int fbla_k_decode_deep_of(int batch, int kv_heads, int vg, int qg, long long tokens);)
 // out[row][ch] = bf16(partial[row][ch] / partial[row][128]) for rows rows of FBLA_K_PSTRIDE floats
 // total[i] = log2 sum over shards of 2^mass[s][i]
 FBLA_HOST_API(cudaError_t fbla_k_total_mass_launch(const float *mass, float *total, int shards, int rows, cudaStream_t stream);)

@@ -54,6 +54,15 @@ def test_rows_are_folded_per_cta_for_few_heads_only(lib):
     assert split_of(lib, 4, 4, 8, 2, 65536)[1] == 0
 
 
+def test_the_shape_follows_the_groups_a_warp_streams(lib):
+    """Eight warps with a whole group in flight where twelve would not leave a warp less than three quarters of the groups."""
+    deep = lambda batch, heads, qg, tokens: lib.fbla_k_decode_deep_of(batch, heads, 1, qg, ctypes.c_longlong(tokens))  # noqa: E731
+    for heads, tokens, qg, want in [(8, 60000, 4, 1), (8, 150000, 4, 1), (8, 20000, 4, 1), (8, 20000, 1, 0), (8, 131072, 4, 0), (8, 266667, 4, 0),
+                                    (1, 65000, 4, 1), (1, 65000, 1, 1), (8, 1 << 20, 4, 0), (1, 512, 1, 1)]:
+        assert deep(1, heads, qg, tokens) == want, (heads, tokens, qg)
+    assert not deep(64, 8, 4, 65536) and not deep(8, 8, 4, 131072)
+
+
 class Deal(ctypes.Structure):
     _fields_ = [("cluster", ctypes.c_int), ("above", ctypes.c_int), ("tiles", ctypes.c_int)]
 
