@@ -105,7 +105,7 @@ ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_
   ScratchMap m{};
   const int ratio = c->q_heads / c->kv_heads, qg = queries_per_virtual_head(ratio);
   // (the size does not depend on the call's tau: room for the weights where the format's own asks for them)
-  m.two = two_sweeps && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * (ratio / qg), c->capacity ? c->capacity : tokens, usual_tau(c));
+  m.two = two_sweeps && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * (ratio / qg), qg, c->capacity ? c->capacity : tokens, usual_tau(c));
   const size_t vheads = (size_t)c->batch * c->kv_heads * (ratio / qg);
   m.nblocks = (int)(groups_of(tokens) * kBlocksPerGroup);
   m.nslices = (m.nblocks + FBLA_K_SLICE - 1) / FBLA_K_SLICE;
@@ -210,7 +210,7 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   const float threshold = c->tau != 0.f ? c->tau : usual_tau(c);
   a.log2_tau = log2f(threshold);
   // (a shard's two phases share the scratch but only the second one uses tau: they decide by the format's own)
-  a.dense = m.two && (!wants_output || fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * a.vg, room, threshold));
+  a.dense = m.two && (!wants_output || fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * a.vg, a.qg, room, threshold));
   return MLOPS_FBLA_OK;
 }
 mlops_fbla_status enqueue_decode(const char *fn, fbla_k_decode &a, cudaStream_t stream) {

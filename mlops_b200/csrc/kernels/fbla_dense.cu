@@ -96,10 +96,23 @@ extern "C" cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pass i
 }
 
 // A sub-block of a row of N tokens holds 16 / N of the mass on average. Where that is not far below tau most sub-blocks are selected
-// (the mass is spread unevenly): adding each once is then the faster way; beyond, the coarse planes carry most of the sum and
-// one sweep over them costs less than two. Measured on B200 with 32 query / 8 KV heads, us per step one sweep / two, by N tau / 16: 3+3
-// batch 8 1.2: 348 / 234, 2.5: 404 / 404, batch 1 1.2: 79 / 55, 2.5: 82 / 76; 4+2 batch 8 2: 131 / 112, 4.1: 166 / 189, batch 1 4.1: 50 / 48.
-extern "C" int fbla_k_two_sweeps(int batch, int vheads, long long tokens, float tau) {
+// (how many beyond that the values decide), and adding each once is the faster way; else the coarse planes carry most of the sum and one
+// sweep over them costs less than two. The host does not know the values, so the line lies where the worse of two kinds of values loses
+// least: N(0, 1), few sub-blocks far above the average, and the same with four outlier channels, many. The two sweeps' work per group is the
+// same for one query as for four, one sweep's is not: a line per query count. One sweep is a launch and a chain of round trips
+// longer, some 8 us, so that with few groups per CTA the line lies further out. Measured on B200, us per step one sweep / two, N(0, 1)
+// and outliers, 32 / 8 heads unless said; N tau in front:
+//   batch 8, 3+3:  20: 309 / 227, 324 / 229    25: 264 / 261, 331 / 273    30: 242 / 294, 340 / 313    39: 263 / 367, 362 / 389
+//   batch 8, 4+2:  20: 111 / 81, 114 / 81      25: 97 / 92, 116 / 94       30: 91 / 103, 119 / 106     39: 96 / 124, 123 / 127
+//   batch 1, 3+3:  20: 77 / 55, 79 / 56        30: 66 / 62, 80 / 65        39: 63 / 72, 78 / 75        60: 79 / 95, 92 / 98
+//   batch 1, 4+2:  20: 41 / 32, 42 / 32        30: 36 / 35, 41 / 36        39: 38 / 38, 42 / 39        60: 42 / 46, 46 / 46
+//   batch 8, 16 / 8 heads, 3+3:  20: 238 / 237, 252 / 239    23: 220 / 259, 256 / 266     4+2:  16: 99 / 77, 92 / 77    23: 82 / 92, 93 / 93
+//   batch 8, 8 / 8 heads, 3+3:   13: 222 / 178, 187 / 176    16: 207 / 205, 193 / 204     4+2:  13: 79 / 73, 70 / 73    16: 78 / 82, 72 / 82
+extern "C" int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens, float tau) {
   const long long groups = (tokens + fbla::G - 1) / fbla::G;
-  return batch <= FBLA_K_DENSE_MAX_BATCH && (long long)vheads * groups * fbla::dense::PAIRS < (1ll << 29) && (double)tokens * tau <= 2.5 * 16;
+  const double n_tau = (double)tokens * tau;
+  const int line = qg == 4 ? 27 : qg == 2 ? 22 : 15;
+  const int few = qg == 4 ? 52 : qg == 2 ? 20 : 12, few_line = qg == 4 ? 40 : qg == 2 ? 30 : 20;  // groups per CTA of a B200, whatever the device
+  return batch <= FBLA_K_DENSE_MAX_BATCH && (long long)vheads * groups * fbla::dense::PAIRS < (1ll << 29) &&
+         (n_tau <= line || (n_tau <= few_line && (long long)vheads * groups <= few * 148));
 }

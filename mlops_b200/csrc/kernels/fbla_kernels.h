@@ -82,8 +82,8 @@ FBLA_HOST_API(void fbla_k_decode_split(fbla_k_decode *a, long long tokens);)
 // followed by 2 x cells block maxima and 2 x cells x 16 bytes of weights: FBLA_K_TWO_FLOATS floats per cell in all.
 static inline __host__ __device__ size_t fbla_k_two_cells(size_t vheads, int nblocks, int qg) { return (vheads * nblocks * qg + 63) / 64 * 64; }
 #define FBLA_K_TWO_FLOATS 11
-// whether a decode of rows of about `tokens` tokens with selection threshold tau runs in two sweeps
-FBLA_HOST_API(int fbla_k_two_sweeps(int batch, int vheads, long long tokens, float tau);)
+// whether a decode of rows of about `tokens` tokens with selection threshold tau runs in two sweeps (vheads: virtual heads of the call, qg queries each)
+FBLA_HOST_API(int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens, float tau);)
 // the dense passes (0 scores, 1 rows' masses, 2 values, 3 merge): a whole decode or shard phase; one pass
 FBLA_HOST_API(cudaError_t fbla_k_dense_launch(const fbla_k_decode *a, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_dense_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)

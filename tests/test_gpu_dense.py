@@ -1,12 +1,15 @@
 """The dense decode (scores first, then every sub-block's value once) and the decode that corrects coarse sums, at the
 lengths where dealing or table look-ups can go wrong, against the oracle: no closed group, one, runs that end inside a
 group; 1, 2 and 4 queries per virtual head; ragged rows; selection of none, some and all sub-blocks; shards of such rows."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from tests import datagen
 from tests import gpu_util as gu
+from tests import items_util as iu
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +49,27 @@ def test_dense_ragged_rows(ours, oracle, lens):
     want = oracle.decode(q, o, lengths=np.array(lens, np.int32))
     for b in range(B):
         gu.check_close(gu.bits_of(got)[b], want[b], f"row {b} of {lens}")
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("outliers", [False, True])
+@pytest.mark.parametrize("QH,N,cap,tau,first", [(8, 3000, 3000, 0.0, "dense::score_item"), (8, 3000, 400000, 0.0, "coarse_item"),  # most sub-blocks selected
+                                                (8, 6000, 6000, 4e-3, "dense::score_item"), (8, 6000, 6000, 3e-2, "coarse_item"),   # few
+                                                (2, 6000, 6000, 2e-3, "dense::score_item"), (2, 6000, 6000, 3e-2, "coarse_item"), (4, 20000, 20000, 3e-2, "coarse_item")])
+def test_both_sides_of_the_line(ours, oracle, mode, outliers, QH, N, cap, tau, first):
+    """The same rows in two sweeps and in one (a large slot, a caller's threshold), with most sub-blocks selected and with few, for values
+    that spread the mass evenly and for values that do not; which way a call takes is read off its plan."""
+    KH = 2
+    q, k, v = datagen.baseline_case(90 + N, 1, QH, KH, N, outliers=outliers)
+    qd = gu.bf16_tensor(q)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=cap)
+    got = ours.decode(c, qd, tau=tau)
+    length = torch.tensor([N], dtype=torch.int32, device="cuda")
+    assert torch.equal(got, ours.decode_at(c, qd, length, tau=tau))
+    torch.cuda.synchronize()
+    gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode, capacity=cap), tau=tau), f"{mode} {N} of {cap}, tau {tau}")
+    cfg, kc, passes, vp = gu.Config(1, QH, KH, 0, 0, tau, gu.FORMATS[mode][2], cap, 0, 0, 0, 0, 0), ours._cache(c), (iu.Items * 4)(), ctypes.c_void_p
+    scratch = ours.last_scratch
+    assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(got.data_ptr()),
+                                               vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
+    assert passes[0].entry.decode().startswith("fbla::" + first)

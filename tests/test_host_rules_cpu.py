@@ -54,6 +54,21 @@ def test_rows_are_folded_per_cta_for_few_heads_only(lib):
     assert split_of(lib, 4, 4, 8, 2, 65536)[1] == 0
 
 
+@pytest.mark.parametrize("qg", [1, 2, 4])
+def test_two_sweeps_up_to_a_line(lib, qg):
+    """Rows up to a number of tokens are decoded in two sweeps, longer ones in one; the line follows N tau, and few groups move it out."""
+    two = lambda vheads, tokens, tau, batch=1: lib.fbla_k_two_sweeps(batch, vheads, qg, ctypes.c_longlong(tokens), ctypes.c_float(tau))  # noqa: E731
+    for tau in (3e-4, 1e-3, 0.2):
+        for vheads in (1, 2, 8, 64, 512):
+            picks = [two(vheads, n, tau) for n in range(1, 300000, 997)]
+            assert picks == sorted(picks, reverse=True)  # (one line: two sweeps below it)
+            line = {1: 15, 2: 22, 4: 27}[qg] / tau
+            assert two(vheads, int(0.99 * line), tau) and not two(vheads, int(1.6 * line), tau)
+    assert two(8, 100, 3e-4, batch=1024) and not two(8, 100, 3e-4, batch=1025)  # (prefix sums of the batch in shared memory)
+    assert not two(1 << 15, 1 << 20, 1e-9)                                     # (pairs of all heads below 2^29)
+    assert two(8, 4096, 3e-4) and two(512, 8192, 1e-3) and not two(8, 131072, 3e-4) and not two(8, 1 << 20, 1e-3)
+
+
 def test_the_shape_follows_the_groups_a_warp_streams(lib):
     """Eight warps with a whole group in flight where twelve would not leave a warp less than three quarters of the groups."""
     deep = lambda batch, heads, qg, tokens: lib.fbla_k_decode_deep_of(batch, heads, 1, qg, ctypes.c_longlong(tokens))  # noqa: E731
