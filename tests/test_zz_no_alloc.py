@@ -85,3 +85,29 @@ def test_static_scratch_rejects_large_configurations():
     assert st == 1 and "scratch" in err and str(limit) in err, (st, err)
     st, _, err = _static_decode(lib, c, gu.bf16_tensor(q))
     assert st == 0 and err == ""
+
+
+def test_static_scratch_too_small_for_the_weights():
+    """Rows whose weights between two sweeps do not fit the built-in array are decoded in one sweep: the same attention within the rule for
+    outputs, against mlops_fbla_decode (two sweeps) on every row and against the oracle on one."""
+    from oracle import fbla_oracle
+    lib = gu.CLib(gu.OURS)
+    lib.lib.mlops_fbla_decode_static_scratch_limit.restype = ctypes.c_size_t
+    B, QH, KH, N, mode = 8, 32, 2, 49152, "3+3"
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(8)
+    k, v = (torch.randn((B, KH, N, 128), generator=gen, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    q = torch.randn((B, QH, 128), generator=gen, dtype=torch.bfloat16, device="cuda")
+    c = lib.encode(k, v, mode)
+    assert lib.scratch(c, QH).numel() > lib.lib.mlops_fbla_decode_static_scratch_limit()
+    want = lib.decode(c, q)
+    for _ in range(2):
+        st, out, err = _static_decode(lib, c, q)
+        assert st == 0, err
+    again = _static_decode(lib, c, q)[1]
+    torch.cuda.synchronize()
+    assert torch.equal(out, again)
+    a, b = (datagen.bf16_to_f32(gu.bits_of(x)).astype(np.float64) for x in (out, want))
+    assert (np.abs(a - b) <= 2e-3 * np.abs(b).max() + gu.bf16_ulp(b)).all()
+    row = fbla_oracle.encode(gu.bits_of(k[:1]), gu.bits_of(v[:1]), mode)
+    gu.check_close(gu.bits_of(out[:1]), fbla_oracle.decode(gu.bits_of(q[:1]), row), "static, one sweep")
