@@ -28,7 +28,7 @@
 // per cycle and scheduler); the tensor-core share of a pass is about as long as its exp2 share alone. Measured at batch 4 x
 // 8192 (32 / 8 heads, 4+2): sixteen warps doing softmax and requantisation in turn 5.66 ms = 388 TFLOP/s; roles of their
 // own 5.35; BF16 operands with all loads in flight 5.21; biases on tensor cores 4.75; two sweeps over eight rows of a lane
-// with one reduction 4.59 = 479 TFLOP/s. (64 registers per thread: 29 warps. Halving the softmax warps so that the tiles
+// with one reduction 4.54 = 484 TFLOP/s. (64 registers per thread: 29 warps. Halving the softmax warps so that the tiles
 // alternate, or one copy of the unpacking code for both records of an operand warp, measured slower.)
 // Every wait is bounded: on a timeout the thread raises a flag, everybody drains, tensor memory is freed, the kernel
 // returns and the host sees fbla_k_attend_tc_status() != 0.
@@ -43,10 +43,7 @@ namespace tc {
 
 constexpr int ROWS = 128;                 // rows of a tile
 constexpr int CTA_ROWS = 2 * ROWS;
-#ifndef FBLA_PF_PRODUCERS
-#define FBLA_PF_PRODUCERS 4  /* operand warps. Measured: 4 (21 warps, 80 registers, 28 bytes of spills) 336.5 TFLOP/s; 3 (96 registers, none) 324.8 */
-#endif
-constexpr int PRODUCERS = FBLA_PF_PRODUCERS, PT = 32 * PRODUCERS;  // operand warps and threads
+constexpr int PRODUCERS = 4, PT = 32 * PRODUCERS;  // operand warps (two of a group's eight records each) and threads
 constexpr int QUANT_WARP0 = 16, PRODUCER_WARP0 = 24, ISSUER_WARP = 24 + PRODUCERS;
 constexpr int THREADS = (25 + PRODUCERS) * 32;
 constexpr int SLAB = ROWS * 128;          // bytes of one K slab (128 rows x 128 bytes): 64 FP16 / BF16 of the K extent
