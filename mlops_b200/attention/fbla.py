@@ -51,7 +51,7 @@ def _allocate(make, batch, kv_heads, capacity, mode, device) -> FBLACache:
     coarse_bits, fine_bits, fmt = planes
     groups = -(-capacity // GROUP)
     records = 8 * groups
-    sink_k, sink_v, open_k, open_v = make((4, batch, kv_heads, GROUP, HEAD_DIM), dtype=torch.bfloat16, device=device).unbind(0)
+    sink_k, sink_v, open_k, open_v = (make((batch, kv_heads, GROUP, HEAD_DIM), dtype=torch.bfloat16, device=device) for _ in range(4))
     return FBLACache(coarse=make((batch, kv_heads, records, 512 * coarse_bits), dtype=torch.uint8, device=device),
                      fine=make((batch, kv_heads, records, 512 * fine_bits), dtype=torch.uint8, device=device),
                      meta=make((batch, kv_heads, groups, 512), dtype=torch.bfloat16, device=device),
