@@ -148,7 +148,7 @@ typedef struct {
   float sl;
   // 0: the attention pass serves every count. > 0 (a chunk whose count lives on the device): the attention is two
   // passes and the count decides on the device which of them works -- the tensor-core pass when count * queries per KV
-  // head >= tc_min_rows, the warp-per-row pass below that -- so that a device-count call takes the kernel the host-count
+  // head >= tc_min_rows, the few-row pass below that -- so that a device-count call takes the kernel the host-count
   // call of the same chunk takes and the two stay bit-identical.
   int tc_min_rows;
   // > 0 (a chunk that starts a cache whose arrays have no initial contents): the groups per KV head that the layout has

@@ -21,6 +21,15 @@ namespace tc {
 template <int CB, int FB, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) attend_tc_kernel(const fbla_k_prefill a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  // A launch that the count does not ask for is gone before its turn: the close pass, which comes first in every call with a count on the
+  // device, lets the next kernel begin behind its own wait, so count and length are what they will be. One CTA keeps the order: the kernel
+  // after this one may not begin before the close pass is complete. (512 tokens at 128 in a cache with room for 64K, us: one launch 52;
+  // two 59 with both waiting first, 54 so.)
+  if (a.dcount && !serves(a)) {
+    allow_next_pass();
+    if (blockIdx.x == 0 && blockIdx.y == 0) wait_previous_pass();
+    return;
+  }
   wait_previous_pass();
   allow_next_pass();
   attend_tiles<CB, FB, SPLIT ? CLUSTER : WHOLE>(a, smem_raw);
@@ -73,9 +82,9 @@ extern "C" cudaError_t fbla_k_attend_tc_launch(const fbla_k_prefill *a, cudaStre
     const bool split = args.cluster > 1;
     const auto kernel = a->cb == 3 ? split ? attend_tc_kernel<3, 3, true> : attend_tc_kernel<3, 3, false> : split ? attend_tc_kernel<4, 2, true> : attend_tc_kernel<4, 2, false>;
     const int wide = deal[i].tiles * args.cluster;
-    // launched dependent where one wave holds the grid (a 777-token prompt 69.5 -> 67.8 us); several waves that began among the
-    // CTAs of the kernel before measured 3 % slower (batch 4 x 8192 4.55 -> 4.69 ms)
-    const cudaError_t e = fbla::launch(wide * heads <= 148, args.cluster, kernel, dim3(wide, heads), THREADS, smem, stream, args);
+    // launched dependent where one wave holds the grid (a 777-token prompt 69.5 -> 67.8 us), or where it is likely not the one that
+    // works; several waves that began among the CTAs of the kernel before measured 3 % slower (batch 4 x 8192 4.55 -> 4.69 ms)
+    const cudaError_t e = fbla::launch(wide * heads <= 148 || i + 1 < launches, args.cluster, kernel, dim3(wide, heads), THREADS, smem, stream, args);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -193,6 +193,13 @@ __device__ __forceinline__ int shares_of(const fbla_k_prefill &a, int rows, int 
   return tile_shares((long long)((rows + CTA_ROWS - 1) / CTA_ROWS) * a.batch * a.kv_heads, (n1 - 1) / G + 1, FBLA_K_TILE_SHARES);
 }
 
+// whether a launch for a count on the device is the one that serves it (the same for every CTA of the grid)
+__device__ __forceinline__ bool serves(const fbla_k_prefill &a) {
+  const int count = FBLA_POS::ro(a.dcount), n1 = (a.length ? FBLA_POS::ro(a.length) : 0) + a.n0 + count, rows = count * (a.q_heads / a.kv_heads);
+  const int shares = shares_of(a, rows, n1);
+  return rows >= a.tc_min_rows && shares > a.above && shares <= a.cluster;
+}
+
 template <int CB, int FB, Way WAY>
 __device__ __forceinline__ void attend_tiles(const fbla_k_prefill &a, uint8_t *smem_raw, int turn = 0, Kept *kept = nullptr) {
   constexpr bool SPLIT = WAY != WHOLE;
@@ -214,8 +221,8 @@ __device__ __forceinline__ void attend_tiles(const fbla_k_prefill &a, uint8_t *s
   const int n_pass = n_closed + 1 + max(own_max - own_lo + 1, 0);
   // this CTA's share of them: passes [p_lo, p_hi), of which [p_lo, c_hi) closed, [x_lo, p_hi) BF16
   const int shares = shares_of(a, rows, n1);
-  // (the same for every CTA of the grid, and of a cluster those leave that have no share: its barriers wait for threads that have not exited)
-  if (WAY == WHOLE ? shares > 1 : WAY == CLUSTER && (shares <= a.above || shares > cluster || rank >= shares)) return;
+  // (of a cluster those leave that have no share: its barriers wait for threads that have not exited)
+  if (WAY == CLUSTER ? shares <= a.above || shares > cluster || rank >= shares : WAY == WHOLE && shares > 1) return;
   const int p_lo = !SPLIT ? 0 : (int)((long long)n_pass * rank / shares);
   const int p_hi = !SPLIT ? n_pass : (int)((long long)n_pass * (rank + 1) / shares);
   const int c_hi = SPLIT ? min(n_closed, p_hi) : n_closed, x_lo = SPLIT ? max(n_closed, p_lo) : n_closed;
