@@ -118,7 +118,7 @@ _KINDS = ((torch.uint8, _RECORDS),) * 2 + ((torch.bfloat16, _ROWS),) * 5
 
 def _arrays(c):
     """A cache's arrays, checked as `decode` and `prefill` check theirs: the structure that names them to the library, their device.
-    (Looked at in every call -- 2 us of the host's time -- and nothing of it kept: a cache is a plain record that its user may change,
+    (Looked at in every call -- 4 us of the host's time -- and nothing of it kept: a cache is a plain record that its user may change,
     copy and save.)"""
     arrays = c.coarse, c.fine, c.meta, c.sink_k, c.sink_v, c.open_k, c.open_v
     device = arrays[0].device
@@ -278,8 +278,9 @@ def encode(k, v, coarse, fine, meta, sink_k, sink_v, open_k, open_v, capacity, f
     dev = k.device
     _tensor(k, dev, torch.bfloat16, "k")
     _tensor(v, dev, torch.bfloat16, "v")
+    if torch._C._cuda_getDevice() != dev.index:
+        with torch.cuda.device(dev):
+            return encode(k, v, coarse, fine, meta, sink_k, sink_v, open_k, open_v, capacity, format)
     cfg = _config(k.size(0), k.size(1), k.size(1), 0, format, capacity, 0.0, 0.0)
     cache = _cache(coarse, fine, meta, sink_k, sink_v, open_k, open_v)
-    with torch.cuda.device(dev):
-        st = _lib.mlops_fbla_encode(ctypes.byref(cfg), k.size(2), k.data_ptr(), v.data_ptr(), ctypes.byref(cache), _stream(dev))
-    _raise(st, "mlops_fbla_encode")
+    _raise(_lib.mlops_fbla_encode(ctypes.byref(cfg), k.size(2), k.data_ptr(), v.data_ptr(), ctypes.byref(cache), _raw_stream(dev.index)), "mlops_fbla_encode")

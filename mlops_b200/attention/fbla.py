@@ -43,15 +43,16 @@ def _require_kv(k, v):
         raise ValueError(f"k and v have to live on the same CUDA device (k: {k.device}, v: {v.device})")
 
 
-def _allocate(make, batch, kv_heads, capacity, mode, device) -> FBLACache:
-    """The arrays of a cache for ``capacity`` tokens, each from ``make(shape, dtype=, device=)``."""
+def _allocate(make, like, batch, kv_heads, capacity, mode, device) -> FBLACache:
+    """The arrays of a cache for ``capacity`` tokens, each from ``make(shape, dtype=, device=)`` or ``like(another)``."""
     planes = _PLANES.get(mode)
     if planes is None:
         raise ValueError(f"unknown mode {mode!r}: choose '3+3' or '4+2'")
     coarse_bits, fine_bits, fmt = planes
     groups = -(-capacity // GROUP)
     records = 8 * groups
-    sink_k, sink_v, open_k, open_v = (make((batch, kv_heads, GROUP, HEAD_DIM), dtype=torch.bfloat16, device=device) for _ in range(4))
+    sink_k = make((batch, kv_heads, GROUP, HEAD_DIM), dtype=torch.bfloat16, device=device)
+    sink_v, open_k, open_v = like(sink_k), like(sink_k), like(sink_k)
     return FBLACache(coarse=make((batch, kv_heads, records, 512 * coarse_bits), dtype=torch.uint8, device=device),
                      fine=make((batch, kv_heads, records, 512 * fine_bits), dtype=torch.uint8, device=device),
                      meta=make((batch, kv_heads, groups, 512), dtype=torch.bfloat16, device=device),
@@ -60,7 +61,7 @@ def _allocate(make, batch, kv_heads, capacity, mode, device) -> FBLACache:
 
 def empty(batch: int, kv_heads: int, capacity: int, mode: str = "3+3", device="cuda") -> FBLACache:
     """A cache with room for ``capacity`` tokens and none stored. All arrays start as zeros."""
-    cache = _allocate(torch.zeros, batch, kv_heads, capacity, mode, device)
+    cache = _allocate(torch.zeros, torch.zeros_like, batch, kv_heads, capacity, mode, device)
     with torch.cuda.device(torch.device(device)):
         image_bytes = _C.images_bytes(batch, kv_heads, -(-capacity // GROUP) * GROUP)
     if image_bytes > 0:
@@ -95,7 +96,7 @@ def encode(k: torch.Tensor, v: torch.Tensor, mode: str = "3+3", capacity: Option
         _extend(cache, k, v)
         return cache
     # (the call that stores the tokens also zeroes what they leave of the arrays)
-    cache = _allocate(torch.empty, batch, kv_heads, room, mode, k.device)
+    cache = _allocate(torch.empty, torch.empty_like, batch, kv_heads, room, mode, k.device)
     _C.encode(k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous(), cache.coarse, cache.fine, cache.meta, cache.sink_k,
               cache.sink_v, cache.open_k, cache.open_v, room, cache.format)
     cache.tokens = n

@@ -34,7 +34,7 @@ def test_one_buffer_per_stream_and_a_bounded_number(package):
 def test_the_arrays_of_a_cache_are_tensors_of_their_own(package):
     """Each can be written, saved and given back without the others (a window that was a view of all four could not be written while autograd
     records)."""
-    cache = package.fbla._allocate(torch.zeros, 1, 2, 300, "4+2", "cpu")
+    cache = package.fbla._allocate(torch.zeros, torch.zeros_like, 1, 2, 300, "4+2", "cpu")
     arrays = [cache.coarse, cache.fine, cache.meta, cache.sink_k, cache.sink_v, cache.open_k, cache.open_v]
     assert len({a.untyped_storage().data_ptr() for a in arrays}) == 7
     assert all(a.untyped_storage().nbytes() == a.numel() * a.element_size() for a in arrays)
