@@ -51,6 +51,16 @@ def test_dense_ragged_rows(ours, oracle, lens):
         gu.check_close(gu.bits_of(got)[b], want[b], f"row {b} of {lens}")
 
 
+def first_entry(ours, c, qd, mode, tau):
+    """the first pass of a decode's plan"""
+    length, vp, passes = torch.tensor([c["tokens"]], dtype=torch.int32, device="cuda"), ctypes.c_void_p, (iu.Items * 4)()
+    cfg, kc = gu.Config(c["batch"], qd.shape[1], c["kv_heads"], 0, 0, tau, gu.FORMATS[mode][2], c["capacity"], 0, 0, 0, 0, 0), ours._cache(c)
+    scratch, out = ours.scratch(dict(c, tokens=c["capacity"]), qd.shape[1]), torch.empty_like(qd)
+    assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
+                                               vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
+    return passes[0].entry.decode()
+
+
 @pytest.mark.parametrize("mode", ["3+3", "4+2"])
 @pytest.mark.parametrize("outliers", [False, True])
 @pytest.mark.parametrize("QH,N,cap,tau,first", [(8, 3000, 3000, 0.0, "dense::score_item"), (8, 3000, 400000, 0.0, "coarse_item"),  # most sub-blocks selected
@@ -68,8 +78,18 @@ def test_both_sides_of_the_line(ours, oracle, mode, outliers, QH, N, cap, tau, f
     assert torch.equal(got, ours.decode_at(c, qd, length, tau=tau))
     torch.cuda.synchronize()
     gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode, capacity=cap), tau=tau), f"{mode} {N} of {cap}, tau {tau}")
-    cfg, kc, passes, vp = gu.Config(1, QH, KH, 0, 0, tau, gu.FORMATS[mode][2], cap, 0, 0, 0, 0, 0), ours._cache(c), (iu.Items * 4)(), ctypes.c_void_p
-    scratch = ours.last_scratch
-    assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(got.data_ptr()),
-                                               vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
-    assert passes[0].entry.decode().startswith("fbla::" + first)
+    assert first_entry(ours, c, qd, mode, tau).startswith("fbla::" + first)
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("QH,KH,N,deal,deep", [(8, 8, 20000, 1, 0), (16, 8, 52000, 2, 0), (8, 8, 9000, 1, 1), (16, 8, 30000, 1, 1), (32, 8, 17000, 2, 1), (32, 8, 24000, 1, 1), (16, 2, 200000, 2, 0)])
+def test_shapes_of_the_coarse_sweep(ours, oracle, mode, QH, KH, N, deal, deep):
+    """One sweep with one, two and four queries per virtual head, twelve warps and eight, with the windows on a warp of their own and dealt by cost."""
+    q, k, v = datagen.uneven_case(70 + QH, 1, QH, KH, N)
+    qd, tau = gu.bf16_tensor(q), 1e-2
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode)
+    assert first_entry(ours, c, qd, mode, tau).endswith(f"{deal}, {deep}>")
+    got = ours.decode(c, qd, tau=tau)
+    assert torch.equal(got, ours.decode_at(c, qd, torch.tensor([N], dtype=torch.int32, device="cuda"), tau=tau))
+    torch.cuda.synchronize()
+    gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode), tau=tau), f"{mode} {N}")
