@@ -91,6 +91,10 @@ fbla_k_cache kernel_cache(const mlops_fbla_cache *k) {
 }
 long long groups_of(long long tokens) { return (tokens + kGroup - 1) / kGroup; }
 
+// The tokens by which a decode's way is chosen (fbla_k_two_sweeps): the room of the cache, for host and device lengths alike, so that both
+// calls on one cache run the same kernels and return the same bits. Rows of lengths of their own are taken to fill two thirds of it.
+long long typical_tokens(long long room, bool own_lengths) { return own_lengths ? (2 * room + 2) / 3 : room; }
+
 // ---- decode scratch ------------------------------------------------------------------------------------------------------------
 // Byte offsets of the arrays fbla_kernels.h describes, in this order, inside the caller's scratch.
 struct ScratchMap {
@@ -104,8 +108,8 @@ struct ScratchMap {
 ScratchMap map_scratch(const mlops_fbla_config *c, long long tokens, const fbla_k_decode &shape, int extra_rows, bool two_sweeps) {
   ScratchMap m{};
   const int ratio = c->q_heads / c->kv_heads, qg = queries_per_virtual_head(ratio);
-  // (the size does not depend on the call's tau: room for the weights where the format's own asks for them)
-  m.two = two_sweeps && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * (ratio / qg), qg, c->capacity ? c->capacity : tokens, usual_tau(c));
+  // (the size depends neither on the call's tau nor on its kind of lengths: room for the weights where the format's own tau asks for them)
+  m.two = two_sweeps && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * (ratio / qg), qg, typical_tokens(c->capacity ? c->capacity : tokens, true), usual_tau(c));
   const size_t vheads = (size_t)c->batch * c->kv_heads * (ratio / qg);
   m.nblocks = (int)(groups_of(tokens) * kBlocksPerGroup);
   m.nslices = (m.nblocks + FBLA_K_SLICE - 1) / FBLA_K_SLICE;
@@ -210,7 +214,7 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   const float threshold = c->tau != 0.f ? c->tau : usual_tau(c);
   a.log2_tau = log2f(threshold);
   // (a shard's two phases share the scratch but only the second one uses tau: they decide by the format's own)
-  a.dense = m.two && (!wants_output || fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * a.vg, a.qg, room, threshold));
+  a.dense = m.two && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * a.vg, a.qg, typical_tokens(room, c->length_stride != 0), wants_output ? threshold : usual_tau(c));
   return MLOPS_FBLA_OK;
 }
 mlops_fbla_status enqueue_decode(const char *fn, fbla_k_decode &a, cudaStream_t stream) {

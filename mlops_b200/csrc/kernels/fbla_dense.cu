@@ -108,10 +108,13 @@ extern "C" cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pass i
 //   batch 1, 4+2:  20: 41 / 32, 42 / 32        30: 36 / 35, 41 / 36        39: 38 / 38, 42 / 39        60: 42 / 46, 46 / 46
 //   batch 8, 16 / 8 heads, 3+3:  20: 238 / 237, 252 / 239    23: 220 / 259, 256 / 266     4+2:  16: 99 / 77, 92 / 77    23: 82 / 92, 93 / 93
 //   batch 8, 8 / 8 heads, 3+3:   13: 222 / 178, 187 / 176    16: 207 / 205, 193 / 204     4+2:  13: 79 / 73, 70 / 73    16: 78 / 82, 72 / 82
+// Rows of lengths of their own are shorter than the room that the host sees. Evenly spread up to it they break even at about twice these
+// lines, all of them full at the lines themselves; the host asks with two thirds of the room, where either loses about as much (N tau of the
+// room, us one / two, batch 8, 32 / 8 heads, 3+3, N(0, 1): spread 31: 262 / 188, 40: 264 / 235, 54: 278 / 303; full 31: 245 / 302, 40: 263 / 374).
 extern "C" int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens, float tau) {
   const long long groups = (tokens + fbla::G - 1) / fbla::G;
   const double n_tau = (double)tokens * tau;
-  const int line = qg == 4 ? 27 : qg == 2 ? 22 : 15;
+  const int line = qg == 4 ? 28 : qg == 2 ? 22 : 15;
   const int few = qg == 4 ? 52 : qg == 2 ? 20 : 12, few_line = qg == 4 ? 40 : qg == 2 ? 30 : 20;  // groups per CTA of a B200, whatever the device
   return batch <= FBLA_K_DENSE_MAX_BATCH && (long long)vheads * groups * fbla::dense::PAIRS < (1ll << 29) &&
          (n_tau <= line || (n_tau <= few_line && (long long)vheads * groups <= few * 148));

@@ -51,10 +51,10 @@ def test_dense_ragged_rows(ours, oracle, lens):
         gu.check_close(gu.bits_of(got)[b], want[b], f"row {b} of {lens}")
 
 
-def first_entry(ours, c, qd, mode, tau):
+def first_entry(ours, c, qd, mode, tau, length_stride=0):
     """the first pass of a decode's plan"""
-    length, vp, passes = torch.tensor([c["tokens"]], dtype=torch.int32, device="cuda"), ctypes.c_void_p, (iu.Items * 4)()
-    cfg, kc = gu.Config(c["batch"], qd.shape[1], c["kv_heads"], 0, 0, tau, gu.FORMATS[mode][2], c["capacity"], 0, 0, 0, 0, 0), ours._cache(c)
+    length, vp, passes = torch.tensor([c["tokens"]] * c["batch"], dtype=torch.int32, device="cuda"), ctypes.c_void_p, (iu.Items * 4)()
+    cfg, kc = gu.Config(c["batch"], qd.shape[1], c["kv_heads"], 0, 0, tau, gu.FORMATS[mode][2], c["capacity"], 0, 0, 0, 0, length_stride), ours._cache(c)
     scratch, out = ours.scratch(dict(c, tokens=c["capacity"]), qd.shape[1]), torch.empty_like(qd)
     assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
                                                vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
@@ -93,3 +93,25 @@ def test_shapes_of_the_coarse_sweep(ours, oracle, mode, QH, KH, N, deal, deep):
     assert torch.equal(got, ours.decode_at(c, qd, torch.tensor([N], dtype=torch.int32, device="cuda"), tau=tau))
     torch.cuda.synchronize()
     gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode), tau=tau), f"{mode} {N}")
+
+
+def test_rows_of_their_own_lengths_fill_part_of_the_room(ours, oracle):
+    """A room beyond the line: rows of one length are decoded in one sweep, rows of lengths of their own in two, in the scratch that the size
+    query gives for either."""
+    mode, QH, KH, cap, lens = "4+2", 2, 2, 22000, [300, 9000, 21000]
+    q, k, v = datagen.uneven_case(12, len(lens), QH, KH, max(lens))
+    qd, B = gu.bf16_tensor(q), len(lens)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=cap)
+    assert first_entry(ours, c, qd, mode, 0.0).startswith("fbla::coarse_item") and first_entry(ours, c, qd, mode, 0.0, 1).startswith("fbla::dense::score_item")
+    out = ours.decode_at(c, qd, torch.tensor([max(lens)], dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    gu.check_close(gu.bits_of(out), oracle.decode(q, oracle.encode(k, v, mode, capacity=cap)), "one length")
+    for b, n in enumerate(lens):  # the rows' own caches
+        row = ours.encode(gu.bf16_tensor(k[b:b + 1, :, :n]), gu.bf16_tensor(v[b:b + 1, :, :n]), mode, capacity=cap)
+        for key in ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v"):
+            c[key][b].copy_(row[key][0])
+    out = ours.decode_at(c, qd, torch.tensor(lens, dtype=torch.int32, device="cuda"), length_stride=1)
+    torch.cuda.synchronize()
+    for b, n in enumerate(lens):
+        want = oracle.decode(q[b:b + 1], oracle.encode(k[b:b + 1, :, :n], v[b:b + 1, :, :n], mode, capacity=cap))
+        gu.check_close(gu.bits_of(out)[b:b + 1], want, f"row of {n}")

@@ -62,7 +62,7 @@ def test_two_sweeps_up_to_a_line(lib, qg):
         for vheads in (1, 2, 8, 64, 512):
             picks = [two(vheads, n, tau) for n in range(1, 300000, 997)]
             assert picks == sorted(picks, reverse=True)  # (one line: two sweeps below it)
-            line = {1: 15, 2: 22, 4: 27}[qg] / tau
+            line = {1: 15, 2: 22, 4: 28}[qg] / tau
             assert two(vheads, int(0.99 * line), tau) and not two(vheads, int(1.6 * line), tau)
     assert two(8, 100, 3e-4, batch=1024) and not two(8, 100, 3e-4, batch=1025)  # (prefix sums of the batch in shared memory)
     assert not two(1 << 15, 1 << 20, 1e-9)                                     # (pairs of all heads below 2^29)
