@@ -112,21 +112,32 @@ def scratch_bytes(batch, q_heads, kv_heads, tokens, format, capacity):
 
 
 # ---- calls on a whole cache object --------------------------------------------------------------------------------------------
-_RECORDS, _ROWS = "packed cache records", "cache metadata / exact group"
-_KINDS = ((torch.uint8, _RECORDS),) * 2 + ((torch.bfloat16, _ROWS),) * 5
+_U8, _BF16 = torch.uint8, torch.bfloat16
 
 
 def _arrays(c):
-    """A cache's arrays, checked as `decode` and `prefill` check theirs: the structure that names them to the library, their device.
-    (Looked at in every call -- 4 us of the host's time -- and nothing of it kept: a cache is a plain record that its user may change,
+    """A cache's arrays, checked as `decode` and `prefill` check theirs: the structure that names them to the library, their device's index.
+    (Looked at in every call -- 3 us of the host's time -- and nothing of it kept: a cache is a plain record that its user may change,
     copy and save.)"""
-    arrays = c.coarse, c.fine, c.meta, c.sink_k, c.sink_v, c.open_k, c.open_v
-    device = arrays[0].device
-    index = arrays[0].get_device()
-    for x, (dtype, what) in zip(arrays, _KINDS):
-        if index < 0 or x.get_device() != index or x.dtype is not dtype or not x.is_contiguous():
-            _tensor(x, device, dtype, what)
-    return _cache(*arrays, c.images), device
+    k, f, m, sk, sv, ok, ov = c.coarse, c.fine, c.meta, c.sink_k, c.sink_v, c.open_k, c.open_v
+    index = k.get_device()
+    if not (0 <= index == f.get_device() == m.get_device() == sk.get_device() == sv.get_device() == ok.get_device() == ov.get_device()
+            and k.dtype is f.dtype is _U8 and m.dtype is sk.dtype is sv.dtype is ok.dtype is ov.dtype is _BF16
+            and k.is_contiguous() and f.is_contiguous() and m.is_contiguous() and sk.is_contiguous() and sv.is_contiguous()
+            and ok.is_contiguous() and ov.is_contiguous()):
+        for x in (k, f):
+            _tensor(x, k.device, _U8, "packed cache records")
+        for x in (m, sk, sv, ok, ov):
+            _tensor(x, k.device, _BF16, "cache metadata / exact group")
+    images = c.images
+    return Cache(k.data_ptr(), f.data_ptr(), m.data_ptr(), sk.data_ptr(), sv.data_ptr(), ok.data_ptr(), ov.data_ptr(),
+                 images.data_ptr() if images is not None else None), index
+
+
+def _rows(x, index, what):
+    """as _tensor, for a BF16 operand on the cache's device"""
+    if x.get_device() != index or x.dtype is not _BF16 or not x.is_contiguous():
+        _tensor(x, torch.device("cuda", index), _BF16, what)
 
 
 _scratch_bytes = functools.lru_cache(maxsize=256)(lambda device, *shape: scratch_bytes(*shape))
@@ -175,22 +186,22 @@ _pool = _ScratchPool()
 
 def decode_cache(q, c, scale, tau):
     """decode of a whole cache object with the pool's scratch"""
-    struct, device = _arrays(c)
+    struct, index = _arrays(c)
     if q.dim() != 3 or q.size(2) != 128:
         raise ValueError(f"q must be [batch, q_heads, 128], got {tuple(q.shape)}")
     if not q.is_contiguous():
         q = q.contiguous()
-    if q.device != device:
-        raise ValueError(f"q: expected a CUDA tensor on {device}")
-    if torch._C._cuda_getDevice() != device.index:
-        with torch.cuda.device(device.index):
+    if q.get_device() != index:
+        raise ValueError(f"q: expected a CUDA tensor on cuda:{index}")
+    if torch._C._cuda_getDevice() != index:
+        with torch.cuda.device(index):
             return decode_cache(q, c, scale, tau)
     batch, q_heads, kv_heads = q.size(0), q.size(1), c.meta.size(1)
     tokens, capacity = int(c.tokens), int(c.capacity)
     room = min(capacity, -(-tokens // 16384) * 16384)  # (asked for once in 16 384 tokens; a slot may have room for far more than it holds)
-    need = _scratch_bytes(device.index, batch, q_heads, kv_heads, room, c.format, capacity)
-    stream = _raw_stream(device.index)
-    scratch = _pool.get(device, stream, need)
+    need = _scratch_bytes(index, batch, q_heads, kv_heads, room, c.format, capacity)
+    stream = _raw_stream(index)
+    scratch = _pool.get(q.device, stream, need)
     out = torch.empty_like(q)
     cfg = Config(batch, q_heads, kv_heads, tokens, float(scale), float(tau), int(c.format), capacity, 0, 0, 0, 0, 0)
     with scratch.lock:
@@ -201,22 +212,22 @@ def decode_cache(q, c, scale, tau):
 
 def prefill_cache(q, k, v, c, scale):
     """prefill (append for q None) on a whole cache object; k and v contiguous BF16 of the cache's batch and KV heads"""
-    struct, device = _arrays(c)
-    _tensor(k, device, torch.bfloat16, "k")
-    _tensor(v, device, torch.bfloat16, "v")
-    if torch._C._cuda_getDevice() != device.index:
-        with torch.cuda.device(device.index):
+    struct, index = _arrays(c)
+    _rows(k, index, "k")
+    _rows(v, index, "v")
+    if torch._C._cuda_getDevice() != index:
+        with torch.cuda.device(index):
             return prefill_cache(q, k, v, c, scale)
     batch, kv_heads, n, out = c.meta.size(0), c.meta.size(1), k.size(2), None
     q_heads = kv_heads
     if q is not None:
         if q.dim() != 4 or q.size(0) != batch or q.size(2) != n or q.size(3) != 128:
             raise ValueError(f"q must be [batch, q_heads, n, 128] matching k, got {tuple(q.shape)}")
-        _tensor(q, device, torch.bfloat16, "q")
+        _rows(q, index, "q")
         q_heads, out = q.size(1), torch.empty_like(q)
     cfg = Config(batch, q_heads, kv_heads, int(c.tokens), float(scale), 0.0, int(c.format), int(c.capacity), 0, 0, 0, 0, 0)
     _raise(_lib.mlops_fbla_prefill(ctypes.byref(cfg), n, q.data_ptr() if q is not None else None, k.data_ptr(), v.data_ptr(), ctypes.byref(struct),
-                                   out.data_ptr() if out is not None else None, _raw_stream(device.index)), "mlops_fbla_prefill")
+                                   out.data_ptr() if out is not None else None, _raw_stream(index)), "mlops_fbla_prefill")
     return out
 
 

@@ -36,11 +36,16 @@ class FBLACache:
 
 def _require_kv(k, v):
     """K and V of one chunk: equal 4-D shapes with a head dimension of 128, on one CUDA device."""
-    same = k.ndim == 4 and tuple(k.shape) == tuple(v.shape) and k.shape[-1] == HEAD_DIM
-    if not same:
+    shape = k.shape
+    if not (len(shape) == 4 and shape == v.shape and shape[3] == HEAD_DIM):
         raise ValueError(f"expected k and v of one shape [B, Hkv, n, {HEAD_DIM}]; k is {tuple(k.shape)}, v is {tuple(v.shape)}")
-    if not (k.is_cuda and v.is_cuda and k.device == v.device):
+    if not (k.is_cuda and v.is_cuda and k.get_device() == v.get_device()):
         raise ValueError(f"k and v have to live on the same CUDA device (k: {k.device}, v: {v.device})")
+
+
+def _dense(x):
+    """as the library reads K and V: BF16, contiguous"""
+    return x if x.dtype is torch.bfloat16 and x.is_contiguous() else x.to(torch.bfloat16).contiguous()
 
 
 def _allocate(make, like, batch, kv_heads, capacity, mode, device) -> FBLACache:
@@ -72,13 +77,12 @@ def empty(batch: int, kv_heads: int, capacity: int, mode: str = "3+3", device="c
 def _extend(cache, k, v, q=None, scale=0.0):
     """One library call: store the chunk (k, v) behind the cache's tokens and, given q, attend from its positions."""
     _require_kv(k, v)
-    held = tuple(cache.meta.shape[:2])
-    if tuple(k.shape[:2]) != held:
-        raise ValueError(f"the chunk is [batch, kv_heads] = {tuple(k.shape[:2])} but the cache was built for {held}")
-    added = int(k.shape[2])
+    meta, added = cache.meta, k.size(2)
+    if k.size(0) != meta.size(0) or k.size(1) != meta.size(1):
+        raise ValueError(f"the chunk is [batch, kv_heads] = {tuple(k.shape[:2])} but the cache was built for {tuple(meta.shape[:2])}")
     if cache.tokens + added > cache.capacity:
         raise ValueError(f"{added} more tokens do not fit: the cache holds {cache.tokens} of {cache.capacity}")
-    result = _C.prefill_cache(q, k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous(), cache, scale)
+    result = _C.prefill_cache(q, _dense(k), _dense(v), cache, scale)
     cache.tokens += added
     return result
 
@@ -97,7 +101,7 @@ def encode(k: torch.Tensor, v: torch.Tensor, mode: str = "3+3", capacity: Option
         return cache
     # (the call that stores the tokens also zeroes what they leave of the arrays)
     cache = _allocate(torch.empty, torch.empty_like, batch, kv_heads, room, mode, k.device)
-    _C.encode(k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous(), cache.coarse, cache.fine, cache.meta, cache.sink_k,
+    _C.encode(_dense(k), _dense(v), cache.coarse, cache.fine, cache.meta, cache.sink_k,
               cache.sink_v, cache.open_k, cache.open_v, room, cache.format)
     cache.tokens = n
     return cache
@@ -116,7 +120,7 @@ def append(cache: FBLACache, k: torch.Tensor, v: torch.Tensor) -> FBLACache:
 def prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: FBLACache, *, scale: float = 0.0) -> torch.Tensor:
     """Causal attention of a chunk. ``k, v [B, Hkv, n, 128]`` are stored in ``cache`` first; the query of chunk
     position i (absolute position ``tokens + i``) sees every token up to its own. Returns ``[B, Hq, n, 128]`` BF16."""
-    fits = q.dtype == torch.bfloat16 and q.ndim == 4 and q.shape[0] == k.shape[0] and q.shape[2] == k.shape[2]
+    fits = q.dtype == torch.bfloat16 and q.ndim == 4 and k.ndim > 2 and q.size(0) == k.size(0) and q.size(2) == k.size(2)
     if not fits:
         raise ValueError(f"q has to be a bfloat16 [B, Hq, n, {HEAD_DIM}] tensor with the batch and length of k {tuple(k.shape)}; "
                          f"it is {q.dtype} {tuple(q.shape)}")
