@@ -116,11 +116,8 @@ __device__ __forceinline__ long long head_offset(const fbla_k_decode &a, int hpr
 }
 __device__ __forceinline__ long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
-// q row (batch b, virtual head hir = kh * vg + j, query qi) in q / out
-__device__ __forceinline__ int q_row(const fbla_k_decode &a, int b, int hir, int qi) {
-  const int kh = hir / a.vg, j = hir - kh * a.vg;
-  return b * a.q_heads + kh * (a.q_heads / a.kv_heads) + j * a.qg + qi;
-}
+// q row (batch b, virtual head hir = kh * vg + j, query qi) in q / out: kh (vg qg) + j qg + qi within the batch row
+__device__ __forceinline__ int q_row(const fbla_k_decode &a, int b, int hir, int qi) { return b * a.q_heads + hir * a.qg + qi; }
 
 // ---- per-group query quantization (the definition of include/mlops_fbla.h) --------------------------------------------
 // Lane l holds channels 4 l .. 4 l + 3: km = the lane's 16 metadata bytes of K (4 bases, 4 steps), q4 = its 4 q values.

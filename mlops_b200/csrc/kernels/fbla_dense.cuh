@@ -225,6 +225,26 @@ __device__ __forceinline__ float2 merge_mass(float2 x, float2 y) {  // (m, l) pa
   return make_float2(m, x.y * ex2(x.x - m) + y.y * ex2(y.x - m));
 }
 
+// The heads whose rows the CTA's warps have left: warp x's run of work is the end of vh[x][0] (all of it if vh[x][1] < 0) and, behind
+// heads of its own, the beginning of vh[x][1]; -1: none (idle warps lie before or behind the others). A head is folded by its first warp.
+struct Runs {
+  int first, last;   // of warp `lane`
+  uint32_t mask0, mask1;  // bit x: warp x is the first of the head in vh[x][0], vh[x][1]
+  __device__ __forceinline__ Runs(const int (*vh)[2], int warps, int lane) {
+    first = lane < warps ? vh[lane][0] : -1;
+    last = lane < warps ? vh[lane][1] : -1;
+    const int before = __shfl_up_sync(FULL, last >= 0 ? last : first, 1);
+    mask0 = __ballot_sync(FULL, first >= 0 && (lane == 0 || before != first));
+    mask1 = __ballot_sync(FULL, last >= 0);
+  }
+  // the warps, from x on, that hold rows of the head in vh[x][r] (the same x and r in every lane)
+  __device__ __forceinline__ int length(int x, int r) const {
+    const int lane = FBLA_POS::tid() & 31, f = __shfl_sync(FULL, first, x), l = __shfl_sync(FULL, last, x);
+    const uint32_t more = __ballot_sync(FULL, lane > x && first == (r ? l : f));
+    return 1 + (r == 0 && l >= 0 ? 0 : __popc(more));
+  }
+};
+
 // The CTA's share of the score pass: pieces of groups (units of NB sub-blocks) [first, first + count) and window chunk
 // numbers [chunk, chunk + chunks); warp w of the CTA takes chunk number w and the run [lo, hi) of the pieces.
 template <int QG>
@@ -435,24 +455,22 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
     sm.stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
-  // rows of heads that may continue in neighbouring warps, in warp order (as coarse_item's fold)
+  // rows of heads that may continue in neighbouring warps: a lane per (warp, query), merged by a butterfly (one after the other: 1 us)
+  const Runs runs(sm.stage_vh, SCORE_WARPS, lane);
 #pragma unroll 1
   for (int r = 0; r < 2; ++r) {
-    const int v = sm.stage_vh[warp][r];
-    if (v < 0) continue;
-    if (r == 0 && warp > 0) {
-      const int prev = sm.stage_vh[warp - 1][1] >= 0 ? sm.stage_vh[warp - 1][1] : sm.stage_vh[warp - 1][0];
-      if (prev == v) continue;
+    if (!((r ? runs.mask1 : runs.mask0) >> warp & 1)) continue;
+    const int v = sm.stage_vh[warp][r], n = runs.length(warp, r);
+    float2 acc = make_float2(-FBLA_INF, 0.f);
+#pragma unroll
+    for (int e = lane; e < SCORE_WARPS * QG; e += 32)
+      if (e / QG < n) acc = merge_mass(acc, sm.stage[warp + e / QG][e < QG ? r : 0][e % QG]);
+#pragma unroll
+    for (int o = QG; o < 32; o <<= 1) {
+      const float2 y = make_float2(__shfl_xor_sync(FULL, acc.x, o), __shfl_xor_sync(FULL, acc.y, o));
+      acc = (lane & o) ? merge_mass(y, acc) : merge_mass(acc, y);
     }
-    if (lane < QG) {
-      float2 acc = sm.stage[warp][r][lane];
-      if (r == 1 || sm.stage_vh[warp][1] < 0)
-        for (int x = warp + 1; x < SCORE_WARPS && sm.stage_vh[x][0] == v; ++x) {
-          acc = merge_mass(acc, sm.stage[x][0][lane]);
-          if (sm.stage_vh[x][1] >= 0) break;
-        }
-      mass_pair(a, cta + v)[lane] = acc;
-    }
+    if (lane < QG) mass_pair(a, cta + v)[lane] = acc;
   }
 }
 
@@ -484,13 +502,13 @@ __device__ __forceinline__ float row_mass(const fbla_k_decode &a, const Rows &r,
     float2 v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int i = i0 + j * (32 / QG);
-      v[j] = make_float2(-FBLA_INF, 0.f);
-      if (i < nm) v[j] = __ldcg(mass_pair(a, r.m0 + i + vh) + q);
-      else if (i < n) v[j] = __ldcg(reinterpret_cast<const float2 *>(window_row(a, r.x0 + i - nm + vh) + q * PSTRIDE + D));
+      const int i = min(i0 + j * (32 / QG), n - 1);
+      const float2 *const pair = mass_pair(a, r.m0 + i + vh) + q, *const window = reinterpret_cast<const float2 *>(window_row(a, r.x0 + i - nm + vh) + q * PSTRIDE + D);
+      v[j] = __ldcg(i < nm ? pair : window);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc = merge_mass(acc, v[j]);
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j * (32 / QG) < n) acc = merge_mass(acc, v[j]);
   }
 #pragma unroll
   for (int o = QG; o < 32; o <<= 1) {
@@ -555,10 +573,10 @@ struct __align__(16) ValueWarp {
   // The current head's sums (Sums, [word][lane]): in registers they would halve the warps that an SM holds. At the end: the last
   // head's row set.
   float2 run[17][32];
-  int stage_vh[2];
 };
 struct ValueSmem {
   ValueWarp w[VALUE_WARPS];
+  int stage_vh[VALUE_WARPS][2];
   Table table;
 };
 static_assert(sizeof(ValueSmem) + 128 <= 227 * 1024, "one CTA's shared memory");
@@ -786,29 +804,38 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     write_sums<QG>(cur_vh == first_vh ? &w.stage[0][0] : reinterpret_cast<float *>(w.run), r, lane);
   }
   if (lane == 0) {
-    w.stage_vh[0] = first_vh;
-    w.stage_vh[1] = cur_vh != first_vh ? cur_vh : -1;
+    sm.stage_vh[warp][0] = first_vh;
+    sm.stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
+  // rows of heads that may continue in neighbouring warps, added in warp order: a head by four warps, 16 bytes a thread. (By its first
+  // warp alone the rows of sixteen warps took 5 us: 8 x 16K 4+2 70.5 -> 63.0 us, 1 x 12K 24.1 -> 21.3.)
+  const Runs runs(sm.stage_vh, VALUE_WARPS, lane);
+  const int t = FBLA_POS::tid() & 127, quad = FBLA_POS::tid() >> 7;
+  uint64_t left = (uint64_t)runs.mask1 << 32 | runs.mask0;
 #pragma unroll 1
-  for (int r = 0; r < 2; ++r) {  // rows of heads that may continue in neighbouring warps, added in warp order
-    const int v = w.stage_vh[r];
-    if (v < 0) continue;
-    if (r == 0 && warp > 0) {
-      const ValueWarp &prev = sm.w[warp - 1];
-      if ((prev.stage_vh[1] >= 0 ? prev.stage_vh[1] : prev.stage_vh[0]) == v) continue;
+  for (int k = 0; left; ++k) {
+    const int bit = __ffsll((long long)left) - 1, r = bit >> 5, x = bit & 31;
+    left &= left - 1;
+    if (k % (VALUE_WARPS / 4) != quad) continue;
+    const int n = runs.length(x, r);
+    float *const dst = value_row(a, cta + sm.stage_vh[x][r]);
+    const float *src = r ? reinterpret_cast<const float *>(sm.w[x].run) : &sm.w[x].stage[0][0];
+    const int at = (t >> 5) * PSTRIDE + 4 * (t & 31);  // query t / 32, channels 4 (t % 32) ..
+    if (t < 32 * QG) {
+      float4 s = *reinterpret_cast<const float4 *>(src + at);
+#pragma unroll 4
+      for (int y = 1; y < n; ++y) {
+        const float4 z = *reinterpret_cast<const float4 *>(&sm.w[x + y].stage[0][0] + at);
+        s.x += z.x; s.y += z.y; s.z += z.z; s.w += z.w;
+      }
+      *reinterpret_cast<float4 *>(dst + at) = s;
     }
-    const bool open = r == 1 || w.stage_vh[1] < 0;
-    float *dst = value_row(a, cta + v);
-    for (int i = lane; i < QG * (PSTRIDE / 4); i += 32) {
-      float4 s = reinterpret_cast<const float4 *>(r ? reinterpret_cast<const float *>(w.run) : &w.stage[0][0])[i];
-      if (open)
-        for (int x = warp + 1; x < VALUE_WARPS && sm.w[x].stage_vh[0] == v; ++x) {
-          const float4 y = reinterpret_cast<const float4 *>(&sm.w[x].stage[0][0])[i];
-          s.x += y.x; s.y += y.y; s.z += y.z; s.w += y.w;
-          if (sm.w[x].stage_vh[1] >= 0) break;
-        }
-      reinterpret_cast<float4 *>(dst)[i] = s;
+    if (t < QG) {
+      float s = src[t * PSTRIDE + D];
+#pragma unroll 4
+      for (int y = 1; y < n; ++y) s += sm.w[x + y].stage[t][D];
+      dst[t * PSTRIDE + D] = s;
     }
   }
 }

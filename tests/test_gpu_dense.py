@@ -32,6 +32,16 @@ def test_dense_sizes(ours, oracle, mode, B, QH, KH, N, tau):
     gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode), tau=tau), f"{mode} {N}")
 
 
+@pytest.mark.parametrize("B,QH,KH,N", [(64, 32, 8, 300), (70, 16, 8, 700), (100, 8, 8, 390), (148, 16, 4, 513)])
+def test_heads_folded_inside_a_cta(ours, oracle, B, QH, KH, N):
+    """several heads per CTA, each of several warps, of one, and across the CTA's border"""
+    q, k, v = datagen.baseline_case(5 + N, B, QH, KH, N)
+    for mode in ("3+3", "4+2"):
+        got = ours.decode(ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode), gu.bf16_tensor(q))
+        torch.cuda.synchronize()
+        gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode)), f"{mode} {B} x {N}")
+
+
 @pytest.mark.parametrize("lens", [[1, 2000, 129, 16], [300] * 3 + [1], [256, 257, 4000, 255, 31]])
 def test_dense_ragged_rows(ours, oracle, lens):
     B, QH, KH, cap, mode = len(lens), 8, 2, 4096, "3+3"
