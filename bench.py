@@ -322,7 +322,7 @@ def run_decode(D, cfg, args, headline):
     peak, peak_kind = hbm_peak()
     rec = dict(ms_per_step=ms, blocks=blocks, clocks=clocks, share=share, ms_e2e=ms_e2e, h2d=q_host.numel() * 2 * world, d2h=out_host.numel() * 2 * world,
                abytes=abytes, parts=parts, peak=peak, peak_kind=peak_kind, pass_us=pass_us, ref_us=ref_us, world=world,
-               dense=b"dense" in passes[0].entry)
+               dense=b"dense" in passes[0].entry, one_kernel=passes[0].entry.endswith(b"true>"))
     return rec
 
 
@@ -376,6 +376,8 @@ def decode_record(cfg, rec, n_gpus):
         else:
             names = ["coarse_kernel", "select_kernel", "refine_kernel", "merge_kernel"]
             bytes_of = [parts["coarse_and_meta"] + parts["bf16_windows"], None, parts["refine"], None]
+        if rec["one_kernel"]:
+            names, us, bytes_of = ["head_kernel"], us[:1], [rec["abytes"]]
         top = int(np.argmax(us))
         roof["passes_us"] = dict(zip(names, us))
         roof["dominant_kernel"] = dict(name=names[top], us=us[top], share_of_passes=us[top] / sum(us))

@@ -249,18 +249,18 @@ struct WindowTile {
   uint4 v[8];
   int count;  // attended tokens of the sub-block (1 .. 16)
 };
-// The window sub-blocks [lo, hi) of the flattened list, c the cursor of `lo`; the partial rows of virtual head vh go to
-// rows + vh QG PSTRIDE. AHEAD: the next sub-block's loads are issued before the current one is computed (64 registers
+// The window sub-blocks [lo, hi) of the flattened list, c the cursor of `lo`; the partial rows of virtual head vh go to row_at(vh) (the
+// place of the last head's may be sm.v). AHEAD: the next sub-block's loads are issued before the current one is computed (64 registers
 // more: for the kernels with few warps per SM).
-template <int QG, bool AHEAD>
-__device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, long long lo, long long hi, Cursor c, float *rows) {
+template <int QG, bool AHEAD, class RowAt>
+__device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, long long lo, long long hi, Cursor c, RowAt row_at) {
   const int hpr = a.kv_heads * a.vg;
   if (lo >= hi) return;
   const int gid = lane >> 2, tig = lane & 3;
   int cur_vh = -1;
   float m[2], l[2], o[8][4];  // queries 2 tig + e; o[tile]: channels 16 tile + gid (.0, .1), + 8 (.2, .3) x the two queries
   auto flush = [&]() {
-    float *p = rows + (size_t)cur_vh * QG * PSTRIDE;
+    float *p = row_at(cur_vh);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int qi = 2 * tig + e;
@@ -360,6 +360,7 @@ __device__ void exact_range(const fbla_k_decode &a, ExactWarp &sm, int lane, lon
     }
     if (AHEAD) cur = nxt;
   }
+  __syncwarp();  // (the V rows have been read)
   flush();
 }
 // window slots lie after the coarse slots: slot xw + virtual head of window warp xw
@@ -370,7 +371,7 @@ __device__ __forceinline__ float *window_rows(const fbla_k_decode &a, int qg, in
 template <int QG>
 __device__ __forceinline__ void exact_warp(const fbla_k_decode &a, ExactWarp &sm, int lane, int xw, int nxw) {
   const long long total = total_units<true>(a, a.kv_heads * a.vg), per = ceil_div(total, nxw), lo = (long long)xw * per;
-  if (lo < total) exact_range<QG, true>(a, sm, lane, lo, min(total, lo + per), locate<true>(a, a.kv_heads * a.vg, lo), window_rows(a, QG, xw));
+  if (lo < total) exact_range<QG, true>(a, sm, lane, lo, min(total, lo + per), locate<true>(a, a.kv_heads * a.vg, lo), [&](int vh) { return window_rows(a, QG, xw) + (size_t)vh * QG * PSTRIDE; });
 }
 
 // ---- one closed group on the tensor cores ----------------------------------------------------------------------------------
@@ -638,7 +639,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
     long long xlo, xhi;
     gw = (long long)FBLA_POS::x() * sw + warp;
     deal_range(d, gw, xlo, xhi, lo, hi);
-    if (xlo < xhi) exact_range<QG, true>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, xlo, xhi, locate<true>(a, hpr, xlo), window_rows(a, QG, (int)gw));
+    if (xlo < xhi) exact_range<QG, true>(a, *reinterpret_cast<ExactWarp *>(&sm.w[warp]), lane, xlo, xhi, locate<true>(a, hpr, xlo), [&](int vh) { return window_rows(a, QG, (int)gw) + (size_t)vh * QG * PSTRIDE; });
     __syncwarp();
   }
   StreamWarp<CB, SHAPE> &w = sm.w[warp];

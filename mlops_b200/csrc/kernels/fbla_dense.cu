@@ -11,6 +11,12 @@ __global__ void __launch_bounds__(32 * SCORE_WARPS, 1) score_kernel(const fbla_k
   score_item<CB, FB, QG>(a, smem_raw);
 }
 
+template <int CB, int FB, int QG>
+__global__ void __launch_bounds__(32 * SCORE_WARPS, 1) head_kernel(const fbla_k_decode a) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  head_passes<CB, FB, QG>(a, smem_raw);
+}
+
 template <int QG>
 __global__ void __launch_bounds__(256) mass_kernel(const fbla_k_decode a) {
   mass_item<QG>(a, nullptr);
@@ -36,11 +42,19 @@ template <int CB, int FB, int QG> struct Kernels {
     if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(score_kernel<CB, FB, QG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCORE_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(value_kernel<CB, FB, QG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VALUE_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(head_kernel<CB, FB, QG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HeadSmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(head_kernel<CB, FB, QG>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = 1;
     return e;
   }
+  static cudaError_t whole(fbla_k_decode a, bool dependent, cudaStream_t stream) {
+    a.status = nullptr;  // (no wait of this kernel gives up)
+    a.mass_given = 0;
+    return launch(dependent, a.head_ctas, head_kernel<CB, FB, QG>, dim3(a.head_ctas, a.kv_heads * a.vg, a.batch), 32 * SCORE_WARPS, sizeof(HeadSmem), stream, a);
+  }
   static cudaError_t pass(const fbla_k_decode &a, int which, bool dependent, cudaStream_t stream) {
     const int vheads = a.batch * a.kv_heads * a.vg;
+    if (a.head_ctas) return which == 0 ? whole(a, dependent, stream) : cudaSuccess;
     switch (which) {
       case 0: return launch(dependent, 1, score_kernel<CB, FB, QG>, dim3(a.coarse_ctas), 32 * SCORE_WARPS, SCORE_SMEM, stream, a);
       case 1: return launch(dependent, 1, mass_kernel<QG>, dim3((vheads + 7) / 8), 256, 0, stream, a);
@@ -51,6 +65,7 @@ template <int CB, int FB, int QG> struct Kernels {
   }
   static cudaError_t all(const fbla_k_decode &a, cudaStream_t stream) {
     cudaError_t e = configure();
+    if (a.head_ctas && e == cudaSuccess) return whole(a, true, stream);
     if (a.phase != 2 && e == cudaSuccess) e = pass(a, 0, true, stream);
     if (e != cudaSuccess) return e;
     if (a.phase == 1) return pass(a, 1, true, stream);
@@ -73,6 +88,13 @@ template <int CB, int FB, int QG> struct Kernels {
     snprintf(p[0].entry, sizeof p[0].entry, "fbla::dense::score_item<%d, %d, %d>", CB, FB, QG);
     snprintf(p[1].entry, sizeof p[1].entry, "fbla::dense::mass_item<%d>", QG);
     snprintf(p[2].entry, sizeof p[2].entry, "fbla::dense::value_item<%d, %d, %d>", CB, FB, QG);
+    if (a.head_ctas && e == cudaSuccess) {
+      e = describe(head_kernel<CB, FB, QG>, a.head_ctas, 32 * SCORE_WARPS, sizeof(HeadScoreSmem), p + 0);
+      if (e == cudaSuccess) e = describe(head_kernel<CB, FB, QG>, a.head_ctas, 32 * VALUE_WARPS, sizeof(HeadValueSmem), p + 2);
+      for (int i = 0; i <= 2; i += 2) { p[i].gy = a.kv_heads * a.vg; p[i].gz = a.batch; }
+      snprintf(p[0].entry, sizeof p[0].entry, "fbla::dense::score_item<%d, %d, %d, true>", CB, FB, QG);
+      snprintf(p[2].entry, sizeof p[2].entry, "fbla::dense::value_item<%d, %d, %d, true>", CB, FB, QG);
+    }
     snprintf(p[3].entry, sizeof p[3].entry, "fbla::dense::gather_item<%d>", QG);
     return e;
   }
@@ -118,4 +140,24 @@ extern "C" int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens
   const int few = qg == 4 ? 52 : qg == 2 ? 20 : 12, few_line = qg == 4 ? 40 : qg == 2 ? 30 : 20;  // groups per CTA of a B200, whatever the device
   return batch <= FBLA_K_DENSE_MAX_BATCH && (long long)vheads * groups * fbla::dense::PAIRS < (1ll << 29) &&
          (n_tau <= line || (n_tau <= few_line && (long long)vheads * groups <= few * 148));
+}
+
+// A short decode is mostly launches and the chains of round trips at their borders. One kernel with a cluster per virtual head has neither,
+// but its heads' CTAs leave SMs idle and a head's work cannot move to another's. CTAs per head: as many as let all clusters run at once (of n
+// CTAs with an SM each a B200 holds n: 1: 148, 2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 8: 15, 10: 11, 16: 7). Groups per CTA up to which it is the
+// faster way (the room's: rows of lengths of their own wait for the longest). Device time on B200, us, three kernels / one, 3+3, 32 / 8 heads
+// unless said:
+//   batch 1, 10 CTAs: 250 tokens 11.0 / 7.2    4 096: 18.7 / 12.4    12 000 (9 groups per CTA): 21.9 / 19.7    30 000 (23): 31.1 / 31.3    80 000: 52 / 77
+//   batch 2, 6 CTAs:  250: 11.2 / 7.3          4 096: 20.5 / 14.7    12 000 (16): 27.7 / 24.8                  30 000 (39): 44.6 / 52.1
+//   batch 4, 4 CTAs:  250: 11.4 / 7.3          4 096: 23.9 / 17.5    12 000 (23): 36.1 / 34.0                  30 000 (58): 68.7 / 77.4
+//   batch 9, 2 CTAs:  250: 12.2 / 8.1          4 000: 31.8 / 24.6    8 000 (31): 49.5 / 47.3
+//   batch 12, 1 CTA:  250: 12.8 / 8.7          2 000 (14): 27.7 / 23.8    4 000 (30): 37.7 / 41.3
+//   8 / 2 heads, 16:  250: 8.6 / 6.9           4 096: 18.8 / 11.0    12 000 (6): 21.1 / 16.0    30 000 (15): 24.8 / 23.7    80 000 (39): 31.8 / 42.7
+//   4+2, batch 1:     4 096: 18.1 / 11.6       30 000: 27.8 / 26.2    batch 4: 12 000: 32.2 / 28.6    batch 8, 2 CTAs: 12 000 (47): 50.6 / 53.1
+//   rows of their own lengths, batch 8: 1 000 to 4 000 (16): 30.2 / 26.0    300 to 8 000 (32): 39.4 / 43.2
+extern "C" int fbla_k_head_ctas(int vheads, long long tokens) {
+  static const struct { int ctas, vheads; } held[] = {{16, 7}, {10, 11}, {8, 15}, {6, 22}, {5, 26}, {4, 33}, {3, 45}, {2, 74}, {1, 148}};
+  for (const auto &h : held)
+    if (vheads <= h.vheads) return (tokens + fbla::G - 1) / fbla::G <= (h.ctas == 16 ? 16 : 20) * h.ctas ? h.ctas : 0;
+  return 0;
 }

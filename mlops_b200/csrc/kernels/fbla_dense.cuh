@@ -93,6 +93,20 @@ template <bool EXACT> __device__ __forceinline__ Cursor find(const fbla_k_decode
   return c;
 }
 
+// Where every virtual head has CTAs of its own (a.head_ctas of them: the grid is CTAs x heads of a batch row x batch rows): the head of this
+// item's CTA, and the CTA's rank among the head's. `slot`: the CTA's number among all.
+struct Own {
+  int ctas, rank, hir, b, vh, slot;
+  Row row;
+  __device__ __forceinline__ explicit Own(const fbla_k_decode &a) : ctas(FBLA_POS::nx()), rank(FBLA_POS::x()), hir(FBLA_POS::y()), b(FBLA_POS::z()) {
+    vh = b * (int)FBLA_POS::ny() + hir;
+    slot = vh * ctas + rank;
+    row = row_of(a, b);
+  }
+};
+// the KV head of virtual head vh
+__device__ __forceinline__ int kv_of(const fbla_k_decode &a, int vh) { return a.vg == 1 ? vh : vh / a.vg; }
+
 // ---- scratch (`lse`; the rest inside the decode's `part` and `dpart` arrays) -----------------------------------------------------------------
 // Window chunks: the flattened window sub-blocks in runs of `run`; chunk c leaves one (m, l, o) row per virtual head it meets, at
 // slot c + vh. Value rows (o, l in units of 2^-R) and the score pass's (m, l) pairs: one per (CTA, virtual head), slot cta + vh.
@@ -212,17 +226,21 @@ struct ScoreWarp {
     } s;
   };
 };
-struct __align__(16) ScoreSmem {
-  ScoreWarp w[SCORE_WARPS];
-  Table table;
+struct ScoreFold {
   float2 stage[SCORE_WARPS][2][4];  // (m, l) of the first and the last virtual head of a warp's run
   int stage_vh[SCORE_WARPS][2];
+  float2 window[SCORE_WARPS][4];    // a head's own CTAs: (m, l) of the warp's window sub-block
 };
+struct __align__(16) ScoreSmem {
+  ScoreWarp w[SCORE_WARPS];
+  ScoreFold fold;
+  Table table;
+};
+struct __align__(16) HeadScoreSmem { ScoreWarp w[SCORE_WARPS]; ScoreFold fold; };
 
 __device__ __forceinline__ float2 merge_mass(float2 x, float2 y) {  // (m, l) pairs; symmetric in its arguments up to the order of one sum
-  const float m = fmaxf(x.x, y.x);
-  if (m == -FBLA_INF) return x;
-  return make_float2(m, x.y * ex2(x.x - m) + y.y * ex2(y.x - m));
+  const float m = fmaxf(x.x, y.x), by = m == -FBLA_INF ? 0.f : m;  // (nothing on either side: 2^-inf = 0)
+  return make_float2(m, x.y * ex2(x.x - by) + y.y * ex2(y.x - by));
 }
 
 // The heads whose rows the CTA's warps have left: warp x's run of work is the end of vh[x][0] (all of it if vh[x][1] < 0) and, behind
@@ -245,11 +263,20 @@ struct Runs {
   }
 };
 
+// lane l's pair becomes that of query l % QG over all lanes
+template <int QG> __device__ __forceinline__ float2 merge_lanes(float2 acc, int lane) {
+#pragma unroll
+  for (int o = QG; o < 32; o <<= 1) {
+    const float2 y = make_float2(__shfl_xor_sync(FULL, acc.x, o), __shfl_xor_sync(FULL, acc.y, o));
+    acc = (lane & o) ? merge_mass(y, acc) : merge_mass(acc, y);
+  }
+  return acc;
+}
+
 // The CTA's share of the score pass: pieces of groups (units of NB sub-blocks) [first, first + count) and window chunk
 // numbers [chunk, chunk + chunks); warp w of the CTA takes chunk number w and the run [lo, hi) of the pieces.
 template <int QG>
-__device__ __forceinline__ void score_item_units(const fbla_k_decode &a, int total, int x_total, int run, int warp, int &chunk, int &lo, int &hi) {
-  const int ctas = FBLA_POS::nx(), cta = FBLA_POS::x();
+__device__ __forceinline__ void score_item_units(int ctas, int cta, int total, int x_total, int run, int warp, int &chunk, int &lo, int &hi) {
   const int per = (total + ctas - 1) / ctas, first = min(total, cta * per), count = min(total, first + per) - first;
   const int chunks = (x_total + run - 1) / run, cper = (chunks + ctas - 1) / ctas, c0 = min(chunks, cta * cper), nc = min(chunks, c0 + cper) - c0;
   chunk = warp < nc ? c0 + warp : -1;
@@ -266,29 +293,58 @@ __device__ __forceinline__ void score_item_units(const fbla_k_decode &a, int tot
   hi = first + min(count, at + (warp < nc ? with : without));
 }
 
-template <int CB, int FB, int QG>
-__device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem_raw) {
+// What the CTAs of one head hand on, in a plan's passes: through the scratch
+template <int QG> struct ScratchVia {
+  const fbla_k_decode &a;
+  int ctas, vh, slot;
+  __device__ __forceinline__ explicit ScratchVia(const fbla_k_decode &a_) : a(a_) { const Own own(a); ctas = own.ctas; vh = own.vh; slot = own.slot; }
+  __device__ __forceinline__ ScratchVia(const fbla_k_decode &a_, int vh_) : a(a_), ctas(a_.head_ctas), vh(vh_), slot(0) {}
+  __device__ __forceinline__ void ready() const {}
+  __device__ __forceinline__ float *window(int x) const { return window_row(a, vh * SCORE_WARPS + x + vh); }  // the head's window sub-block x: [QG][PSTRIDE]
+  // the CTA's (m, l) of query lane % QG
+  __device__ __forceinline__ void put_mass(float2 mass, int lane) const { if (lane < QG) mass_pair(a, slot + vh)[lane] = mass; }
+  __device__ __forceinline__ float2 mass(int cta, int q) const { return __ldcg(mass_pair(a, vh * ctas + cta + vh) + q); }
+  // the CTA's sum of query q, channel ch (D: l), and that of CTA cta
+  __device__ __forceinline__ void put(int q, int ch, float x) const { value_row(a, slot + vh)[q * PSTRIDE + ch] = x; }
+  __device__ __forceinline__ float sum(int cta, int q, int ch) const { return __ldcg(value_row(a, vh * ctas + cta + vh) + q * PSTRIDE + ch); }
+};
+struct NoVia { __device__ __forceinline__ void ready() const {} };
+
+// HEAD: every virtual head has CTAs of its own; else the work is dealt over all CTAs, `table` the batch's prefix sums
+// (Via: how the parts of a head's own CTAs hand their results on)
+template <int CB, int FB, int QG, bool HEAD, class Via>
+__device__ __forceinline__ void score_units(const fbla_k_decode &a, ScoreWarp *ws, ScoreFold &fold, const Table *table, const Via &via) {
   constexpr int NB = 8 / QG, UPG = QG;  // sub-blocks per unit, units per group
   constexpr float HOFF = .5f * ((1 << FB) - 1);
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
-  ScoreSmem &sm = *reinterpret_cast<ScoreSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
-  const int hpr = a.kv_heads * a.vg;
-  wait_previous_pass();  // (lengths, queries and the cache may come from the kernel before)
-  allow_next_pass();     // (behind the wait: the value pass then finds everything before this call complete)
-  if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status) { a.status[0] = 0; a.status[1] = 0; }
-  build_table(a, sm.table, 32 * SCORE_WARPS);
-  if (FBLA_POS::x() == 0 && a.lstride)
-    for (int i = FBLA_POS::tid(); i <= a.batch; i += 32 * SCORE_WARPS) { table_of(a)[i] = sm.table.closed[i]; table_of(a)[a.batch + 1 + i] = sm.table.exact[i]; }
-  const int total = UPG * total_of<false>(a, sm.table.closed, hpr), x_total = total_of<true>(a, sm.table.exact, hpr), run = window_run(a, x_total);
-  int chunk, lo, hi;
-  score_item_units<QG>(a, total, x_total, run, warp, chunk, lo, hi);
-  if (chunk >= 0) exact_range<QG, false>(a, sm.w[warp].exact, lane, chunk * run, min(x_total, (chunk + 1) * run), find<true>(a, sm.table.exact, hpr, chunk * run), window_row(a, chunk));
+  const int hpr = HEAD ? (int)FBLA_POS::ny() : a.kv_heads * a.vg;
+  int chunk, lo, hi, cta;
+  Cursor c{0, 0, 0, 0};
+  if constexpr (HEAD) {
+    const Own own(a);
+    cta = own.slot;
+    score_item_units<QG>(own.ctas, own.rank, UPG * own.row.closed, own.row.exact, 1, warp, chunk, lo, hi);
+    float2 mass = make_float2(-FBLA_INF, 0.f);
+    if (chunk >= 0) {
+      float *const row = via.window(chunk);
+      exact_range<QG, false>(a, ws[warp].exact, lane, chunk, chunk + 1, Cursor{own.b, own.hir, chunk, own.row.exact}, [&](int) { return row; });
+      __syncwarp();
+      if (lane < QG) mass = make_float2(row[lane * PSTRIDE + D], row[lane * PSTRIDE + D + 1]);
+    }
+    if (lane < QG) fold.window[warp][lane] = mass;
+    c = Cursor{own.b, own.hir, lo / UPG, own.row.closed};
+  } else {
+    cta = FBLA_POS::x();
+    const int total = UPG * total_of<false>(a, table->closed, hpr), x_total = total_of<true>(a, table->exact, hpr), run = window_run(a, x_total);
+    score_item_units<QG>(FBLA_POS::nx(), cta, total, x_total, run, warp, chunk, lo, hi);
+    if (chunk >= 0) exact_range<QG, false>(a, ws[warp].exact, lane, chunk * run, min(x_total, (chunk + 1) * run), find<true>(a, table->exact, hpr, chunk * run),
+                                             [&](int vh) { return window_row(a, chunk + vh); });
+  }
   __syncwarp();
-  uint8_t *const qst = sm.w[warp].s.qst;
-  uint8_t (*const pst)[128] = sm.w[warp].s.pst;
+  uint8_t *const qst = ws[warp].s.qst;
+  uint8_t (*const pst)[128] = ws[warp].s.pst;
 
-  const int cta = FBLA_POS::x();
   int first_vh = -1, cur_vh = -1;
   float m[2] = {-FBLA_INF, -FBLA_INF}, l[2] = {0.f, 0.f};  // of the thread's two columns
   // (m, l) of every query of the head into dst[0 .. QG): columns of one query are merged over the threads that hold them
@@ -309,7 +365,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
     }
   };
   if (lo < hi) {
-    Cursor c = find<false>(a, sm.table.closed, hpr, lo / UPG);
+    if constexpr (!HEAD) c = find<false>(a, table->closed, hpr, lo / UPG);
     int piece = lo % UPG;
     // Where the next unit's words lie, and the cells of the unit in work: pointers that run on, set anew with every head only.
     const uint8_t *kp, *fp, *mp;
@@ -319,7 +375,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
     const long long k_skip = (long long)(a.gs - 1) * SBG * RC, f_skip = (long long)(a.gs - 1) * SBG * RF, m_step = (long long)a.gs * 1024;
     const int k_tail = KWords<3>::tail(tig);
     auto place_records = [&](const Cursor &x, int pc) {
-      const size_t unit = (size_t)((x.b * hpr + x.hir) / a.vg) * a.hs + (size_t)group_of(a, x) * a.gs;
+      const size_t unit = (size_t)kv_of(a, x.b * hpr + x.hir) * a.hs + (size_t)group_of(a, x) * a.gs;
       kp = a.c.coarse + (unit * SBG + pc * NB) * RC + KWords<CB>::offset(gid, tig);
       fp = a.c.fine + (unit * SBG + pc * NB) * RF + KWords<FB>::offset(gid, tig);
       mp = reinterpret_cast<const uint8_t *>(a.c.meta) + unit * 1024 + 16 * lane;
@@ -345,7 +401,7 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
     for (int u = lo; u < hi; ++u) {
       const int vh = c.b * hpr + c.hir;
       if (vh != cur_vh) {
-        if (cur_vh >= 0) leave(cur_vh == first_vh ? sm.stage[warp][0] : mass_pair(a, cta + cur_vh));
+        if (cur_vh >= 0) leave(cur_vh == first_vh ? fold.stage[warp][0] : mass_pair(a, cta + cur_vh));
         else first_vh = vh;
         cur_vh = vh;
         m[0] = m[1] = -FBLA_INF; l[0] = l[1] = 0.f;
@@ -448,29 +504,56 @@ __device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem
       wp[4 * n_cells] = lds32(pst[1] + 4 * lane);
       lp += 8; wp += 32;
     }
-    leave(sm.stage[warp][cur_vh == first_vh ? 0 : 1]);
+    leave(fold.stage[warp][cur_vh == first_vh ? 0 : 1]);
   }
   if (lane == 0) {
-    sm.stage_vh[warp][0] = first_vh;
-    sm.stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
+    fold.stage_vh[warp][0] = first_vh;
+    fold.stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
   // rows of heads that may continue in neighbouring warps: a lane per (warp, query), merged by a butterfly (one after the other: 1 us)
-  const Runs runs(sm.stage_vh, SCORE_WARPS, lane);
-#pragma unroll 1
-  for (int r = 0; r < 2; ++r) {
-    if (!((r ? runs.mask1 : runs.mask0) >> warp & 1)) continue;
-    const int v = sm.stage_vh[warp][r], n = runs.length(warp, r);
-    float2 acc = make_float2(-FBLA_INF, 0.f);
+  via.ready();
+  if constexpr (HEAD) {  // one head: its pairs of all warps, and of the CTA's window sub-blocks (a CTA without either leaves -inf)
+    if (warp == 0) {
+      float2 acc = make_float2(-FBLA_INF, 0.f);
 #pragma unroll
-    for (int e = lane; e < SCORE_WARPS * QG; e += 32)
-      if (e / QG < n) acc = merge_mass(acc, sm.stage[warp + e / QG][e < QG ? r : 0][e % QG]);
-#pragma unroll
-    for (int o = QG; o < 32; o <<= 1) {
-      const float2 y = make_float2(__shfl_xor_sync(FULL, acc.x, o), __shfl_xor_sync(FULL, acc.y, o));
-      acc = (lane & o) ? merge_mass(y, acc) : merge_mass(acc, y);
+      for (int e = lane; e < SCORE_WARPS * QG; e += 32) {
+        if (fold.stage_vh[e / QG][0] >= 0) acc = merge_mass(acc, fold.stage[e / QG][0][e % QG]);
+        acc = merge_mass(acc, fold.window[e / QG][e % QG]);
+      }
+      acc = merge_lanes<QG>(acc, lane);
+      via.put_mass(acc, lane);
     }
-    if (lane < QG) mass_pair(a, cta + v)[lane] = acc;
+  } else {
+    const Runs runs(fold.stage_vh, SCORE_WARPS, lane);
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {
+      if (!((r ? runs.mask1 : runs.mask0) >> warp & 1)) continue;
+      const int v = fold.stage_vh[warp][r], n = runs.length(warp, r);
+      float2 acc = make_float2(-FBLA_INF, 0.f);
+#pragma unroll
+      for (int e = lane; e < SCORE_WARPS * QG; e += 32)
+        if (e / QG < n) acc = merge_mass(acc, fold.stage[warp + e / QG][e < QG ? r : 0][e % QG]);
+      acc = merge_lanes<QG>(acc, lane);
+      if (lane < QG) mass_pair(a, cta + v)[lane] = acc;
+    }
+  }
+}
+
+template <int CB, int FB, int QG, bool HEAD = false>
+__device__ __forceinline__ void score_item(const fbla_k_decode &a, uint8_t *smem_raw) {
+  wait_previous_pass();  // (lengths, queries and the cache may come from the kernel before)
+  allow_next_pass();     // (behind the wait: the value pass then finds everything before this call complete)
+  if (FBLA_POS::x() == 0 && FBLA_POS::y() == 0 && FBLA_POS::z() == 0 && FBLA_POS::tid() == 0 && a.status) { a.status[0] = 0; a.status[1] = 0; }
+  if constexpr (HEAD) {
+    HeadScoreSmem &sm = *reinterpret_cast<HeadScoreSmem *>(smem_raw);
+    score_units<CB, FB, QG, true>(a, sm.w, sm.fold, nullptr, ScratchVia<QG>(a));
+  } else {
+    ScoreSmem &sm = *reinterpret_cast<ScoreSmem *>(smem_raw);
+    build_table(a, sm.table, 32 * SCORE_WARPS);
+    if (FBLA_POS::x() == 0 && a.lstride)
+      for (int i = FBLA_POS::tid(); i <= a.batch; i += 32 * SCORE_WARPS) { table_of(a)[i] = sm.table.closed[i]; table_of(a)[a.batch + 1 + i] = sm.table.exact[i]; }
+    score_units<CB, FB, QG, false>(a, sm.w, sm.fold, &sm.table, NoVia());
   }
 }
 
@@ -510,12 +593,15 @@ __device__ __forceinline__ float row_mass(const fbla_k_decode &a, const Rows &r,
     for (int j = 0; j < 4; ++j)
       if (i0 + j * (32 / QG) < n) acc = merge_mass(acc, v[j]);
   }
-#pragma unroll
-  for (int o = QG; o < 32; o <<= 1) {
-    const float2 y = make_float2(__shfl_xor_sync(FULL, acc.x, o), __shfl_xor_sync(FULL, acc.y, o));
-    acc = (lane & o) ? merge_mass(y, acc) : merge_mass(acc, y);
-  }
+  acc = merge_lanes<QG>(acc, lane);
   return acc.x + lg2(acc.y);  // (-inf for a shard that holds nothing of the row)
+}
+// the same where the head has CTAs of its own
+template <int QG, class Via> __device__ __forceinline__ float head_mass(const Via &via, int ctas, int lane) {
+  float2 acc = make_float2(-FBLA_INF, 0.f);
+  for (int i = lane / QG; i < ctas; i += 32 / QG) acc = merge_mass(acc, via.mass(i, lane % QG));
+  acc = merge_lanes<QG>(acc, lane);
+  return acc.x + lg2(acc.y);
 }
 // the rows' masses into row_r: a shard's first phase, and a pass of its own under an executor. One warp per virtual head.
 template <int QG>
@@ -525,7 +611,7 @@ __device__ __forceinline__ void mass_item(const fbla_k_decode &a, uint8_t *smem_
   wait_previous_pass();
   if (vh >= a.batch * hpr) return;
   const int *t = table_of(a);
-  const float R = row_mass<QG>(a, rows_of<QG>(a, t, t + a.batch + 1, hpr, vh), vh, lane);
+  const float R = a.head_ctas ? head_mass<QG>(ScratchVia<QG>(a, vh), a.head_ctas, lane) : row_mass<QG>(a, rows_of<QG>(a, t, t + a.batch + 1, hpr, vh), vh, lane);
   if (lane < QG) a.row_r[vh * QG + lane] = R;
 }
 
@@ -579,6 +665,7 @@ struct ValueSmem {
   int stage_vh[VALUE_WARPS][2];
   Table table;
 };
+struct __align__(16) HeadValueSmem { ValueWarp w[VALUE_WARPS]; };
 static_assert(sizeof(ValueSmem) + 128 <= 227 * 1024, "one CTA's shared memory");
 
 // the sums of one virtual head over the warp's pairs, in units of 2^-R: thread (gid, tig) holds channels 4 (8 u + gid) + cc of
@@ -607,30 +694,50 @@ template <int QG> __device__ __forceinline__ void write_sums(float *p, const Sum
   }
 }
 
-template <int CB, int FB, int QG>
-__device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem_raw) {
+// `wait` returns when the score pass's results may be read; what does not depend on them is asked for before.
+template <int CB, int FB, int QG, bool HEAD, class Via, class Wait>
+__device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *ws, int (*stage_vh)[2], const Table *table, const Via &via, Wait wait) {
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
   constexpr float HOFF = .5f * ((1 << FB) - 1);
-  ValueSmem &sm = *reinterpret_cast<ValueSmem *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
-  const int hpr = a.kv_heads * a.vg, cta = FBLA_POS::x();
-  ValueWarp &w = sm.w[warp];
-  allow_next_pass();
-  build_table(a, sm.table, 32 * VALUE_WARPS);
-  const int total = PAIRS * total_of<false>(a, sm.table.closed, hpr), per = (total + (int)FBLA_POS::nx() - 1) / (int)FBLA_POS::nx();
-  const int c_lo = min(total, cta * per), c_n = min(total, c_lo + per) - c_lo, wper = (c_n + VALUE_WARPS - 1) / VALUE_WARPS;
-  const int lo = c_lo + min(c_n, warp * wper), hi = c_lo + min(c_n, (warp + 1) * wper);
-  wait_previous_pass();
+  const int hpr = HEAD ? (int)FBLA_POS::ny() : a.kv_heads * a.vg;
+  ValueWarp &w = ws[warp];
+  int cta, total, c_lo, c_n;
+  Cursor c{0, 0, 0, 0};
+  if constexpr (HEAD) {
+    const Own own(a);
+    cta = own.slot; total = PAIRS * own.row.closed;
+    const int per = (QG * own.row.closed + own.ctas - 1) / own.ctas * (PAIRS / QG);  // the sub-blocks that the CTA has scored
+    c_lo = min(total, own.rank * per); c_n = min(total, c_lo + per) - c_lo;
+    c = Cursor{own.b, own.hir, 0, own.row.closed};
+  } else {
+    cta = FBLA_POS::x(); total = PAIRS * total_of<false>(a, table->closed, hpr);
+    const int per = (total + (int)FBLA_POS::nx() - 1) / (int)FBLA_POS::nx();
+    c_lo = min(total, cta * per); c_n = min(total, c_lo + per) - c_lo;
+  }
+  const int wper = (c_n + VALUE_WARPS - 1) / VALUE_WARPS, lo = c_lo + min(c_n, warp * wper), hi = c_lo + min(c_n, (warp + 1) * wper);
+  float R = 0.f;  // lane l: of query l % QG of the current head
+  // (HEAD: every warp asks for it, also one without pairs: the CTA's window sub-blocks need it)
+  auto mass_of = [&](int vh) {
+    if (a.mass_given) return __ldcg(a.row_r + vh * QG + lane % QG);
+    if constexpr (HEAD) return head_mass<QG>(via, (int)FBLA_POS::nx(), lane);
+    else return row_mass<QG>(a, rows_of<QG>(a, table->closed, table->exact, hpr, vh), vh, lane);
+  };
+  if (lo >= hi) {
+    wait();
+    if (HEAD) R = mass_of(c.b * hpr + c.hir);
+  }
   int first_vh = -1, cur_vh = -1;
   if (lo < hi) {
-    Cursor c = find<false>(a, sm.table.closed, hpr, lo / PAIRS);
+    if constexpr (HEAD) c.i = lo / PAIRS;
+    else c = find<false>(a, table->closed, hpr, lo / PAIRS);
     const int groups = (hi - 1) / PAIRS - lo / PAIRS + 1;
     int left = hi - lo;  // pairs
     // The sums of integer products are taken as they are: a nonnegative s32 below 2^23 read as FP32 is the subnormal s 2^-149, and a
     // weight times 2^75 brings the product back into range; the group's sums come out times 2^-74.
     constexpr float UP = 37778931862957161709568.f /* 2^75 */, BACK = 18889465931478580854784.f /* 2^74 */;
     // a group's place: its unit, and its first cell
-    auto unit_of = [&](const Cursor &x) { return (size_t)((x.b * hpr + x.hir) / a.vg) * a.hs + (size_t)group_of(a, x) * a.gs; };
+    auto unit_of = [&](const Cursor &x) { return (size_t)kv_of(a, x.b * hpr + x.hir) * a.hs + (size_t)group_of(a, x) * a.gs; };
     auto cell_of = [&](const Cursor &x) { return ((size_t)(x.b * hpr + x.hir) * a.nblocks + (size_t)group_of(a, x) * SBG) * QG; };
     const size_t n_cells = cells_of(a);
     const int pcol = (gid >> 2) * QG + (gid & 3);  // the lane's column of a pair's P words: sub-block gid / 4, query gid % 4
@@ -653,8 +760,6 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
                    ::"r"(smem_u32(w.meta[buf] + 16 * lane)), "l"(reinterpret_cast<const uint8_t *>(a.c.meta) + un * 1024 + 512 + 16 * lane) : "memory");
     };
     int J = lo % PAIRS;
-    ask(cell);
-    ask_p(cell, J);
     fetch_meta(unit, 0);
     // where the words of the next pair (coarse) and of the pair in work (fine) lie: pointers that run on within a head
     const uint8_t *cp = a.c.coarse + (unit * SBG + 2 * J) * RC + VWords<CB>::offset(gid, tig), *fp = a.c.fine + (unit * SBG + 2 * J) * RF + VWords<FB>::offset(gid, tig);
@@ -667,7 +772,22 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
       cp += 2 * RC;
     };
     load_coarse();
-    float R = 0.f;  // lane l: of query l % QG of the current head
+    VWords<FB> fa, fb;
+    auto load_fine = [&] {
+      fa.load(fp, d1, d2);
+      fb.load(fp + RF, d1, d2);
+      fp += 2 * RF;
+    };
+    if constexpr (HEAD) {  // (the CTA's own cells: complete. Short rows, most sub-blocks selected: the fine words do not wait for R)
+      load_fine();
+      ask(cell);
+      ask_p(cell, J);
+      wait();
+    } else {
+      wait();
+      ask(cell);
+      ask_p(cell, J);
+    }
     auto sums = [&] {
       Sums r;
       r.l = w.run[16][lane];
@@ -686,11 +806,8 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
         cur_vh = vh;
 #pragma unroll
         for (int x = 0; x < 17; ++x) w.run[x][lane] = make_float2(0.f, 0.f);
-        if (a.mass_given) R = __ldcg(a.row_r + vh * QG + lane % QG);
-        else {
-          R = row_mass<QG>(a, rows_of<QG>(a, sm.table.closed, sm.table.exact, hpr, vh), vh, lane);
-          if (lane < QG) a.row_r[vh * QG + lane] = R;  // for the merge (every warp of the head writes the same)
-        }
+        R = mass_of(vh);
+        if (!HEAD && !a.mass_given && lane < QG) a.row_r[vh * QG + lane] = R;  // for the merge (every warp of the head writes the same)
       }
       const uint32_t mask = __ballot_sync(FULL, lse_n - R > a.log2_tau);  // bit cell: selected
       float wl = ex2(((mask >> lane) & 1 ? mf_n : mc_n) - R) * UP;          // lane: the weight of its cell
@@ -713,12 +830,10 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
 #pragma unroll 1
       for (; J < j1; ++J, --left) {
         const uint32_t pm = (mask >> (2 * QG * J)) & ((1u << (2 * QG)) - 1u);  // the pair's selections
-        VWords<FB> fa, fb;
-        if (pm) {
-          fa.load(fp, d1, d2);
-          fb.load(fp + RF, d1, d2);
+        if constexpr (!HEAD) {
+          if (pm) load_fine();
+          else fp += 2 * RF;
         }
-        fp += 2 * RF;
         uint32_t pw = (pm >> pcol) & 1 ? pf : pc;
         if (!has) pw = 0u;
         const bool last = J + 1 >= PAIRS;
@@ -780,6 +895,7 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
             add(x, y, f, A[u]);
           }
         }
+        if (HEAD && left > 1) load_fine();
       }
       J = 0;
       if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -803,14 +919,41 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     __syncwarp();
     write_sums<QG>(cur_vh == first_vh ? &w.stage[0][0] : reinterpret_cast<float *>(w.run), r, lane);
   }
+  if constexpr (HEAD) {
+    // One head: a thread per (query, channel) adds the CTA's window sub-blocks, brought to units of 2^-R, and the warps' rows.
+    const Own own(a);
+    const int q = warp >> 2, ch = FBLA_POS::tid() & 127, x_per = (own.row.exact + own.ctas - 1) / own.ctas;
+    const int x0 = min(own.row.exact, own.rank * x_per), x1 = min(own.row.exact, x0 + x_per), rows = wper ? (c_n + wper - 1) / wper : 0;
+    const float Rq = __shfl_sync(FULL, R, q % QG);
+    float o = 0.f, l = 0.f;
+    if (q < QG)
+      for (int x = x0; x < x1; ++x) {
+        const float *const row = via.window(x) + q * PSTRIDE;
+        const float e = ex2(row[D] - Rq);
+        o = fmaf(e, row[ch], o);
+        l = fmaf(e, row[D + 1], l);
+      }
+    __syncthreads();
+    if (q < QG) {
+#pragma unroll 4
+      for (int x = 0; x < rows; ++x) o += ws[x].stage[q][ch];
+      via.put(q, ch, o);
+      if (ch == 0) {
+#pragma unroll 4
+        for (int x = 0; x < rows; ++x) l += ws[x].stage[q][D];
+        via.put(q, D, l);
+      }
+    }
+    return;
+  }
   if (lane == 0) {
-    sm.stage_vh[warp][0] = first_vh;
-    sm.stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
+    stage_vh[warp][0] = first_vh;
+    stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
   // rows of heads that may continue in neighbouring warps, added in warp order: a head by four warps, 16 bytes a thread. (By its first
   // warp alone the rows of sixteen warps took 5 us: 8 x 16K 4+2 70.5 -> 63.0 us, 1 x 12K 24.1 -> 21.3.)
-  const Runs runs(sm.stage_vh, VALUE_WARPS, lane);
+  const Runs runs(stage_vh, VALUE_WARPS, lane);
   const int t = FBLA_POS::tid() & 127, quad = FBLA_POS::tid() >> 7;
   uint64_t left = (uint64_t)runs.mask1 << 32 | runs.mask0;
 #pragma unroll 1
@@ -819,14 +962,14 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     left &= left - 1;
     if (k % (VALUE_WARPS / 4) != quad) continue;
     const int n = runs.length(x, r);
-    float *const dst = value_row(a, cta + sm.stage_vh[x][r]);
-    const float *src = r ? reinterpret_cast<const float *>(sm.w[x].run) : &sm.w[x].stage[0][0];
+    float *const dst = value_row(a, cta + stage_vh[x][r]);
+    const float *src = r ? reinterpret_cast<const float *>(ws[x].run) : &ws[x].stage[0][0];
     const int at = (t >> 5) * PSTRIDE + 4 * (t & 31);  // query t / 32, channels 4 (t % 32) ..
     if (t < 32 * QG) {
       float4 s = *reinterpret_cast<const float4 *>(src + at);
 #pragma unroll 4
       for (int y = 1; y < n; ++y) {
-        const float4 z = *reinterpret_cast<const float4 *>(&sm.w[x + y].stage[0][0] + at);
+        const float4 z = *reinterpret_cast<const float4 *>(&ws[x + y].stage[0][0] + at);
         s.x += z.x; s.y += z.y; s.z += z.z; s.w += z.w;
       }
       *reinterpret_cast<float4 *>(dst + at) = s;
@@ -834,23 +977,48 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
     if (t < QG) {
       float s = src[t * PSTRIDE + D];
 #pragma unroll 4
-      for (int y = 1; y < n; ++y) s += sm.w[x + y].stage[t][D];
+      for (int y = 1; y < n; ++y) s += ws[x + y].stage[t][D];
       dst[t * PSTRIDE + D] = s;
     }
+  }
+}
+
+template <int CB, int FB, int QG, bool HEAD = false>
+__device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem_raw) {
+  allow_next_pass();
+  if constexpr (HEAD) {  // (a plan's items only: the stream call's kernel is head_passes)
+    value_units<CB, FB, QG, true>(a, reinterpret_cast<HeadValueSmem *>(smem_raw)->w, nullptr, nullptr, ScratchVia<QG>(a), [] {});
+  } else {
+    ValueSmem &sm = *reinterpret_cast<ValueSmem *>(smem_raw);
+    build_table(a, sm.table, 32 * VALUE_WARPS);
+    if (a.phase != 0) wait_previous_pass();  // (a whole decode: the score pass let this one begin when all before the call was complete)
+    value_units<CB, FB, QG, false>(a, sm.w, sm.stage_vh, &sm.table, NoVia(), [&] { if (a.phase == 0) wait_previous_pass(); });
   }
 }
 
 // ---- merge: out = (sum 2^(m_x - R) o_x + sum o_v) / (sum 2^(m_x - R) l_x + sum l_v), BF16 -----------------------------------
 // One CTA of four warps per output row: warp s sums rows s, s + 4, ... of the head's window and value rows, lane c channels
 // 4 c .. 4 c + 3; the four sums are added in order.
+// the same where the head has CTAs of its own: thread ch of 128 adds their sums(cta, channel or D for l)
+template <class Sum> __device__ __forceinline__ void write_row(const fbla_k_decode &a, int vh, int qi, int ch, int ctas, Sum sums) {
+  float o = 0.f, l = 0.f;
+#pragma unroll 4
+  for (int i = 0; i < ctas; ++i) { o += sums(i, ch); l += sums(i, D); }
+  a.out[((size_t)vh * a.qg + qi) * D + ch] = f32_to_bf16(__fdividef(o, l));  // (the row of query qi of virtual head vh)
+}
 template <int QG>
 __device__ __forceinline__ void gather_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   __shared__ float4 so[4][32];
   __shared__ float sl[4];
   const int vh = FBLA_POS::x() / QG, qi = FBLA_POS::x() % QG, lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5;
-  const int hpr = a.kv_heads * a.vg, b = vh / hpr, hir = vh - b * hpr;
   allow_next_pass();
   wait_previous_pass();
+  if (a.head_ctas) {
+    const ScratchVia<QG> via(a, vh);
+    write_row(a, vh, qi, FBLA_POS::tid(), a.head_ctas, [&](int cta, int ch) { return via.sum(cta, qi, ch); });
+    return;
+  }
+  const int hpr = a.kv_heads * a.vg, b = vh / hpr, hir = vh - b * hpr;
   const int *t = table_of(a);
   const Rows r = rows_of<QG>(a, t, t + a.batch + 1, hpr, vh);
   // (a head without closed groups was nobody's in the value pass)
@@ -894,6 +1062,49 @@ __device__ __forceinline__ void gather_item(const fbla_k_decode &a, uint8_t *sme
   } else {
     a.out[row * D + ch] = failed ? (uint16_t)0x7fc0 : f32_to_bf16(__fdividef(Os, Ls));
   }
+}
+// ---- a short decode: all passes in one kernel -----------------------------------------------------------------------------------
+// A cluster of a.head_ctas CTAs per virtual head does the head's scores, values and output rows: the same code as a plan's passes, hence the
+// same bits, with the cluster's barrier in the place of a kernel boundary and masses and sums stored into the shared memory of the CTAs
+// that read them.
+struct __align__(16) HeadSmem {
+  HeadScoreSmem s;
+  HeadValueSmem v;  // (beside the scores': the first values are asked for before the cluster meets)
+  float2 mass[16][4];  // [CTA][query]
+  // in the scores' place once all CTAs have theirs: a window sub-block's row over its warp's V rows, the CTAs' sums over the queries
+  __device__ __forceinline__ float *window(int warp) { return reinterpret_cast<float *>(&s.w[warp].exact.v[0][0]); }
+  __device__ __forceinline__ float *sums(int slot) { return reinterpret_cast<float *>(&s.w[slot].exact.q[0][0]); }
+};
+static_assert(sizeof(HeadSmem) <= 227 * 1024, "one CTA's shared memory");
+static_assert(SCORE_WARPS == 16 && VALUE_WARPS == 16, "one CTA runs both passes; at most sixteen CTAs of a head");
+static_assert(sizeof(ExactWarp::v) >= 4 * PSTRIDE * sizeof(float) && sizeof(ExactWarp::q) >= PSTRIDE * sizeof(float) && sizeof(ExactWarp::q) >= sizeof(ScoreWarp::s),
+              "a window sub-block's row beside the warp's later queries and P bytes");
+template <int QG> struct ClusterVia {
+  HeadSmem &sm;
+  int ctas, rank, x0;  // x0: the first of the CTA's window sub-blocks
+  __device__ __forceinline__ void ready() const { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }  // (every CTA has begun)
+  __device__ __forceinline__ float *window(int x) const { return sm.window(x - x0); }
+  __device__ __forceinline__ void put_mass(float2 mass, int lane) const {
+    for (int i = lane / QG; i < ctas; i += 32 / QG) st_remote2(remote(&sm.mass[rank][lane % QG], i), mass);
+  }
+  __device__ __forceinline__ float2 mass(int cta, int q) const { return sm.mass[cta][q]; }
+  // query q is CTA q % ctas's, its (q / ctas)-th
+  __device__ __forceinline__ void put(int q, int ch, float x) const { st_remote1(remote(sm.sums(q / ctas * ctas + rank) + ch, q % ctas), x); }
+};
+template <int CB, int FB, int QG>
+__device__ __forceinline__ void head_passes(const fbla_k_decode &a, uint8_t *smem_raw) {
+  HeadSmem &sm = *reinterpret_cast<HeadSmem *>(smem_raw);
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  wait_previous_pass();
+  allow_next_pass();
+  const Own own(a);
+  const int x_per = (own.row.exact + own.ctas - 1) / own.ctas;
+  const ClusterVia<QG> via{sm, own.ctas, own.rank, min(own.row.exact, own.rank * x_per)};
+  score_units<CB, FB, QG, true>(a, sm.s.w, sm.s.fold, nullptr, via);
+  value_units<CB, FB, QG, true>(a, sm.v.w, nullptr, nullptr, via, [] { cluster_meet(); });
+  cluster_meet();
+  const int quad = FBLA_POS::tid() >> 7, qi = own.rank + own.ctas * quad;
+  if (qi < QG) write_row(a, own.vh, qi, FBLA_POS::tid() & 127, own.ctas, [&](int cta, int ch) { return sm.sums(quad * own.ctas + cta)[ch]; });
 }
 
 }  // namespace dense

@@ -190,6 +190,8 @@ __device__ __forceinline__ float2 ld_remote2(uint32_t p) {
   asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void st_remote1(uint32_t p, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory"); }
+__device__ __forceinline__ void st_remote2(uint32_t p, float2 v) { asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" ::"r"(p), "f"(v.x), "f"(v.y) : "memory"); }
 __device__ __forceinline__ int ld_remote1(uint32_t p) {
   int v;
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");

@@ -58,7 +58,8 @@ typedef struct {
   short status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
   char fold;           // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
   char deep;           // the coarse pass's shape: 1: few warps with a whole group in flight each; 0: more warps (fbla_decode.cuh)
-  short dense;         // 1: two sweeps, weights kept between them (fbla_dense.cuh); 0: coarse sums, then corrections (fbla_decode.cuh)
+  char dense;          // 1: two sweeps, weights kept between them (fbla_dense.cuh); 0: coarse sums, then corrections (fbla_decode.cuh)
+  char head_ctas;      // two sweeps: n > 0: every virtual head has n CTAs of its own (coarse_ctas in all), in a stream call a cluster of one kernel; 0: the work is dealt over all CTAs
   short deal;          // how the coarse pass's warps share the work, FBLA_K_DEAL_*
 } fbla_k_decode;
 #define FBLA_K_DEAL_LENGTHS 0 /* a CTA's warps are split between windows and groups by the rows' lengths (short contexts) */
@@ -84,7 +85,9 @@ static inline __host__ __device__ size_t fbla_k_two_cells(size_t vheads, int nbl
 #define FBLA_K_TWO_FLOATS 11
 // whether a decode of rows of about `tokens` tokens with selection threshold tau runs in two sweeps (vheads: virtual heads of the call, qg queries each)
 FBLA_HOST_API(int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens, float tau);)
-// the dense passes (0 scores, 1 rows' masses, 2 values, 3 merge): a whole decode or shard phase; one pass
+// CTAs per virtual head of a decode in two sweeps that runs as one kernel; 0: it runs as three (pure host arithmetic)
+FBLA_HOST_API(int fbla_k_head_ctas(int vheads, long long tokens);)
+// the dense passes (0 scores, 1 rows' masses, 2 values, 3 merge): a whole decode or shard phase; one pass (of a decode in one kernel: 0 all of it)
 FBLA_HOST_API(cudaError_t fbla_k_dense_launch(const fbla_k_decode *a, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_dense_pass_launch(const fbla_k_decode *a, int pass, cudaStream_t stream);)
 // the same choice for a shape given by its numbers (pure host arithmetic: no device is touched): deal and fold as fbla_k_decode_split sets them

@@ -42,6 +42,60 @@ def test_heads_folded_inside_a_cta(ours, oracle, B, QH, KH, N):
         gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode)), f"{mode} {B} x {N}")
 
 
+# a cluster of 16, 10, 8, 6, 5, 4, 3, 2, 1 CTAs per head; CTAs without groups, without windows, with less and with more than a unit per warp
+OWN = [(1, 4, 1, 130, 16), (1, 2, 1, 385, 16), (2, 3, 3, 9000, 16), (2, 16, 4, 2600, 10), (3, 8, 4, 3001, 8), (3, 24, 6, 257, 6), (5, 10, 5, 2999, 5), (8, 16, 4, 1700, 4),
+       (9, 4, 4, 2049, 3), (9, 32, 4, 1500, 2), (16, 32, 8, 640, 1), (30, 8, 4, 2300, 1), (74, 4, 2, 17, 1)]
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("B,QH,KH,N,ctas", OWN)
+def test_heads_with_ctas_of_their_own(ours, oracle, mode, B, QH, KH, N, ctas):
+    q, k, v = datagen.baseline_case(11 + N, B, QH, KH, N)
+    qd = gu.bf16_tensor(q)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=N)
+    got = ours.decode(c, qd)
+    assert torch.equal(got, ours.decode_at(c, qd, torch.tensor([N], dtype=torch.int32, device="cuda")))
+    torch.cuda.synchronize()
+    gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode, capacity=N)), f"{mode} {B} x {N}")
+    assert ours.lib.fbla_k_head_ctas(B * KH * (QH // KH // gu_group(QH // KH)), ctypes.c_longlong(N)) == ctas
+    assert first_entry(ours, c, qd, mode, 0.0).endswith(", true>")
+
+
+def gu_group(ratio):
+    """queries per virtual head"""
+    return ratio if ratio in (1, 2, 4) else 4 if ratio % 4 == 0 else 2 if ratio % 2 == 0 else 1
+
+
+@pytest.mark.parametrize("B,QH,KH,N,ctas", [OWN[2], OWN[3], OWN[5], OWN[10]])
+def test_own_ctas_lengths_and_plans(ours, oracle, B, QH, KH, N, ctas):
+    """Rows shorter than the room (down to one token, no closed group), each against its own decode in a cache of the same room; the plan's
+    passes bit for bit the stream call, one CTA per item and as loops of three."""
+    mode, lens = "4+2", [max(1, N * i // B - 3 * i) for i in range(B)]
+    q, k, v = datagen.uneven_case(21, B, QH, KH, N)
+    qd = gu.bf16_tensor(q)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=N)
+    want = []
+    for b, n in enumerate(lens):
+        row = ours.encode(gu.bf16_tensor(k[b:b + 1, :, :n]), gu.bf16_tensor(v[b:b + 1, :, :n]), mode, capacity=N)
+        for key in ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v"):
+            c[key][b].copy_(row[key][0])
+        want.append(oracle.decode(q[b:b + 1], oracle.encode(k[b:b + 1, :, :n], v[b:b + 1, :, :n], mode, capacity=N)))
+    length, vp, passes = torch.tensor(lens, dtype=torch.int32, device="cuda"), ctypes.c_void_p, (iu.Items * 4)()
+    got = ours.decode_at(c, qd, length, length_stride=1)
+    torch.cuda.synchronize()
+    for b in range(B):
+        gu.check_close(gu.bits_of(got)[b:b + 1], want[b], f"row of {lens[b]}")
+    cfg, kc = gu.Config(B, QH, KH, 0, 0, 0, gu.FORMATS[mode][2], N, 0, 0, 0, 0, 1), ours._cache(c)
+    for loops in (None, 3):
+        scratch, out = ours.scratch(dict(c, tokens=N), QH), torch.empty_like(qd)
+        scratch.fill_(0xFF)
+        assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
+                                                   vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
+        iu.run_plan(ours.lib, passes, 4, torch.cuda.current_stream().cuda_stream, loops)
+        torch.cuda.synchronize()
+        assert torch.equal(out, got)
+
+
 @pytest.mark.parametrize("lens", [[1, 2000, 129, 16], [300] * 3 + [1], [256, 257, 4000, 255, 31]])
 def test_dense_ragged_rows(ours, oracle, lens):
     B, QH, KH, cap, mode = len(lens), 8, 2, 4096, "3+3"

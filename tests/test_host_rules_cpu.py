@@ -69,6 +69,20 @@ def test_two_sweeps_up_to_a_line(lib, qg):
     assert two(8, 4096, 3e-4) and two(512, 8192, 1e-3) and not two(8, 131072, 3e-4) and not two(8, 1 << 20, 1e-3)
 
 
+def test_short_rows_have_ctas_of_their_own_heads(lib):
+    """As many CTAs per head as let all clusters run at once, up to a number of groups each; longer rows are dealt over all CTAs."""
+    ctas = lambda vheads, tokens: lib.fbla_k_head_ctas(vheads, ctypes.c_longlong(tokens))  # noqa: E731
+    for vheads in list(range(1, 160)) + [1000]:
+        c = ctas(vheads, 1)
+        assert (c > 0) == (vheads <= 148) and c * vheads <= 148 and c <= 16
+        picks = [ctas(vheads, n) for n in range(1, 60000, 127)]
+        assert set(picks) <= {c, 0} and picks == sorted(picks, reverse=True)  # (one line)
+        if c:
+            line = 128 * c * (16 if c == 16 else 20)
+            assert ctas(vheads, line) == c and ctas(vheads, line + 1) == 0
+    assert [ctas(v, 1) for v in (1, 8, 15, 16, 26, 32, 45, 64, 148)] == [16, 10, 8, 6, 5, 4, 3, 2, 1]
+
+
 def test_the_shape_follows_the_groups_a_warp_streams(lib):
     """Eight warps with a whole group in flight where twelve would not leave a warp less than three quarters of the groups."""
     deep = lambda batch, heads, qg, tokens: lib.fbla_k_decode_deep_of(batch, heads, 1, qg, ctypes.c_longlong(tokens))  # noqa: E731
