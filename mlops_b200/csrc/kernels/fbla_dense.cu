@@ -48,7 +48,6 @@ template <int CB, int FB, int QG> struct Kernels {
     return e;
   }
   static cudaError_t whole(fbla_k_decode a, bool dependent, cudaStream_t stream) {
-    a.status = nullptr;  // (no wait of this kernel gives up)
     a.mass_given = 0;
     return launch(dependent, a.head_ctas, head_kernel<CB, FB, QG>, dim3(a.head_ctas, a.kv_heads * a.vg, a.batch), 32 * SCORE_WARPS, sizeof(HeadSmem), stream, a);
   }

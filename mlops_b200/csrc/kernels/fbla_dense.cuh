@@ -1097,6 +1097,7 @@ __device__ __forceinline__ void head_passes(const fbla_k_decode &a, uint8_t *sme
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   wait_previous_pass();
   allow_next_pass();
+  if (FBLA_POS::x() == 0 && FBLA_POS::y() == 0 && FBLA_POS::z() == 0 && FBLA_POS::tid() == 0 && a.status) { a.status[0] = 0; a.status[1] = 0; }  // (no wait here gives up)
   const Own own(a);
   const int x_per = (own.row.exact + own.ctas - 1) / own.ctas;
   const ClusterVia<QG> via{sm, own.ctas, own.rank, min(own.row.exact, own.rank * x_per)};
