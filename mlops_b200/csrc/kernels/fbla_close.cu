@@ -17,18 +17,18 @@ template <class K> cudaError_t pass_of(K kernel, int gx, int gy, int threads, si
 namespace fbla {
 template <int CB, int FB>
 __global__ void __launch_bounds__(CLOSE_THREADS, 2) close_kernel(const fbla_k_prefill a) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
+  extern __shared__ __align__(128) uint8_t smem_raw[];
   wait_previous_pass();
   allow_next_pass();
   close_item<CB, FB>(a, smem_raw);
 }
 
 template <int CB, int FB>
-__global__ void __launch_bounds__(CLOSE_THREADS, 2) write_kernel(const fbla_k_prefill a) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
+__global__ void __launch_bounds__(TENSOR_THREADS, 4) write_kernel(const fbla_k_prefill a, int blocks) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
   wait_previous_pass();
   allow_next_pass();
-  write_item<CB, FB>(a, smem_raw);
+  write_chunk<CB, FB>(a, smem_raw, blocks);
 }
 
 __global__ void __launch_bounds__(CLOSE_THREADS) finish_kernel(const fbla_k_prefill a) {
@@ -37,33 +37,38 @@ __global__ void __launch_bounds__(CLOSE_THREADS) finish_kernel(const fbla_k_pref
   finish_item(a, nullptr);
 }
 
-// the kernels' shared memory is above the default limit: asked for once per device and host thread
-static cudaError_t configure() {
-  static thread_local int configured[64] = {0};
-  int dev = 0;
+// the write kernels' shared memory is above the default limit: asked for once per device and host thread; *sms: the device's SMs
+static cudaError_t configure(int *sms) {
+  static thread_local int configured[64] = {0};  // (its SMs, once configured)
+  int dev = 0, n = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-  for (auto kernel : {close_kernel<3, 3>, close_kernel<4, 2>, write_kernel<3, 3>, write_kernel<4, 2>})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CloseSmem));
-  if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = 1;
+  if (dev >= 0 && dev < 64 && configured[dev]) { *sms = configured[dev]; return cudaSuccess; }
+  cudaError_t e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  for (auto kernel : {write_kernel<3, 3>, write_kernel<4, 2>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
+  if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = n;
+  *sms = n;
   return e;
 }
 }  // namespace fbla
 
 extern "C" cudaError_t fbla_k_close_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream) {
   if (close_blocks <= 0) return cudaSuccess;
-  const cudaError_t e = fbla::configure();
-  if (e != cudaSuccess) return e;
+  static_assert(2 * sizeof(fbla::CloseSmem) <= 48 * 1024, "within the default limit");
   const dim3 grid(close_blocks, a->batch * a->kv_heads);
-  return fbla::launch(true, 1, a->cb == 3 ? fbla::close_kernel<3, 3> : fbla::close_kernel<4, 2>, grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream, *a);
+  return fbla::launch(true, 1, a->cb == 3 ? fbla::close_kernel<3, 3> : fbla::close_kernel<4, 2>, grid, fbla::CLOSE_THREADS, 2 * sizeof(fbla::CloseSmem), stream, *a);
 }
 
 extern "C" cudaError_t fbla_k_write_launch(const fbla_k_prefill *a, int close_blocks, cudaStream_t stream) {
-  const cudaError_t e = fbla::configure();
+  int sms = 0;
+  const cudaError_t e = fbla::configure(&sms);
   if (e != cudaSuccess) return e;
-  const dim3 grid(close_blocks > 0 ? close_blocks : 1, a->batch * a->kv_heads);
-  return fbla::launch(true, 1, a->cb == 3 ? fbla::write_kernel<3, 3> : fbla::write_kernel<4, 2>, grid, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream, *a);
+  // as many CTAs as the SMs hold at once (four each), no more than there are units to close or to clear
+  const int blocks = close_blocks > 0 ? close_blocks : 1;
+  const long long heads = (long long)a->batch * a->kv_heads, units = 2 * blocks * heads;
+  const long long clear = a->clear_groups ? heads * (a->clear_groups - (a->count - 1) / fbla::G) : 0, work = units > clear ? units : clear;
+  const int ctas = (int)(work < 4 * sms ? work : 4 * sms);
+  return fbla::launch(true, 1, a->cb == 3 ? fbla::write_kernel<3, 3> : fbla::write_kernel<4, 2>, dim3(ctas), fbla::TENSOR_THREADS, sizeof(fbla::WriteSmem), stream, *a, blocks);
 }
 
 extern "C" cudaError_t fbla_k_finish_launch(const fbla_k_prefill *a, cudaStream_t stream) {
@@ -72,8 +77,8 @@ extern "C" cudaError_t fbla_k_finish_launch(const fbla_k_prefill *a, cudaStream_
 
 extern "C" cudaError_t fbla_k_close_pass(const fbla_k_prefill *a, int close_blocks, fbla_k_pass *info) {
   const int heads = a->batch * a->kv_heads;
-  if (a->cb == 3) return pass_of(fbla::close_kernel<3, 3>, close_blocks, heads, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), "fbla::close_item<3, 3>", info);
-  return pass_of(fbla::close_kernel<4, 2>, close_blocks, heads, fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), "fbla::close_item<4, 2>", info);
+  if (a->cb == 3) return pass_of(fbla::close_kernel<3, 3>, close_blocks, heads, fbla::CLOSE_THREADS, 2 * sizeof(fbla::CloseSmem), "fbla::close_item<3, 3>", info);
+  return pass_of(fbla::close_kernel<4, 2>, close_blocks, heads, fbla::CLOSE_THREADS, 2 * sizeof(fbla::CloseSmem), "fbla::close_item<4, 2>", info);
 }
 
 extern "C" cudaError_t fbla_k_finish_pass(const fbla_k_prefill *a, fbla_k_pass *info) {

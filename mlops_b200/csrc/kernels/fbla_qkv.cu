@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(CLOSE_THREADS) qkv_step_kernel(const fbla_k_pr
   const int bh = blockIdx.x;
   const Chunk ch = chunk_of(closing, bh / closing.kv_heads);
   const int g = closing_group(ch, 0);
-  if (g >= 0) close_group<CB, FB>(closing, *reinterpret_cast<CloseSmem *>(smem_raw), bh, g, ch.n0);
+  if (g >= 0) close_group<CB, FB>(closing, *reinterpret_cast<CloseSmem (*)[2]>(smem_raw), bh, g, ch.n0);
   qkv_token_item<NORM>(a, nullptr);
 }
 
@@ -43,11 +43,11 @@ template <int CB, int FB, bool NORM> static cudaError_t launch_step(const fbla_k
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(fbla::qkv_step_kernel<CB, FB, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(fbla::CloseSmem));
+    const cudaError_t e = cudaFuncSetAttribute(fbla::qkv_step_kernel<CB, FB, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)sizeof(fbla::CloseSmem));
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  return fbla::launch(true, 1, fbla::qkv_step_kernel<CB, FB, NORM>, dim3(a.batch * a.kv_heads), fbla::CLOSE_THREADS, sizeof(fbla::CloseSmem), stream, closing, a);
+  return fbla::launch(true, 1, fbla::qkv_step_kernel<CB, FB, NORM>, dim3(a.batch * a.kv_heads), fbla::CLOSE_THREADS, 2 * sizeof(fbla::CloseSmem), stream, closing, a);
 }
 extern "C" cudaError_t fbla_k_qkv_step_launch(const fbla_k_prefill *closing, const fbla_k_token *a, cudaStream_t stream) {
   if (closing->cb == 3) return a->q_norm ? launch_step<3, 3, true>(*closing, *a, stream) : launch_step<3, 3, false>(*closing, *a, stream);

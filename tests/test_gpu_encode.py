@@ -37,3 +37,25 @@ def test_encode_starts_an_empty_cache_only():
     cfg = _C._config(1, 1, 1, 5, 0, 256, 0.0, 0.0)
     assert _C.lib.mlops_fbla_encode(ctypes.byref(cfg), 1, c.open_k.data_ptr(), c.open_v.data_ptr(), ctypes.byref(kc), None) == _C.INVALID_VALUE
     assert "tokens has to be 0" in _C.last_error()
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("heads,n,n0", [(8, 12300, 0), (3, 40001, 0), (5, 9000, 77)])
+def test_many_units_per_cta(oracle, mode, heads, n, n0):
+    """More (group, tensor) units than CTAs: the later ones come through shared memory; a chunk that starts inside a group; channels whose
+    steps are subnormal, have a subnormal reciprocal, or none (a constant channel, a range beyond the largest float) beside ordinary ones."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    scale = 2.0 ** torch.randint(-12, 3, (1, heads, 1, 128), generator=gen, device="cuda").double()
+    scale[..., 3], scale[..., 50], scale[..., 90], scale[..., 127] = 2.0 ** -131, 2.0 ** -124, 2.0 ** 124, 2.0 ** 127
+    k, v = ((torch.randn((1, heads, n0 + n, 128), generator=gen, device="cuda").clamp(-1.9, 1.9).double() * scale).to(torch.bfloat16) for _ in range(2))
+    k[..., 17], v[..., 18] = 0.5, 0.0
+    c = attention.empty(1, heads, n0 + n + 300, mode)
+    if n0:
+        attention.append(c, k[:, :, :n0], v[:, :, :n0])
+    attention.append(c, k[:, :, n0:], v[:, :, n0:])
+    bits = lambda x: x.view(torch.int16).cpu().numpy().view("uint16")  # noqa: E731
+    want = oracle.encode(bits(k), bits(v), mode, capacity=n0 + n + 300)
+    for a in ARRAYS:
+        x, y = getattr(c, a).view(torch.uint8).cpu().numpy().reshape(-1), want[a].view("uint8").reshape(-1)
+        assert x.size == y.size and (x == y).all(), a
