@@ -180,10 +180,11 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   a.qg = queries_per_virtual_head(ratio);
   a.vg = ratio / a.qg;
   // the refine pass keeps one prefix entry per (virtual head, slice of 16 384 tokens) in shared memory
-  const long long entries = (long long)c->batch * c->kv_heads * a.vg * m.nslices, entry_limit = fbla_k_refine_entry_limit(a.cb);
+  const long long entries = (long long)c->batch * c->kv_heads * a.vg * m.nslices, entry_limit = fbla_k_refine_entry_limit(a.cb, 0);
   if (entries > entry_limit)
     return refuse(fn, "batch * kv_heads * virtual heads * slices of 16384 tokens = %lld is more than the %lld one call handles: split the batch",
                   entries, entry_limit);
+  a.refine_fold = entries <= fbla_k_refine_entry_limit(a.cb, 1);
   a.c = kernel_cache(k);
   a.q = q;
   a.out = out;
@@ -226,7 +227,6 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   return MLOPS_FBLA_OK;
 }
 mlops_fbla_status enqueue_decode(const char *fn, fbla_k_decode &a, cudaStream_t stream) {
-  a.status_cleared = 1;  // the launcher zeroes the status word on the stream, ahead of the first pass
   const cudaError_t e = fbla_k_decode_launch(&a, stream);
   return e == cudaSuccess ? accepted() : device_failure(fn, e);
 }
@@ -609,12 +609,10 @@ mlops_fbla_status mlops_fbla_shard_step(const mlops_fbla_config *c, const mlops_
   sum_pass = mass_pass;
   mass_pass.phase = 1;  // coarse pass; the rows' local masses
   mass_pass.row_r = reinterpret_cast<float *>(own + M.local_mass);
-  mass_pass.status_cleared = 1;
   sum_pass.mass_given = 1;
   sum_pass.phase = 2;   // select with the common masses, refine, the shard's sums
   sum_pass.row_r = reinterpret_cast<float *>(own + M.total);
   sum_pass.out_partial = reinterpret_cast<float *>(own + M.local_part);
-  sum_pass.status_cleared = 1;
   cudaError_t e = fbla_k_decode_launch(&mass_pass, stream);
   if (e == cudaSuccess) e = fbla_k_link_push_mass(&L, stream);
   if (e == cudaSuccess) e = fbla_k_link_gather_mass(&L, stream);

@@ -48,10 +48,13 @@ template <int CB, int FB, int QG> CoarseBuild coarse_build(int deal, int deep) {
   return deep ? coarse_build<CB, FB, QG, DEEP>(deal) : coarse_build<CB, FB, QG, WIDE>(deal);
 }
 
-constexpr int REFINE_SMEM_MAX = 220 * 1024;  // dynamic shared memory of the refine pass (its ring + the slice prefix)
+constexpr int REFINE_SMEM_MAX = 220 * 1024;  // dynamic shared memory of the refine pass (its ring + the slice prefix + the first heads' row sets)
+template <int CB, int FB> size_t refine_smem(const fbla_k_decode &a) {
+  return (sizeof(RefineWarp<CB, FB>) + (a.refine_fold ? REFINE_SET_BYTES : 0)) * RefineShape<CB, FB>::WARPS + refine_prefix_bytes((size_t)a.batch * a.kv_heads * a.vg * a.nslices);
+}
 template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a, cudaStream_t stream) {
   const int vheads = a.batch * a.kv_heads * a.vg;
-  const size_t rsm = sizeof(RefineWarp<CB, FB>) * RefineShape<CB, FB>::WARPS + sizeof(int) * ((size_t)vheads * a.nslices + 1);
+  const size_t rsm = refine_smem<CB, FB>(a);
   static thread_local int configured[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -69,15 +72,9 @@ template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a,
   }
   if (rsm > REFINE_SMEM_MAX) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
-  if (a.status_cleared && a.phase != 2) {  // ordered before every report of this call (a bounded wait that gives up); a shard's second
-                                           // phase keeps what its first phase may have reported
-    e = cudaMemsetAsync(a.status, 0, 16, stream);
-    if (e != cudaSuccess) return e;
-  }
   if (a.phase != 2) {
     const CoarseBuild c = coarse_build<CB, FB, QG>(a.deal, a.deep);
-    c.kernel<<<a.coarse_ctas, c.threads, c.smem, stream>>>(a);
-    e = cudaGetLastError();
+    e = launch(true, 1, c.kernel, dim3(a.coarse_ctas), c.threads, c.smem, stream, a);
     if (e == cudaSuccess) e = launch(true, 1, select_kernel<QG>, dim3(a.phase == 1 ? 1 : a.nslices, vheads), 256, 0, stream, a);
     if (a.phase == 1) return e;
   } else {
@@ -92,7 +89,7 @@ template <int CB, int FB, int QG> cudaError_t launch_all(const fbla_k_decode &a,
 // one pass alone, as an ordinary launch (no overlap with its neighbours): for measurements pass by pass
 template <int CB, int FB, int QG> cudaError_t launch_one(const fbla_k_decode &a, int pass, cudaStream_t stream) {
   const int vheads = a.batch * a.kv_heads * a.vg;
-  const size_t rsm = sizeof(RefineWarp<CB, FB>) * RefineShape<CB, FB>::WARPS + sizeof(int) * ((size_t)vheads * a.nslices + 1);
+  const size_t rsm = refine_smem<CB, FB>(a);
   if (rsm > REFINE_SMEM_MAX) return cudaErrorInvalidValue;
   switch (pass) {
     case 0: {
@@ -110,7 +107,7 @@ template <int CB, int FB, int QG> cudaError_t launch_one(const fbla_k_decode &a,
 
 template <int CB, int FB, int QG> cudaError_t passes_of(const fbla_k_decode &a, fbla_k_pass *p) {
   const int vheads = a.batch * a.kv_heads * a.vg;
-  const size_t rsm = sizeof(RefineWarp<CB, FB>) * RefineShape<CB, FB>::WARPS + sizeof(int) * ((size_t)vheads * a.nslices + 1) + 128;
+  const size_t rsm = refine_smem<CB, FB>(a) + 128;
   if (rsm - 128 > REFINE_SMEM_MAX) return cudaErrorInvalidValue;
   char e[96];
   const CoarseBuild c = coarse_build<CB, FB, QG>(a.deal, a.deep);
@@ -154,10 +151,12 @@ extern "C" cudaError_t fbla_k_combine_launch(const float *partial, uint16_t *out
   return cudaGetLastError();
 }
 
-extern "C" long long fbla_k_refine_entry_limit(int cb) {
+extern "C" long long fbla_k_refine_entry_limit(int cb, int fold) {
   using namespace fbla;
   const size_t ring = cb == 3 ? sizeof(RefineWarp<3, 3>) * RefineShape<3, 3>::WARPS : sizeof(RefineWarp<4, 2>) * RefineShape<4, 2>::WARPS;
-  return (long long)((REFINE_SMEM_MAX - ring) / sizeof(int)) - 1;
+  const size_t sets = fold ? REFINE_SET_BYTES * RefineShape<4, 2>::WARPS : 0;
+  static_assert(REFINE_SMEM_MAX % 16 == 0 && REFINE_SET_BYTES % 16 == 0 && sizeof(RefineWarp<3, 3>) % 16 == 0 && sizeof(RefineWarp<4, 2>) % 16 == 0, "the prefix may fill its room");
+  return (long long)((REFINE_SMEM_MAX - ring - sets) / sizeof(int)) - 1;
 }
 
 extern "C" cudaError_t fbla_k_decode_shape(fbla_k_decode *a) {

@@ -154,9 +154,8 @@ template <int CB, int SHAPE> struct __align__(128) StreamWarp {
   uint64_t bar_pair[Sh::NP], bar_meta[2];
   // The partial rows of the first and the last virtual head of the warp's run, which neighbouring warps of the CTA may
   // share: they are folded into one row per (CTA, virtual head) before they leave the CTA. stage_vh: the rows' virtual
-  // heads (-1: no such row).
+  // heads (-1: no such row) are kept beside.
   __align__(16) float stage[2][4][FBLA_K_PSTRIDE];
-  int stage_vh[2];
 };
 struct __align__(16) ExactWarp {
   uint16_t q[8][D + 8];   // the virtual head's queries in BF16 (rows >= QG: zero); rows 272 bytes apart: 16-byte aligned, conflict-free
@@ -585,29 +584,76 @@ template <int QG> __device__ __forceinline__ void write_partial(float *p, const 
 }
 
 
-// dst (scratch) = the staged row set `own` merged with the first staged row sets of the next `more` warps (`next` points at
-// the first of them, the following ones lie one StreamWarp further each): per query the usual log-sum-exp merge of
-// (m, l, o[128]), taken in warp order. Lane l owns channels 4 l .. 4 l + 3.
-template <int QG>
-__device__ __forceinline__ void fold_rows(float *dst, const float *own, const float *next, int more, int lane, size_t warp_stride_floats) {
-#pragma unroll
-  for (int qi = 0; qi < QG; ++qi) {
-    const float *p = own + qi * PSTRIDE;
-    float4 o = *reinterpret_cast<const float4 *>(p + 4 * lane);
-    float m = p[D], l = p[D + 1];
-    for (int x = 0; x < more; ++x) {
-      const float *n = next + (size_t)x * warp_stride_floats + qi * PSTRIDE;
-      const float4 o2 = *reinterpret_cast<const float4 *>(n + 4 * lane);
-      const float m2 = n[D], l2 = n[D + 1];
-      const float mn = fmaxf(m, m2), sa = ex2(m - mn), sb = ex2(m2 - mn);
-      o.x = fmaf(o.x, sa, o2.x * sb); o.y = fmaf(o.y, sa, o2.y * sb); o.z = fmaf(o.z, sa, o2.z * sb); o.w = fmaf(o.w, sa, o2.w * sb);
-      l = fmaf(l, sa, l2 * sb);
-      m = mn;
-    }
-    float *d = dst + qi * PSTRIDE;
-    *reinterpret_cast<float4 *>(d + 4 * lane) = o;
-    if (lane == 0) { d[D] = m; d[D + 1] = l; }
+// ---- rows of heads that several warps of a CTA hold -------------------------------------------------------------------------
+// The heads whose rows the CTA's warps have left: warp x's run of work is the end of vh[x][0] (all of it if vh[x][1] < 0) and, behind
+// heads of its own, the beginning of vh[x][1]; -1: none (idle warps lie before or behind the others). A head is folded into one row.
+struct Runs {
+  int first, last;   // of warp `lane`
+  uint32_t mask0, mask1;  // bit x: warp x is the first of the head in vh[x][0], vh[x][1]
+  __device__ __forceinline__ Runs(const int (*vh)[2], int warps, int lane) {
+    first = lane < warps ? vh[lane][0] : -1;
+    last = lane < warps ? vh[lane][1] : -1;
+    const int before = __shfl_up_sync(FULL, last >= 0 ? last : first, 1);
+    mask0 = __ballot_sync(FULL, first >= 0 && (lane == 0 || before != first));
+    mask1 = __ballot_sync(FULL, last >= 0);
   }
+  // the warps, from x on, that hold rows of the head in vh[x][r] (the same x and r in every lane)
+  __device__ __forceinline__ int length(int x, int r) const {
+    const int lane = FBLA_POS::tid() & 31, f = __shfl_sync(FULL, first, x), l = __shfl_sync(FULL, last, x);
+    const uint32_t more = __ballot_sync(FULL, lane > x && first == (r ? l : f));
+    return 1 + (r == 0 && l >= 0 ? 0 : __popc(more));
+  }
+};
+
+// f(x, r, n, t) for every head that this thread's quad of warps folds (of `quads`; all their threads are here): rows of the head in
+// vh[x][r], held by the n warps from x on; t: the thread among 128. (The head's first warp alone, warp after warp, took 2 to 5 us.)
+template <class F> __device__ __forceinline__ void fold_heads(const int (*vh)[2], int warps, int quads, F f) {
+  const Runs runs(vh, warps, FBLA_POS::tid() & 31);
+  uint64_t left = (uint64_t)runs.mask1 << 32 | runs.mask0;
+#pragma unroll 1
+  for (int k = 0; left; ++k) {
+    const int bit = __ffsll((long long)left) - 1, r = bit >> 5, x = bit & 31;
+    left &= left - 1;
+    if (k % quads == FBLA_POS::tid() >> 7) f(x, r, runs.length(x, r), FBLA_POS::tid() & 127);
+  }
+}
+// dst = the n row sets row(0 ..) in shared memory, added in order: sums in the same units, (o, l). Thread t of 128: query t / 32, channels 4 (t % 32) ..
+template <int QG, class RowOf> __device__ __forceinline__ void add_sets(float *dst, int n, int t, RowOf row) {
+  const int at = (t >> 5) * PSTRIDE + 4 * (t & 31);
+  if (t < 32 * QG) {
+    float4 s = *reinterpret_cast<const float4 *>(row(0) + at);
+#pragma unroll 4
+    for (int y = 1; y < n; ++y) {
+      const float4 z = *reinterpret_cast<const float4 *>(row(y) + at);
+      s.x += z.x; s.y += z.y; s.z += z.z; s.w += z.w;
+    }
+    *reinterpret_cast<float4 *>(dst + at) = s;
+  }
+  if (t < QG) {
+    float s = row(0)[t * PSTRIDE + D];
+#pragma unroll 4
+    for (int y = 1; y < n; ++y) s += row(y)[t * PSTRIDE + D];
+    dst[t * PSTRIDE + D] = s;
+  }
+}
+// the same of running softmax sums (m, l, o): brought to the largest m first
+template <int QG, class RowOf> __device__ __forceinline__ void merge_sets(float *dst, int n, int t, RowOf row) {
+  const int at = (t >> 5) * PSTRIDE, c = 4 * (t & 31);
+  if (t >= 32 * QG) return;
+  float m = row(0)[at + D], l = 0.f;
+#pragma unroll 4
+  for (int y = 1; y < n; ++y) m = fmaxf(m, row(y)[at + D]);
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int y = 0; y < n; ++y) {
+    const float *p = row(y) + at;
+    const float4 z = *reinterpret_cast<const float4 *>(p + c);
+    const float e = ex2(p[D] - m);
+    o.x = fmaf(e, z.x, o.x); o.y = fmaf(e, z.y, o.y); o.z = fmaf(e, z.z, o.z); o.w = fmaf(e, z.w, o.w);
+    l = fmaf(e, p[D + 1], l);
+  }
+  *reinterpret_cast<float4 *>(dst + at + c) = o;
+  if (c == 0) { dst[at + D] = m; dst[at + D + 1] = l; }
 }
 
 // DEAL: how the work is dealt to the warps (FBLA_K_DEAL_*, the host's choice in fbla_k_decode::deal; one build per way, so
@@ -615,11 +661,12 @@ __device__ __forceinline__ void fold_rows(float *dst, const float *own, const fl
 template <int CB, int FB, int QG, int DEAL, int SHAPE = WIDE>
 __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   using Sh = CoarseShape<CB, SHAPE>;
-  allow_next_pass();
+  wait_previous_pass();  // (lengths, queries and the cache may come from the kernel before)
+  allow_next_pass();     // (behind the wait: the later passes then find everything before this call complete)
   smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;  // (an executor's storage is 16-byte aligned; an offset keeps the pointer's address space known)
   CoarseSmem<CB, SHAPE> &sm = *reinterpret_cast<CoarseSmem<CB, SHAPE> *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5;
-  if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status && !a.status_cleared) { a.status[0] = 0; a.status[1] = 0; }
+  if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status) { a.status[0] = 0; a.status[1] = 0; }
   const int hpr = a.kv_heads * a.vg;
   int sw = Sh::TOTAL;                 // streaming warps of this CTA
   long long gw, lo, hi;               // the warp's index among the grid's streaming warps and its run of the flattened groups
@@ -669,6 +716,7 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
   // of virtual heads that lie wholly inside the warp's run go straight to the scratch; the run's first and last virtual
   // head may continue in the neighbouring warps, so their rows are staged in shared memory and folded below, in warp order
   // (a fixed order: the result is reproducible bit for bit). Otherwise: one row per (warp, virtual head), slot gw + vh.
+  __shared__ int stage_vh[Sh::TOTAL][2];
   const int cta = FBLA_POS::x();
   int first_vh = -1, cur_vh = -1;
   bool ok = true;
@@ -709,34 +757,15 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
   }
   if (ok) retire();  // (after a wait that gave up a copy may still be in flight: the barriers stay as they are)
   if (lane == 0) {
-    w.stage_vh[0] = ok ? first_vh : -1;
-    w.stage_vh[1] = ok && cur_vh != first_vh ? cur_vh : -1;
+    stage_vh[warp][0] = ok ? first_vh : -1;
+    stage_vh[warp][1] = ok && cur_vh != first_vh ? cur_vh : -1;
   }
   // every streaming warp of the CTA has staged its rows
   asm volatile("bar.sync 1, %0;" ::"r"(32 * sw) : "memory");
-  // Row r of this warp is folded here unless an earlier warp does it: the first row belongs to the first warp that
-  // touched its virtual head, the last row (a later virtual head) always to this warp. The rows that continue it are
-  // the first rows of the following warps, as long as those warps stay inside the same virtual head.
-#pragma unroll 1
-  for (int r = 0; r < 2; ++r) {
-    const int v = w.stage_vh[r];
-    if (v < 0) continue;
-    if (r == 0 && warp > 0) {
-      const StreamWarp<CB, SHAPE> &prev = sm.w[warp - 1];
-      const int prev_last = prev.stage_vh[1] >= 0 ? prev.stage_vh[1] : prev.stage_vh[0];
-      if (prev_last == v) continue;
-    }
-    if (r == 0 && w.stage_vh[1] >= 0) {  // the virtual head ends inside this warp's run: nothing to fold
-      fold_rows<QG>(a.part + (size_t)(cta + v) * QG * PSTRIDE, &w.stage[0][0][0], nullptr, 0, lane, 0);
-      continue;
-    }
-    int more = 0;
-    for (int x = warp + 1; x < sw && sm.w[x].stage_vh[0] == v; ++x) {
-      ++more;
-      if (sm.w[x].stage_vh[1] >= 0) break;
-    }
-    fold_rows<QG>(a.part + (size_t)(cta + v) * QG * PSTRIDE, &w.stage[r][0][0], warp + 1 < sw ? &sm.w[warp + 1].stage[0][0][0] : nullptr, more, lane, sizeof(w) / sizeof(float));
-  }
+  if (warp >= sw / 4 * 4) return;  // (folded by quads of warps)
+  fold_heads(stage_vh, sw, sw / 4, [&](int x, int r, int n, int t) {
+    merge_sets<QG>(a.part + (size_t)(cta + stage_vh[x][r]) * QG * PSTRIDE, n, t, [&](int y) { return &sm.w[x + y].stage[y ? 0 : r][0][0]; });
+  });
 }
 
 // ---- which partial slots belong to a virtual head ------------------------------------------------------------------------
@@ -874,51 +903,19 @@ template <int CB, int FB> struct __align__(128) RefineWarp {
   uint8_t pst[128];  // rows 0..3: P under the full scores, rows 4..7: under the coarse scores; 16 tokens each
   uint64_t bar[RefineShape<CB, FB>::NST];
 };
+// behind the warps: the prefix of `entries` counts; with a.refine_fold, per warp the row set of its run's first virtual head (the last one's:
+// in the ring, at the end)
+__host__ __device__ constexpr size_t refine_prefix_bytes(size_t entries) { return (sizeof(int) * (entries + 1) + 15) / 16 * 16; }
+constexpr size_t REFINE_SET_BYTES = 4 * FBLA_K_PSTRIDE * sizeof(float);
 
+// The items [lo, hi) of one warp; the heads' row sets to dpart, slot `slot` + head, but with `first` given: the first head's (first_vh) there, the
+// last one's, if it is another (last_vh, else -1), in w.stage. False: a wait gave up.
 template <int CB, int FB, int QG>
-__device__ __forceinline__ void refine_item(const fbla_k_decode &a, uint8_t *smem_raw) {
+__device__ __forceinline__ bool refine_run(const fbla_k_decode &a, RefineWarp<CB, FB> &w, const int *pre, int entries, int lo, int hi, int slot, float *first, int &first_vh, int &last_vh) {
   using Sh = RefineShape<CB, FB>;
   constexpr float HOFF = .5f * ((1 << FB) - 1);
-  smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;  // (an executor's storage is 16-byte aligned; an offset keeps the pointer's address space known)
-  RefineWarp<CB, FB> *ws = reinterpret_cast<RefineWarp<CB, FB> *>(smem_raw);
-  int *pre = reinterpret_cast<int *>(smem_raw + sizeof(RefineWarp<CB, FB>) * Sh::WARPS);  // [entries + 1]
-  __shared__ int chunk_sum[256];
-  const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
-  const int hpr = a.kv_heads * a.vg, vheads = a.batch * hpr, entries = vheads * a.nslices;
-  allow_next_pass();
-  wait_previous_pass();
-  // exclusive prefix of the slices' counts: pre[e], e = vh * nslices + slice
-  {
-    const int per = (entries + 255) / 256, e0 = FBLA_POS::tid() * per, e1 = min(entries, e0 + per);
-    int sum = 0;
-    for (int e = e0; e < e1; ++e) sum += __ldcg(a.counts + e);
-    if (FBLA_POS::tid() < 256) chunk_sum[FBLA_POS::tid()] = sum;  // (threads past 256 own no entries)
-    __syncthreads();
-    if (warp == 0) {
-      int run = 0;
-      for (int i0 = 0; i0 < 256; i0 += 32) {
-        const int v = chunk_sum[i0 + lane];
-        int x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(FULL, x, o); x += lane >= o ? y : 0; }
-        chunk_sum[i0 + lane] = run + x - v;
-        run += __shfl_sync(FULL, x, 31);
-      }
-      if (!lane) pre[entries] = run;
-    }
-    __syncthreads();
-    int acc = FBLA_POS::tid() < 256 ? chunk_sum[FBLA_POS::tid()] : 0;
-    for (int e = e0; e < e1; ++e) { pre[e] = acc; acc += __ldcg(a.counts + e); }
-    __syncthreads();
-    if (FBLA_POS::x() == 0)  // for the merge: the first item of every virtual head, and the total
-      for (int v = FBLA_POS::tid(); v <= vheads; v += 32 * Sh::WARPS) a.item_off[v] = pre[v * a.nslices];
-  }
-  const int total = pre[entries];
-  const long long rw = (long long)FBLA_POS::nx() * Sh::WARPS;
-  const int per = (int)ceil_div(total, rw), gw = FBLA_POS::x() * Sh::WARPS + warp;
-  const int lo = gw * per, hi = min(total, lo + per);
-  if (lo >= hi) return;
-  RefineWarp<CB, FB> &w = ws[warp];
+  const int lane = FBLA_POS::tid() & 31, gid = lane >> 2, tig = lane & 3, hpr = a.kv_heads * a.vg;
+  static_assert(sizeof(w.stage) >= 4 * PSTRIDE * sizeof(float), "a row set fits the ring");
   for (int i = lane; i < (int)sizeof(w.qst) / 4; i += 32) reinterpret_cast<uint32_t *>(w.qst)[i] = 0u;
   reinterpret_cast<uint32_t *>(w.pst)[lane] = 0u;
   if (lane == 0) {
@@ -996,7 +993,8 @@ __device__ __forceinline__ void refine_item(const fbla_k_decode &a, uint8_t *sme
     int ce;
     const int it = item_at(k, ce), vh = ce / a.nslices, sb = it >> 4;
     if (vh != cur_vh) {
-      if (cur_vh >= 0) write_partial<QG>(a.dpart + (size_t)(gw + cur_vh) * QG * PSTRIDE, run, lane, true);
+      if (cur_vh >= 0) write_partial<QG>(first && cur_vh == first_vh ? first : a.dpart + (size_t)(slot + cur_vh) * QG * PSTRIDE, run, lane, true);
+      else first_vh = vh;
       cur_vh = vh; cur_unit = -1;
       reset<QG>(run);
       const int b = vh / hpr, hir = vh - b * hpr;
@@ -1009,10 +1007,7 @@ __device__ __forceinline__ void refine_item(const fbla_k_decode &a, uint8_t *sme
       for (int e = 0; e < 2; ++e) Rq[e] = query_valid<QG>(tig, e) ? __ldcg(a.row_r + vh * QG + 2 * (tig & 1) + e) : 0.f;
     }
     const bool ok = mbar_wait_bounded(&w.bar[s], ((k - lo) / Sh::NST) & 1);
-    if (!__all_sync(FULL, ok)) {
-      if (lane == 0) report(a, 3);
-      return;
-    }
+    if (!__all_sync(FULL, ok)) return false;
     const uint8_t *crec = w.stage[s], *frec = crec + Sh::RC;
     const long long unit = (long long)vh * a.nblocks + sb / SBG;
     if (unit != cur_unit2) { cur_unit2 = unit; cur_par ^= 1; }  // (the same sequence of groups as the issuing side)
@@ -1131,14 +1126,72 @@ __device__ __forceinline__ void refine_item(const fbla_k_decode &a, uint8_t *sme
       if (lane == 0) { fence_async_smem(); issue(ahead, ne, s); }
     }
   }
-  write_partial<QG>(a.dpart + (size_t)(gw + cur_vh) * QG * PSTRIDE, run, lane, true);
-  __syncwarp();
+  __syncwarp();  // (the last records have been read)
+  write_partial<QG>(!first ? a.dpart + (size_t)(slot + cur_vh) * QG * PSTRIDE : cur_vh == first_vh ? first : reinterpret_cast<float *>(w.stage), run, lane, true);
+  if (cur_vh != first_vh) last_vh = cur_vh;
   if (lane == 0) {  // (as the coarse pass: no live barrier is left behind for the CTA's next item)
 #pragma unroll
     for (int s = 0; s < Sh::NST; ++s) mbar_inval(&w.bar[s]);
   }
+  return true;
 }
 
+template <int CB, int FB, int QG>
+__device__ __forceinline__ void refine_item(const fbla_k_decode &a, uint8_t *smem_raw) {
+  using Sh = RefineShape<CB, FB>;
+  smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;  // (an executor's storage is 16-byte aligned; an offset keeps the pointer's address space known)
+  RefineWarp<CB, FB> *ws = reinterpret_cast<RefineWarp<CB, FB> *>(smem_raw);
+  int *pre = reinterpret_cast<int *>(smem_raw + sizeof(RefineWarp<CB, FB>) * Sh::WARPS);  // [entries + 1]
+  __shared__ int warp_sum[8], stage_vh[Sh::WARPS][2];
+  const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5;
+  const int hpr = a.kv_heads * a.vg, vheads = a.batch * hpr, entries = vheads * a.nslices;
+  allow_next_pass();
+  wait_previous_pass();
+  // exclusive prefix of the slices' counts: pre[e], e = vh * nslices + slice (256 threads, equal runs of entries)
+  {
+    const int per = (entries + 255) / 256, e0 = FBLA_POS::tid() * per, e1 = min(entries, e0 + per), head = e0 < e1 ? __ldcg(a.counts + e0) : 0;
+    int sum = head;
+    for (int e = e0 + 1; e < e1; ++e) sum += __ldcg(a.counts + e);
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(FULL, x, o); x += lane >= o ? y : 0; }
+    if (lane == 31 && warp < 8) warp_sum[warp] = x;
+    __syncthreads();
+    int acc = x - sum, all = 0;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) { if (v < warp) acc += warp_sum[v]; all += warp_sum[v]; }
+    for (int e = e0; e < e1; ++e) { pre[e] = acc; acc += e == e0 ? head : __ldcg(a.counts + e); }
+    if (FBLA_POS::tid() == 0) pre[entries] = all;
+    __syncthreads();
+    if (FBLA_POS::x() == 0)  // for the merge: the first item of every virtual head, and the total
+      for (int v = FBLA_POS::tid(); v <= vheads; v += 32 * Sh::WARPS) a.item_off[v] = pre[v * a.nslices];
+  }
+  const int total = pre[entries];
+  const long long rw = (long long)FBLA_POS::nx() * Sh::WARPS;
+  const int per = (int)ceil_div(total, rw), gw = FBLA_POS::x() * Sh::WARPS + warp;
+  const int lo = min(total, gw * per), hi = min(total, lo + per), cta = FBLA_POS::x();
+  if (cta * Sh::WARPS * per >= total) return;  // (nothing for the whole CTA)
+  RefineWarp<CB, FB> &w = ws[warp];
+  // a.refine_fold: a head's corrections leave the CTA as one row set, slot cta + vh: those of heads wholly inside a warp's run directly, the first
+  // and the last head's folded over the warps. (A row set per warp, as where the prefix leaves no room: the merge reads some two hundred of
+  // them per head of a 128K context.)
+  float *const firsts = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(pre) + refine_prefix_bytes(entries)), *const first = a.refine_fold ? firsts + (size_t)warp * 4 * PSTRIDE : nullptr;
+  int first_vh = -1, last_vh = -1;
+  if (lo < hi) {
+    const bool ok = refine_run<CB, FB, QG>(a, w, pre, entries, lo, hi, a.refine_fold ? cta : gw, first, first_vh, last_vh);
+    if (!ok) {
+      if (lane == 0) report(a, 3);
+      first_vh = last_vh = -1;
+    }
+  }
+  if (!a.refine_fold) return;
+  if (lane == 0) { stage_vh[warp][0] = first_vh; stage_vh[warp][1] = last_vh; }
+  __syncthreads();
+  fold_heads(stage_vh, Sh::WARPS, Sh::WARPS / 4, [&](int x, int r, int n, int t) {
+    add_sets<QG>(a.dpart + (size_t)(cta + stage_vh[x][r]) * QG * PSTRIDE, n, t,
+                 [&](int y) { return y == 0 && r ? reinterpret_cast<const float *>(ws[x].stage) : firsts + (size_t)(x + y) * 4 * PSTRIDE; });
+  });
+}
 // ---- merge: out = (sum 2^(m_c - R) o_c + sum do) / (sum 2^(m_c - R) l_c + sum dl), BF16 ---------------------------------
 // One CTA per output row (virtual head, query): thread (c4, sl) sums the partial rows sl, sl + 16, ... of channels
 // 4 c4 .. 4 c4 + 3, the sixteen sums of a channel are then added in a fixed order.
@@ -1150,6 +1203,7 @@ __device__ __forceinline__ void merge_item(const fbla_k_decode &a, uint8_t *smem
   __shared__ Slots ss;
   const int vh = FBLA_POS::x() / QG, qi = FBLA_POS::x() % QG, c4 = FBLA_POS::tid() & 31, sl = FBLA_POS::tid() >> 5;
   const int hpr = a.kv_heads * a.vg, vheads = a.batch * hpr, b = vh / hpr, hir = vh - b * hpr;
+  allow_next_pass();
   if (FBLA_POS::tid() == 0) ss = slots_of(a, vh);  // (from the lengths alone: before the previous pass has completed)
   __syncthreads();
   wait_previous_pass();
@@ -1162,7 +1216,7 @@ __device__ __forceinline__ void merge_item(const fbla_k_decode &a, uint8_t *smem
   float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
   float L = 0.f;
   const int nc = s.c1 - s.c0 + 1, nx = s.x1 - s.x0 + 1, n = nc + nx;
-  // (a long sequence at a small batch gives a head some tens of partial rows and a few hundred correction rows: NS * MJ
+  // (a long sequence at a small batch gives a head some tens of partial rows: NS * MJ
   // rows of the CTA in flight keep the number of dependent round trips to memory small; the summation order is fixed
   // by the loops alone)
   for (int i0 = sl; i0 < n; i0 += NS * MJ) {
@@ -1182,12 +1236,12 @@ __device__ __forceinline__ void merge_item(const fbla_k_decode &a, uint8_t *smem
         O.x = fmaf(e, o[j].x, O.x); O.y = fmaf(e, o[j].y, O.y); O.z = fmaf(e, o[j].z, O.z); O.w = fmaf(e, o[j].w, O.w);
       }
   }
-  int w0 = 0, w1 = -1;  // the refine warps whose runs of items met this head
+  int w0 = 0, w1 = -1;  // the refine CTAs (warps) whose runs of items met this head
   if (it1 > it0) {
-    const int per = (int)ceil_div(total, (long long)a.refine_ctas * a.refine_warps);
+    const int per = (int)ceil_div(total, (long long)a.refine_ctas * a.refine_warps) * (a.refine_fold ? a.refine_warps : 1);
     w0 = it0 / per; w1 = (it1 - 1) / per;
   }
-  for (int i0 = w0 + sl; i0 <= w1; i0 += NS * MJ) {  // (one correction row per refine warp that met the head)
+  for (int i0 = w0 + sl; i0 <= w1; i0 += NS * MJ) {  // (one correction row per refine CTA that met the head)
     float l[MJ];
     float4 o[MJ];
 #pragma unroll

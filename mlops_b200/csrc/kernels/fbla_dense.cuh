@@ -243,26 +243,6 @@ __device__ __forceinline__ float2 merge_mass(float2 x, float2 y) {  // (m, l) pa
   return make_float2(m, x.y * ex2(x.x - by) + y.y * ex2(y.x - by));
 }
 
-// The heads whose rows the CTA's warps have left: warp x's run of work is the end of vh[x][0] (all of it if vh[x][1] < 0) and, behind
-// heads of its own, the beginning of vh[x][1]; -1: none (idle warps lie before or behind the others). A head is folded by its first warp.
-struct Runs {
-  int first, last;   // of warp `lane`
-  uint32_t mask0, mask1;  // bit x: warp x is the first of the head in vh[x][0], vh[x][1]
-  __device__ __forceinline__ Runs(const int (*vh)[2], int warps, int lane) {
-    first = lane < warps ? vh[lane][0] : -1;
-    last = lane < warps ? vh[lane][1] : -1;
-    const int before = __shfl_up_sync(FULL, last >= 0 ? last : first, 1);
-    mask0 = __ballot_sync(FULL, first >= 0 && (lane == 0 || before != first));
-    mask1 = __ballot_sync(FULL, last >= 0);
-  }
-  // the warps, from x on, that hold rows of the head in vh[x][r] (the same x and r in every lane)
-  __device__ __forceinline__ int length(int x, int r) const {
-    const int lane = FBLA_POS::tid() & 31, f = __shfl_sync(FULL, first, x), l = __shfl_sync(FULL, last, x);
-    const uint32_t more = __ballot_sync(FULL, lane > x && first == (r ? l : f));
-    return 1 + (r == 0 && l >= 0 ? 0 : __popc(more));
-  }
-};
-
 // lane l's pair becomes that of query l % QG over all lanes
 template <int QG> __device__ __forceinline__ float2 merge_lanes(float2 acc, int lane) {
 #pragma unroll
@@ -951,36 +931,11 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
     stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
-  // rows of heads that may continue in neighbouring warps, added in warp order: a head by four warps, 16 bytes a thread. (By its first
-  // warp alone the rows of sixteen warps took 5 us: 8 x 16K 4+2 70.5 -> 63.0 us, 1 x 12K 24.1 -> 21.3.)
-  const Runs runs(stage_vh, VALUE_WARPS, lane);
-  const int t = FBLA_POS::tid() & 127, quad = FBLA_POS::tid() >> 7;
-  uint64_t left = (uint64_t)runs.mask1 << 32 | runs.mask0;
-#pragma unroll 1
-  for (int k = 0; left; ++k) {
-    const int bit = __ffsll((long long)left) - 1, r = bit >> 5, x = bit & 31;
-    left &= left - 1;
-    if (k % (VALUE_WARPS / 4) != quad) continue;
-    const int n = runs.length(x, r);
-    float *const dst = value_row(a, cta + stage_vh[x][r]);
-    const float *src = r ? reinterpret_cast<const float *>(ws[x].run) : &ws[x].stage[0][0];
-    const int at = (t >> 5) * PSTRIDE + 4 * (t & 31);  // query t / 32, channels 4 (t % 32) ..
-    if (t < 32 * QG) {
-      float4 s = *reinterpret_cast<const float4 *>(src + at);
-#pragma unroll 4
-      for (int y = 1; y < n; ++y) {
-        const float4 z = *reinterpret_cast<const float4 *>(&ws[x + y].stage[0][0] + at);
-        s.x += z.x; s.y += z.y; s.z += z.z; s.w += z.w;
-      }
-      *reinterpret_cast<float4 *>(dst + at) = s;
-    }
-    if (t < QG) {
-      float s = src[t * PSTRIDE + D];
-#pragma unroll 4
-      for (int y = 1; y < n; ++y) s += ws[x + y].stage[t][D];
-      dst[t * PSTRIDE + D] = s;
-    }
-  }
+  // rows of heads that may continue in neighbouring warps, added in warp order (by the head's first warp alone: 8 x 16K 4+2 70.5 us, so 63.0)
+  fold_heads(stage_vh, VALUE_WARPS, VALUE_WARPS / 4, [&](int x, int r, int n, int t) {
+    add_sets<QG>(value_row(a, cta + stage_vh[x][r]), n, t,
+                 [&](int y) { return y == 0 && r ? reinterpret_cast<const float *>(ws[x].run) : &ws[x + y].stage[0][0]; });
+  });
 }
 
 template <int CB, int FB, int QG, bool HEAD = false>

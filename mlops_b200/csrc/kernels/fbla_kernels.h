@@ -25,7 +25,7 @@ typedef struct {
 //   lse    [VH][nblocks][qg]  float  log2 mass of every closed sub-block under the coarse scores (two sweeps: then the weights, fbla_dense.cuh)
 //   part   [2 TW + 2 VH][qg][132] float  (o[128], m, l) partials: slot w + vh for streaming warp (or, folded, CTA) w,
 //          coarse_ctas * coarse_warps + VH + x + vh for window warp x; TW = coarse_ctas * coarse_warps
-//   dpart  [RW + VH][qg][129] float  (dl, do[128]) corrections of refine warp w at slot w + vh
+//   dpart  [RW + VH][qg][132] float  (do[128], dl) corrections of refine warp (or, folded, CTA) w at slot w + vh
 //   row_r  [VH][qg]           float  log2 of the row's total coarse mass
 //   counts [VH][nslices]      int    selected sub-blocks per slice of 1024 sub-blocks
 //   items  [VH][nslices][1024] int   (sub-block << 4) | query mask, in sub-block order
@@ -55,7 +55,7 @@ typedef struct {
   short shard_on, sh_windows, phase;
   short mass_given;    // dense: the rows' masses are in row_r (a pass before, or a shard's caller) instead of formed by the value pass
   float *out_partial;  // [rows][FBLA_K_PSTRIDE] floats (phase 2)
-  short status_cleared;  // 1: the launcher zeroes the status word on the stream before the first pass; 0: CTA 0 of the coarse pass does
+  short refine_fold;   // 1: the refine pass leaves one row of corrections per (CTA, virtual head) instead of one per (warp, virtual head)
   char fold;           // 1: the coarse pass leaves one partial row per (CTA, virtual head) instead of one per (warp, virtual head)
   char deep;           // the coarse pass's shape: 1: few warps with a whole group in flight each; 0: more warps (fbla_decode.cuh)
   char dense;          // 1: two sweeps, weights kept between them (fbla_dense.cuh); 0: coarse sums, then corrections (fbla_decode.cuh)
@@ -99,7 +99,8 @@ FBLA_HOST_API(int fbla_k_decode_deep_of(int batch, int kv_heads, int vg, int qg,
 FBLA_HOST_API(cudaError_t fbla_k_total_mass_launch(const float *mass, float *total, int shards, int rows, cudaStream_t stream);)
 FBLA_HOST_API(cudaError_t fbla_k_combine_launch(const float *partial, uint16_t *out, int rows, cudaStream_t stream);)
 // the most (virtual head, slice) entries one decode may have: the refine pass keeps their prefix sums in shared memory
-FBLA_HOST_API(long long fbla_k_refine_entry_limit(int cb);)
+// (fold: with room for the row sets of refine_fold)
+FBLA_HOST_API(long long fbla_k_refine_entry_limit(int cb, int fold);)
 // occupancy-derived launch shape for the current device; fills coarse_ctas .. refine_warps from cb / qg
 FBLA_HOST_API(cudaError_t fbla_k_decode_shape(fbla_k_decode *a);)
 

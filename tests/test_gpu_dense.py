@@ -159,6 +159,26 @@ def test_shapes_of_the_coarse_sweep(ours, oracle, mode, QH, KH, N, deal, deep):
     gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode), tau=tau), f"{mode} {N}")
 
 
+@pytest.mark.parametrize("extra", [0, 1])
+def test_corrections_with_and_without_room_to_fold(ours, oracle, extra):
+    """One sweep with the most (head, slice) entries whose prefix leaves the refine pass room for its row sets, and with more: a few rows of the batch"""
+    mode, KH, N = "4+2", 16, 270
+    limit = ours.lib.fbla_k_refine_entry_limit
+    limit.restype = ctypes.c_longlong
+    B = limit(4, 1) // KH + extra
+    assert B > 1024 and (B * KH > limit(4, 1)) == bool(extra) and B * KH <= limit(4, 0)
+    q, k, v = datagen.uneven_case(8, 3, KH, KH, N)
+    rows = torch.arange(B, device="cuda") % 3
+    c = ours.encode(*(gu.bf16_tensor(x)[rows].contiguous() for x in (k, v)), mode)
+    qd = gu.bf16_tensor(q)[rows].contiguous()
+    assert first_entry(ours, c, qd, mode, 0.0).startswith("fbla::coarse_item")
+    got = ours.decode(c, qd)
+    torch.cuda.synchronize()
+    want = oracle.decode(q, oracle.encode(k, v, mode))
+    for b in (0, 1, B // 2, B - 1):
+        gu.check_close(gu.bits_of(got)[b], want[b % 3], f"row {b} of {B}")
+
+
 def test_rows_of_their_own_lengths_fill_part_of_the_room(ours, oracle):
     """A room beyond the line: rows of one length are decoded in one sweep, rows of lengths of their own in two, in the scratch that the size
     query gives for either."""
