@@ -27,8 +27,8 @@
 // integer rounding and the requantisation of the row's 128 query channels (about 17 000 warp instructions per pass at 0.6
 // per cycle and scheduler); the tensor-core share of a pass is about as long as its exp2 share alone. Measured at batch 4 x
 // 8192 (32 / 8 heads, 4+2): sixteen warps doing softmax and requantisation in turn 5.66 ms = 388 TFLOP/s; roles of their
-// own 5.35; BF16 operands with all loads in flight 5.21; biases on tensor cores 4.75; two sweeps over eight rows of a lane
-// with one reduction 4.54 = 484 TFLOP/s. (64 registers per thread: 29 warps. Halving the softmax warps so that the tiles
+// own 5.35; BF16 operands with all loads in flight 5.21; biases on tensor cores 4.75; a lane's eight rows requantised with one
+// reduction, read twice, 4.60; four at a time, read once, 4.39 = 501 TFLOP/s. (64 registers per thread: 29 warps. Halving the softmax warps so that the tiles
 // alternate, or one copy of the unpacking code for both records of an operand warp, measured slower.)
 // Every wait is bounded: on a timeout the thread raises a flag, everybody drains, tensor memory is freed, the kernel
 // returns and the host sees fbla_k_attend_tc_status() != 0.
@@ -381,11 +381,11 @@ __device__ __forceinline__ void attend_tiles(const fbla_k_prefill &a, uint8_t *s
     }
     const float2 mg = splat(MAGICF), ng = splat(-MAGICF);
     const float sl127 = __fmul_rn(a.sl, 1.f / 127.f);
-    const uint8_t *const meta = reinterpret_cast<const uint8_t *>(a.c.meta) + head * 1024 + 32 * qc;
-    uint4 ma = make_uint4(0u, 0u, 0u, 0u), mb = ma;  // K metadata of channels 8 qc .. + 7: per four channels, four BF16 bases (unused here) then four BF16 steps
+    const uint8_t *const meta = reinterpret_cast<const uint8_t *>(a.c.meta) + head * 1024 + 32 * qc + 8;
+    uint2 ma = make_uint2(0u, 0u), mb = ma;  // K's steps of channels 8 qc .. + 7 (the metadata: per four channels, four BF16 bases then four BF16 steps)
     auto load_meta = [&](int g) {
-      ma = __ldcg(reinterpret_cast<const uint4 *>(meta + (size_t)g * a.gs * 1024));
-      mb = __ldcg(reinterpret_cast<const uint4 *>(meta + (size_t)g * a.gs * 1024 + 16));
+      ma = __ldcg(reinterpret_cast<const uint2 *>(meta + (size_t)g * a.gs * 1024));
+      mb = __ldcg(reinterpret_cast<const uint2 *>(meta + (size_t)g * a.gs * 1024 + 16));
     };
     if (p_lo < c_hi) load_meta(1 + p_lo);
     __syncwarp();  // (the warp's own rows of the q tiles are in place)
@@ -408,64 +408,51 @@ __device__ __forceinline__ void attend_tiles(const fbla_k_prefill &a, uint8_t *s
           for (int i = 0; i < 4; ++i) sm.qbias[(k >> 3) & 1][2 * (lane & 3) + (i & 1)][X][16 * qw + (lane >> 2) + 8 * (i >> 1)] = __fmul_rn(d[i], a.sl);
         }
       }
-      const float4 s0 = make_float4(bf_lo(ma.z), bf_hi(ma.z), bf_lo(ma.w), bf_hi(ma.w));
-      const float4 s1 = make_float4(bf_lo(mb.z), bf_hi(mb.z), bf_lo(mb.w), bf_hi(mb.w));
+      const float4 s0 = make_float4(bf_lo(ma.x), bf_hi(ma.x), bf_lo(ma.y), bf_hi(ma.y));
+      const float4 s1 = make_float4(bf_lo(mb.x), bf_hi(mb.x), bf_lo(mb.y), bf_hi(mb.y));
       if (n + 1 < c_hi) load_meta(g + 1);
 #pragma unroll 1
       for (int X = 0; X < 2; ++X) {
         // the tile's qhat buffer is free once the S product of the pass before is complete
         if (k > 0) wait(sm, &sm.bar_s[X], (k - 1) & 1);
         if (g < tile_own[X]) {
-          // z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16. First sweep: the lane's shares of max |z| for
-          // its eight rows; a butterfly over a row's 16 lanes that hands half of the rows on in
-          // every step leaves row `it` = 4 b3 + 2 b2 + b1 in the lanes with those bits, which form its r once.
-          auto z_of = [&](int it, int h, float2 (&z)[4]) -> uint32_t {  // row it + 4 h of the lane's eight
-            const uint32_t off = qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4));
-            const uint4 qv = *reinterpret_cast<const uint4 *>(sm.q[X] + off);
-            z[0] = mul2(bf2(qv.x), make_float2(s0.x, s0.y)); z[1] = mul2(bf2(qv.y), make_float2(s0.z, s0.w));
-            z[2] = mul2(bf2(qv.z), make_float2(s1.x, s1.y)); z[3] = mul2(bf2(qv.w), make_float2(s1.z, s1.w));
-            return off;
-          };
-          float amax[4] = {0.f, 0.f, 0.f, 0.f}, before[4];
+          // z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16: four of the lane's eight rows at a time, their z in registers.
+          // The lane's shares of max |z|; a butterfly over a row's 16 lanes that hands half of the rows on in each of its first two
+          // steps leaves row 2 b3 + b2 in the lanes with those bits, which form its r once.
 #pragma unroll 1
-          for (int h = 0; h < 2; ++h)
+          for (int h = 0; h < 2; ++h) {
+            float2 z[4][4];
+            float amax[4];
 #pragma unroll
             for (int it = 0; it < 4; ++it) {
-              float2 z[4];
-              z_of(it, h, z);
-              before[it] = amax[it];
-              amax[it] = max3_abs(max3_abs(z[0].x, z[0].y, z[1].x), max3_abs(z[1].y, z[2].x, z[2].y), fmaxf(fabsf(z[3].x), fabsf(z[3].y)));
+              const uint4 qv = *reinterpret_cast<const uint4 *>(sm.q[X] + qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4)));
+              z[it][0] = mul2(bf2(qv.x), make_float2(s0.x, s0.y)); z[it][1] = mul2(bf2(qv.y), make_float2(s0.z, s0.w));
+              z[it][2] = mul2(bf2(qv.z), make_float2(s1.x, s1.y)); z[it][3] = mul2(bf2(qv.w), make_float2(s1.z, s1.w));
+              amax[it] = max3_abs(max3_abs(z[it][0].x, z[it][0].y, z[it][1].x), max3_abs(z[it][1].y, z[it][2].x, z[it][2].y), fmaxf(fabsf(z[it][3].x), fabsf(z[it][3].y)));
             }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {  // lane bit 3 decides which four rows are kept, bits 2 and 1 which half of what is left
-            const bool up = lane & 8;
-            const float keep = up ? amax[i] : before[i], send = up ? before[i] : amax[i];
-            amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 8));
-          }
+            for (int w = 2; w; w >>= 1) {
+              const bool up = lane & (4 * w);
 #pragma unroll
-          for (int w = 2; w; w >>= 1) {
-            const bool up = lane & (2 * w);
-#pragma unroll
-            for (int i = 0; i < w; ++i) {
-              const float keep = up ? amax[i + w] : amax[i], send = up ? amax[i] : amax[i + w];
-              amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 2 * w));
+              for (int i = 0; i < w; ++i) {
+                const float keep = up ? amax[i + w] : amax[i], send = up ? amax[i] : amax[i + w];
+                amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 4 * w));
+              }
             }
-          }
-          const float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 1));
-          const float rq = quotient_127(am);
-          if (!(lane & 1)) sm.qscale[k & 1][X][qrow0 + (lane & 14)] = __fmul_rn(am, sl127);  // (row qrow0 + 2 it)
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h)
+            float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 2));
+            am = fmaxf(am, __shfl_xor_sync(FULL, am, 1));
+            const float rq = quotient_127(am);
+            if (!(lane & 3)) sm.qscale[k & 1][X][qrow0 + 8 * h + ((lane & 12) >> 1)] = __fmul_rn(am, sl127);  // (row qrow0 + 8 h + 2 it)
 #pragma unroll
             for (int it = 0; it < 4; ++it) {
-              float2 z[4];
-              const uint32_t off = z_of(it, h, z);
               // rint(z r) as the exact float (t - 1.5 * 2^23), then FP16 (an integer of magnitude <= 127: exact)
-              const float2 rr2 = splat(__shfl_sync(FULL, rq, (lane & 16) | (8 * h + 2 * it)));
-              const float2 t0 = add2(fma2(z[0], rr2, mg), ng), t1 = add2(fma2(z[1], rr2, mg), ng);
-              const float2 t2 = add2(fma2(z[2], rr2, mg), ng), t3 = add2(fma2(z[3], rr2, mg), ng);
-              *reinterpret_cast<uint4 *>(sm.qp[X] + off) = make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
+              const float2 rr2 = splat(__shfl_sync(FULL, rq, (lane & 16) | (4 * it)));
+              const float2 t0 = add2(fma2(z[it][0], rr2, mg), ng), t1 = add2(fma2(z[it][1], rr2, mg), ng);
+              const float2 t2 = add2(fma2(z[it][2], rr2, mg), ng), t3 = add2(fma2(z[it][3], rr2, mg), ng);
+              *reinterpret_cast<uint4 *>(sm.qp[X] + qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4))) =
+                  make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
             }
+          }
         }
         fence_async_smem();
         mbar_arrive(&sm.bar_q[X]);
