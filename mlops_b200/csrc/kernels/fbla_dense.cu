@@ -89,7 +89,7 @@ template <int CB, int FB, int QG> struct Kernels {
     snprintf(p[2].entry, sizeof p[2].entry, "fbla::dense::value_item<%d, %d, %d>", CB, FB, QG);
     if (a.head_ctas && e == cudaSuccess) {
       e = describe(head_kernel<CB, FB, QG>, a.head_ctas, 32 * SCORE_WARPS, sizeof(HeadScoreSmem), p + 0);
-      if (e == cudaSuccess) e = describe(head_kernel<CB, FB, QG>, a.head_ctas, 32 * VALUE_WARPS, sizeof(HeadValueSmem), p + 2);
+      if (e == cudaSuccess) e = describe(head_kernel<CB, FB, QG>, a.head_ctas, 32 * VALUE_WARPS, sizeof(HeadValueItemSmem), p + 2);
       for (int i = 0; i <= 2; i += 2) { p[i].gy = a.kv_heads * a.vg; p[i].gz = a.batch; }
       snprintf(p[0].entry, sizeof p[0].entry, "fbla::dense::score_item<%d, %d, %d, true>", CB, FB, QG);
       snprintf(p[2].entry, sizeof p[2].entry, "fbla::dense::value_item<%d, %d, %d, true>", CB, FB, QG);

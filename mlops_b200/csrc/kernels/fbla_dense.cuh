@@ -161,7 +161,9 @@ __device__ __forceinline__ void quantize_group(uint4 km, const uint2 (&q)[QG], u
 // ---- score pass -----------------------------------------------------------------------------------------------------------------
 // K words of one sub-block in registers: what thread (gid, tig) supplies to the products, for tokens gid and gid + 8.
 // 4 and 2 bits: the thread's slots are 4 t + i and 8 + 4 t + i (i = 0..3, t = tig % 2) of channel half tig / 2, so that a token's words
-// come in 16-byte pieces (2 bits: both t read the same piece); 3 bits: the words of qk_tile<3>.
+// come in 16-byte pieces (2 bits: both t read the same piece). 3 bits: the thread's words are W[2 t], W[2 t + 1] and W[4 + t] of half tig / 2:
+// slots 2 t, + 1, 6 + 2 t, + 1, 12 + 2 t, + 1, 4 + t and 10 + t, whole. (Every thread on W[tig] of both halves took two words and twice the
+// loads more; with the values' tails in shared memory: 32 sequences of 300 to 6 000 tokens 82.5 -> 75.8 us, 16 / 8 heads 16 x 4 000 54.2 -> 43.9.)
 template <int BITS> struct KWords {
   uint4 a, a8;
   static __device__ __forceinline__ int offset(int gid, int tig) { return (BITS == 4 ? 512 * (tig & 1) : 0) + 256 * (tig >> 1) + 16 * gid; }
@@ -171,13 +173,13 @@ template <int BITS> struct KWords {
   }
 };
 template <> struct KWords<3> {
-  uint32_t a, a8, c, c8, e, e8, f, f8;
-  static __device__ __forceinline__ int offset(int gid, int tig) { return 16 * gid + 4 * tig; }
-  static __device__ __forceinline__ int tail(int tig) { return 1024 + 4 * (tig >> 1) - 4 * tig; }  // from there to the words 4 + tig / 2
-  __device__ __forceinline__ void load(const uint8_t *p8, int tail) {
-    const uint32_t *p = reinterpret_cast<const uint32_t *>(p8), *q = reinterpret_cast<const uint32_t *>(p8 + tail);
-    a = __ldg(p); a8 = __ldg(p + 32); c = __ldg(p + 64); c8 = __ldg(p + 96);
-    e = __ldg(q); e8 = __ldg(q + 32); f = __ldg(q + 2); f8 = __ldg(q + 34);
+  uint2 a, a8;      // W[2 t], W[2 t + 1] of tokens gid and gid + 8
+  uint32_t e, e8;   // W[4 + t]
+  static __device__ __forceinline__ int offset(int gid, int tig) { return 256 * (tig >> 1) + 16 * gid + 8 * (tig & 1); }
+  static __device__ __forceinline__ int tail(int tig) { return 1024 + 8 * (tig >> 1) + 4 * (tig & 1) - 256 * (tig >> 1) - 8 * (tig & 1); }  // from there to W[4 + t]
+  __device__ __forceinline__ void load(const uint8_t *p, int tail) {
+    a = __ldg(reinterpret_cast<const uint2 *>(p)); a8 = __ldg(reinterpret_cast<const uint2 *>(p + 128));
+    e = __ldg(reinterpret_cast<const uint32_t *>(p + tail)); e8 = __ldg(reinterpret_cast<const uint32_t *>(p + tail + 128));
   }
 };
 // the qhat words matching KWords
@@ -187,7 +189,9 @@ template <int CB> __device__ __forceinline__ void score_frag(const uint8_t *qst,
     const uint4 lo = lds128(p), hi = lds128(p + 32);
     B[0] = lo.x; B[1] = lo.y; B[2] = lo.z; B[3] = lo.w; B[4] = hi.x; B[5] = hi.y; B[6] = hi.z; B[7] = hi.w;
   } else {
-    qhat_frag<3>(qst, row, tig, B);
+    const uint8_t *p = qst + QST_ROW * row + 64 * (tig >> 1) + 8 * (tig & 1), *r = p - 4 * (tig & 1);
+    const uint2 x = lds64(p), y = lds64(p + 24), z = lds64(p + 48);
+    B[0] = x.x; B[1] = x.y; B[2] = y.x; B[3] = y.y; B[4] = z.x; B[5] = z.y; B[6] = lds32(r + 16); B[7] = lds32(r + 40);
   }
 }
 // The sub-block's products, in accumulators of the low and of the high class (times 16, 3 bits: 8): set (FIRST) or added to.
@@ -207,13 +211,12 @@ __device__ __forceinline__ void score_products(const KWords<BITS> &k, const uint
     mma_u8s8_k32(lo, a.z & L, a8.z & L, a.w & L, a8.w & L, b[2], b[3]);
     mma_u8s8_k32(hi, a.z & H, a8.z & H, a.w & H, a8.w & H, b[6], b[7]);
   } else {
-    const int sh = 4 + (tig & 1), se = 3 * (tig & 1);
     constexpr uint32_t L = 0x07070707u, M = 0x38383838u, T2 = 0x03030303u, T1 = 0x04040404u;
-    mma_step<FIRST>(lo, k.a & L, k.a8 & L, k.c & L, k.c8 & L, b[0], b[1]);
-    mma_step<FIRST>(hi, k.a & M, k.a8 & M, k.c & M, k.c8 & M, b[2], b[3]);
-    mma_u8s8_k32(lo, ((k.a >> 6) & T2) | ((k.e >> sh) & T1), ((k.a8 >> 6) & T2) | ((k.e8 >> sh) & T1),
-                 ((k.c >> 6) & T2) | ((k.f >> sh) & T1), ((k.c8 >> 6) & T2) | ((k.f8 >> sh) & T1), b[4], b[5]);
-    mma_u8s8_k32(lo, (k.e >> se) & L, (k.e8 >> se) & L, (k.f >> se) & L, (k.f8 >> se) & L, b[6], b[7]);
+    mma_step<FIRST>(lo, k.a.x & L, k.a8.x & L, k.a.y & L, k.a8.y & L, b[0], b[1]);
+    mma_step<FIRST>(hi, k.a.x & M, k.a8.x & M, k.a.y & M, k.a8.y & M, b[2], b[3]);
+    mma_u8s8_k32(lo, ((k.a.x >> 6) & T2) | ((k.e >> 4) & T1), ((k.a8.x >> 6) & T2) | ((k.e8 >> 4) & T1),
+                 ((k.a.y >> 6) & T2) | ((k.e >> 5) & T1), ((k.a8.y >> 6) & T2) | ((k.e8 >> 5) & T1), b[4], b[5]);
+    mma_u8s8_k32(lo, k.e & L, k.e8 & L, (k.e >> 3) & L, (k.e8 >> 3) & L, b[6], b[7]);
   }
 }
 
@@ -596,14 +599,14 @@ __device__ __forceinline__ void mass_item(const fbla_k_decode &a, uint8_t *smem_
 }
 
 // ---- value pass -------------------------------------------------------------------------------------------------------------------
-// V words of a record in registers: what thread (gid, tig) supplies to the products for record lanes 8 u + gid, u = 0..3, and its
-// slots (as v_slots of fbla_frag.cuh).
+// V words of a record: what thread (gid, tig) supplies to the products for record lanes 8 u + gid, u = 0..3, and its slots (as v_slots of
+// fbla_frag.cuh). In registers; of 3 bits the record lanes' words W[4], W[5] lie in shared memory (`tail`: 8 bytes per record lane; the
+// warp copies a record's 256 bytes there, 8 a lane): in registers they were two thirds of the words, each held by four threads, and the
+// kernel spilled.
 template <int BITS> struct VWords {
-  uint32_t w[4][BITS == 2 ? 1 : BITS == 4 ? 2 : 3];
+  uint32_t w[4][BITS == 4 ? 2 : 1];
   static __device__ __forceinline__ int offset(int gid, int tig) { return BITS == 4 ? 1024 + 512 * (tig >> 1) + 16 * gid + 8 * (tig & 1) : 512 + 16 * gid + 4 * tig; }
-  // p: the record + offset; 3 bits: d1, d2 from there to W[4 + tig / 2] (the top bit of slot 12 + tig) and W[4 + tig % 2] (slot 4 + tig
-  // for tig < 2, 10 + tig - 2 beyond)
-  __device__ __forceinline__ void load(const uint8_t *p, int d1, int d2) {
+  __device__ __forceinline__ void load(const uint8_t *p) {  // p: the record + offset
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if constexpr (BITS == 4) {
@@ -611,28 +614,26 @@ template <int BITS> struct VWords {
         w[u][0] = y.x; w[u][1] = y.y;
       } else {
         w[u][0] = __ldg(reinterpret_cast<const uint32_t *>(p + 128 * u));
-        if constexpr (BITS == 3) {
-          w[u][1] = __ldg(reinterpret_cast<const uint32_t *>(p + d1 + 64 * u));
-          w[u][2] = __ldg(reinterpret_cast<const uint32_t *>(p + d2 + 64 * u));
-        }
       }
     }
   }
-  __device__ __forceinline__ void slots(int u, int tig, uint32_t (&v)[4]) const {
+  __device__ __forceinline__ void slots(int u, int tig, const uint8_t *tail, uint32_t (&v)[4]) const {
     const uint32_t a = w[u][0];
     if constexpr (BITS == 4) {
       const uint32_t b = w[u][1];
       v[0] = a & 0x0f0f0f0fu; v[1] = b & 0x0f0f0f0fu; v[2] = a & 0xf0f0f0f0u; v[3] = b & 0xf0f0f0f0u;
     } else if constexpr (BITS == 2) {
       v[0] = a & 0x03030303u; v[1] = a & 0x0c0c0c0cu; v[2] = a & 0x30303030u; v[3] = a & 0xc0c0c0c0u;
-    } else {
+    } else {  // W[4 + tig / 2]: the top bit of slot 12 + tig; W[4 + tig % 2]: slot 4 + tig for tig < 2, 10 + tig - 2 beyond
       v[0] = a & 0x07070707u;
       v[1] = a & 0x38383838u;
-      v[2] = (w[u][2] >> (3 * (tig >> 1))) & 0x07070707u;
-      v[3] = ((a >> 6) & 0x03030303u) | ((w[u][1] >> (4 + (tig & 1))) & 0x04040404u);
+      v[2] = (lds32(tail + 64 * u + 4 * (tig & 1)) >> (3 * (tig >> 1))) & 0x07070707u;
+      v[3] = ((a >> 6) & 0x03030303u) | ((lds32(tail + 64 * u + 4 * (tig >> 1)) >> (4 + (tig & 1))) & 0x04040404u);
     }
   }
 };
+constexpr int TAIL_BYTES = 256;               // of a record's V half
+constexpr int TAILS_BYTES = 8 * TAIL_BYTES;   // of a warp: [coarse, fine][pair, alternating][sub-block of the pair]
 struct __align__(16) ValueWarp {
   uint8_t meta[2][512];        // V's metadata of the group in work and of the next
   float stage[4][PSTRIDE];     // the row set of the first virtual head of the warp's run
@@ -642,10 +643,12 @@ struct __align__(16) ValueWarp {
 };
 struct ValueSmem {
   ValueWarp w[VALUE_WARPS];
+  uint8_t tails[VALUE_WARPS][TAILS_BYTES];
   int stage_vh[VALUE_WARPS][2];
   Table table;
 };
 struct __align__(16) HeadValueSmem { ValueWarp w[VALUE_WARPS]; };
+struct __align__(16) HeadValueItemSmem { HeadValueSmem s; uint8_t tails[VALUE_WARPS][TAILS_BYTES]; };
 static_assert(sizeof(ValueSmem) + 128 <= 227 * 1024, "one CTA's shared memory");
 
 // the sums of one virtual head over the warp's pairs, in units of 2^-R: thread (gid, tig) holds channels 4 (8 u + gid) + cc of
@@ -674,9 +677,9 @@ template <int QG> __device__ __forceinline__ void write_sums(float *p, const Sum
   }
 }
 
-// `wait` returns when the score pass's results may be read; what does not depend on them is asked for before.
+// `wait` returns when the score pass's results may be read; what does not depend on them is asked for before. tails: the warp's.
 template <int CB, int FB, int QG, bool HEAD, class Via, class Wait>
-__device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *ws, int (*stage_vh)[2], const Table *table, const Via &via, Wait wait) {
+__device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *ws, uint8_t *tails, int (*stage_vh)[2], const Table *table, const Via &via, Wait wait) {
   constexpr int RC = record_bytes(CB), RF = record_bytes(FB);
   constexpr float HOFF = .5f * ((1 << FB) - 1);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5, gid = lane >> 2, tig = lane & 3;
@@ -735,31 +738,56 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
       if (has) { pc = __ldcg(w0 + (at + 2 * QG * J) * 4); pf = __ldcg(w1 + (at + 2 * QG * J) * 4); }
     };
     size_t unit = unit_of(c);
+    // Asynchronous copies, 3 bits: they leave in the order of a pair's coarse tails, its fine tails, the next pair's coarse tails, ... -- a group
+    // of copies each (empty where there is nothing to copy), the metadata of the next group of tokens with one of them -- so that waiting for
+    // all but the last group is waiting for what the pair in work needs next. Else: the metadata alone.
+    constexpr bool TAILS = CB == 3;
+    auto close_copies = [] { if (TAILS) asm volatile("cp.async.commit_group;" ::: "memory"); };
+    auto arrived = [] {
+      if (TAILS) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+      }
+    };
     auto fetch_meta = [&](size_t un, int buf) {  // V's 512 bytes of metadata
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n\tcp.async.commit_group;"
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;"
                    ::"r"(smem_u32(w.meta[buf] + 16 * lane)), "l"(reinterpret_cast<const uint8_t *>(a.c.meta) + un * 1024 + 512 + 16 * lane) : "memory");
+      if (!TAILS) asm volatile("cp.async.commit_group;" ::: "memory");
     };
     int J = lo % PAIRS;
     fetch_meta(unit, 0);
     // where the words of the next pair (coarse) and of the pair in work (fine) lie: pointers that run on within a head
     const uint8_t *cp = a.c.coarse + (unit * SBG + 2 * J) * RC + VWords<CB>::offset(gid, tig), *fp = a.c.fine + (unit * SBG + 2 * J) * RF + VWords<FB>::offset(gid, tig);
     const long long c_skip = (long long)(a.gs - 1) * SBG * RC, f_skip = (long long)(a.gs - 1) * SBG * RF;
-    const int d1 = 1280 - 512 - 8 * gid - 4 * tig + 4 * (tig >> 1), d2 = 1280 - 512 - 8 * gid - 4 * tig + 4 * (tig & 1);
     VWords<CB> va, vb;
-    auto load_coarse = [&] {
-      va.load(cp, d1, d2);
-      vb.load(cp + RC, d1, d2);
+    VWords<FB> fa, fb;
+    int turn = 0;  // the pair's place among the tails
+    uint8_t *const ctail = tails + 8 * gid, *const ftail = ctail + 4 * TAIL_BYTES;
+    auto fetch_tails = [&](const uint8_t *rec, int bytes, uint8_t *to) {  // rec: this thread's place in the first record
+      if constexpr (TAILS) {
+        const uint8_t *const from = rec - VWords<3>::offset(gid, tig) + 1280 + 8 * lane;
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(to - 8 * gid + 8 * lane + TAIL_BYTES * b)), "l"(from + bytes * b) : "memory");
+      }
+    };
+    auto load_coarse = [&](int at) {
+      va.load(cp);
+      vb.load(cp + RC);
+      fetch_tails(cp, RC, ctail + 2 * TAIL_BYTES * at);
       cp += 2 * RC;
     };
-    load_coarse();
-    VWords<FB> fa, fb;
-    auto load_fine = [&] {
-      fa.load(fp, d1, d2);
-      fb.load(fp + RF, d1, d2);
+    auto load_fine = [&](int at) {
+      fa.load(fp);
+      fb.load(fp + RF);
+      fetch_tails(fp, RF, ftail + 2 * TAIL_BYTES * at);
       fp += 2 * RF;
     };
+    load_coarse(0);
+    close_copies();
     if constexpr (HEAD) {  // (the CTA's own cells: complete. Short rows, most sub-blocks selected: the fine words do not wait for R)
-      load_fine();
+      load_fine(0);
+      close_copies();
       ask(cell);
       ask_p(cell, J);
       wait();
@@ -811,9 +839,12 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
       for (; J < j1; ++J, --left) {
         const uint32_t pm = (mask >> (2 * QG * J)) & ((1u << (2 * QG)) - 1u);  // the pair's selections
         if constexpr (!HEAD) {
-          if (pm) load_fine();
+          if (pm) load_fine(turn);
           else fp += 2 * RF;
+          close_copies();
         }
+        arrived();  // the pair's coarse tails
+        const uint8_t *const ct = ctail + 2 * TAIL_BYTES * turn, *const ft = ftail + 2 * TAIL_BYTES * turn;
         uint32_t pw = (pm >> pcol) & 1 ? pf : pc;
         if (!has) pw = 0u;
         const bool last = J + 1 >= PAIRS;
@@ -848,8 +879,8 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             uint32_t x[4], y[4];
-            va.slots(u, tig, x);
-            vb.slots(u, tig, y);
+            va.slots(u, tig, ct, x);
+            vb.slots(u, tig, ct + TAIL_BYTES, y);
             add(x, y, f, A[u]);
           }
         }
@@ -861,8 +892,10 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
               fp = a.c.fine + unit_n * SBG * RF + VWords<FB>::offset(gid, tig);
             }
           }
-          load_coarse();
+          load_coarse(turn ^ 1);
         }
+        close_copies();
+        arrived();  // the pair's fine tails
         if (pm) {
           float2 f[4];
 #pragma unroll
@@ -870,17 +903,23 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             uint32_t x[4], y[4];
-            fa.slots(u, tig, x);
-            fb.slots(u, tig, y);
+            fa.slots(u, tig, ft, x);
+            fb.slots(u, tig, ft + TAIL_BYTES, y);
             add(x, y, f, A[u]);
           }
         }
-        if (HEAD && left > 1) load_fine();
+        if constexpr (HEAD) {
+          if (left > 1) load_fine(turn ^ 1);
+          close_copies();
+        }
+        turn ^= 1;
       }
       J = 0;
-      if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
-      else asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncwarp();
+      if (!TAILS) {  // (else the metadata has come with the tails)
+        if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+      }
       const uint8_t *meta = w.meta[k & 1];
       L = __fmul2_rn(L, splat(BACK)); Hc = __fmul2_rn(Hc, splat(HOFF * BACK));
       w.run[16][lane] = __fadd2_rn(w.run[16][lane], L);
@@ -942,12 +981,13 @@ template <int CB, int FB, int QG, bool HEAD = false>
 __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   allow_next_pass();
   if constexpr (HEAD) {  // (a plan's items only: the stream call's kernel is head_passes)
-    value_units<CB, FB, QG, true>(a, reinterpret_cast<HeadValueSmem *>(smem_raw)->w, nullptr, nullptr, ScratchVia<QG>(a), [] {});
+    HeadValueItemSmem &sm = *reinterpret_cast<HeadValueItemSmem *>(smem_raw);
+    value_units<CB, FB, QG, true>(a, sm.s.w, sm.tails[FBLA_POS::tid() >> 5], nullptr, nullptr, ScratchVia<QG>(a), [] {});
   } else {
     ValueSmem &sm = *reinterpret_cast<ValueSmem *>(smem_raw);
     build_table(a, sm.table, 32 * VALUE_WARPS);
     if (a.phase != 0) wait_previous_pass();  // (a whole decode: the score pass let this one begin when all before the call was complete)
-    value_units<CB, FB, QG, false>(a, sm.w, sm.stage_vh, &sm.table, NoVia(), [&] { if (a.phase == 0) wait_previous_pass(); });
+    value_units<CB, FB, QG, false>(a, sm.w, sm.tails[FBLA_POS::tid() >> 5], sm.stage_vh, &sm.table, NoVia(), [&] { if (a.phase == 0) wait_previous_pass(); });
   }
 }
 
@@ -1028,12 +1068,13 @@ struct __align__(16) HeadSmem {
   float2 mass[16][4];  // [CTA][query]
   // in the scores' place once all CTAs have theirs: a window sub-block's row over its warp's V rows, the CTAs' sums over the queries
   __device__ __forceinline__ float *window(int warp) { return reinterpret_cast<float *>(&s.w[warp].exact.v[0][0]); }
+  __device__ __forceinline__ uint8_t *tails(int warp) { return reinterpret_cast<uint8_t *>(window(warp) + 4 * PSTRIDE); }  // behind that row
   __device__ __forceinline__ float *sums(int slot) { return reinterpret_cast<float *>(&s.w[slot].exact.q[0][0]); }
 };
 static_assert(sizeof(HeadSmem) <= 227 * 1024, "one CTA's shared memory");
 static_assert(SCORE_WARPS == 16 && VALUE_WARPS == 16, "one CTA runs both passes; at most sixteen CTAs of a head");
-static_assert(sizeof(ExactWarp::v) >= 4 * PSTRIDE * sizeof(float) && sizeof(ExactWarp::q) >= PSTRIDE * sizeof(float) && sizeof(ExactWarp::q) >= sizeof(ScoreWarp::s),
-              "a window sub-block's row beside the warp's later queries and P bytes");
+static_assert(sizeof(ExactWarp::v) >= 4 * PSTRIDE * sizeof(float) + TAILS_BYTES && sizeof(ExactWarp::q) >= PSTRIDE * sizeof(float) && sizeof(ExactWarp::q) >= sizeof(ScoreWarp::s),
+              "a window sub-block's row and the tails beside the warp's later queries and P bytes");
 template <int QG> struct ClusterVia {
   HeadSmem &sm;
   int ctas, rank, x0;  // x0: the first of the CTA's window sub-blocks
@@ -1057,7 +1098,7 @@ __device__ __forceinline__ void head_passes(const fbla_k_decode &a, uint8_t *sme
   const int x_per = (own.row.exact + own.ctas - 1) / own.ctas;
   const ClusterVia<QG> via{sm, own.ctas, own.rank, min(own.row.exact, own.rank * x_per)};
   score_units<CB, FB, QG, true>(a, sm.s.w, sm.s.fold, nullptr, via);
-  value_units<CB, FB, QG, true>(a, sm.v.w, nullptr, nullptr, via, [] { cluster_meet(); });
+  value_units<CB, FB, QG, true>(a, sm.v.w, sm.tails(FBLA_POS::tid() >> 5), nullptr, nullptr, via, [] { cluster_meet(); });
   cluster_meet();
   const int quad = FBLA_POS::tid() >> 7, qi = own.rank + own.ctas * quad;
   if (qi < QG) write_row(a, own.vh, qi, FBLA_POS::tid() & 127, own.ctas, [&](int cta, int ch) { return sm.sums(quad * own.ctas + cta)[ch]; });
