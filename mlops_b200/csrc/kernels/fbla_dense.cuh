@@ -738,10 +738,13 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
       if (has) { pc = __ldcg(w0 + (at + 2 * QG * J) * 4); pf = __ldcg(w1 + (at + 2 * QG * J) * 4); }
     };
     size_t unit = unit_of(c);
-    // Asynchronous copies, 3 bits: they leave in the order of a pair's coarse tails, its fine tails, the next pair's coarse tails, ... -- a group
-    // of copies each (empty where there is nothing to copy), the metadata of the next group of tokens with one of them -- so that waiting for
-    // all but the last group is waiting for what the pair in work needs next. Else: the metadata alone.
-    constexpr bool TAILS = CB == 3;
+    // Asynchronous copies, 3 bits (TAILS): they leave in the order of a pair's coarse tails, its fine tails, the next pair's coarse tails, ... -- a
+    // group of copies each (empty where there is nothing to copy), the metadata of the next group of tokens with one of them -- so that
+    // waiting for all but the last group is waiting for what the pair in work needs next. Else: the metadata alone.
+    // AHEAD: both planes of a pair, one group of copies, a whole pair ahead instead of a plane half a pair ahead, in registers that the tails
+    // do not take: 64 rows of 1K to 64K 811 -> 749 us, 32 of 300 to 6 000 75.8 -> 72.9, 16 x 8 000 70.2 -> 66.7; but with two queries 16 x 4 000
+    // 44.3 -> 45.6, and in the one kernel of a short decode, whose warps have a pair or two, 4K 11.5 -> 12.3.
+    constexpr bool TAILS = CB == 3, AHEAD = TAILS && !HEAD && QG == 4;
     auto close_copies = [] { if (TAILS) asm volatile("cp.async.commit_group;" ::: "memory"); };
     auto arrived = [] {
       if (TAILS) {
@@ -771,23 +774,25 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
           asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(to - 8 * gid + 8 * lane + TAIL_BYTES * b)), "l"(from + bytes * b) : "memory");
       }
     };
-    auto load_coarse = [&](int at) {
-      va.load(cp);
-      vb.load(cp + RC);
+    auto load_coarse = [&](VWords<CB> &x, VWords<CB> &y, int at) {
+      x.load(cp);
+      y.load(cp + RC);
       fetch_tails(cp, RC, ctail + 2 * TAIL_BYTES * at);
       cp += 2 * RC;
     };
-    auto load_fine = [&](int at) {
-      fa.load(fp);
-      fb.load(fp + RF);
+    auto load_fine = [&](VWords<FB> &x, VWords<FB> &y, int at) {
+      x.load(fp);
+      y.load(fp + RF);
       fetch_tails(fp, RF, ftail + 2 * TAIL_BYTES * at);
       fp += 2 * RF;
     };
-    load_coarse(0);
-    close_copies();
-    if constexpr (HEAD) {  // (the CTA's own cells: complete. Short rows, most sub-blocks selected: the fine words do not wait for R)
-      load_fine(0);
+    load_coarse(va, vb, 0);
+    if (!AHEAD) close_copies();
+    if (HEAD || AHEAD) {  // (whether it is selected is not known yet; mostly it is)
+      load_fine(fa, fb, 0);
       close_copies();
+    }
+    if constexpr (HEAD) {  // (the CTA's own cells: complete)
       ask(cell);
       ask_p(cell, J);
       wait();
@@ -838,8 +843,26 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
 #pragma unroll 1
       for (; J < j1; ++J, --left) {
         const uint32_t pm = (mask >> (2 * QG * J)) & ((1u << (2 * QG)) - 1u);  // the pair's selections
-        if constexpr (!HEAD) {
-          if (pm) load_fine(turn);
+        const bool last = J + 1 >= PAIRS;
+        auto move_on = [&] {  // from the group's last pair to the next group
+          if (stay) { cp += c_skip; fp += f_skip; }
+          else {
+            cp = a.c.coarse + unit_n * SBG * RC + VWords<CB>::offset(gid, tig);
+            fp = a.c.fine + unit_n * SBG * RF + VWords<FB>::offset(gid, tig);
+          }
+        };
+        VWords<CB> na, nb;
+        VWords<FB> ma, mb;
+        if constexpr (AHEAD) {
+          if (left > 1) {
+            if (last) move_on();
+            load_coarse(na, nb, turn ^ 1);
+            if (last || ((mask >> (2 * QG * (J + 1))) & ((1u << (2 * QG)) - 1u))) load_fine(ma, mb, turn ^ 1);  // (the next group's selections are not known yet)
+            else fp += 2 * RF;
+          }
+          close_copies();
+        } else if constexpr (!HEAD) {
+          if (pm) load_fine(fa, fb, turn);
           else fp += 2 * RF;
           close_copies();
         }
@@ -847,7 +870,6 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
         const uint8_t *const ct = ctail + 2 * TAIL_BYTES * turn, *const ft = ftail + 2 * TAIL_BYTES * turn;
         uint32_t pw = (pm >> pcol) & 1 ? pf : pc;
         if (!has) pw = 0u;
-        const bool last = J + 1 >= PAIRS;
         if (left > 1) ask_p(last ? cell_n : cell, last ? 0 : J + 1);
         // the thread's two columns: sub-block tig >> 1, queries 2 (tig & 1) + e
         const int own = QG * (tig >> 1) + 2 * (tig & 1);
@@ -884,18 +906,14 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
             add(x, y, f, A[u]);
           }
         }
-        if (left > 1) {
-          if (last) {
-            if (stay) { cp += c_skip; fp += f_skip; }
-            else {
-              cp = a.c.coarse + unit_n * SBG * RC + VWords<CB>::offset(gid, tig);
-              fp = a.c.fine + unit_n * SBG * RF + VWords<FB>::offset(gid, tig);
-            }
+        if constexpr (!AHEAD) {
+          if (left > 1) {
+            if (last) move_on();
+            load_coarse(va, vb, turn ^ 1);
           }
-          load_coarse(turn ^ 1);
+          close_copies();
+          arrived();  // the pair's fine tails
         }
-        close_copies();
-        arrived();  // the pair's fine tails
         if (pm) {
           float2 f[4];
 #pragma unroll
@@ -908,8 +926,10 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
             add(x, y, f, A[u]);
           }
         }
-        if constexpr (HEAD) {
-          if (left > 1) load_fine(turn ^ 1);
+        if constexpr (AHEAD) {
+          va = na; vb = nb; fa = ma; fb = mb;
+        } else if constexpr (HEAD) {
+          if (left > 1) load_fine(fa, fb, turn ^ 1);
           close_copies();
         }
         turn ^= 1;
