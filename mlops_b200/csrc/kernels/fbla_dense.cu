@@ -145,7 +145,7 @@ extern "C" int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens
 // but its heads' CTAs leave SMs idle and a head's work cannot move to another's. CTAs per head: as many as let all clusters run at once (of n
 // CTAs with an SM each a B200 holds n: 1: 148, 2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 8: 15, 10: 11, 16: 7). Groups per CTA up to which it is the
 // faster way (the room's: rows of lengths of their own wait for the longest). Device time on B200, us, three kernels / one, 3+3, 32 / 8 heads
-// unless said:
+// unless said, when the line was set (3+3 has become faster on both sides since: 4 096 tokens in one kernel 11.8):
 //   batch 1, 10 CTAs: 250 tokens 11.0 / 7.2    4 096: 18.7 / 12.4    12 000 (9 groups per CTA): 21.9 / 19.7    30 000 (23): 31.1 / 31.3    80 000: 52 / 77
 //   batch 2, 6 CTAs:  250: 11.2 / 7.3          4 096: 20.5 / 14.7    12 000 (16): 27.7 / 24.8                  30 000 (39): 44.6 / 52.1
 //   batch 4, 4 CTAs:  250: 11.4 / 7.3          4 096: 23.9 / 17.5    12 000 (23): 36.1 / 34.0                  30 000 (58): 68.7 / 77.4

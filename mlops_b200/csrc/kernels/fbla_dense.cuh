@@ -14,8 +14,9 @@
 // arithmetic runs once per eight (sub-block, query) columns on full warps. Semantics, formats and the definition of every
 // number are fbla_decode.cuh's; only the order of the sums differs.
 // Work is dealt in contiguous runs of the flattened (virtual head, group, piece of a group) list: first to CTAs, then to
-// the CTA's warps, so that a head's partial rows are one per CTA, folded in warp order (reproducible bit for bit).
-// Bound by instruction issue: see the figures at the two passes.
+// the CTA's warps, so that a head's partial rows are one per CTA, folded in warp order (reproducible bit for bit). Short rows: every head
+// has CTAs of its own, and one kernel does both passes and the output rows (head_passes).
+// Bound by latency: four warps per scheduler issue 0.44 to 0.5 instructions per cycle, waiting for loads and for their own results.
 #pragma once
 #include "fbla_decode.cuh"
 
