@@ -863,7 +863,7 @@ int mlops_fbla_item_access(const mlops_fbla_items *passes, int npasses, int pass
       for (int h = 0; h < heads; ++h) head_windows(r, h, 0, true, true);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 1, lse, part - lse);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 1, part, dpart - part);
-      r.add(MLOPS_FBLA_ARG_SCRATCH, 1, status, 16);
+      r.add(MLOPS_FBLA_ARG_SCRATCH, 1, dpart + (long long)x * 4, 4);  // (the CTA's report word)
     } else if (p.kind == MLOPS_FBLA_ITEM_SELECT) {
       const long long per = (long long)a.nblocks * a.qg * 4;
       r.add(MLOPS_FBLA_ARG_SCRATCH, 0, lse + y * per, per);
@@ -871,6 +871,10 @@ int mlops_fbla_item_access(const mlops_fbla_items *passes, int npasses, int pass
       r.add(MLOPS_FBLA_ARG_SCRATCH, 1, row_r + (long long)y * a.qg * 4, a.qg * 4);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 1, counts + ((long long)y * a.nslices + x) * 4, 4);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 1, items + ((long long)y * a.nslices + x) * FBLA_K_SLICE * 4, FBLA_K_SLICE * 4);
+      if (x == 0 && y == 0) {
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 0, dpart, (long long)a.coarse_ctas * 4);
+        r.add(MLOPS_FBLA_ARG_SCRATCH, 1, status, 16);
+      }
     } else if (p.kind == MLOPS_FBLA_ITEM_REFINE) {
       r.add(MLOPS_FBLA_ARG_SCRATCH, 0, row_r, (long long)vheads * a.qg * 4);
       r.add(MLOPS_FBLA_ARG_SCRATCH, 0, counts, (long long)vheads * a.nslices * 4);

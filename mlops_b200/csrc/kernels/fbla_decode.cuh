@@ -218,8 +218,13 @@ __device__ __forceinline__ Split split_of(const fbla_k_decode &a, int hpr) {
   return Split{total - xw, xw};
 }
 
+// A wait of pass 1 (coarse) or 3 (refine) gave up. The coarse pass's CTAs report in a word of their own each, which they clear themselves: a
+// status word cleared by one of them would not be ordered against the others' reports (a plan's items run in any order). The words lie
+// in dpart, which nothing else uses before the refine pass; the select pass makes the status word of them.
+__device__ __forceinline__ int *coarse_reports(const fbla_k_decode &a) { return reinterpret_cast<int *>(a.dpart); }  // [coarse_ctas]
 __device__ __forceinline__ void report(const fbla_k_decode &a, int pass) {
-  if (a.status) { atomicCAS(a.status, 0, pass); a.status[1] = FBLA_POS::x(); }
+  if (pass == 1) coarse_reports(a)[FBLA_POS::x()] = 1;
+  else if (a.status) { atomicCAS(a.status, 0, pass); a.status[1] = FBLA_POS::x(); }
 }
 
 // ---- the BF16 windows ---------------------------------------------------------------------------------------------------
@@ -666,7 +671,8 @@ __device__ __forceinline__ void coarse_item(const fbla_k_decode &a, uint8_t *sme
   smem_raw += (128u - (smem_u32(smem_raw) & 127u)) & 127u;  // (an executor's storage is 16-byte aligned; an offset keeps the pointer's address space known)
   CoarseSmem<CB, SHAPE> &sm = *reinterpret_cast<CoarseSmem<CB, SHAPE> *>(smem_raw);
   const int lane = FBLA_POS::tid() & 31, warp = FBLA_POS::tid() >> 5;
-  if (FBLA_POS::x() == 0 && FBLA_POS::tid() == 0 && a.status) { a.status[0] = 0; a.status[1] = 0; }
+  if (FBLA_POS::tid() == 0) coarse_reports(a)[FBLA_POS::x()] = 0;
+  __syncthreads();  // (ahead of every report of this CTA)
   const int hpr = a.kv_heads * a.vg;
   int sw = Sh::TOTAL;                 // streaming warps of this CTA
   long long gw, lo, hi;               // the warp's index among the grid's streaming warps and its run of the flattened groups
@@ -823,6 +829,12 @@ __device__ __forceinline__ void select_item(const fbla_k_decode &a, uint8_t *sme
     const float *p = a.lse + ((size_t)vh * a.nblocks + (closed ? sb : 0)) * QG;
 #pragma unroll
     for (int qi = 0; qi < QG; ++qi) x[i][qi] = closed ? __ldcg(p + qi) : -FBLA_INF;
+  }
+  if (vh == 0 && slice == 0 && warp == 7 && a.phase != 2 && a.status) {  // the coarse pass's reports (the second phase of a shard keeps the first one's)
+    int who = -1;
+    for (int i = lane; i < a.coarse_ctas; i += 32) who = __ldcg(coarse_reports(a) + i) ? i : who;
+    who = __reduce_max_sync(FULL, who);
+    if (!lane) { a.status[0] = who >= 0; a.status[1] = max(who, 0); }
   }
   if (a.phase == 2) {  // the rows' (global) log2 mass is given
     if (FBLA_POS::tid() < QG) R[FBLA_POS::tid()] = __ldcg(a.row_r + vh * QG + FBLA_POS::tid());

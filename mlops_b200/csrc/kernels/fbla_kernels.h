@@ -25,7 +25,8 @@ typedef struct {
 //   lse    [VH][nblocks][qg]  float  log2 mass of every closed sub-block under the coarse scores (two sweeps: then the weights, fbla_dense.cuh)
 //   part   [2 TW + 2 VH][qg][132] float  (o[128], m, l) partials: slot w + vh for streaming warp (or, folded, CTA) w,
 //          coarse_ctas * coarse_warps + VH + x + vh for window warp x; TW = coarse_ctas * coarse_warps
-//   dpart  [RW + VH][qg][132] float  (do[128], dl) corrections of refine warp (or, folded, CTA) w at slot w + vh
+//   dpart  [RW + VH][qg][132] float  (do[128], dl) corrections of refine warp (or, folded, CTA) w at slot w + vh; before that pass its first
+//          words are the coarse CTAs' reports (nonzero: a bounded wait gave up)
 //   row_r  [VH][qg]           float  log2 of the row's total coarse mass
 //   counts [VH][nslices]      int    selected sub-blocks per slice of 1024 sub-blocks
 //   items  [VH][nslices][1024] int   (sub-block << 4) | query mask, in sub-block order

@@ -88,16 +88,18 @@ def item_call(lib, p):
     return buf.value.decode()
 
 
-def run_plan(lib, passes, n, stream, ctas=None, around=None):
+def run_plan(lib, passes, n, stream, ctas=None, around=None, edit=None):
     """Compiles one kernel per pass and launches them in order on `stream` (a CUDA stream handle): an executor whose only
     dependency rule is 'every item of a pass after every item of the pass before' (stream order). ctas: run every pass
-    as a persistent loop on that many CTAs instead of one CTA per item. around(i): a context manager for pass i."""
+    as a persistent loop on that many CTAs instead of one CTA per item. around(i): a context manager for pass i. edit(i, call):
+    the statements that take the place of the call of pass i."""
     import contextlib
 
     import numpy as np
     import torch
     from cuda.bindings import driver
-    src = POLICY + "".join(kernel_source(f"pass_{i}", passes[i].threads, item_call(lib, passes[i]), None if ctas is None else passes[i].items)
+    calls = [item_call(lib, passes[i]) for i in range(n)]
+    src = POLICY + "".join(kernel_source(f"pass_{i}", passes[i].threads, edit(i, calls[i]) if edit else calls[i], None if ctas is None else passes[i].items)
                            for i in range(n))
     cubin = compile_program(src)
     err, module = driver.cuModuleLoadData(cubin)

@@ -125,6 +125,38 @@ def test_decode_passes_read_what_they_declare(ours, mode, N, cap):
     assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("given_up", [False, True])
+def test_a_report_of_the_coarse_pass_outlasts_its_other_items(ours, mode, given_up):
+    """The coarse pass's items run in any order: here the last one first, and it reports (as after a wait that gave up) before the others run.
+    The rows are then not plausible numbers, and the status word names the pass."""
+    QH, KH, N, cap = 8, 2, 3000, 163840
+    q, k, v = datagen.baseline_case(45, 1, QH, KH, N)
+    qd = gu.bf16_tensor(q)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=cap)
+    length, out = _i32(N), torch.full_like(qd, -9.0)
+    want = ours.decode_at(c, qd, length)
+    lib, vp, kc, passes = ours.lib, ctypes.c_void_p, ours._cache(c), (iu.Items * 4)()
+    nbytes = lib.mlops_fbla_decode_scratch_bytes(ctypes.byref(gu.Config(1, QH, KH, cap, 0, 0, gu.FORMATS[mode][2], cap, 0, 0, 0, 0, 0)))
+    scratch = torch.full((nbytes,), 0xA5, dtype=torch.uint8, device="cuda")
+    assert lib.mlops_fbla_decode_at_items(ctypes.byref(_cfg(c, QH)), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
+                                          vp(scratch.data_ptr()), ctypes.c_size_t(nbytes), 0, passes, 4) == 4, ours.error()
+    assert passes[0].entry.startswith(b"fbla::coarse_item")
+
+    def edit(i, call):
+        if i:
+            return call
+        call = call.replace("position(item,", f"position({passes[0].items - 1} - item,")
+        return call + (" __syncthreads(); if (item == 0 && threadIdx.x == 0) fbla::report(*reinterpret_cast<const fbla_k_decode *>(args), 1);" if given_up else "")
+
+    iu.run_plan(lib, passes, 4, _stream(), ctas=1, edit=edit)
+    status = scratch[passes[0].geom[4]:][:16].view(torch.int32).tolist()
+    if given_up:
+        assert torch.isnan(out.float()).all() and status[:2] == [1, passes[0].items - 1]
+    else:
+        assert torch.equal(out, want) and status[:2] == [0, 0]
+
+
 @pytest.mark.parametrize("mode,count,ctas", [("4+2", 300, None), ("3+3", 5, None), ("3+3", 700, 3)])
 def test_prefill_plan_equals_prefill_at(ours, mode, count, ctas):
     """count 300 / 700: the tensor-core pass (TC) -- with ctas = 3 as a persistent loop, so that one CTA runs several
