@@ -855,6 +855,7 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
         VWords<CB> na, nb;
         VWords<FB> ma, mb;
         if constexpr (AHEAD) {
+          __syncwarp();  // (every lane has read the tails of the pair before: the next one's take their place)
           if (left > 1) {
             if (last) move_on();
             load_coarse(na, nb, turn ^ 1);

@@ -66,11 +66,12 @@ def gu_group(ratio):
     return ratio if ratio in (1, 2, 4) else 4 if ratio % 4 == 0 else 2 if ratio % 2 == 0 else 1
 
 
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
 @pytest.mark.parametrize("B,QH,KH,N,ctas", [OWN[2], OWN[3], OWN[5], OWN[10]])
-def test_own_ctas_lengths_and_plans(ours, oracle, B, QH, KH, N, ctas):
+def test_own_ctas_lengths_and_plans(ours, oracle, mode, B, QH, KH, N, ctas):
     """Rows shorter than the room (down to one token, no closed group), each against its own decode in a cache of the same room; the plan's
     passes bit for bit the stream call, one CTA per item and as loops of three."""
-    mode, lens = "4+2", [max(1, N * i // B - 3 * i) for i in range(B)]
+    lens = [max(1, N * i // B - 3 * i) for i in range(B)]
     q, k, v = datagen.uneven_case(21, B, QH, KH, N)
     qd = gu.bf16_tensor(q)
     c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=N)
@@ -113,6 +114,57 @@ def test_dense_ragged_rows(ours, oracle, lens):
     want = oracle.decode(q, o, lengths=np.array(lens, np.int32))
     for b in range(B):
         gu.check_close(gu.bits_of(got)[b], want[b], f"row {b} of {lens}")
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("QH,KH,lens,tau,scale", [(40, 40, [1, 2000, 129, 16], 0.0, 0.0), (80, 40, [1, 2000, 129, 16], 0.0, 0.0), (160, 40, [1, 2000, 129, 16], 0.0, 0.0),
+                                                  (160, 40, [300] * 3 + [1], 0.0, 0.0), (120, 10, [256, 257, 1300, 255, 31], 0.0, 0.0),  # (three virtual heads per KV head)
+                                                  # some sub-blocks selected; even masses: all of the short rows', none of the longest one's
+                                                  (40, 40, [256, 257, 4000, 255], 5e-3, 0.0), (80, 40, [256, 257, 4000, 255], 5e-3, 0.0), (160, 40, [256, 257, 4000, 255], 5e-3, 0.0),
+                                                  (40, 40, [385, 4000, 512, 31], 5e-3, 1e-3), (80, 40, [385, 4000, 512, 31], 5e-3, 1e-3), (160, 40, [385, 4000, 512, 31], 5e-3, 1e-3)])
+def test_ragged_rows_dealt_over_all_ctas(ours, oracle, mode, QH, KH, lens, tau, scale):
+    """Two sweeps whose groups are dealt over all CTAs (more virtual heads than SMs): rows without a closed group and of one token, in both
+    formats with one, two and four queries; the plan's passes bit for bit the stream call, one CTA per item or as loops of three."""
+    B, cap, vp, passes = len(lens), 4096, ctypes.c_void_p, (iu.Items * 4)()
+    q, k, v = datagen.uneven_case(31 + QH, B, QH, KH, max(lens))
+    c, o, qd = ours.empty(B, KH, cap, mode), oracle.empty(B, KH, cap, mode), gu.bf16_tensor(q)
+    for b, n in enumerate(lens):
+        row = ours.encode(gu.bf16_tensor(k[b:b + 1, :, :n]), gu.bf16_tensor(v[b:b + 1, :, :n]), mode, capacity=cap)
+        for key in ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v"):
+            c[key][b].copy_(row[key][0])
+        orow = gu.cache_to_numpy(row)  # (the encode's bytes have tests of their own)
+        for key in ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v"):
+            o[key][b * KH:(b + 1) * KH] = orow[key].reshape(o[key][b * KH:(b + 1) * KH].shape)
+    entry = first_entry(ours, c, qd, mode, tau, 1)
+    assert entry.startswith("fbla::dense::score_item") and not entry.endswith(", true>")
+    length = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    got = ours.decode_at(c, qd, length, length_stride=1, tau=tau, scale=scale)
+    torch.cuda.synchronize()
+    o["tokens"] = max(lens)
+    want = oracle.decode(q, o, lengths=np.array(lens, np.int32), tau=tau, scale=scale)
+    for b in range(B):
+        gu.check_close(gu.bits_of(got)[b], want[b], f"row {b} of {lens}")
+    cfg, kc = gu.Config(B, QH, KH, 0, scale, tau, gu.FORMATS[mode][2], cap, 0, 0, 0, 0, 1), ours._cache(c)
+    scratch, out = ours.scratch(dict(c, tokens=cap), QH), torch.empty_like(qd)
+    assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
+                                               vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
+    iu.run_plan(ours.lib, passes, 4, torch.cuda.current_stream().cuda_stream, 3 if scale else None)
+    assert torch.equal(out, got)
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+@pytest.mark.parametrize("QH,KH,cap,N,tau", [(24, 24, 14900, 385, 1e-4), (16, 8, 40000, 9001, 1e-4), (4, 1, 40000, 20011, 1e-4), (24, 2, 40000, 700, 1e-4), (32, 8, 30000, 30000, 1e-3)])
+def test_a_room_beyond_one_kernel(ours, oracle, mode, QH, KH, cap, N, tau):
+    """Two sweeps over few heads, dealt over all CTAs because the room is too large for a head's own: host and device lengths the same bits"""
+    q, k, v = datagen.baseline_case(17 + N, 1, QH, KH, N)
+    qd = gu.bf16_tensor(q)
+    c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=cap)
+    entry = first_entry(ours, c, qd, mode, tau)
+    assert entry.startswith("fbla::dense::score_item") and not entry.endswith(", true>")
+    got = ours.decode(c, qd, tau=tau)
+    assert torch.equal(got, ours.decode_at(c, qd, torch.tensor([N], dtype=torch.int32, device="cuda"), tau=tau))
+    torch.cuda.synchronize()
+    gu.check_close(gu.bits_of(got), oracle.decode(q, oracle.encode(k, v, mode, capacity=cap), tau=tau), f"{mode} {N} of {cap}")
 
 
 def first_entry(ours, c, qd, mode, tau, length_stride=0):
