@@ -319,6 +319,7 @@ __device__ __forceinline__ void write_chunk(const fbla_k_prefill &a, uint8_t *sm
     const int g = closing_group(ch, (at >> 1) - bh * blocks);
     if (g < 0 || g * G < ch.n0) return false;
     if (tid == 0 && !sm.failed) {
+      fence_async_smem();  // (the buffer's rows have been read, behind a barrier)
       mbar_expect_tx(&sm.bar, sizeof sm.in);
       bulk_g2s(sm.in, ((at & 1) ? a.v : a.k) + (size_t)bh * a.count * D + (size_t)(g * G - ch.n0) * D, sizeof sm.in, &sm.bar);
     }
