@@ -59,3 +59,27 @@ def test_many_units_per_cta(oracle, mode, heads, n, n0):
     for a in ARRAYS:
         x, y = getattr(c, a).view(torch.uint8).cpu().numpy().reshape(-1), want[a].view("uint8").reshape(-1)
         assert x.size == y.size and (x == y).all(), a
+
+
+@pytest.mark.parametrize("mode", ["3+3", "4+2"])
+def test_values_that_are_not_numbers_or_infinite(oracle, mode):
+    """Records and metadata byte for byte the oracle's where channels hold NaN (code 0, not part of the range) and infinities (no step: code 0)"""
+    heads, n = 8, 12300
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    k, v = (torch.randn((1, heads, n, 128), generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    for x in (k, v):
+        rare = torch.rand((1, heads, n), generator=gen, device="cuda") < 0.03
+        x[..., 5] = torch.where(rare, float("nan"), x[..., 5])
+        x[..., 70] = torch.where(rare, float("inf"), x[..., 70])
+        x[..., 99] = torch.where(rare, float("-inf"), x[..., 99])
+        x[..., 100] = torch.where(rare, float("nan"), x[..., 99])
+        x[:, :, 256:384, 31] = float("nan")
+        x[:, :, 256:384, 32] = float("-inf")
+    c = attention.empty(1, heads, n, mode)
+    attention.append(c, k, v)
+    bits = lambda x: x.view(torch.int16).cpu().numpy().view("uint16")  # noqa: E731
+    want = oracle.encode(bits(k), bits(v), mode)
+    for a in ARRAYS:
+        x, y = getattr(c, a).view(torch.uint8).cpu().numpy().reshape(-1), want[a].view("uint8").reshape(-1)
+        assert x.size == y.size and (x == y).all(), a
