@@ -47,6 +47,28 @@ template <int CB, int FB, int QG> struct Kernels {
     if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = 1;
     return e;
   }
+  // clusters of `ctas` (1 .. 16) that are at work at once (0: such a cluster cannot be placed); asked for once per device and host thread, as
+  // the attributes (every call: 0.3 us of a 12 us decode)
+  static int clusters(int ctas) {
+    static thread_local short held[64][17] = {};  // the answer + 1
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    const bool known = dev >= 0 && dev < 64;
+    if (known && held[dev][ctas]) return held[dev][ctas] - 1;
+    if (configure() != cudaSuccess) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas); cfg.blockDim = dim3(32 * SCORE_WARPS); cfg.dynamicSmemBytes = sizeof(HeadSmem);
+    cudaLaunchAttribute size = {};
+    size.id = cudaLaunchAttributeClusterDimension;
+    size.val.clusterDim.x = ctas; size.val.clusterDim.y = size.val.clusterDim.z = 1;
+    cfg.attrs = &size; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, head_kernel<CB, FB, QG>, &cfg) != cudaSuccess) {
+      cudaGetLastError();  // (not the call's: it takes three kernels)
+      n = 0;
+    }
+    if (known) held[dev][ctas] = (short)(n + 1);
+    return n;
+  }
   static cudaError_t whole(fbla_k_decode a, bool dependent, cudaStream_t stream) {
     a.mass_given = 0;
     return launch(dependent, a.head_ctas, head_kernel<CB, FB, QG>, dim3(a.head_ctas, a.kv_heads * a.vg, a.batch), 32 * SCORE_WARPS, sizeof(HeadSmem), stream, a);
@@ -99,7 +121,7 @@ template <int CB, int FB, int QG> struct Kernels {
   }
 };
 
-template <class F> cudaError_t dispatch(const fbla_k_decode &a, F f) {
+template <class F> auto dispatch(const fbla_k_decode &a, F f) {
   if (a.cb == 3) return a.qg == 1 ? f(Kernels<3, 3, 1>{}) : a.qg == 2 ? f(Kernels<3, 3, 2>{}) : f(Kernels<3, 3, 4>{});
   return a.qg == 1 ? f(Kernels<4, 2, 1>{}) : a.qg == 2 ? f(Kernels<4, 2, 2>{}) : f(Kernels<4, 2, 4>{});
 }
@@ -159,4 +181,12 @@ extern "C" int fbla_k_head_ctas(int vheads, long long tokens) {
   for (const auto &h : held)
     if (vheads <= h.vheads) return (tokens + fbla::G - 1) / fbla::G <= (h.ctas == 16 ? 16 : 20) * h.ctas ? h.ctas : 0;
   return 0;
+}
+// (the table is a whole B200's; where fewer clusters than heads run at once, or none can be placed, three kernels are the way that always runs)
+extern "C" int fbla_k_head_choice(const fbla_k_decode *a, int vheads, long long tokens, int (*held)(const fbla_k_decode *a, int ctas)) {
+  const int ctas = fbla_k_head_ctas(vheads, tokens);
+  return ctas > 0 && held(a, ctas) >= vheads ? ctas : 0;
+}
+extern "C" int fbla_k_head_clusters(const fbla_k_decode *a, int ctas) {
+  return fbla::dense::dispatch(*a, [&](auto k) { return decltype(k)::clusters(ctas); });
 }

@@ -83,6 +83,23 @@ def test_short_rows_have_ctas_of_their_own_heads(lib):
     assert [ctas(v, 1) for v in (1, 8, 15, 16, 26, 32, 45, 64, 148)] == [16, 10, 8, 6, 5, 4, 3, 2, 1]
 
 
+def test_one_kernel_needs_a_device_that_holds_its_clusters(lib):
+    """A device that holds fewer clusters than there are heads runs the three kernels."""
+    asked = []
+
+    def choice(vheads, tokens, held):
+        fn = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_int)(lambda a, ctas: asked.append(ctas) or held(ctas))
+        return lib.fbla_k_head_choice(None, vheads, ctypes.c_longlong(tokens), fn)
+    for vheads in list(range(1, 150)) + [1000]:
+        for tokens in (1, 4096, 30000):
+            c = lib.fbla_k_head_ctas(vheads, ctypes.c_longlong(tokens))
+            del asked[:]
+            assert choice(vheads, tokens, lambda ctas: 1000) == choice(vheads, tokens, lambda ctas: vheads) == c
+            assert choice(vheads, tokens, lambda ctas: vheads - 1) == choice(vheads, tokens, lambda ctas: 0) == 0
+            assert asked == [c] * 4 if c else not asked  # (no query for what takes three kernels anyway)
+    assert choice(8, 4096, lambda ctas: 8 if ctas <= 8 else 0) == 0  # (ten CTAs: beyond the portable size)
+
+
 def test_the_shape_follows_the_groups_a_warp_streams(lib):
     """Eight warps with a whole group in flight where twelve would not leave a warp less than three quarters of the groups."""
     deep = lambda batch, heads, qg, tokens: lib.fbla_k_decode_deep_of(batch, heads, 1, qg, ctypes.c_longlong(tokens))  # noqa: E731
