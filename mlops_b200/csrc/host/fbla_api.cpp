@@ -218,7 +218,8 @@ mlops_fbla_status make_decode(const char *fn, const mlops_fbla_config *c, const 
   a.dense = m.two && fbla_k_two_sweeps(c->batch, c->batch * c->kv_heads * a.vg, a.qg, typical_tokens(room, c->length_stride != 0), wants_output ? threshold : usual_tau(c));
   // a short one is one kernel, with CTAs of every head's own (by the room too: their number decides the order of the sums)
   if (a.dense && wants_output) {
-    const int vheads = c->batch * c->kv_heads * a.vg, each = fbla_k_head_choice(&a, vheads, room, fbla_k_head_clusters);
+    const int vheads = c->batch * c->kv_heads * a.vg, own_lengths = c->length_stride != 0 && c->batch > 1;
+    const int each = fbla_k_head_choice(&a, vheads, a.qg, own_lengths, room, fbla_k_head_clusters);
     if (each > 0 && each * vheads <= a.coarse_ctas) {
       a.head_ctas = (char)each;
       a.coarse_ctas = each * vheads;

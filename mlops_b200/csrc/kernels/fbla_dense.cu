@@ -165,27 +165,39 @@ extern "C" int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens
 
 // A short decode is mostly launches and the chains of round trips at their borders. One kernel with a cluster per virtual head has neither,
 // but its heads' CTAs leave SMs idle and a head's work cannot move to another's. CTAs per head: as many as let all clusters run at once (of n
-// CTAs with an SM each a B200 holds n: 1: 148, 2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 8: 15, 10: 11, 16: 7). Groups per CTA up to which it is the
-// faster way (the room's: rows of lengths of their own wait for the longest). Device time on B200, us, three kernels / one, 3+3, 32 / 8 heads
-// unless said, when the line was set (3+3 has become faster on both sides since: 4 096 tokens in one kernel 11.8):
-//   batch 1, 10 CTAs: 250 tokens 11.0 / 7.2    4 096: 18.7 / 12.4    12 000 (9 groups per CTA): 21.9 / 19.7    30 000 (23): 31.1 / 31.3    80 000: 52 / 77
-//   batch 2, 6 CTAs:  250: 11.2 / 7.3          4 096: 20.5 / 14.7    12 000 (16): 27.7 / 24.8                  30 000 (39): 44.6 / 52.1
-//   batch 4, 4 CTAs:  250: 11.4 / 7.3          4 096: 23.9 / 17.5    12 000 (23): 36.1 / 34.0                  30 000 (58): 68.7 / 77.4
-//   batch 9, 2 CTAs:  250: 12.2 / 8.1          4 000: 31.8 / 24.6    8 000 (31): 49.5 / 47.3
-//   batch 12, 1 CTA:  250: 12.8 / 8.7          2 000 (14): 27.7 / 23.8    4 000 (30): 37.7 / 41.3
-//   8 / 2 heads, 16:  250: 8.6 / 6.9           4 096: 18.8 / 11.0    12 000 (6): 21.1 / 16.0    30 000 (15): 24.8 / 23.7    80 000 (39): 31.8 / 42.7
-//   4+2, batch 1:     4 096: 18.1 / 11.6       30 000: 27.8 / 26.2    batch 4: 12 000: 32.2 / 28.6    batch 8, 2 CTAs: 12 000 (47): 50.6 / 53.1
-//   rows of their own lengths, batch 8: 1 000 to 4 000 (16): 30.2 / 26.0    300 to 8 000 (32): 39.4 / 43.2
+// CTAs with an SM each a B200 holds n: 1: 148, 2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 8: 15, 10: 11, 16: 7). At most 20 groups per CTA of the room, 16 in
+// clusters of 16. Device time on B200 behind a flush of L2, us, three kernels / one, 3+3, by heads and queries per head:
+//   8 heads, 10 CTAs, 4:   3 groups per CTA 25.6 / 19.0    8: 31.8 / 24.4    13: 33.5 / 28.8    17: 35.9 / 32.9    20: 37.9 / 35.0    24: 37.9 / 38.9    (4+2  20: 36.2 / 34.5)
+//   16 heads, 6 CTAs, 4:   3: 25.6 / 18.7    8: 29.7 / 24.8    13: 35.6 / 30.6    20: 37.9 / 36.4    (4+2  20: 37.9 / 35.1)
+//   33 heads, 4 CTAs, 4:   3: 27.6 / 18.7    13: 37.9 / 30.7    20: 44.3 / 38.6    24: 46.9 / 43.0
+//   74 heads, 2 CTAs, 4:   3: 25.6 / 20.5    13: 37.9 / 32.8    20: 45.8 / 40.9    2: 20: 44.5 / 43.0    148, 1 CTA, 4: 20: 48.4 / 42.7
+//   75 heads, 1 CTA, 4:    3: 25.6 / 20.6    13: 33.8 / 30.9    17: 35.8 / 34.6    20: 37.2 / 38.8       7 heads, 16 CTAs, 4: 17: 37.9 / 34.9
 extern "C" int fbla_k_head_ctas(int vheads, long long tokens) {
   static const struct { int ctas, vheads; } held[] = {{16, 7}, {10, 11}, {8, 15}, {6, 22}, {5, 26}, {4, 33}, {3, 45}, {2, 74}, {1, 148}};
   for (const auto &h : held)
     if (vheads <= h.vheads) return (tokens + fbla::G - 1) / fbla::G <= (h.ctas == 16 ? 16 : 20) * h.ctas ? h.ctas : 0;
   return 0;
 }
-// (the table is a whole B200's; where fewer clusters than heads run at once, or none can be placed, three kernels are the way that always runs)
-extern "C" int fbla_k_head_choice(const fbla_k_decode *a, int vheads, long long tokens, int (*held)(const fbla_k_decode *a, int ctas)) {
-  const int ctas = fbla_k_head_ctas(vheads, tokens);
-  return ctas > 0 && held(a, ctas) >= vheads ? ctas : 0;
+// Fewer groups where the one kernel falls behind sooner: rows of lengths of their own (it waits for the longest; the three kernels deal what there
+// is over all SMs), the more the more SMs its clusters leave idle; and one query per head, where a unit is a whole group, so that a CTA whose
+// groups and window sub-blocks are more than its warps does them in two goes (`one`: what still fits). us, three kernels / one (and, 4+2, as
+// three kernels were before there was one); rows evenly spread from a tenth of the room up to it:
+//   8 heads, 10 CTAs, 4 queries:  13 groups per CTA 31.7 / 28.7    17: 30.7 / 32.3    20: 31.8 / 34.4       75 heads, 1 CTA:  13: 29.7 / 30.5    20: 31.5 / 36.3
+//   8 heads, 2 queries:           12: 29.7 / 28.5    17: 30.0 / 33.8     75 heads:  10: 27.7 / 28.7    20: 31.1 / 37.9    27 heads, 4 CTAs:  12: 31.8 / 28.7    17: 34.8 / 34.9
+//   8 heads, 1 query:             9: 29.7 / 28.7     13: 31.8 / 31.5     17: 32.8 / 38.9 (4+2 31.7 / 40.5, 32)            148 heads, 1 CTA: 13: 39.9 / 35.0    16: 38.0 / 38.7
+//   27 heads, 4 CTAs, 1 query:    12: 33.8 / 32.5    13: 32.4 / 36.8 (4+2 31.8 / 38.6, 33)     75 heads:  9: 29.7 / 29.6    20: 33.8 / 45.0 (4+2 31.8 / 45.1, 34)
+// One length, 1 query:  75 heads: 15: 37.9 / 36.7    20: 40.9 / 45.1    46 heads, 2 CTAs: 10: 35.8 / 30.8    13: 33.8 / 36.7    8 heads: 14: 33.8 / 32.9    15: 33.8 / 36.9    16 heads: 20: 42.0 / 41.3
+// Last, where fewer clusters than heads run at once, or none can be placed, the three kernels are the way that always runs.
+extern "C" int fbla_k_head_choice(const fbla_k_decode *a, int vheads, int qg, int own_lengths, long long tokens, int (*held)(const fbla_k_decode *a, int ctas)) {
+  const int ctas = fbla_k_head_ctas(vheads, tokens), busy = ctas * vheads;
+  if (ctas == 0) return 0;
+  const bool few = busy < 96;  // SMs at work
+  const int one = ctas == 16 ? 15 : ctas >= 8 ? 14 : ctas == 6 ? 13 : ctas >= 4 ? 12 : ctas >= 2 ? 10 : 15;
+  const int line = !own_lengths ? (qg == 1 && few ? one : 20)
+                   : qg == 4    ? (few ? 16 : 20)
+                   : qg == 2    ? (few ? 12 : busy < 132 ? 16 : 20)
+                                : (few ? 9 : one);
+  return (tokens + fbla::G - 1) / fbla::G <= (long long)line * ctas && held(a, ctas) >= vheads ? ctas : 0;
 }
 extern "C" int fbla_k_head_clusters(const fbla_k_decode *a, int ctas) {
   return fbla::dense::dispatch(*a, [&](auto k) { return decltype(k)::clusters(ctas); });

@@ -88,8 +88,9 @@ static inline __host__ __device__ size_t fbla_k_two_cells(size_t vheads, int nbl
 FBLA_HOST_API(int fbla_k_two_sweeps(int batch, int vheads, int qg, long long tokens, float tau);)
 // CTAs per virtual head of a decode in two sweeps that may run as one kernel; 0: it runs as three (pure host arithmetic)
 FBLA_HOST_API(int fbla_k_head_ctas(int vheads, long long tokens);)
-// the same where held(a, ctas) clusters of that many CTAs are at work at once: 0 if the heads are more
-FBLA_HOST_API(int fbla_k_head_choice(const fbla_k_decode *a, int vheads, long long tokens, int (*held)(const fbla_k_decode *a, int ctas));)
+// whether it does, for heads of qg queries and rows of one length or of lengths of their own, where held(a, ctas) clusters of that many CTAs are at
+// work at once: its CTAs per head, or 0
+FBLA_HOST_API(int fbla_k_head_choice(const fbla_k_decode *a, int vheads, int qg, int own_lengths, long long tokens, int (*held)(const fbla_k_decode *a, int ctas));)
 // `held` of the current device
 FBLA_HOST_API(int fbla_k_head_clusters(const fbla_k_decode *a, int ctas);)
 // the dense passes (0 scores, 1 rows' masses, 2 values, 3 merge): a whole decode or shard phase; one pass (of a decode in one kernel: 0 all of it)

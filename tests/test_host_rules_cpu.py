@@ -83,21 +83,41 @@ def test_short_rows_have_ctas_of_their_own_heads(lib):
     assert [ctas(v, 1) for v in (1, 8, 15, 16, 26, 32, 45, 64, 148)] == [16, 10, 8, 6, 5, 4, 3, 2, 1]
 
 
+def head_choice(lib, vheads, qg, own_lengths, tokens, held=lambda ctas: 1000):
+    fn = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_int)(lambda a, ctas: held(ctas))
+    return lib.fbla_k_head_choice(None, vheads, qg, own_lengths, ctypes.c_longlong(tokens), fn)
+
+
 def test_one_kernel_needs_a_device_that_holds_its_clusters(lib):
     """A device that holds fewer clusters than there are heads runs the three kernels."""
     asked = []
-
-    def choice(vheads, tokens, held):
-        fn = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_int)(lambda a, ctas: asked.append(ctas) or held(ctas))
-        return lib.fbla_k_head_choice(None, vheads, ctypes.c_longlong(tokens), fn)
     for vheads in list(range(1, 150)) + [1000]:
         for tokens in (1, 4096, 30000):
             c = lib.fbla_k_head_ctas(vheads, ctypes.c_longlong(tokens))
             del asked[:]
-            assert choice(vheads, tokens, lambda ctas: 1000) == choice(vheads, tokens, lambda ctas: vheads) == c
-            assert choice(vheads, tokens, lambda ctas: vheads - 1) == choice(vheads, tokens, lambda ctas: 0) == 0
+            for held, want in [(1000, c), (vheads, c), (vheads - 1, 0), (0, 0)]:
+                assert head_choice(lib, vheads, 4, 0, tokens, lambda ctas: asked.append(ctas) or held) == want
             assert asked == [c] * 4 if c else not asked  # (no query for what takes three kernels anyway)
-    assert choice(8, 4096, lambda ctas: 8 if ctas <= 8 else 0) == 0  # (ten CTAs: beyond the portable size)
+    assert head_choice(lib, 8, 4, 0, 4096, lambda ctas: 8 if ctas <= 8 else 0) == 0  # (ten CTAs: beyond the portable size)
+
+
+@pytest.mark.parametrize("qg", [1, 2, 4])
+def test_rows_of_their_own_lengths_leave_one_kernel_earlier(lib, qg):
+    """One line per head count, never beyond that of rows of one length; shapes on which the one kernel was measured the slower way take three."""
+    line = {}
+    for vheads in range(1, 149):
+        for own in (0, 1):
+            picks = [head_choice(lib, vheads, qg, own, n) for n in range(1, 60000, 127)]
+            assert set(picks) <= {picks[0], 0} and picks[0] and picks == sorted(picks, reverse=True)
+            line[vheads, own] = sum(p > 0 for p in picks)
+        assert line[vheads, 1] <= line[vheads, 0] and (qg == 1 or line[vheads, 0] == sum(lib.fbla_k_head_ctas(vheads, ctypes.c_longlong(n)) > 0 for n in range(1, 60000, 127)))
+    # (heads, groups per CTA) that were slower, and that were not
+    slower = {4: [(75, 20), (8, 17)], 2: [(75, 17), (8, 17), (46, 17)], 1: [(8, 15), (75, 11), (80, 20), (27, 13), (46, 11), (74, 13)]}[qg]
+    faster = {4: [(8, 13), (27, 20), (148, 20)], 2: [(8, 12), (33, 16), (148, 20)], 1: [(8, 9), (27, 12), (15, 14), (148, 15)]}[qg]
+    for cases, chosen in ((slower, False), (faster, True)):
+        for vheads, groups in cases:
+            ctas = lib.fbla_k_head_ctas(vheads, ctypes.c_longlong(1))
+            assert bool(head_choice(lib, vheads, qg, 1, 128 * groups * ctas)) == chosen, (vheads, groups)
 
 
 def test_the_shape_follows_the_groups_a_warp_streams(lib):
