@@ -66,12 +66,11 @@ def gu_group(ratio):
     return ratio if ratio in (1, 2, 4) else 4 if ratio % 4 == 0 else 2 if ratio % 2 == 0 else 1
 
 
-@pytest.mark.parametrize("mode", ["3+3", "4+2"])
 @pytest.mark.parametrize("B,QH,KH,N,ctas", [OWN[2], OWN[3], OWN[5], OWN[10]])
-def test_own_ctas_lengths_and_plans(ours, oracle, mode, B, QH, KH, N, ctas):
+def test_own_ctas_lengths_and_plans(ours, oracle, B, QH, KH, N, ctas):
     """Rows shorter than the room (down to one token, no closed group), each against its own decode in a cache of the same room; the plan's
     passes bit for bit the stream call, one CTA per item and as loops of three."""
-    lens = [max(1, N * i // B - 3 * i) for i in range(B)]
+    mode, lens = "4+2", [max(1, N * i // B - 3 * i) for i in range(B)]
     q, k, v = datagen.uneven_case(21, B, QH, KH, N)
     qd = gu.bf16_tensor(q)
     c = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=N)
@@ -86,6 +85,38 @@ def test_own_ctas_lengths_and_plans(ours, oracle, mode, B, QH, KH, N, ctas):
     torch.cuda.synchronize()
     for b in range(B):
         gu.check_close(gu.bits_of(got)[b:b + 1], want[b], f"row of {lens[b]}")
+    cfg, kc = gu.Config(B, QH, KH, 0, 0, 0, gu.FORMATS[mode][2], N, 0, 0, 0, 0, 1), ours._cache(c)
+    for loops in (None, 3):
+        scratch, out = ours.scratch(dict(c, tokens=N), QH), torch.empty_like(qd)
+        scratch.fill_(0xFF)
+        assert ours.lib.mlops_fbla_decode_at_items(ctypes.byref(cfg), vp(length.data_ptr()), vp(qd.data_ptr()), ctypes.byref(kc), vp(out.data_ptr()),
+                                                   vp(scratch.data_ptr()), ctypes.c_size_t(scratch.numel()), 0, passes, 4) == 4, ours.error()
+        iu.run_plan(ours.lib, passes, 4, torch.cuda.current_stream().cuda_stream, loops)
+        torch.cuda.synchronize()
+        assert torch.equal(out, got)
+
+
+@pytest.mark.parametrize("B,QH,KH,N,ctas", [OWN[2], OWN[3], OWN[5], OWN[10]])
+def test_own_ctas_lengths_and_plans_of_three_bit_words(ours, oracle, B, QH, KH, N, ctas):
+    """The same in 3+3, whose values' tails lie in shared memory"""
+    mode, lens = "3+3", [max(1, N * i // B - 3 * i) for i in range(B)]
+    q, k, v = datagen.uneven_case(21, B, QH, KH, N)
+    qd = gu.bf16_tensor(q)
+    c, o = ours.encode(gu.bf16_tensor(k), gu.bf16_tensor(v), mode, capacity=N), oracle.empty(B, KH, N, mode)
+    for b, n in enumerate(lens):
+        row = ours.encode(gu.bf16_tensor(k[b:b + 1, :, :n]), gu.bf16_tensor(v[b:b + 1, :, :n]), mode, capacity=N)
+        orow = oracle.encode(k[b:b + 1, :, :n], v[b:b + 1, :, :n], mode, capacity=N)
+        for key in ("coarse", "fine", "meta", "sink_k", "sink_v", "open_k", "open_v"):
+            c[key][b].copy_(row[key][0])
+            o[key][b * KH:(b + 1) * KH] = orow[key]
+    assert first_entry(ours, c, qd, mode, 0.0, 1).endswith(", true>")
+    length, vp, passes = torch.tensor(lens, dtype=torch.int32, device="cuda"), ctypes.c_void_p, (iu.Items * 4)()
+    got = ours.decode_at(c, qd, length, length_stride=1)
+    torch.cuda.synchronize()
+    o["tokens"] = max(lens)
+    want = oracle.decode(q, o, lengths=np.array(lens, np.int32))
+    for b in range(B):
+        gu.check_close(gu.bits_of(got)[b], want[b], f"row of {lens[b]}")
     cfg, kc = gu.Config(B, QH, KH, 0, 0, 0, gu.FORMATS[mode][2], N, 0, 0, 0, 0, 1), ours._cache(c)
     for loops in (None, 3):
         scratch, out = ours.scratch(dict(c, tokens=N), QH), torch.empty_like(qd)
