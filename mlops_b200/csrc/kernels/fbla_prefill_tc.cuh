@@ -416,41 +416,82 @@ __device__ __forceinline__ void attend_tiles(const fbla_k_prefill &a, uint8_t *s
         // the tile's qhat buffer is free once the S product of the pass before is complete
         if (k > 0) wait(sm, &sm.bar_s[X], (k - 1) & 1);
         if (g < tile_own[X]) {
-          // z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16: four of the lane's eight rows at a time, their z in registers.
-          // The lane's shares of max |z|; a butterfly over a row's 16 lanes that hands half of the rows on in each of its first two
-          // steps leaves row 2 b3 + b2 in the lanes with those bits, which form its r once.
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h) {
-            float2 z[4][4];
-            float amax[4];
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              const uint4 qv = *reinterpret_cast<const uint4 *>(sm.q[X] + qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4)));
-              z[it][0] = mul2(bf2(qv.x), make_float2(s0.x, s0.y)); z[it][1] = mul2(bf2(qv.y), make_float2(s0.z, s0.w));
-              z[it][2] = mul2(bf2(qv.z), make_float2(s1.x, s1.y)); z[it][3] = mul2(bf2(qv.w), make_float2(s1.z, s1.w));
-              amax[it] = max3_abs(max3_abs(z[it][0].x, z[it][0].y, z[it][1].x), max3_abs(z[it][1].y, z[it][2].x, z[it][2].y), fmaxf(fabsf(z[it][3].x), fabsf(z[it][3].y)));
-            }
+          // z = q * step_K, r = fl(127 / max|z|), rint(z r) written as FP16. The lane's shares of max |z|; a butterfly over a row's 16
+          // lanes that hands half of the rows on in each of its first steps leaves one row in each group of lanes, which form its r once.
+          auto place = [&](int it, int h) { return qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4)); };  // of row it + 4 h of the lane's eight
+          auto z_of = [&](int it, int h, float2 (&z)[4]) {
+            const uint4 qv = *reinterpret_cast<const uint4 *>(sm.q[X] + place(it, h));
+            z[0] = mul2(bf2(qv.x), make_float2(s0.x, s0.y)); z[1] = mul2(bf2(qv.y), make_float2(s0.z, s0.w));
+            z[2] = mul2(bf2(qv.z), make_float2(s1.x, s1.y)); z[3] = mul2(bf2(qv.w), make_float2(s1.z, s1.w));
+          };
+          auto max_of = [](const float2 (&z)[4]) { return max3_abs(max3_abs(z[0].x, z[0].y, z[1].x), max3_abs(z[1].y, z[2].x, z[2].y), fmaxf(fabsf(z[3].x), fabsf(z[3].y))); };
+          auto write = [&](int it, int h, const float2 (&z)[4], float r) {  // rint(z r) as the exact float (t - 1.5 * 2^23), then FP16 (an integer of magnitude <= 127: exact)
+            const float2 rr2 = splat(r);
+            const float2 t0 = add2(fma2(z[0], rr2, mg), ng), t1 = add2(fma2(z[1], rr2, mg), ng);
+            const float2 t2 = add2(fma2(z[2], rr2, mg), ng), t3 = add2(fma2(z[3], rr2, mg), ng);
+            *reinterpret_cast<uint4 *>(sm.qp[X] + place(it, h)) = make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
+          };
+          auto hand_on = [&](float (&amax)[4], int bit) {  // four rows to one: lane bits `bit` and bit / 2 decide which
 #pragma unroll
             for (int w = 2; w; w >>= 1) {
-              const bool up = lane & (4 * w);
+              const int o = bit * w / 2;
+              const bool up = lane & o;
 #pragma unroll
               for (int i = 0; i < w; ++i) {
                 const float keep = up ? amax[i + w] : amax[i], send = up ? amax[i] : amax[i + w];
-                amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 4 * w));
+                amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, o));
               }
             }
-            float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 2));
-            am = fmaxf(am, __shfl_xor_sync(FULL, am, 1));
-            const float rq = quotient_127(am);
-            if (!(lane & 3)) sm.qscale[k & 1][X][qrow0 + 8 * h + ((lane & 12) >> 1)] = __fmul_rn(am, sl127);  // (row qrow0 + 8 h + 2 it)
+          };
+          // Whole tiles: four rows at a time, their z in registers (2 x 4 000 tokens 714 -> 677 us). A tile's shares, whose passes are no
+          // faster so: all eight rows in one butterfly, q read twice (400 tokens behind 60 000, 32 / 8 heads 1 107 -> 1 021 us, 100 behind
+          // 20 000 163 -> 155; 4+2: 1 088 -> 1 032, 159 -> 153).
+          if constexpr (SPLIT) {  // (row 4 b3 + 2 b2 + b1 in the lanes with those bits)
+            float amax[4] = {0.f, 0.f, 0.f, 0.f}, before[4];
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              // rint(z r) as the exact float (t - 1.5 * 2^23), then FP16 (an integer of magnitude <= 127: exact)
-              const float2 rr2 = splat(__shfl_sync(FULL, rq, (lane & 16) | (4 * it)));
-              const float2 t0 = add2(fma2(z[it][0], rr2, mg), ng), t1 = add2(fma2(z[it][1], rr2, mg), ng);
-              const float2 t2 = add2(fma2(z[it][2], rr2, mg), ng), t3 = add2(fma2(z[it][3], rr2, mg), ng);
-              *reinterpret_cast<uint4 *>(sm.qp[X] + qoff + 1024 * h + 2 * it * 128 + (qcx ^ (((2 * it) & 7) << 4))) =
-                  make_uint4(pack_half2(t0.x, t0.y), pack_half2(t1.x, t1.y), pack_half2(t2.x, t2.y), pack_half2(t3.x, t3.y));
+              for (int it = 0; it < 4; ++it) {
+                float2 z[4];
+                z_of(it, h, z);
+                before[it] = amax[it];
+                amax[it] = max_of(z);
+              }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const bool up = lane & 8;
+              const float keep = up ? amax[i] : before[i], send = up ? before[i] : amax[i];
+              amax[i] = fmaxf(keep, __shfl_xor_sync(FULL, send, 8));
+            }
+            hand_on(amax, 4);
+            const float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 1));
+            const float rq = quotient_127(am);
+            if (!(lane & 1)) sm.qscale[k & 1][X][qrow0 + (lane & 14)] = __fmul_rn(am, sl127);  // (row qrow0 + 2 it)
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int it = 0; it < 4; ++it) {
+                float2 z[4];
+                z_of(it, h, z);
+                write(it, h, z, __shfl_sync(FULL, rq, (lane & 16) | (8 * h + 2 * it)));
+              }
+          } else {  // (row 2 b3 + b2 in the lanes with those bits)
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              float2 z[4][4];
+              float amax[4];
+#pragma unroll
+              for (int it = 0; it < 4; ++it) {
+                z_of(it, h, z[it]);
+                amax[it] = max_of(z[it]);
+              }
+              hand_on(amax, 8);
+              float am = fmaxf(amax[0], __shfl_xor_sync(FULL, amax[0], 2));
+              am = fmaxf(am, __shfl_xor_sync(FULL, am, 1));
+              const float rq = quotient_127(am);
+              if (!(lane & 3)) sm.qscale[k & 1][X][qrow0 + 8 * h + ((lane & 12) >> 1)] = __fmul_rn(am, sl127);  // (row qrow0 + 8 h + 2 it)
+#pragma unroll
+              for (int it = 0; it < 4; ++it) write(it, h, z[it], __shfl_sync(FULL, rq, (lane & 16) | (4 * it)));
             }
           }
         }
