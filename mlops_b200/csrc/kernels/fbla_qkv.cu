@@ -22,11 +22,14 @@ template <int CB, int FB, bool NORM>
 __global__ void __launch_bounds__(CLOSE_THREADS) qkv_step_kernel(const fbla_k_prefill closing, const fbla_k_token a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   wait_previous_pass();
-  allow_next_pass();
   const int bh = blockIdx.x;
   const Chunk ch = chunk_of(closing, bh / closing.kv_heads);
   const int g = closing_group(ch, 0);
   if (g >= 0) close_group<CB, FB>(closing, *reinterpret_cast<CloseSmem (*)[2]>(smem_raw), bh, g, ch.n0);
+  // The decode behind this step is let in here, not at the top: launched together with this kernel, while neither's code was in L2 yet, it ran
+  // 4 to 10 us longer (us of the step behind a read of 256 MB, 3+3, top / here: 16 rows of 240 to 2 400 tokens, 8 / 8 heads 53.2 / 41.5; 32 of 300
+  // to 6 000, 32 / 8 heads 77.8 / 71.6; one of 1 999 27.7 / 19.5; nothing evicted between: 34.2 / 34.2, 67.2 / 66.9, 13.0 / 13.0).
+  allow_next_pass();
   qkv_token_item<NORM>(a, nullptr);
 }
 
