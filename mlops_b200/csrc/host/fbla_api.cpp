@@ -276,7 +276,7 @@ void fill_chunk(const mlops_fbla_config *c, int count, long long room, const uin
   a.room = (int)room;
 }
 // The passes in the order that keeps them correct: closing groups reads the windows as they were, the attention reads
-// them too, and only then are the windows rewritten. Without queries one launch does both (fbla_close.cuh: write_item).
+// them too, and only then are the windows rewritten. Without queries one launch does both (fbla_close.cuh: write_chunk).
 mlops_fbla_status enqueue_chunk(const char *fn, fbla_k_prefill &a, int closable_groups, cudaStream_t stream) {
   a.early = closable_groups > 0;
   if (!a.q) {

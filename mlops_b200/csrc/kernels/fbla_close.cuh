@@ -9,8 +9,9 @@
 // lane) reads its lane's 16 slot words and packs both planes' words from them, stored 64 or 128 bits at a time.
 // 64 KiB read, 25 KiB written per (head, group). A CTA per group, two per SM, idled HBM while both packed codes: 8 heads x 32 768 tokens 57.4
 // us. A chunk without queries (write_chunk) is dealt over CTAs that stay, one tensor at a time (fewer threads at a barrier), the next unit
-// on its way meanwhile, and the codes' bounds come with a saturating product: 43.9 us = 4.2 TB/s, now bound by the instructions issued (0.58
-// per cycle and scheduler). Two threads per channel for base and step: 48.7 -> 50.0 (two tensors per CTA).
+// on its way meanwhile, and the codes' bounds come with a saturating product: 43.9 us = 4.2 TB/s, now bound by the latency of its
+// barriers and of shared memory (0.58 instructions issued per cycle and scheduler; stalls per issue: barrier 2.0, short scoreboard 1.9). Two
+// threads per channel for base and step: 48.7 -> 50.0 (two tensors per CTA).
 // A form with a thread per channel reading the 128 tokens of its channel from shared memory, and packing byte by byte from a
 // byte-per-code tile, was bound by those single-byte accesses: 307 us.
 // Replaces the reference's close_kernel / finish_kernel (attention/fbla/src/fbla_prefill.cuh:63-164); results are

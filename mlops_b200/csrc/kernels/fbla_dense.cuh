@@ -495,8 +495,8 @@ __device__ __forceinline__ void score_units(const fbla_k_decode &a, ScoreWarp *w
     fold.stage_vh[warp][1] = cur_vh != first_vh ? cur_vh : -1;
   }
   __syncthreads();
-  // rows of heads that may continue in neighbouring warps: a lane per (warp, query), merged by a butterfly (one after the other: 1 us)
   via.ready();
+  // the warps' pairs: a lane per (warp, query), merged by a butterfly (one after the other: 1 us)
   if constexpr (HEAD) {  // one head: its pairs of all warps, and of the CTA's window sub-blocks (a CTA without either leaves -inf)
     if (warp == 0) {
       float2 acc = make_float2(-FBLA_INF, 0.f);
@@ -508,7 +508,7 @@ __device__ __forceinline__ void score_units(const fbla_k_decode &a, ScoreWarp *w
       acc = merge_lanes<QG>(acc, lane);
       via.put_mass(acc, lane);
     }
-  } else {
+  } else {  // rows of heads that may continue in neighbouring warps
     const Runs runs(fold.stage_vh, SCORE_WARPS, lane);
 #pragma unroll 1
     for (int r = 0; r < 2; ++r) {
@@ -743,7 +743,7 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
     // group of copies each (empty where there is nothing to copy), the metadata of the next group of tokens with one of them -- so that
     // waiting for all but the last group is waiting for what the pair in work needs next. Else: the metadata alone.
     // AHEAD: both planes of a pair, one group of copies, a whole pair ahead instead of a plane half a pair ahead, in registers that the tails
-    // do not take: 64 rows of 1K to 64K 811 -> 749 us, 32 of 300 to 6 000 75.8 -> 72.9, 16 x 8 000 70.2 -> 66.7; but with two queries 16 x 4 000
+    // do not take: 64 rows of 1K to 64K 811 -> 749 us (behind a flush of L2), 32 of 300 to 6 000 75.8 -> 72.9, 16 x 8 000 70.2 -> 66.7; but with two queries 16 x 4 000
     // 44.3 -> 45.6, and in the one kernel of a short decode, whose warps have a pair or two, 4K 11.5 -> 12.3.
     constexpr bool TAILS = CB == 3, AHEAD = TAILS && !HEAD && QG == 4;
     auto close_copies = [] { if (TAILS) asm volatile("cp.async.commit_group;" ::: "memory"); };
@@ -1014,15 +1014,15 @@ __device__ __forceinline__ void value_item(const fbla_k_decode &a, uint8_t *smem
 }
 
 // ---- merge: out = (sum 2^(m_x - R) o_x + sum o_v) / (sum 2^(m_x - R) l_x + sum l_v), BF16 -----------------------------------
-// One CTA of four warps per output row: warp s sums rows s, s + 4, ... of the head's window and value rows, lane c channels
-// 4 c .. 4 c + 3; the four sums are added in order.
-// the same where the head has CTAs of its own: thread ch of 128 adds their sums(cta, channel or D for l)
+// Where the head has CTAs of its own: thread ch of 128 adds their sums(cta, channel or D for l), in order.
 template <class Sum> __device__ __forceinline__ void write_row(const fbla_k_decode &a, int vh, int qi, int ch, int ctas, Sum sums) {
   float o = 0.f, l = 0.f;
 #pragma unroll 4
   for (int i = 0; i < ctas; ++i) { o += sums(i, ch); l += sums(i, D); }
   a.out[((size_t)vh * a.qg + qi) * D + ch] = f32_to_bf16(__fdividef(o, l));  // (the row of query qi of virtual head vh)
 }
+// Else one CTA of four warps per output row: warp s sums rows s, s + 4, ... of the head's window and value rows, lane c channels
+// 4 c .. 4 c + 3; the four sums are added in order.
 template <int QG>
 __device__ __forceinline__ void gather_item(const fbla_k_decode &a, uint8_t *smem_raw) {
   __shared__ float4 so[4][32];
