@@ -27,7 +27,9 @@ template <int CB, int FB>
 __global__ void __launch_bounds__(TENSOR_THREADS, 4) write_kernel(const fbla_k_prefill a, int blocks) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   wait_previous_pass();
-  allow_next_pass();
+  // The next kernel is not let in before this one is through: a decode's CTAs want an SM each, and were placed as these CTAs left. us per append and
+  // decode, 32 / 8 heads, let in at the top / not, and behind a read of 256 MB: 1 x 100 000 + 1 4+2 49.6 / 45.1, 59.4 / 49.2; 4 x 60 000 + 1 3+3
+  // 122.5 / 111.7, 132.1 / 115.8; 4 x 3 000 + 1 3+3 26.3 / 26.9 (Python's), 33.8 / 23.6. At the end of a CTA: 129.0 at 4 x 60 000, behind the read.
   write_chunk<CB, FB>(a, smem_raw, blocks);
 }
 
