@@ -145,7 +145,7 @@ extern "C" cudaError_t fbla_k_dense_passes(const fbla_k_decode *a, fbla_k_pass i
 // same for one query as for four, one sweep's is not: a line per query count. One sweep is a launch and a chain of round trips
 // longer, some 8 us, so that with few groups per CTA the line lies further out. Measured on B200 when the lines were set, us per step one sweep /
 // two, N(0, 1) and outliers, 32 / 8 heads unless said; N tau in front (since then one sweep has become some 7 us shorter at batch 1, two in 3+3 by
-// about a tenth; the lines have stayed):
+// a tenth or more; the lines have stayed):
 //   batch 8, 3+3:  20: 309 / 227, 324 / 229    25: 264 / 261, 331 / 273    30: 242 / 294, 340 / 313    39: 263 / 367, 362 / 389
 //   batch 8, 4+2:  20: 111 / 81, 114 / 81      25: 97 / 92, 116 / 94       30: 91 / 103, 119 / 106     39: 96 / 124, 123 / 127
 //   batch 1, 3+3:  20: 77 / 55, 79 / 56        30: 66 / 62, 80 / 65        39: 63 / 72, 78 / 75        60: 79 / 95, 92 / 98

@@ -743,8 +743,8 @@ __device__ __forceinline__ void value_units(const fbla_k_decode &a, ValueWarp *w
     // group of copies each (empty where there is nothing to copy), the metadata of the next group of tokens with one of them -- so that
     // waiting for all but the last group is waiting for what the pair in work needs next. Else: the metadata alone.
     // AHEAD: both planes of a pair, one group of copies, a whole pair ahead instead of a plane half a pair ahead, in registers that the tails
-    // do not take: 64 rows of 1K to 64K 811 -> 749 us (behind a flush of L2), 32 of 300 to 6 000 75.8 -> 72.9, 16 x 8 000 70.2 -> 66.7; but with two queries 16 x 4 000
-    // 44.3 -> 45.6, and in the one kernel of a short decode, whose warps have a pair or two, 4K 11.5 -> 12.3.
+    // do not take: 64 rows of 1K to 64K 811 -> 749 us (behind a flush of L2), 32 of 300 to 6 000 75.8 -> 72.9, 16 x 8 000 70.2 -> 66.7; but with
+    // two queries 16 x 4 000 44.3 -> 45.6, and in the one kernel of a short decode, whose warps have a pair or two, 4K 11.5 -> 12.3.
     constexpr bool TAILS = CB == 3, AHEAD = TAILS && !HEAD && QG == 4;
     auto close_copies = [] { if (TAILS) asm volatile("cp.async.commit_group;" ::: "memory"); };
     auto arrived = [] {
